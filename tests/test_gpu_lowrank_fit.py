@@ -102,3 +102,26 @@ def test_fit_rejects_non_finite_inputs():
     assert bool((fq[1] == 0).all()) and bool((fk[1] == 0).all()) and bool(fq[0].abs().sum() > 0)
     with pytest.raises(ValueError):
         online_u(q, k, 16)
+
+
+@pytest.mark.parametrize("N", [2048, 2177, 8192 + 1])
+@pytest.mark.parametrize("spread_q, spread_k", [(1.0, 1.0), (3e-3, 1.0), (1e-6, 3e-3), (1.0, 1e-6)])
+def test_fit_on_both_factor_routes(N, spread_q, spread_k):
+    """Cholesky factor and clamped symmetric root, in every combination of the two sides: smallest second moments of
+    0.3 and 4e-6 (Cholesky: the trace of the inverse is 3e6) and of 5e-13 (below the clamp).  Several and ragged slabs.  The oracle works in float64 on the same bfloat16 values; the kernels' second moments are fp32 sums per
+    slab (2^-24 per addition, 2^-17 for a slab of thousands of rows at worst), and the fit divides by the gap between
+    the singular values 32 and 33 (a quarter and more here): 1e-3 of the largest logit, as above."""
+    from token2tile_b200.deploy_step import online_u
+    g = torch.Generator().manual_seed(N)
+    H = 2
+    ramp = torch.linspace(0.0, 1.0, 128)
+    step = torch.where(torch.arange(128) < 32, 1.0, 0.7)      # a gap between the kept and the dropped values
+    mix = torch.block_diag(torch.linalg.qr(torch.randn(64, 64, generator=g)).Q, torch.eye(64))      # bfloat16 keeps the small ones
+    q = ((torch.randn(H, N, 128, generator=g) * step * spread_q ** ramp) @ mix.T).to(BF)
+    k = ((torch.randn(H, N, 128, generator=g) * step * spread_k ** ramp) @ mix.T).to(BF)
+    Uq, Uk = online_u(q.to(DEV), k.to(DEV), 32)
+    oq, ok = O.online_u(q.double(), k.double(), 32)
+    # the logits' approximation is what is determined: clamped directions carry no data
+    want = (q.double() @ _product(oq, ok)) @ k.double().transpose(1, 2)
+    got = (q.double() @ _product(Uq, Uk)) @ k.double().transpose(1, 2)
+    assert (got - want).abs().max() <= 1e-3 * want.abs().max()

@@ -10,19 +10,18 @@
 //                      as BOTH operands of a 128 x 128 x 128 product (A = tile^T, B = tile, both
 //                      MN-major views of the same shared-memory tile); fp32 accumulator in TMEM.
 //                      HBM-bound: every input row is read once.
-//   sym_roots_kernel   sums the slabs in a fixed order in fp64 (M = G / N, deterministic), then finds
-//                      M = V diag(e) V^T by one-sided Jacobi in shared memory and writes
-//                      M^(1/2) (and M^(-1/2) for the query side) with the eigenvalues clamped at 1e-8.
-//   lowrank_kernel     C = Mq^(1/2) Mk^(1/2), its singular triplets by one-sided Jacobi, the 32 largest:
-//                      Uq = Mq^(-1/2) U_r S_r^(1/2),  Uk = Mk^(-1/2) V_r S_r^(1/2) = Mq^(1/2) U_r S_r^(-1/2)
-//                      (V = C^T U S^-1 and Mk^(-1/2) Mk^(1/2) = I).
+//   factor_kernel      sums the slabs in a fixed order in fp64 (M = G / N, deterministic) and writes F with
+//                      F F^T = M and, for the query side, F^-T: the Cholesky factor, or the symmetric root
+//                      with the eigenvalues clamped at 1e-8 where the clamp may matter.
+//   lowrank_kernel     C = Fq^T Fk, its singular triplets by one-sided Jacobi, the 32 largest:
+//                      Uq = Fq^-T U_r S_r^(1/2),  Uk = Fk^-T V_r S_r^(1/2) = Fq U_r S_r^(-1/2)
+//                      (V = C^T U S^-1 and Fk^-T Fk^T = I).
 //
 // One-sided (Hestenes) Jacobi orthogonalises the columns of W by plane rotations, W <- W J: for a
 // symmetric positive semi-definite M the columns of the limit are e_i v_i, for a general C they are
-// s_i u_i.  64 disjoint column pairs rotate per round (round-robin schedule, 127 rounds per sweep),
-// 16 threads per pair, all in fp64.  Eigenvectors of clamped eigenvalues are never normalised:
-// because every clamped eigenvalue has the same value c, their joint contribution to f(M) is
-// f(c) (I - sum of the other v v^T), whatever basis spans them.
+// s_i u_i.  Eigenvectors of clamped eigenvalues are never normalised: because every clamped eigenvalue has
+// the same value c, their joint contribution to f(M) is f(c) (I - sum of the other v v^T), whatever basis
+// spans them.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -35,15 +34,23 @@ namespace t2t {
 // Gram matrices
 // ---------------------------------------------------------------------------
 constexpr int GR_ROWS = 128;                 // rows per tile
-constexpr int GR_SLAB_TILES = 64;            // tiles per CTA: 8192 rows in one fp32 accumulation
+constexpr int GR_SLAB_TILES = 64;            // tiles per CTA, at most: 8192 rows in one fp32 accumulation
 constexpr int GR_TILE = GR_ROWS * kD * 2;    // 32 KB
 constexpr int GR_STAGES = 3;
 constexpr int GR_SMEM = GR_STAGES * GR_TILE + 128 + 1024;
 
-__host__ __device__ inline int gram_slabs(int N) { return cdiv(cdiv(N, GR_ROWS), GR_SLAB_TILES); }
+// Tiles per slab: both sides' slabs should fill the chip twice over, but each costs 64 KB written and read again, so
+// four tiles (1024 rows' worth of input bytes, as much as the slab itself) are the least.  At 2 heads x 4096 rows one
+// CTA per head took 15 us a side.
+inline int gram_slab_tiles(int H, int N) {
+  const int even = cdiv(2 * H * cdiv(N, GR_ROWS), 2 * 148);
+  return even < 4 ? 4 : (even > GR_SLAB_TILES ? GR_SLAB_TILES : even);
+}
+inline int gram_slabs(int H, int N) { return cdiv(cdiv(N, GR_ROWS), gram_slab_tiles(H, N)); }
 
-__global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUtensorMap mapX, float* __restrict__ partial,
-                                                   int N, int* __restrict__ status) {
+__global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUtensorMap mapQ,
+                                                   const __grid_constant__ CUtensorMap mapK, float* __restrict__ partial,
+                                                   int N, int slab_tiles, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
@@ -55,8 +62,10 @@ __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUten
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int slab = blockIdx.x, h = blockIdx.y, slabs = gridDim.x;
-  const int tile0 = slab * GR_SLAB_TILES;
-  const int ntiles = min(GR_SLAB_TILES, cdiv(N, GR_ROWS) - tile0);
+  const int m = blockIdx.z * gridDim.y + h;      // matrix: the query side's first, then the key side's
+  const CUtensorMap* map = blockIdx.z ? &mapK : &mapQ;
+  const int tile0 = slab * slab_tiles;
+  const int ntiles = min(slab_tiles, cdiv(N, GR_ROWS) - tile0);
 
   if (warp == 0) {
     tmem_alloc(tmem_slot, 128);
@@ -79,8 +88,8 @@ __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUten
       if (t >= GR_STAGES && !mbar_wait(freeb + st, ((t / GR_STAGES) - 1) & 1, abort_flag)) break;
       mbar_arrive_expect_tx(full + st, GR_TILE);
       const uint32_t dst = base + st * GR_TILE;
-      tma_load_tile3(dst, &mapX, 0, (tile0 + t) * GR_ROWS, h, full + st);
-      tma_load_tile3(dst + GR_ROWS * 128, &mapX, 64, (tile0 + t) * GR_ROWS, h, full + st);
+      tma_load_tile3(dst, map, 0, (tile0 + t) * GR_ROWS, h, full + st);
+      tma_load_tile3(dst + GR_ROWS * 128, map, 64, (tile0 + t) * GR_ROWS, h, full + st);
     }
   } else if (tid == 32) {
     // ---- products: G += tile^T tile, eight steps of 16 rows ----
@@ -102,7 +111,7 @@ __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUten
   const bool ok = mbar_wait(done, 0, abort_flag);
   tc_fence_after();
   if (ok) {
-    float* dst = partial + ((size_t)h * slabs + slab) * (kD * kD) + (size_t)tid * kD;
+    float* dst = partial + ((size_t)m * slabs + slab) * (kD * kD) + (size_t)tid * kD;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       uint32_t v[32];
@@ -124,131 +133,350 @@ __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUten
 // one-sided Jacobi on a 128 x 128 fp64 matrix in shared memory
 // ---------------------------------------------------------------------------
 constexpr int JD = 128;                  // matrix order
-constexpr int JLD = JD + 1;              // column stride in doubles: an odd stride spreads the pairs over the banks
-constexpr int J_THREADS = 1024;          // 64 pairs x 16 threads
+constexpr int JLD = JD + 1;              // column stride in doubles: odd, so that rows can be walked as well as columns
+constexpr int J_THREADS = 256;
 constexpr int J_MAX_SWEEPS = 18;
-constexpr int J_SMEM = JD * JLD * 8 + 2 * JD * 8 + 64;
+constexpr double kJacobiDone2 = 9.0e-16;   // (3e-8)^2: see jacobi_orthogonalise
+constexpr int J_SMEM = JD * JLD * 8 + 2 * JD * 8 + 8 * 8 * 16 + 4 * JD * 8 + 64;
 
 __device__ __forceinline__ double shfl_xor_d(double v, int m) {
-  return __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(v), m, 16),
-                          __shfl_xor_sync(0xffffffffu, __double2loint(v), m, 16));
+  return __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(v), m),
+                          __shfl_xor_sync(0xffffffffu, __double2loint(v), m));
 }
 
 // Squared norms of the columns of W into nrm2[0..127] (every thread calls it).
 __device__ void column_norms2(const double* W, double* nrm2) {
-  const int tid = threadIdx.x, col = tid >> 3, sub = tid & 7;
+  const int tid = threadIdx.x, col = tid >> 1, sub = tid & 1;
   double acc = 0.0;
-#pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    const double x = W[col * JLD + sub + 8 * m];
+#pragma unroll 8
+  for (int m = 0; m < 64; ++m) {
+    const double x = W[col * JLD + sub + 2 * m];
     acc = fma(x, x, acc);
   }
-  acc += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(acc), 4, 8), __shfl_xor_sync(0xffffffffu, __double2loint(acc), 4, 8));
-  acc += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(acc), 2, 8), __shfl_xor_sync(0xffffffffu, __double2loint(acc), 2, 8));
-  acc += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(acc), 1, 8), __shfl_xor_sync(0xffffffffu, __double2loint(acc), 1, 8));
+  acc += shfl_xor_d(acc, 1);
   if (sub == 0) nrm2[col] = acc;
   __syncthreads();
 }
 
-// Rotates column pairs of W (column j at W + j * JLD) until all columns are mutually orthogonal
-// to working precision.  Every thread of the 1024-thread CTA calls it.
-__device__ void jacobi_orthogonalise(double* W, double* nrm2, int* flag) {
-  const int tid = threadIdx.x, pi = tid >> 4, sub = tid & 15;
+// The eight column pairs (x_i, y_i) of a round among the sixteen columns e that a warp holds in registers (lane l:
+// rows l, l + 32, l + 64, l + 96 of every column).  CROSS: column i of the first block with column i + R of the second
+// (mod 8); otherwise round R of the seven that bring every pair inside each block together.
+template <bool CROSS, int R>
+struct Round {
+  static __host__ __device__ constexpr int inner_x(int i) { return i == 0 ? 7 : (R + i) % 7; }
+  static __host__ __device__ constexpr int inner_y(int i) { return i == 0 ? R : (R + 7 - i) % 7; }
+  static __host__ __device__ constexpr int x(int i) { return CROSS ? i : (i & 4) * 2 + inner_x(i & 3); }
+  static __host__ __device__ constexpr int y(int i) { return CROSS ? 8 + ((i + R) & 7) : (i & 4) * 2 + inner_y(i & 3); }
+};
+
+// One round.  A, B: the two blocks' numbers (column 8 A + i is e[i], column 8 B + i is e[8 + i]); lane l works out the
+// angle of pair l & 7.
+//
+// The angle itself only steers convergence, so it comes from fp32 arithmetic (relative error 1e-7 leaves 1e-7 of
+// the pair's product for the next visit); (c, s) is then normalised in fp64, so every rotation is orthogonal to
+// fp64 precision and nothing of the result depends on fp32.
+template <bool CROSS, int R>
+__device__ __forceinline__ void rotate8(double (&e)[16][4], int A, int B, double* nrm2, double2* cs, double tiny2,
+                                        float scale, bool& again) {
+  using P = Round<CROSS, R>;
+  const int lane = threadIdx.x & 31, p = lane & 7;
+  const int px = CROSS ? p : P::inner_x(p & 3), py = CROSS ? (p + R) & 7 : P::inner_y(p & 3);
+  const int cx = 8 * (CROSS || p < 4 ? A : B) + px, cy = 8 * (CROSS || p >= 4 ? B : A) + py;
+  double g[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    g[i] = e[P::x(i)][0] * e[P::y(i)][0];
+#pragma unroll
+    for (int m = 1; m < 4; ++m) g[i] = fma(e[P::x(i)][m], e[P::y(i)][m], g[i]);
+  }
+  // eight sums over the warp: lane l ends up with that of pair l & 7
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+  double u[4], v[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) u[i] = (b0 ? g[2 * i + 1] : g[2 * i]) + shfl_xor_d(b0 ? g[2 * i] : g[2 * i + 1], 1);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) v[i] = (b1 ? u[2 * i + 1] : u[2 * i]) + shfl_xor_d(b1 ? u[2 * i] : u[2 * i + 1], 2);
+  double gamma = (b2 ? v[1] : v[0]) + shfl_xor_d(b2 ? v[0] : v[1], 4);
+  gamma += shfl_xor_d(gamma, 8);
+  gamma += shfl_xor_d(gamma, 16);
+  const double alpha = nrm2[cx], beta = nrm2[cy];
+  const double g2rel = gamma * gamma, ab = alpha * beta;
+  const bool live = alpha > tiny2 && beta > tiny2 && g2rel > 1.0e-27 * ab;
+  if (!__any_sync(0xffffffffu, live)) return;
+  again = again || (live && g2rel > kJacobiDone2 * ab);
+  double c = 1.0, s = 0.0;
+  if (live) {
+    // tan of the rotation: the smaller root of t^2 + (beta - alpha) / gamma t - 1 = 0
+    const double dx = beta - alpha, dy = 2.0 * gamma;
+    const float fx = fabsf((float)(dx * scale)), fy = fabsf((float)(dy * scale));
+    const float lo = fminf(fx, fy) / fmaxf(fx, fy), root = sqrtf(fmaf(lo, lo, 1.0f));
+    const float tf = fy <= fx ? lo / (1.0f + root) : 1.0f / (lo + root);
+    const double t = ((dx >= 0.0) == (dy >= 0.0)) ? (double)tf : -(double)tf;
+    const double a = fma(t, t, 1.0);
+    double r = (double)rsqrtf((float)a);
+    r = r * fma(-0.5 * a, r * r, 1.5);
+    r = r * fma(-0.5 * a, r * r, 1.5);
+    c = r;
+    s = r * t;
+    if (lane < 8) {
+      nrm2[cx] = fmax(fma(-t, gamma, alpha), 0.0);
+      nrm2[cy] = fmax(fma(t, gamma, beta), 0.0);
+    }
+  }
+  if (lane < 8) cs[lane] = make_double2(c, s);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const double2 r = cs[i];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const double a = e[P::x(i)][m], b = e[P::y(i)][m];
+      e[P::x(i)][m] = fma(r.x, a, -(r.y * b));
+      e[P::y(i)][m] = fma(r.y, a, r.x * b);
+    }
+  }
+  __syncwarp();      // cs and nrm2 may be written again
+}
+
+// Rotates column pairs of W (column j at W + j * JLD) until all columns are mutually orthogonal.  Every thread of
+// the 256-thread CTA calls it.
+//
+// 16 blocks of eight columns meet pairwise in 15 steps a sweep (round-robin); a warp loads the sixteen columns of a
+// block pair into registers, runs the eight rounds of eight disjoint pairs (and, in a sweep's first step, the seven
+// rounds inside the blocks) and writes them back, so shared memory carries the matrix once per eight rounds.  What
+// bounds a round: 160 warp-wide fp64 operations for the products and rotations on a pipe that takes two cycles each,
+// then the reduction's shuffles; the angle's arithmetic is done once per pair, one lane in eight of a warp's four
+// repeats.  (Blocks of four columns and 16 warps: 295 instructions for four pairs and half the shared-memory saving; the whole
+// fit 1.62 instead of 1.57 ms at 2 heads, both bound by the rounds' chain of dependent steps.)
+// A sweep in which no pair's cosine exceeded sqrt(kJacobiDone2) = 3e-8 leaves cosines of the order of its square
+// (inside a cluster of equal singular values, at most 3e-8), below the rounding of the fp32 factors: it is the last.
+__device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  double2* cs = cs_all + warp * 8;
   __syncthreads();      // W was just written by other threads
+  column_norms2(W, nrm2);
   // columns whose squared norm is below (1e-14 of the largest column)^2 are numerically zero: rotating
   // them against each other never settles and changes nothing that is used
-  column_norms2(W, nrm2);
   double big = 0.0;
   for (int j = 0; j < JD; ++j) big = fmax(big, nrm2[j]);
   const double tiny2 = 1.0e-28 * big;
+  const float scale = big > 0.0 ? (float)fmin(1.0e18 / big, 1.0e38) : 1.0f;      // keeps the fp32 angles in range
   for (int sweep = 0; sweep < J_MAX_SWEEPS; ++sweep) {
-    __syncthreads();
-    if (tid == 0) *flag = 0;
-    __syncthreads();
-    bool rotated = false;
-    for (int round = 0; round < JD - 1; ++round) {
-      // round-robin pairing of 128 players: player 127 stays, the others move round a ring of 127
-      int p, q;
-      if (pi == 0) { p = JD - 1; q = round; }
-      else { p = (round + pi) % (JD - 1); q = (round + (JD - 1) - pi) % (JD - 1); }
-      double* wp = W + p * JLD;
-      double* wq = W + q * JLD;
-      double alpha = 0.0, beta = 0.0, gamma = 0.0;
+    bool again = false;
+    for (int step = 0; step < 15; ++step) {
+      // round-robin pairing of 16 blocks: block 15 stays, the others move round a ring of 15
+      int A, B;
+      if (warp == 0) { A = 15; B = step; }
+      else { A = (step + warp) % 15; B = (step + 15 - warp) % 15; }
+      double e[16][4];
 #pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        const double a = wp[sub + 16 * m], b = wq[sub + 16 * m];
-        alpha = fma(a, a, alpha);
-        beta = fma(b, b, beta);
-        gamma = fma(a, b, gamma);
-      }
+      for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int d = 8; d > 0; d >>= 1) {
-        alpha += shfl_xor_d(alpha, d);
-        beta += shfl_xor_d(beta, d);
-        gamma += shfl_xor_d(gamma, d);
-      }
-      // all 16 threads of the pair hold the same sums (xor reductions add in the same tree order)
-      if (alpha > tiny2 && beta > tiny2 && gamma * gamma > 1.0e-27 * alpha * beta) {
-        const double zeta = (beta - alpha) / (2.0 * gamma);
-        const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-          const double a = wp[sub + 16 * m], b = wq[sub + 16 * m];
-          wp[sub + 16 * m] = c * a - s * b;
-          wq[sub + 16 * m] = s * a + c * b;
+        for (int m = 0; m < 4; ++m) {
+          e[j][m] = W[(8 * A + j) * JLD + lane + 32 * m];
+          e[8 + j][m] = W[(8 * B + j) * JLD + lane + 32 * m];
         }
-        rotated = true;
+      if (step == 0) {      // every block is held by some warp: the pairs inside the blocks
+        rotate8<false, 0>(e, A, B, nrm2, cs, tiny2, scale, again);
+        rotate8<false, 1>(e, A, B, nrm2, cs, tiny2, scale, again);
+        rotate8<false, 2>(e, A, B, nrm2, cs, tiny2, scale, again);
+        rotate8<false, 3>(e, A, B, nrm2, cs, tiny2, scale, again);
+        rotate8<false, 4>(e, A, B, nrm2, cs, tiny2, scale, again);
+        rotate8<false, 5>(e, A, B, nrm2, cs, tiny2, scale, again);
+        rotate8<false, 6>(e, A, B, nrm2, cs, tiny2, scale, again);
       }
+      rotate8<true, 0>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 1>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 2>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 3>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 4>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 5>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 6>(e, A, B, nrm2, cs, tiny2, scale, again);
+      rotate8<true, 7>(e, A, B, nrm2, cs, tiny2, scale, again);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          W[(8 * A + j) * JLD + lane + 32 * m] = e[j][m];
+          W[(8 * B + j) * JLD + lane + 32 * m] = e[8 + j][m];
+        }
       __syncthreads();
     }
-    if (rotated) *flag = 1;
-    __syncthreads();
-    if (*flag == 0) break;
+    if (!__syncthreads_or(again ? 1 : 0)) break;
+    column_norms2(W, nrm2);      // the running norms pick up rounding
   }
   __syncthreads();
 }
 
 constexpr double kEigFloor = 1.0e-8;     // clamp of the reference (deploy_step.py:137-138)
 
-// One CTA per second-moment matrix (blockIdx.x < H: query side, else key side).
-//   roots    [2 H][128][128] fp64: M^(1/2)
-//   invroots [H][128][128] fp64:   M^(-1/2), query side only
+// Steps 8 M .. 8 M + 7 of cholesky_inverse (which registers hold row and column k must be known when compiling).
+template <int M>
+__device__ __forceinline__ void cholesky_steps(double (&e)[16][4], double* Lc, double* pub, bool& ok) {
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+#pragma unroll 1
+  for (int kk = 0; kk < 8 && ok; ++kk) {
+    const int k = 8 * M + kk;
+    double* col = pub + (k & 1) * 2 * JD;      // two sets in turn: one barrier a step
+    double* row = col + JD;                    // multipliers of step k by column
+    if (l == (k & 31)) {
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        const int i = w + 8 * m;
+        if (i >= k) {
+          col[i] = e[m][M / 4];
+          if (i > k) row[i] = e[m][M / 4];
+        }
+      }
+    }
+    if (w == kk) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int j = l + 32 * n;
+        if (j <= k) row[j] = j == k ? 1.0 : e[M][n];
+      }
+    }
+    __syncthreads();
+    const double piv = col[k];
+    ok = piv > 0.0;                            // the same value in every thread
+    if (ok) {
+      const double isq = rsqrt(piv), inv = isq * isq;
+      if (tid < JD) Lc[k * JLD + tid] = tid >= k ? col[tid] * isq : 0.0;
+      double rr[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) rr[n] = row[l + 32 * n] * inv;
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        const int i = w + 8 * m;
+        if (i > k) {
+          const double c = col[i];
+#pragma unroll
+          for (int n = 0; n < 4; ++n) e[m][n] = fma(-c, rr[n], l + 32 * n == k ? 0.0 : e[m][n]);
+        } else if (i == k) {
+#pragma unroll
+          for (int n = 0; n < 4; ++n) e[m][n] = l + 32 * n < k ? e[m][n] * isq : (l + 32 * n == k ? isq : 0.0);
+        }
+      }
+    }
+  }
+}
+
+// Cholesky factor and its inverse of the matrix whose lower triangle is in e: thread (warp w, lane l) holds the
+// elements (w + 8 m, l + 32 n).  An element belongs to A until its column's step, to X = L^-1 afterwards: step k
+// publishes column k of A and row k of X, and every later row i subtracts A_ik / A_kk times (A_kj for j > k, 1 for
+// j = k, X_kj for j < k).  L goes to Lc (column k at Lc + k * JLD, zeros above the diagonal).  pub: 4 x 128 doubles.
+// Returns false when a pivot is not positive; otherwise e holds X and the Frobenius norm^2 of X (the trace of the
+// inverse matrix) is in *trace.
+__device__ __forceinline__ bool cholesky_inverse(double (&e)[16][4], double* Lc, double* pub, double* red, double* trace) {
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  bool ok = true;
+  cholesky_steps<0>(e, Lc, pub, ok);
+  cholesky_steps<1>(e, Lc, pub, ok);
+  cholesky_steps<2>(e, Lc, pub, ok);
+  cholesky_steps<3>(e, Lc, pub, ok);
+  cholesky_steps<4>(e, Lc, pub, ok);
+  cholesky_steps<5>(e, Lc, pub, ok);
+  cholesky_steps<6>(e, Lc, pub, ok);
+  cholesky_steps<7>(e, Lc, pub, ok);
+  cholesky_steps<8>(e, Lc, pub, ok);
+  cholesky_steps<9>(e, Lc, pub, ok);
+  cholesky_steps<10>(e, Lc, pub, ok);
+  cholesky_steps<11>(e, Lc, pub, ok);
+  cholesky_steps<12>(e, Lc, pub, ok);
+  cholesky_steps<13>(e, Lc, pub, ok);
+  cholesky_steps<14>(e, Lc, pub, ok);
+  cholesky_steps<15>(e, Lc, pub, ok);
+  if (!ok) return false;
+  double acc = 0.0;
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+      if (l + 32 * n <= w + 8 * m) acc = fma(e[m][n], e[m][n], acc);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) acc += shfl_xor_d(acc, d);
+  if (l == 0) red[w] = acc;
+  __syncthreads();
+  double sum = 0.0;
+  for (int i = 0; i < 8; ++i) sum += red[i];
+  *trace = sum;
+  return true;
+}
+
+// One CTA per second-moment matrix M (blockIdx.x < H: query side, else key side).
+//   roots    [2 H][128][128] fp64: F with F F^T = M (eigenvalues clamped), row-major
+//   invroots [H][128][128] fp64:   F^-T, query side only
 //   bad      [2 H] int: 1 when the matrix holds a non-finite value (non-finite input)
-__global__ void __launch_bounds__(J_THREADS, 1) sym_roots_kernel(const float* __restrict__ partial, int slabs, int H,
-                                                                 double inv_n, double* __restrict__ roots,
-                                                                 double* __restrict__ invroots, int* __restrict__ bad) {
+//
+// Any factor serves: with Fq = Mq^(1/2) Oq and Fk = Mk^(1/2) Ok for orthogonal Oq, Ok, the singular value
+// decomposition of Fq^T Fk = Oq^T (Mq^(1/2) Mk^(1/2)) Ok has the same S, its U is Oq^T times the other one, and
+// Fq^-T U is the same matrix.  The Cholesky factor takes 128 short steps; the symmetric root needs all
+// eigenvectors (0.9 ms), and is left for the matrices the clamp may touch: those whose inverse has a trace
+// (an upper bound of 1 / smallest eigenvalue) of 1 / kEigFloor or more.
+// The whole fit took 5.9 ms at 2 heads x 4096 rows and 6.3 at 40 x 75,600 when every matrix needed its eigenvectors
+// and the Jacobi walked shared memory for each pair; 1.57 and 1.90 ms now (3.6 and 3.7 where both routes are needed).
+__global__ void __launch_bounds__(J_THREADS, 1) factor_kernel(const float* __restrict__ partial, int slabs, int H,
+                                                              double inv_n, double* __restrict__ roots,
+                                                              double* __restrict__ invroots, int* __restrict__ bad) {
   extern __shared__ __align__(16) uint8_t jsm[];
   double* W = reinterpret_cast<double*>(jsm);
   double* nrm2 = W + JD * JLD;
   double* coef = nrm2 + JD;
-  int* flag = reinterpret_cast<int*>(coef + JD);
+  double2* cs = reinterpret_cast<double2*>(coef + JD);
+  double* pub = reinterpret_cast<double*>(cs + 8 * 8);
   const int tid = threadIdx.x, m = blockIdx.x;
+  const bool want_inv = m < H;
 
   // M = (sum of the slabs, in slab order) / N; symmetric, so rows can be read as columns
   const float* src = partial + (size_t)m * slabs * (JD * JD);
-  bool finite = true;
-  for (int e = tid; e < JD * JD; e += J_THREADS) {
+  auto moment = [&](int idx) {
     double acc = 0.0;
-    for (int s = 0; s < slabs; ++s) acc += (double)src[(size_t)s * (JD * JD) + e];
-    acc *= inv_n;
-    finite = finite && isfinite(acc);
-    W[(e >> 7) * JLD + (e & 127)] = acc;
+    for (int s = 0; s < slabs; ++s) acc += (double)src[(size_t)s * (JD * JD) + idx];
+    return acc * inv_n;
+  };
+  double* Fo = roots + (size_t)m * JD * JD;
+  double* Io = invroots + (size_t)m * JD * JD;
+  {
+    double e[16][4];
+    bool finite = true;
+#pragma unroll
+    for (int a = 0; a < 16; ++a)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        e[a][n] = moment(((tid >> 5) + 8 * a) * JD + (tid & 31) + 32 * n);
+        finite = finite && isfinite(e[a][n]);
+      }
+    const int any_bad = __syncthreads_or(finite ? 0 : 1);
+    if (tid == 0) bad[m] = any_bad;
+    if (any_bad) return;      // the host raises; nothing below would converge on NaNs
+    double trace = 0.0;
+    const bool ok = cholesky_inverse(e, W, pub, nrm2, &trace);
+    __syncthreads();
+    if (ok && trace < 1.0 / kEigFloor) {
+      for (int i = tid; i < JD * JD; i += J_THREADS) Fo[i] = W[(i & 127) * JLD + (i >> 7)];
+      if (want_inv) {
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < 16; ++a)
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            const int i = (tid >> 5) + 8 * a, j = (tid & 31) + 32 * n;
+            W[j * JLD + i] = j <= i ? e[a][n] : 0.0;
+          }
+        __syncthreads();
+        for (int i = tid; i < JD * JD; i += J_THREADS) Io[i] = W[(i >> 7) * JLD + (i & 127)];
+      }
+      return;
+    }
   }
-  const int any_bad = __syncthreads_or(finite ? 0 : 1);
-  if (any_bad) {          // the host raises; nothing below would converge on NaNs
-    if (tid == 0) bad[m] = 1;
-    return;
-  }
-  if (tid == 0) bad[m] = 0;
 
-  jacobi_orthogonalise(W, nrm2, flag);
+  for (int i = tid; i < JD * JD; i += J_THREADS) W[(i >> 7) * JLD + (i & 127)] = moment(i);
+  jacobi_orthogonalise(W, nrm2, cs);
   column_norms2(W, nrm2);
   // column i of W is e_i v_i: with l_i = max(e_i, floor),
   //   M^(1/2)  = sqrt(floor) I + sum_i (sqrt(l_i) - sqrt(floor)) v_i v_i^T
   //   M^(-1/2) = floor^(-1/2) I + sum_i (l_i^(-1/2) - floor^(-1/2)) v_i v_i^T
   // and v_i v_i^T = w_i w_i^T / e_i^2; the terms of clamped eigenvalues vanish.
-  const bool want_inv = m < H;
   for (int pass = 0; pass < (want_inv ? 2 : 1); ++pass) {
     if (tid < JD) {
       const double e2 = nrm2[tid], e = sqrt(e2);
@@ -257,19 +485,19 @@ __global__ void __launch_bounds__(J_THREADS, 1) sym_roots_kernel(const float* __
       coef[tid] = f;
     }
     __syncthreads();
-    const int col = tid & 127, r0 = (tid >> 7) * 16;      // 16 rows x 1 column per thread
-    double acc[16];
+    const int col = tid & 127, r0 = (tid >> 7) * 64;      // 64 rows x 1 column per thread
+    double acc[64];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.0;
+    for (int i = 0; i < 64; ++i) acc[i] = 0.0;
     for (int k = 0; k < JD; ++k) {
       const double f = coef[k] * W[k * JLD + col];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i] = fma(f, W[k * JLD + r0 + i], acc[i]);
+      for (int i = 0; i < 64; ++i) acc[i] = fma(f, W[k * JLD + r0 + i], acc[i]);
     }
     const double diag = pass == 0 ? sqrt(kEigFloor) : 1.0 / sqrt(kEigFloor);
-    double* dst = pass == 0 ? roots + (size_t)m * JD * JD : invroots + (size_t)m * JD * JD;
+    double* dst = pass == 0 ? Fo : Io;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) dst[(size_t)(r0 + i) * JD + col] = acc[i] + (r0 + i == col ? diag : 0.0);
+    for (int i = 0; i < 64; ++i) dst[(size_t)(r0 + i) * JD + col] = acc[i] + (r0 + i == col ? diag : 0.0);
     __syncthreads();
   }
 }
@@ -283,28 +511,28 @@ __global__ void __launch_bounds__(J_THREADS, 1) lowrank_kernel(const double* __r
   double* W = reinterpret_cast<double*>(jsm);
   double* nrm2 = W + JD * JLD;
   double* coef = nrm2 + JD;                 // reused: the column chosen for each of the 32 ranks
-  int* flag = reinterpret_cast<int*>(coef + JD);
+  double2* cs = reinterpret_cast<double2*>(coef + JD);
   const int tid = threadIdx.x, h = blockIdx.x;
   if (bad[h] | bad[H + h]) return;
-  const double* Rq = roots + (size_t)h * JD * JD;
-  const double* Rk = roots + (size_t)(H + h) * JD * JD;
-  const double* Rqi = invroots + (size_t)h * JD * JD;
+  const double* Fq = roots + (size_t)h * JD * JD;
+  const double* Fk = roots + (size_t)(H + h) * JD * JD;
+  const double* Iq = invroots + (size_t)h * JD * JD;
 
-  // C = Rq^T Rk = Rq Rk (both symmetric); column j of C goes to W + j * JLD
+  // C = Fq^T Fk; column j of C goes to W + j * JLD
   {
-    const int col = tid & 127, r0 = (tid >> 7) * 16;
-    double acc[16];
+    const int col = tid & 127, r0 = (tid >> 7) * 64;
+    double acc[64];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.0;
+    for (int i = 0; i < 64; ++i) acc[i] = 0.0;
     for (int k = 0; k < JD; ++k) {
-      const double b = Rk[(size_t)k * JD + col];
+      const double b = Fk[(size_t)k * JD + col];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i] = fma(Rq[(size_t)(r0 + i) * JD + k], b, acc[i]);
+      for (int i = 0; i < 64; ++i) acc[i] = fma(Fq[(size_t)k * JD + r0 + i], b, acc[i]);
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) W[col * JLD + r0 + i] = acc[i];
+    for (int i = 0; i < 64; ++i) W[col * JLD + r0 + i] = acc[i];
   }
-  jacobi_orthogonalise(W, nrm2, flag);
+  jacobi_orthogonalise(W, nrm2, cs);
   column_norms2(W, nrm2);      // column j is s_j u_j
 
   // rank of every column by decreasing singular value (ties: lower column first)
@@ -319,15 +547,16 @@ __global__ void __launch_bounds__(J_THREADS, 1) lowrank_kernel(const double* __r
     if (rank < kR) pick[rank] = tid;
   }
   __syncthreads();
-  // Uq[:, r] = Rqi w / sqrt(s),  Uk[:, r] = Rq w / s^(3/2)     (w = s u, the chosen column)
+  // Uq[:, r] = Fq^-T w / sqrt(s),  Uk[:, r] = Fk^-T v sqrt(s) = Fq w / s^(3/2)     (w = s u, the chosen column;
+  // v = C^T u / s and Fk^-T Fk^T = I)
   for (int e = tid; e < JD * kR; e += J_THREADS) {
     const int d = e >> 5, r = e & 31, j = pick[r];
     const double s2 = nrm2[j], s = sqrt(s2);
     double aq = 0.0, ak = 0.0;
     for (int k = 0; k < JD; ++k) {
       const double w = W[j * JLD + k];
-      aq = fma(Rqi[(size_t)d * JD + k], w, aq);
-      ak = fma(Rq[(size_t)d * JD + k], w, ak);
+      aq = fma(Iq[(size_t)d * JD + k], w, aq);
+      ak = fma(Fq[(size_t)d * JD + k], w, ak);
     }
     const bool live = s > 0.0;
     Uq[((size_t)h * JD + d) * kR + r] = live ? (float)(aq / sqrt(s)) : 0.f;
@@ -339,7 +568,7 @@ __global__ void __launch_bounds__(J_THREADS, 1) lowrank_kernel(const double* __r
 
 using namespace t2t;
 
-static size_t fit_off_roots(int H, int N) { return (((size_t)2 * H * gram_slabs(N) * kD * kD * 4) + 255) & ~(size_t)255; }
+static size_t fit_off_roots(int H, int N) { return (((size_t)2 * H * gram_slabs(H, N) * kD * kD * 4) + 255) & ~(size_t)255; }
 static size_t fit_off_inv(int H, int N) { return fit_off_roots(H, N) + (size_t)2 * H * kD * kD * 8; }
 
 extern "C" size_t t2t_lowrank_fit_ws_bytes(int H, int N) { return fit_off_inv(H, N) + (size_t)H * kD * kD * 8; }
@@ -360,18 +589,17 @@ extern "C" int t2t_lowrank_fit_strided(const void* q, const void* k, long long r
   float* partial = reinterpret_cast<float*>(w);
   double* roots = reinterpret_cast<double*>(w + fit_off_roots(H, N));
   double* invroots = reinterpret_cast<double*>(w + fit_off_inv(H, N));
-  const int slabs = gram_slabs(N);
+  const int slabs = gram_slabs(H, N);
   if (cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(sym_roots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(lowrank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess)
     return T2T_ERR_CUDA;
   CUtensorMap mq, mk;
   if (!make_head_tile_map(&mq, q, (uint64_t)N, (uint64_t)H, GR_ROWS, (uint64_t)row_stride, (uint64_t)head_stride) ||
       !make_head_tile_map(&mk, k, (uint64_t)N, (uint64_t)H, GR_ROWS, (uint64_t)row_stride, (uint64_t)head_stride))
     return T2T_ERR_CUDA;
-  gram_kernel<<<dim3(slabs, H), 128, GR_SMEM, st>>>(mq, partial, N, d_status);
-  gram_kernel<<<dim3(slabs, H), 128, GR_SMEM, st>>>(mk, partial + (size_t)H * slabs * kD * kD, N, d_status);
-  sym_roots_kernel<<<2 * H, J_THREADS, J_SMEM, st>>>(partial, slabs, H, 1.0 / (double)N, roots, invroots, d_bad);
+  gram_kernel<<<dim3(slabs, H, 2), 128, GR_SMEM, st>>>(mq, mk, partial, N, gram_slab_tiles(H, N), d_status);
+  factor_kernel<<<2 * H, J_THREADS, J_SMEM, st>>>(partial, slabs, H, 1.0 / (double)N, roots, invroots, d_bad);
   lowrank_kernel<<<H, J_THREADS, J_SMEM, st>>>(roots, invroots, H, d_bad, Uq, Uk);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
