@@ -11,8 +11,8 @@
 //                      MN-major views of the same shared-memory tile); fp32 accumulator in TMEM.
 //                      HBM-bound: every input row is read once.
 //   factor_kernel      sums the slabs in a fixed order in fp64 (M = G / N, deterministic) and writes F with
-//                      F F^T = M and, for the query side, F^-T: the Cholesky factor, or the symmetric root
-//                      with the eigenvalues clamped at 1e-8 where the clamp may matter.
+//                      F F^T = M: the symmetric root with the eigenvalues clamped at 1e-8, or, on the query side
+//                      and where the clamp cannot matter, the Cholesky factor; for the query side F^-T too.
 //   lowrank_kernel     C = Fq^T Fk, its singular triplets by one-sided Jacobi, the 32 largest:
 //                      Uq = Fq^-T U_r S_r^(1/2),  Uk = Fk^-T V_r S_r^(1/2) = Fq U_r S_r^(-1/2)
 //                      (V = C^T U S^-1 and Fk^-T Fk^T = I).
@@ -34,23 +34,16 @@ namespace t2t {
 // Gram matrices
 // ---------------------------------------------------------------------------
 constexpr int GR_ROWS = 128;                 // rows per tile
-constexpr int GR_SLAB_TILES = 64;            // tiles per CTA, at most: 8192 rows in one fp32 accumulation
+constexpr int GR_SLAB_TILES = 64;            // tiles per CTA: 8192 rows in one fp32 accumulation
 constexpr int GR_TILE = GR_ROWS * kD * 2;    // 32 KB
 constexpr int GR_STAGES = 3;
 constexpr int GR_SMEM = GR_STAGES * GR_TILE + 128 + 1024;
 
-// Tiles per slab: both sides' slabs should fill the chip twice over, but each costs 64 KB written and read again, so
-// four tiles (1024 rows' worth of input bytes, as much as the slab itself) are the least.  At 2 heads x 4096 rows one
-// CTA per head took 15 us a side.
-inline int gram_slab_tiles(int H, int N) {
-  const int even = cdiv(2 * H * cdiv(N, GR_ROWS), 2 * 148);
-  return even < 4 ? 4 : (even > GR_SLAB_TILES ? GR_SLAB_TILES : even);
-}
-inline int gram_slabs(int H, int N) { return cdiv(cdiv(N, GR_ROWS), gram_slab_tiles(H, N)); }
+__host__ __device__ inline int gram_slabs(int N) { return cdiv(cdiv(N, GR_ROWS), GR_SLAB_TILES); }
 
 __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUtensorMap mapQ,
                                                    const __grid_constant__ CUtensorMap mapK, float* __restrict__ partial,
-                                                   int N, int slab_tiles, int* __restrict__ status) {
+                                                   int N, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
@@ -64,8 +57,8 @@ __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUten
   const int slab = blockIdx.x, h = blockIdx.y, slabs = gridDim.x;
   const int m = blockIdx.z * gridDim.y + h;      // matrix: the query side's first, then the key side's
   const CUtensorMap* map = blockIdx.z ? &mapK : &mapQ;
-  const int tile0 = slab * slab_tiles;
-  const int ntiles = min(slab_tiles, cdiv(N, GR_ROWS) - tile0);
+  const int tile0 = slab * GR_SLAB_TILES;
+  const int ntiles = min(GR_SLAB_TILES, cdiv(N, GR_ROWS) - tile0);
 
   if (warp == 0) {
     tmem_alloc(tmem_slot, 128);
@@ -158,36 +151,25 @@ __device__ void column_norms2(const double* W, double* nrm2) {
   __syncthreads();
 }
 
-// The eight column pairs (x_i, y_i) of a round among the sixteen columns e that a warp holds in registers (lane l:
-// rows l, l + 32, l + 64, l + 96 of every column).  CROSS: column i of the first block with column i + R of the second
-// (mod 8); otherwise round R of the seven that bring every pair inside each block together.
-template <bool CROSS, int R>
-struct Round {
-  static __host__ __device__ constexpr int inner_x(int i) { return i == 0 ? 7 : (R + i) % 7; }
-  static __host__ __device__ constexpr int inner_y(int i) { return i == 0 ? R : (R + 7 - i) % 7; }
-  static __host__ __device__ constexpr int x(int i) { return CROSS ? i : (i & 4) * 2 + inner_x(i & 3); }
-  static __host__ __device__ constexpr int y(int i) { return CROSS ? 8 + ((i + R) & 7) : (i & 4) * 2 + inner_y(i & 3); }
+// The two column segments a warp holds in registers: lane l has rows l, l + 32, l + 64, l + 96 of every column.  After R
+// rounds the top column of pair i (0..7) is in t[(i + R) % 8], the bottom one in b[(i - R) % 8].
+struct Columns {
+  double t[8][4], b[8][4];
 };
 
-// One round.  A, B: the two blocks' numbers (column 8 A + i is e[i], column 8 B + i is e[8 + i]); lane l works out the
-// angle of pair l & 7.
-//
-// The angle itself only steers convergence, so it comes from fp32 arithmetic (relative error 1e-7 leaves 1e-7 of
-// the pair's product for the next visit); (c, s) is then normalised in fp64, so every rotation is orthogonal to
-// fp64 precision and nothing of the result depends on fp32.
-template <bool CROSS, int R>
-__device__ __forceinline__ void rotate8(double (&e)[16][4], int A, int B, double* nrm2, double2* cs, double tiny2,
-                                        float scale, bool& again) {
-  using P = Round<CROSS, R>;
-  const int lane = threadIdx.x & 31, p = lane & 7;
-  const int px = CROSS ? p : P::inner_x(p & 3), py = CROSS ? (p + R) & 7 : P::inner_y(p & 3);
-  const int cx = 8 * (CROSS || p < 4 ? A : B) + px, cy = 8 * (CROSS || p >= 4 ? B : A) + py;
+// One round: the eight disjoint pairs (top, bottom) of a warp.  cx, cy: column numbers of pair lane & 7, whose angle
+// this lane works out.  The angle comes from fp32 arithmetic and one Newton step in fp64 (relative error 1e-13);
+// (c, s) is normalised in fp64 to its last bits, so every rotation is orthogonal to fp64 precision.
+template <int R>
+__device__ __forceinline__ void rotate8(Columns& w, int cx, int cy, double* nrm2, double2* cs, double tiny2, float scale,
+                                        bool& again) {
+  const int lane = threadIdx.x & 31;
   double g[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    g[i] = e[P::x(i)][0] * e[P::y(i)][0];
+    g[i] = w.t[(i + R) & 7][0] * w.b[(i + 8 - R) & 7][0];
 #pragma unroll
-    for (int m = 1; m < 4; ++m) g[i] = fma(e[P::x(i)][m], e[P::y(i)][m], g[i]);
+    for (int m = 1; m < 4; ++m) g[i] = fma(w.t[(i + R) & 7][m], w.b[(i + 8 - R) & 7][m], g[i]);
   }
   // eight sums over the warp: lane l ends up with that of pair l & 7
   const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
@@ -207,17 +189,21 @@ __device__ __forceinline__ void rotate8(double (&e)[16][4], int A, int B, double
   double c = 1.0, s = 0.0;
   if (live) {
     // tan of the rotation: the smaller root of t^2 + (beta - alpha) / gamma t - 1 = 0
-    const double dx = beta - alpha, dy = 2.0 * gamma;
-    const float fx = fabsf((float)(dx * scale)), fy = fabsf((float)(dy * scale));
+    const double dx = beta - alpha;
+    const float fd = (float)(dx * scale), fg = (float)(gamma * scale);
+    const float fx = fabsf(fd), fy = 2.0f * fabsf(fg);
     const float lo = fminf(fx, fy) / fmaxf(fx, fy), root = sqrtf(fmaf(lo, lo, 1.0f));
-    const float tf = fy <= fx ? lo / (1.0f + root) : 1.0f / (lo + root);
-    const double t = ((dx >= 0.0) == (dy >= 0.0)) ? (double)tf : -(double)tf;
+    float tf = fy <= fx ? lo / (1.0f + root) : 1.0f / (lo + root);
+    if (fd != 0.0f && (fd < 0.0f) != (fg < 0.0f)) tf = -tf;
+    // Newton on gamma t^2 + dx t - gamma; the slope is at least dx or gamma in size
+    const double t0 = (double)tf;
+    const double res = fma(fma(gamma, t0, dx), t0, -gamma);
+    const double t = t0 - (double)((float)(res * scale) / fmaf(2.0f * fg, tf, fd));
     const double a = fma(t, t, 1.0);
-    double r = (double)rsqrtf((float)a);
-    r = r * fma(-0.5 * a, r * r, 1.5);
-    r = r * fma(-0.5 * a, r * r, 1.5);
-    c = r;
-    s = r * t;
+    const double y = (double)rsqrtf((float)a);
+    const double h = fma(-a * y, y, 1.0);                  // third-order step: error (1e-7)^3
+    c = fma(y * h, fma(h, 0.375, 0.5), y);
+    s = c * t;
     if (lane < 8) {
       nrm2[cx] = fmax(fma(-t, gamma, alpha), 0.0);
       nrm2[cy] = fmax(fma(t, gamma, beta), 0.0);
@@ -230,26 +216,60 @@ __device__ __forceinline__ void rotate8(double (&e)[16][4], int A, int B, double
     const double2 r = cs[i];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      const double a = e[P::x(i)][m], b = e[P::y(i)][m];
-      e[P::x(i)][m] = fma(r.x, a, -(r.y * b));
-      e[P::y(i)][m] = fma(r.y, a, r.x * b);
+      const double a = w.t[(i + R) & 7][m], b = w.b[(i + 8 - R) & 7][m];
+      w.t[(i + R) & 7][m] = fma(r.x, a, -(r.y * b));
+      w.b[(i + 8 - R) & 7][m] = fma(r.y, a, r.x * b);
     }
   }
   __syncwarp();      // cs and nrm2 may be written again
 }
 
+// Columns held at round r of the round-robin schedule (127 rounds): column 127 stays at the top of pair 0, the others
+// move round a ring of 127.
+__device__ __forceinline__ int top_column(int pair, int r) { return pair == 0 ? JD - 1 : (r + pair) % (JD - 1); }
+__device__ __forceinline__ int bottom_column(int pair, int r) { return (r + (JD - 1) - pair) % (JD - 1); }
+
+// Round R (mod 8) and the hand-over to the next one: one column enters and one leaves each segment of a warp.  The ring
+// runs down the tops (towards pair 0) and up the bottoms: top 1 -> bottom 0, bottom 63 -> top 63.
+template <int R>
+__device__ __forceinline__ void jacobi_round(Columns& w, int& r, double* xch, double* nrm2, double2* cs, double tiny2,
+                                             float scale, bool& again) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pair = 8 * warp + (lane & 7);
+  rotate8<R>(w, top_column(pair, r), bottom_column(pair, r), nrm2, cs, tiny2, scale, again);
+  r = r + 1 < JD - 1 ? r + 1 : 0;
+  constexpr int TI = R & 7, TN = (R + 1) & 7, BI = (15 - R) & 7;      // registers of top 0, of top 1, of bottom 7
+  double* tops = xch + (R & 1) * 16 * JD;                             // [8 warps][128] column leaving the tops
+  double* bots = tops + 8 * JD;                                       // [8 warps][128] column leaving the bottoms
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    tops[warp * JD + lane + 32 * m] = warp == 0 ? w.t[TN][m] : w.t[TI][m];
+    bots[warp * JD + lane + 32 * m] = w.b[BI][m];
+  }
+  if (warp == 0) {      // column 127 keeps its place while the registers' meaning moves on
+#pragma unroll
+    for (int m = 0; m < 4; ++m) w.t[TN][m] = w.t[TI][m];
+  }
+  __syncthreads();
+  const double* from_top = warp < 7 ? tops + (warp + 1) * JD : bots + 7 * JD;
+  const double* from_bot = warp > 0 ? bots + (warp - 1) * JD : tops;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    w.t[TI][m] = from_top[lane + 32 * m];
+    w.b[BI][m] = from_bot[lane + 32 * m];
+  }
+}
+
 // Rotates column pairs of W (column j at W + j * JLD) until all columns are mutually orthogonal.  Every thread of
-// the 256-thread CTA calls it.
+// the 256-thread CTA calls it.  W is overwritten meanwhile.
 //
-// 16 blocks of eight columns meet pairwise in 15 steps a sweep (round-robin); a warp loads the sixteen columns of a
-// block pair into registers, runs the eight rounds of eight disjoint pairs (and, in a sweep's first step, the seven
-// rounds inside the blocks) and writes them back, so shared memory carries the matrix once per eight rounds.  What
-// bounds a round: 160 warp-wide fp64 operations for the products and rotations on a pipe that takes two cycles each,
-// then the reduction's shuffles; the angle's arithmetic is done once per pair, one lane in eight of a warp's four
-// repeats.  (Blocks of four columns and 16 warps: 295 instructions for four pairs and half the shared-memory saving; the whole
-// fit 1.62 instead of 1.57 ms at 2 heads, both bound by the rounds' chain of dependent steps.)
-// A sweep in which no pair's cosine exceeded sqrt(kJacobiDone2) = 3e-8 leaves cosines of the order of its square
-// (inside a cluster of equal singular values, at most 3e-8), below the rounding of the fp32 factors: it is the last.
+// The 64 pairs of a round are disjoint; a warp keeps the sixteen columns of eight neighbouring pairs in registers and
+// passes one column of each segment on per round, so shared memory carries 32 KB a round instead of reading the matrix
+// twice and writing it once (384 KB).  What bounds a round now is its chain of dependent steps: products, a reduction of
+// five shuffles, the angle (worked out once per pair, not by every lane that holds a part of it), the rotation.  The
+// order of the rotations fixes the signs of the result, so it is part of what callers see.
+// A stretch of 128 rounds in which no pair's cosine exceeded sqrt(kJacobiDone2) = 3e-8 leaves cosines of the order of
+// its square (inside a cluster of equal singular values, at most 3e-8), below the rounding of the fp32 factors: it is
+// the last.
 __device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double2* cs = cs_all + warp * 8;
@@ -261,50 +281,60 @@ __device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
   for (int j = 0; j < JD; ++j) big = fmax(big, nrm2[j]);
   const double tiny2 = 1.0e-28 * big;
   const float scale = big > 0.0 ? (float)fmin(1.0e18 / big, 1.0e38) : 1.0f;      // keeps the fp32 angles in range
-  for (int sweep = 0; sweep < J_MAX_SWEEPS; ++sweep) {
+  int r = 0;
+  Columns w;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      w.t[i][m] = W[top_column(8 * warp + i, 0) * JLD + lane + 32 * m];
+      w.b[i][m] = W[bottom_column(8 * warp + i, 0) * JLD + lane + 32 * m];
+    }
+  __syncthreads();      // W now carries the columns that change warps
+#pragma unroll 1
+  for (int stretch = 0; stretch < J_MAX_SWEEPS; ++stretch) {
     bool again = false;
-    for (int step = 0; step < 15; ++step) {
-      // round-robin pairing of 16 blocks: block 15 stays, the others move round a ring of 15
-      int A, B;
-      if (warp == 0) { A = 15; B = step; }
-      else { A = (step + warp) % 15; B = (step + 15 - warp) % 15; }
-      double e[16][4];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          e[j][m] = W[(8 * A + j) * JLD + lane + 32 * m];
-          e[8 + j][m] = W[(8 * B + j) * JLD + lane + 32 * m];
-        }
-      if (step == 0) {      // every block is held by some warp: the pairs inside the blocks
-        rotate8<false, 0>(e, A, B, nrm2, cs, tiny2, scale, again);
-        rotate8<false, 1>(e, A, B, nrm2, cs, tiny2, scale, again);
-        rotate8<false, 2>(e, A, B, nrm2, cs, tiny2, scale, again);
-        rotate8<false, 3>(e, A, B, nrm2, cs, tiny2, scale, again);
-        rotate8<false, 4>(e, A, B, nrm2, cs, tiny2, scale, again);
-        rotate8<false, 5>(e, A, B, nrm2, cs, tiny2, scale, again);
-        rotate8<false, 6>(e, A, B, nrm2, cs, tiny2, scale, again);
-      }
-      rotate8<true, 0>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 1>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 2>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 3>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 4>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 5>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 6>(e, A, B, nrm2, cs, tiny2, scale, again);
-      rotate8<true, 7>(e, A, B, nrm2, cs, tiny2, scale, again);
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          W[(8 * A + j) * JLD + lane + 32 * m] = e[j][m];
-          W[(8 * B + j) * JLD + lane + 32 * m] = e[8 + j][m];
-        }
-      __syncthreads();
+#pragma unroll 1
+    for (int g = 0; g < 16; ++g) {
+      jacobi_round<0>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<1>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<2>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<3>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<4>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<5>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<6>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<7>(w, r, W, nrm2, cs, tiny2, scale, again);
     }
     if (!__syncthreads_or(again ? 1 : 0)) break;
-    column_norms2(W, nrm2);      // the running norms pick up rounding
+    // the running norms pick up rounding
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      double x = 0.0, y = 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        x = fma(w.t[i][m], w.t[i][m], x);
+        y = fma(w.b[i][m], w.b[i][m], y);
+      }
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) {
+        x += shfl_xor_d(x, d);
+        y += shfl_xor_d(y, d);
+      }
+      if (lane == 0) {
+        nrm2[top_column(8 * warp + i, r)] = x;
+        nrm2[bottom_column(8 * warp + i, r)] = y;
+      }
+    }
+    __syncwarp();      // the warp's next round reads its own columns' norms
   }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      W[top_column(8 * warp + i, r) * JLD + lane + 32 * m] = w.t[i][m];
+      W[bottom_column(8 * warp + i, r) * JLD + lane + 32 * m] = w.b[i][m];
+    }
   __syncthreads();
 }
 
@@ -408,13 +438,13 @@ __device__ __forceinline__ bool cholesky_inverse(double (&e)[16][4], double* Lc,
 //   invroots [H][128][128] fp64:   F^-T, query side only
 //   bad      [2 H] int: 1 when the matrix holds a non-finite value (non-finite input)
 //
-// Any factor serves: with Fq = Mq^(1/2) Oq and Fk = Mk^(1/2) Ok for orthogonal Oq, Ok, the singular value
-// decomposition of Fq^T Fk = Oq^T (Mq^(1/2) Mk^(1/2)) Ok has the same S, its U is Oq^T times the other one, and
-// Fq^-T U is the same matrix.  The Cholesky factor takes 128 short steps; the symmetric root needs all
-// eigenvectors (0.9 ms), and is left for the matrices the clamp may touch: those whose inverse has a trace
-// (an upper bound of 1 / smallest eigenvalue) of 1 / kEigFloor or more.
-// The whole fit took 5.9 ms at 2 heads x 4096 rows and 6.3 at 40 x 75,600 when every matrix needed its eigenvectors
-// and the Jacobi walked shared memory for each pair; 1.57 and 1.90 ms now (3.6 and 3.7 where both routes are needed).
+// Query side: any factor serves.  With Fq = Mq^(1/2) O for an orthogonal O, the singular value decomposition of
+// Fq^T Fk = O^T (Mq^(1/2) Fk) has the same S and V, its U is O^T times the other one, and Fq^-T U is the same matrix;
+// one-sided Jacobi, which only sees products of columns, takes the same rotations too.  The Cholesky factor needs 128
+// short steps and gives its inverse on the way; it is taken where the clamp cannot matter: where the trace of the
+// inverse (an upper bound of 1 / smallest eigenvalue) is below 1 / kEigFloor.
+// Key side: the symmetric root (another factor would turn the columns that the rotations work on, and with them the
+// signs of the result).
 __global__ void __launch_bounds__(J_THREADS, 1) factor_kernel(const float* __restrict__ partial, int slabs, int H,
                                                               double inv_n, double* __restrict__ roots,
                                                               double* __restrict__ invroots, int* __restrict__ bad) {
@@ -449,12 +479,12 @@ __global__ void __launch_bounds__(J_THREADS, 1) factor_kernel(const float* __res
     const int any_bad = __syncthreads_or(finite ? 0 : 1);
     if (tid == 0) bad[m] = any_bad;
     if (any_bad) return;      // the host raises; nothing below would converge on NaNs
-    double trace = 0.0;
-    const bool ok = cholesky_inverse(e, W, pub, nrm2, &trace);
-    __syncthreads();
-    if (ok && trace < 1.0 / kEigFloor) {
-      for (int i = tid; i < JD * JD; i += J_THREADS) Fo[i] = W[(i & 127) * JLD + (i >> 7)];
-      if (want_inv) {
+    if (want_inv) {
+      double trace = 0.0;
+      const bool ok = cholesky_inverse(e, W, pub, nrm2, &trace);
+      __syncthreads();
+      if (ok && trace < 1.0 / kEigFloor) {
+        for (int i = tid; i < JD * JD; i += J_THREADS) Fo[i] = W[(i & 127) * JLD + (i >> 7)];
         __syncthreads();
 #pragma unroll
         for (int a = 0; a < 16; ++a)
@@ -465,8 +495,8 @@ __global__ void __launch_bounds__(J_THREADS, 1) factor_kernel(const float* __res
           }
         __syncthreads();
         for (int i = tid; i < JD * JD; i += J_THREADS) Io[i] = W[(i >> 7) * JLD + (i & 127)];
+        return;
       }
-      return;
     }
   }
 
@@ -568,7 +598,7 @@ __global__ void __launch_bounds__(J_THREADS, 1) lowrank_kernel(const double* __r
 
 using namespace t2t;
 
-static size_t fit_off_roots(int H, int N) { return (((size_t)2 * H * gram_slabs(H, N) * kD * kD * 4) + 255) & ~(size_t)255; }
+static size_t fit_off_roots(int H, int N) { return (((size_t)2 * H * gram_slabs(N) * kD * kD * 4) + 255) & ~(size_t)255; }
 static size_t fit_off_inv(int H, int N) { return fit_off_roots(H, N) + (size_t)2 * H * kD * kD * 8; }
 
 extern "C" size_t t2t_lowrank_fit_ws_bytes(int H, int N) { return fit_off_inv(H, N) + (size_t)H * kD * kD * 8; }
@@ -589,7 +619,7 @@ extern "C" int t2t_lowrank_fit_strided(const void* q, const void* k, long long r
   float* partial = reinterpret_cast<float*>(w);
   double* roots = reinterpret_cast<double*>(w + fit_off_roots(H, N));
   double* invroots = reinterpret_cast<double*>(w + fit_off_inv(H, N));
-  const int slabs = gram_slabs(H, N);
+  const int slabs = gram_slabs(N);
   if (cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(lowrank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess)
@@ -598,7 +628,7 @@ extern "C" int t2t_lowrank_fit_strided(const void* q, const void* k, long long r
   if (!make_head_tile_map(&mq, q, (uint64_t)N, (uint64_t)H, GR_ROWS, (uint64_t)row_stride, (uint64_t)head_stride) ||
       !make_head_tile_map(&mk, k, (uint64_t)N, (uint64_t)H, GR_ROWS, (uint64_t)row_stride, (uint64_t)head_stride))
     return T2T_ERR_CUDA;
-  gram_kernel<<<dim3(slabs, H, 2), 128, GR_SMEM, st>>>(mq, mk, partial, N, gram_slab_tiles(H, N), d_status);
+  gram_kernel<<<dim3(slabs, H, 2), 128, GR_SMEM, st>>>(mq, mk, partial, N, d_status);
   factor_kernel<<<2 * H, J_THREADS, J_SMEM, st>>>(partial, slabs, H, 1.0 / (double)N, roots, invroots, d_bad);
   lowrank_kernel<<<H, J_THREADS, J_SMEM, st>>>(roots, invroots, H, d_bad, Uq, Uk);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
