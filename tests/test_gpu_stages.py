@@ -401,3 +401,28 @@ def test_tile_attn_empty_union_is_pure_residual(lib, small_case):
     err = (got.float() - want).abs()
     assert err.max() < 2e-2 and err.mean() < 2e-3
     assert info["pairs"] == 0
+
+
+@pytest.mark.parametrize("H, N", [(1, 1), (2, 127), (3, 129), (1, 2048), (8, 9473), (2, 37889)])
+@pytest.mark.parametrize("Cn", [1, 15, 17, 129, 512, 2048, 2050])
+def test_assign_edges_of_tiles_groups_and_chunks(lib, H, N, Cn):
+    """One and two row tiles per CTA (the last two shapes), ragged rows, centroid counts around a group of 16 and a
+    chunk of 128; a third of the centroids are copies of others - in the same group, in one other group, in many -
+    and a few rows and centroids are not finite.  Labels equal the all-exact kernel's (checked by the helper)."""
+    g = torch.Generator().manual_seed(N + Cn)
+    cen = torch.randn(H, Cn, 32, generator=g)
+    for c in range(0, Cn - 1, 3):
+        cen[:, c + 1] = cen[:, c]                    # same group, mostly
+    for c in range(2, Cn, 48):
+        cen[:, c] = cen[:, (c + 16) % Cn]            # two groups
+    cen[:, ::97] = cen[:, :1]                        # many groups
+    if Cn > 100:
+        cen[0, 77, 5] = float("inf")
+    x = cen[:, torch.randint(0, Cn, (N,), generator=g)] + 0.2 * torch.randn(H, N, 32, generator=g)
+    x[:, :: max(1, N // 7)] = cen[:, :1]             # exact hits
+    if N > 50:
+        x[0, 33] = float("nan")
+        x[0, 34, 2] = float("inf")
+    _assign(lib, x.to(BF).to(DEV), cen.to(BF).to(DEV))
+    finite = torch.nan_to_num(cen, posinf=1.0)       # and with finite centroids, where the bound does its work
+    _assign(lib, x.to(BF).to(DEV), finite.to(BF).to(DEV))

@@ -8,12 +8,11 @@
 
 namespace t2t {
 
-// Tensor-core assignment with exact verification (assign_tc.cu).  `amb` is a
-// scratch list of (H * N + 1) ints: a counter followed by the rows queued for
-// the exact re-evaluation.
+// Tensor-core assignment with exact verification (assign_tc.cu).  `settled`, where given, receives the
+// number of rows that the exact chain had to decide; assign_ws_bytes is what t2t_assign asks of its caller.
 size_t assign_ws_bytes(int H, int N);
 int launch_assign(const __nv_bfloat16* X, const __nv_bfloat16* cen, int* labels, int H, int N, int Cn,
-                  int pin_begin, int pin_label, int* amb, int* d_status, cudaStream_t st);
+                  int pin_begin, int pin_label, int* settled, int* d_status, cudaStream_t st);
 
 // Exact warp-per-row selection of the rows queued in fixq (select.cu).  fixq: per
 // head a count followed by (row, query cluster) pairs, H * (2 N + 1) ints.

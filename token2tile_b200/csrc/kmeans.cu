@@ -450,8 +450,8 @@ struct Carver {
 };
 
 struct KmmWs {
-  int *qlab1, *chist, *cbase_q, *cbase_k, *amb;
-  int *chist_k, *amb_k;      // the key side runs next to the query side and needs scratch of its own
+  int *qlab1, *chist, *cbase_q, *cbase_k;
+  int* chist_k;      // the key side runs next to the query side and needs scratch of its own
   __nv_bfloat16* cq1;
   float *vsum, *bmax;
   size_t total;
@@ -461,9 +461,7 @@ static KmmWs kmm_layout(int H, int N, int CQ, int C, void* base) {
   KmmWs w;
   const int nChunk = cdiv(N, GR_CHUNK);
   w.qlab1 = cv.take<int>((size_t)H * N);
-  w.amb = cv.take<int>((size_t)H * N + 1);
   w.chist = cv.take<int>((size_t)H * nChunk * CQ);
-  w.amb_k = cv.take<int>((size_t)H * N + 1);
   w.chist_k = cv.take<int>((size_t)H * nChunk * C);
   w.cbase_q = cv.take<int>((size_t)H * CQ);
   w.cbase_k = cv.take<int>((size_t)H * C);
@@ -604,7 +602,7 @@ extern "C" int t2t_kmeans_maintain_strided(const void* QU, const void* KU, const
   if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(sk, side->fork, 0) != cudaSuccess)
     return T2T_ERR_CUDA;
   rc = launch_assign((const bf16*)KU, (const bf16*)ck0, (int*)klab, H, N, C, pin_tail > 0 ? N - pin_tail : -1,
-                     C - 1, w.amb_k, d_status, sk);
+                     C - 1, nullptr, d_status, sk);
   if (rc == T2T_OK) {
     launch_group((const int*)klab, w.chist_k, (int*)kcounts, w.cbase_k, (int*)kperm, H, N, C, sk);
     key_mean_kernel<<<kgrid, CS_WARPS * 32, 0, sk>>>((const bf16*)KU, (const int*)kperm, (const int*)kcounts,
@@ -621,13 +619,13 @@ extern "C" int t2t_kmeans_maintain_strided(const void* QU, const void* KU, const
     return rc != T2T_OK ? rc : T2T_ERR_CUDA;
   }
   // queries, pass 1
-  rc = launch_assign((const bf16*)QU, (const bf16*)cq0, w.qlab1, H, N, CQ, -1, 0, w.amb, d_status, st);
+  rc = launch_assign((const bf16*)QU, (const bf16*)cq0, w.qlab1, H, N, CQ, -1, 0, nullptr, d_status, st);
   if (rc != T2T_OK) { join(); return rc; }
   launch_group(w.qlab1, w.chist, (int*)qcounts, w.cbase_q, (int*)qperm, H, N, CQ, st);
   fixed_mean_kernel<<<qgrid, CS_WARPS * 32, 0, st>>>((const bf16*)QU, (const int*)qperm, (const int*)qcounts,
                                                     w.cbase_q, (const bf16*)cq0, w.cq1, N, CQ);
   // queries, pass 2
-  rc = launch_assign((const bf16*)QU, w.cq1, (int*)qlab, H, N, CQ, -1, 0, w.amb, d_status, st);
+  rc = launch_assign((const bf16*)QU, w.cq1, (int*)qlab, H, N, CQ, -1, 0, nullptr, d_status, st);
   if (rc != T2T_OK) { join(); return rc; }
   launch_group((const int*)qlab, w.chist, (int*)qcounts, w.cbase_q, (int*)qperm, H, N, CQ, st);
   fixed_mean_kernel<<<qgrid, CS_WARPS * 32, 0, st>>>((const bf16*)QU, (const int*)qperm, (const int*)qcounts,
