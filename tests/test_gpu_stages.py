@@ -415,14 +415,50 @@ def test_assign_edges_of_tiles_groups_and_chunks(lib, H, N, Cn):
         cen[:, c + 1] = cen[:, c]                    # same group, mostly
     for c in range(2, Cn, 48):
         cen[:, c] = cen[:, (c + 16) % Cn]            # two groups
-    cen[:, ::97] = cen[:, :1]                        # many groups
+    cen[:, ::97] = cen[:, :1].clone()                # many groups
     if Cn > 100:
         cen[0, 77, 5] = float("inf")
     x = cen[:, torch.randint(0, Cn, (N,), generator=g)] + 0.2 * torch.randn(H, N, 32, generator=g)
-    x[:, :: max(1, N // 7)] = cen[:, :1]             # exact hits
+    x[:, :: max(1, N // 7)] = cen[:, :1].clone()     # exact hits
     if N > 50:
         x[0, 33] = float("nan")
         x[0, 34, 2] = float("inf")
     _assign(lib, x.to(BF).to(DEV), cen.to(BF).to(DEV))
     finite = torch.nan_to_num(cen, posinf=1.0)       # and with finite centroids, where the bound does its work
     _assign(lib, x.to(BF).to(DEV), finite.to(BF).to(DEV))
+
+
+@pytest.mark.parametrize("sizes", [(256, 129, 128, 127, 1, 3455 - 256 * 11), (4096,)])
+def test_tile_attn_reference_maximum_far_below_later_scores(lib, sizes):
+    """The softmax keeps its first tile's maximum as reference and corrects when the weights grow: a slow climb
+    (8 bits a tile: the running sum passes 2^24), jumps inside the first half of a tile (20, 40, 150 bits) and inside
+    the second (70 bits: above 2^60; 140 bits: past the largest float), a fall, and rows that see none of it or all of
+    it upside down.  Against a float64 softmax of the same bfloat16 values; the weights are rounded to bfloat16
+    (2^-9 of values around 1, averaged) and so is the output."""
+    N, H = 4096, 1
+    sizes = list(sizes) + [256] * 11 if len(sizes) > 1 else list(sizes)
+    assert sum(sizes) == N
+    g = torch.Generator().manual_seed(N + len(sizes))
+    level = torch.zeros(N)
+    for tile, pos, jump in ((2, 10, 20.0), (4, 3, 40.0), (6, 70, 70.0), (9, 100, 140.0), (12, 0, -200.0), (14, 20, 150.0)):
+        level[tile * 128 + pos:] += jump
+    level[16 * 128:] += 8.0 * (torch.arange(16 * 128) // 128)
+    level += 2.0 * torch.randn(N, generator=g)
+    k = 0.1 * torch.randn(H, N, 128, generator=g)
+    k[0, :, 0] = level * math.sqrt(128.0) / math.log2(math.e) / 16.0
+    q = 0.1 * torch.randn(H, N, 128, generator=g)
+    q[0, :, 0] = 16.0 * torch.tensor([1.0, 0.5, 0.0, -1.0])[torch.randint(0, 4, (N,), generator=g)]
+    v = torch.randn(H, N, 128, generator=g)
+    q, k, v = q.to(BF), k.to(BF), v.to(BF)
+    CQ = len(sizes)
+    ids = torch.arange(N, dtype=torch.int32)[None]
+    km = dict(qcounts=torch.tensor([sizes], dtype=torch.int32), kcounts=torch.full((H, 2048), 2, dtype=torch.int32),
+              qperm=ids, kperm=ids, qlab=torch.repeat_interleave(torch.arange(CQ), torch.tensor(sizes)).int()[None],
+              V_sorted=v, sumv=torch.zeros(H, 2048, 128, dtype=BF), lam=torch.ones(H))
+    full = torch.full((H, CQ, 64), -1, dtype=torch.int32)
+    zeros = torch.zeros(H, N, 32, dtype=BF)
+    _, info = _tile_attn(lib, q, k, v, zeros, km, zeros[:, :2048].contiguous(), full)
+    s = q[0].double() @ k[0].double().T / math.sqrt(128.0)
+    want = torch.softmax(s, 1) @ v[0].double()
+    assert (info["attn_o"][0].double() - want).abs().max() < 2e-2
+    assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-2
