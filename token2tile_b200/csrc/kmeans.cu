@@ -115,27 +115,43 @@ __global__ void __launch_bounds__(AS_THREADS) assign_exact_kernel(const __nv_bfl
 // ---------------------------------------------------------------------------
 // stable grouping: per-chunk histograms -> offsets -> scatter
 // ---------------------------------------------------------------------------
-constexpr int GR_CHUNK = 1024;   // rows per warp
 constexpr int GR_WARPS = 4;
+// Rows per warp: a warp walks its rows 32 at a time, a chain of label -> match -> counter steps of about 100 cycles, and
+// a short problem wants more warps instead (2 heads x 4096 rows ran on two CTAs a side); a long one wants few histograms.
+static int group_chunk(int N) { return N <= 16384 ? 256 : 1024; }
 
+// The labels of a warp's IT x 32 rows, all fetched before the first is used; -1 past the end and for a label outside
+// [0, Cn), which is ignored, never indexed.
+template <int IT>
+__device__ __forceinline__ void load_labels(const int* __restrict__ labh, int r0, int N, int Cn, int (&c)[IT]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const int row = r0 + 32 * i + lane;
+    c[i] = row < N ? labh[row] : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < IT; ++i)
+    if ((unsigned)c[i] >= (unsigned)Cn) c[i] = -1;
+}
+
+template <int IT>
 __global__ void __launch_bounds__(GR_WARPS * 32) hist_kernel(const int* __restrict__ lab,
                                                              int* __restrict__ chist, int N, int Cn,
                                                              int nChunk) {
   extern __shared__ int sh[];
   const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunk = blockIdx.x * GR_WARPS + warp;
+  if (chunk >= nChunk) return;
   int* hh = sh + warp * Cn;
+  int c[IT];
+  load_labels<IT>(lab + (size_t)h * N, chunk * IT * 32, N, Cn, c);
   for (int i = lane; i < Cn; i += 32) hh[i] = 0;
   __syncwarp();
-  if (chunk >= nChunk) return;
-  const int* labh = lab + (size_t)h * N;
-  const int r0 = chunk * GR_CHUNK, r1 = min(N, r0 + GR_CHUNK);
-  for (int r = r0; r < r1; r += 32) {
-    const int row = r + lane;
-    int c = row < r1 ? labh[row] : -1;
-    if ((unsigned)c >= (unsigned)Cn) c = -1;      // a label outside [0, Cn) is ignored, never indexed
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    if (c >= 0 && lane == __ffs(peers) - 1) hh[c] += __popc(peers);
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const unsigned peers = __match_any_sync(0xffffffffu, c[i]);
+    if (c[i] >= 0 && lane == __ffs(peers) - 1) hh[c[i]] += __popc(peers);
     __syncwarp();
   }
   int* out = chist + ((size_t)h * nChunk + chunk) * Cn;
@@ -148,6 +164,7 @@ __global__ void __launch_bounds__(1024) offsets_kernel(int* __restrict__ chist, 
                                                        int* __restrict__ cbase, int Cn, int nChunk) {
   __shared__ int wsum[32];
   __shared__ int carry_s;
+  constexpr int B = 16;      // histogram entries in flight per thread (the offsets replace them, one batch behind)
   const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* ch = chist + (size_t)h * nChunk * Cn;
   if (tid == 0) carry_s = 0;
@@ -156,7 +173,13 @@ __global__ void __launch_bounds__(1024) offsets_kernel(int* __restrict__ chist, 
     const int c = c0 + tid;
     int tot = 0;
     if (c < Cn)
-      for (int k = 0; k < nChunk; ++k) tot += ch[(size_t)k * Cn + c];
+      for (int k0 = 0; k0 < nChunk; k0 += B) {
+        int t[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) t[k] = k0 + k < nChunk ? ch[(size_t)(k0 + k) * Cn + c] : 0;
+#pragma unroll
+        for (int k = 0; k < B; ++k) tot += t[k];
+      }
     int inc = warp_incl_scan(tot, lane);
     if (lane == 31) wsum[warp] = inc;
     __syncthreads();
@@ -172,10 +195,16 @@ __global__ void __launch_bounds__(1024) offsets_kernel(int* __restrict__ chist, 
       counts[(size_t)h * Cn + c] = tot;
       cbase[(size_t)h * Cn + c] = base;
       int r = base;
-      for (int k = 0; k < nChunk; ++k) {
-        const int t = ch[(size_t)k * Cn + c];
-        ch[(size_t)k * Cn + c] = r;
-        r += t;
+      for (int k0 = 0; k0 < nChunk; k0 += B) {
+        int t[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) t[k] = k0 + k < nChunk ? ch[(size_t)(k0 + k) * Cn + c] : 0;
+#pragma unroll
+        for (int k = 0; k < B; ++k)
+          if (k0 + k < nChunk) {
+            ch[(size_t)(k0 + k) * Cn + c] = r;
+            r += t[k];
+          }
       }
     }
     __syncthreads();
@@ -184,6 +213,7 @@ __global__ void __launch_bounds__(1024) offsets_kernel(int* __restrict__ chist, 
   }
 }
 
+template <int IT>
 __global__ void __launch_bounds__(GR_WARPS * 32) scatter_kernel(const int* __restrict__ lab,
                                                                 const int* __restrict__ choff,
                                                                 int* __restrict__ perm, int N, int Cn,
@@ -194,36 +224,40 @@ __global__ void __launch_bounds__(GR_WARPS * 32) scatter_kernel(const int* __res
   if (chunk >= nChunk) return;
   int* cur = sh + warp * Cn;
   const int* off = choff + ((size_t)h * nChunk + chunk) * Cn;
+  int c[IT];
+  load_labels<IT>(lab + (size_t)h * N, chunk * IT * 32, N, Cn, c);
   for (int i = lane; i < Cn; i += 32) cur[i] = off[i];
   __syncwarp();
-  const int* labh = lab + (size_t)h * N;
   int* out = perm + (size_t)h * N;
-  const int r0 = chunk * GR_CHUNK, r1 = min(N, r0 + GR_CHUNK);
-  for (int r = r0; r < r1; r += 32) {
-    const int row = r + lane;
-    int c = row < r1 ? labh[row] : -1;
-    if ((unsigned)c >= (unsigned)Cn) c = -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const unsigned peers = __match_any_sync(0xffffffffu, c[i]);
     const int leader = __ffs(peers) - 1;
     const int rank = __popc(peers & ((1u << lane) - 1u));
     int base = 0;
-    if (c >= 0 && lane == leader) {
-      base = cur[c];
-      cur[c] = base + __popc(peers);
+    if (c[i] >= 0 && lane == leader) {
+      base = cur[c[i]];
+      cur[c[i]] = base + __popc(peers);
     }
     base = __shfl_sync(0xffffffffu, base, leader);
-    if (c >= 0) out[base + rank] = row;
+    if (c[i] >= 0) out[base + rank] = chunk * IT * 32 + 32 * i + lane;
     __syncwarp();
   }
 }
 
+template <int IT>
+static void launch_group_of(const int* lab, int* chist, int* counts, int* cbase, int* perm, int H, int N, int Cn,
+                            cudaStream_t st) {
+  const int nChunk = cdiv(N, IT * 32);
+  const size_t sh = (size_t)GR_WARPS * Cn * sizeof(int);
+  hist_kernel<IT><<<dim3(cdiv(nChunk, GR_WARPS), H), GR_WARPS * 32, sh, st>>>(lab, chist, N, Cn, nChunk);
+  offsets_kernel<<<H, 1024, 0, st>>>(chist, counts, cbase, Cn, nChunk);
+  scatter_kernel<IT><<<dim3(cdiv(nChunk, GR_WARPS), H), GR_WARPS * 32, sh, st>>>(lab, chist, perm, N, Cn, nChunk);
+}
 static void launch_group(const int* lab, int* chist, int* counts, int* cbase, int* perm, int H, int N,
                          int Cn, cudaStream_t st) {
-  const int nChunk = cdiv(N, GR_CHUNK);
-  const size_t sh = (size_t)GR_WARPS * Cn * sizeof(int);
-  hist_kernel<<<dim3(cdiv(nChunk, GR_WARPS), H), GR_WARPS * 32, sh, st>>>(lab, chist, N, Cn, nChunk);
-  offsets_kernel<<<H, 1024, 0, st>>>(chist, counts, cbase, Cn, nChunk);
-  scatter_kernel<<<dim3(cdiv(nChunk, GR_WARPS), H), GR_WARPS * 32, sh, st>>>(lab, chist, perm, N, Cn, nChunk);
+  if (group_chunk(N) == 256) launch_group_of<8>(lab, chist, counts, cbase, perm, H, N, Cn, st);
+  else launch_group_of<32>(lab, chist, counts, cbase, perm, H, N, Cn, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -459,7 +493,7 @@ struct KmmWs {
 static KmmWs kmm_layout(int H, int N, int CQ, int C, void* base) {
   Carver cv(base);
   KmmWs w;
-  const int nChunk = cdiv(N, GR_CHUNK);
+  const int nChunk = cdiv(N, group_chunk(N));
   w.qlab1 = cv.take<int>((size_t)H * N);
   w.chist = cv.take<int>((size_t)H * nChunk * CQ);
   w.chist_k = cv.take<int>((size_t)H * nChunk * C);
@@ -494,7 +528,7 @@ struct UpdWs {
 static UpdWs upd_layout(int H, int N, int Cn, void* base) {
   Carver cv(base);
   UpdWs w;
-  w.chist = cv.take<int>((size_t)H * cdiv(N, GR_CHUNK) * Cn);
+  w.chist = cv.take<int>((size_t)H * cdiv(N, group_chunk(N)) * Cn);
   w.cbase = cv.take<int>((size_t)H * Cn);
   w.perm = cv.take<int>((size_t)H * N);
   w.total = cv.off;

@@ -31,17 +31,20 @@
 
 namespace t2t {
 
-constexpr int ST_THREADS = 512;
-constexpr int ST_CH = 64;                  // centroids per MMA chunk
-constexpr int ST_NCH = kC / ST_CH;         // 32: eight per column group, double-buffered in TMEM
+constexpr int ST_G = 8;                    // column groups of 128 threads (a thread per row of the tile)
+constexpr int ST_THREADS = ST_G * 128;     // 32 warps: the passes are chains of short dependent steps (histogram updates,
+                                           // candidate lists), and 16 warps left a third of the issue slots empty
+constexpr int ST_CH = 32;                  // centroids per MMA chunk
+constexpr int ST_NCH = kC / ST_CH;         // 64: eight per column group, double-buffered in TMEM
 constexpr int ST_B = 64;                   // histogram buckets
 constexpr int ST_CAP = 64;                 // candidates per row
 constexpr int ST_REFINE = 40;              // refine the bucket when it alone holds more clusters than this
 constexpr int ST_MAX_ITERS = 5;
 constexpr int kMomFloats = 32 + 32 * 32;   // per head: mean centroid, second-moment matrix
 constexpr int kMomParts = 8;               // the moments are summed over this many slices of the centroids
-constexpr int ST_TPC = 4;                  // consecutive 128-row tiles of one head per CTA: the head's centroids, sizes
-                                           // and prefix sums are staged once for all of them
+constexpr int ST_MAX_TPC = 8;              // consecutive 128-row tiles of one head per CTA, at most: the head's centroids,
+                                           // sizes and prefix sums are staged once for all of them
+constexpr float ST_SPAN = 0.8f;            // half width of the first histogram range, in standard deviations of a row's scores
 constexpr int ST_STRAGGLERS = 8;           // this few unsettled rows of a tile go to the exact kernel instead of another pass
 
 constexpr int OFF_CK = 0;                               // 1024 rows x 128 B: centroid c in row c % 1024, half c / 1024
@@ -49,14 +52,14 @@ constexpr int OFF_A = OFF_CK + 1024 * 128;              // 128 rows x 128 B (fir
 constexpr int OFF_HIST = OFF_A + 128 * 128;             // [ST_B][128] packed (size << 12 | count); after P2 the
 constexpr int OFF_CAND = OFF_HIST;                      //   same bytes hold [128][ST_CAP] cluster | key << 16
 constexpr int OFF_SIZE = OFF_HIST + ST_B * 128 * 4;     // [2048] (cluster size << 12) + 1
-constexpr int OFF_PART = OFF_SIZE + kC * 4;             // [3][4][128] per-group partial max / sum / sum of squares
-constexpr int OFF_ROW = OFF_PART + 12 * 128 * 4;        // [17][128] per-row scalars
+constexpr int OFF_PART = OFF_SIZE + kC * 4;             // [2][ST_G][128] per-group partial sums
+constexpr int OFF_ROW = OFF_PART + 2 * ST_G * 128 * 4;        // [17][128] per-row scalars
 constexpr int ST_MAXSEG = 8;                            // query clusters one tile may span on the fast path
 constexpr int ST_MAXCQ = 2048;                          // prefix sums of the query-cluster sizes live in smem
 constexpr int OFF_UNION = OFF_ROW + 17 * 128 * 4;       // [ST_MAXSEG][64] segment bitmaps
 constexpr int OFF_PRE = OFF_UNION + ST_MAXSEG * 64 * 4; // [ST_MAXCQ + 1] first sorted row of every query cluster
 constexpr int OFF_MISC = OFF_PRE + (ST_MAXCQ + 4) * 4;  // barriers, segment tables, ...
-constexpr int OFF_MOM = OFF_MISC + 512;                 // [kMomFloats] the head's centroid moments
+constexpr int OFF_MOM = OFF_MISC + 640;                 // [kMomFloats] the head's centroid moments
 constexpr int ST_SMEM = OFF_MOM + kMomFloats * 4 + 1024;
 static_assert(ST_SMEM <= 227 * 1024, "shared memory of select_tc_kernel");
 
@@ -78,12 +81,42 @@ __device__ __forceinline__ int key16_from_score(float s) { return key16_from_hal
 // same slot, hit 32 different banks (the row stride, ST_CAP words, is a multiple of the bank count).
 __device__ __forceinline__ int cand_at(int r, int slot) { return r * ST_CAP + ((slot + r) & (ST_CAP - 1)); }
 
+// Packed fp32 pairs, rounded toward -inf.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma_rm2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add_rm2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Adds to bucket `b` of the histogram column at `col` if there is such a bucket.  (As a conditional atomicAdd this was a
+// branch around every update, 3.4 control instructions a score; predicated it is one.)
+__device__ __forceinline__ void hist_add(uint32_t col, int b, int value) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.lt.u32 p, %1, %3;\n"
+      " @p red.shared::cta.add.u32 [%0], %2;\n}\n" ::"r"(col + (uint32_t)b * 512u),
+      "r"(b), "r"(value), "n"(ST_B)
+      : "memory");
+}
+
 __device__ __forceinline__ void wg_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
 
 __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     const __nv_bfloat16* __restrict__ QU, const __nv_bfloat16* __restrict__ cks,
     const int* __restrict__ kcounts, const int* __restrict__ qperm, const int* __restrict__ tile_sizes,
-    const int* __restrict__ ns_ptr, int* __restrict__ unip, int* __restrict__ rowcnt, int N, int CQ,
+    const int* __restrict__ ns_ptr, int* __restrict__ unip, int* __restrict__ rowcnt, int N, int CQ, int tpc,
     int* __restrict__ fixq, const float* __restrict__ mom, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -97,17 +130,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   int* sRowI = reinterpret_cast<int*>(sm + OFF_ROW);
   uint32_t* sUnion = reinterpret_cast<uint32_t*>(sm + OFF_UNION);             // [ST_MAXSEG][64]
   int* sPre = reinterpret_cast<int*>(sm + OFF_PRE);                           // [CQ + 1]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_MISC);                // [4 groups][2 buffers]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 320);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 324);
-  int* sCmax = reinterpret_cast<int*>(sm + OFF_MISC + 328);                    // max ||cks||^2 as int bits
-  int* sScan = reinterpret_cast<int*>(sm + OFF_MISC + 64);                    // [16] scan scratch
-  int* sSegClu = reinterpret_cast<int*>(sm + OFF_MISC + 128);                 // [ST_MAXSEG] cluster of each segment
-  uint32_t* sSegMask = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 160);      // [4 warps][ST_MAXSEG] lanes of a segment
-  int* sNseg = reinterpret_cast<int*>(sm + OFF_MISC + 288);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_MISC);                // [ST_G groups][2 buffers]
+  int* sScan = reinterpret_cast<int*>(sm + OFF_MISC + 128);                   // [32] scan scratch
+  int* sSegClu = reinterpret_cast<int*>(sm + OFF_MISC + 256);                 // [ST_MAXSEG] cluster of each segment
+  uint32_t* sSegMask = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 288);      // [4 warps][ST_MAXSEG] lanes of a segment
+  int* sNseg = reinterpret_cast<int*>(sm + OFF_MISC + 416);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 420);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC + 424);
+  int* sCmax = reinterpret_cast<int*>(sm + OFF_MISC + 428);                    // max ||cks||^2 as int bits
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = tid >> 7;            // column group: chunks g, g + 4, g + 8, ...
+  const int g = tid >> 7;            // column group: chunks g, g + ST_G, g + 2 ST_G, ...
   const int r = tid & 127;           // row of the tile = TMEM lane
   const int h = blockIdx.y;
   const __nv_bfloat16* ckh = cks + (size_t)h * kC * kR;
@@ -119,10 +152,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   if (tid == 0) {
     *abort_flag = 0;
     *sCmax = 0;
-    for (int i = 0; i < 8; ++i) mbar_init(bars + i, 1);
+    for (int i = 0; i < 2 * ST_G; ++i) mbar_init(bars + i, 1);
     mbar_init_fence();
   }
-  sUnion[tid] = 0u;                                     // ST_MAXSEG * 64 == ST_THREADS words
+  if (tid < ST_MAXSEG * 64) sUnion[tid] = 0u;
   // all 2048 centroids: 16-byte chunk id -> centroid id >> 2, chunk id & 3
 #pragma unroll
   for (int i = 0; i < (kC * 4) / ST_THREADS; ++i) {
@@ -198,12 +231,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   // chunk i + 1 runs while chunk i is scanned.  body(cbase, v) sees 32
   // consecutive approximate scores of this thread's row.
   auto issue = [&](int i) {        // called by the group's first thread
-    const int cc = g + 4 * i, b = i & 1;
+    const int cc = g + ST_G * i, b = i & 1;
     tc_fence_after();
 #pragma unroll
     for (int s2 = 0; s2 < 2; ++s2)
       umma_ss(tmem + g * 2 * ST_CH + b * ST_CH, make_sdesc(sA + s2 * 32, 16, 1024),
-              make_sdesc(sCk + (cc & 15) * (ST_CH * 128) + (cc >> 4) * 64 + s2 * 32, 16, 1024), idesc,
+              make_sdesc(sCk + (cc & (ST_NCH / 2 - 1)) * (ST_CH * 128) + cc / (ST_NCH / 2) * 64 + s2 * 32, 16, 1024), idesc,
               s2 > 0 ? 1u : 0u);
     umma_commit(bars + g * 2 + b);
   };
@@ -211,33 +244,30 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     if (dead) return;
     if (r == 0) issue(0);
 #pragma unroll 1
-    for (int i = 0; i < ST_NCH / 4; ++i) {
-      const int cc = g + 4 * i, b = i & 1;
+    for (int i = 0; i < ST_NCH / ST_G; ++i) {
+      const int cc = g + ST_G * i, b = i & 1;
       // every warp of the group has finished reading the other buffer (chunk i - 1): refill it
       tc_fence_before();
       wg_sync(g);
-      if (r == 0 && i + 1 < ST_NCH / 4) issue(i + 1);
+      if (r == 0 && i + 1 < ST_NCH / ST_G) issue(i + 1);
       if (!mbar_wait(bars + g * 2 + b, b ? ph1 : ph0, abort_flag)) { dead = true; break; }
       if (b) ph1 ^= 1u; else ph0 ^= 1u;
       tc_fence_after();
-#pragma unroll 1      // keeps each pass body at 32 columns of code; fully unrolled the kernel outgrows the I-cache
-      for (int q = 0; q < ST_CH / 32; ++q) {
-        uint32_t v[32];
-        tmem_ld32(t_lane + b * ST_CH + q * 32, v);
-        tmem_wait_ld();
-        body(cc * ST_CH + q * 32, v);
-      }
+      uint32_t v[32];
+      tmem_ld32(t_lane + b * ST_CH, v);
+      tmem_wait_ld();
+      body(cc * ST_CH, v);
     }
     tc_fence_before();
     wg_sync(g);
   };
 
 #pragma unroll 1
-  for (int ti = 0; ti < ST_TPC; ++ti) {
-    const int p0 = (blockIdx.x * ST_TPC + ti) * 128;    // first sorted row of this tile
+  for (int ti = 0; ti < tpc; ++ti) {
+    const int p0 = (blockIdx.x * tpc + ti) * 128;    // first sorted row of this tile
     if (p0 >= N || dead) break;
     const int rows_here = min(128, N - p0);
-    {
+    if (tid < 512) {
       const int ar = tid >> 2, ch = tid & 3;
       const bool valid = ar < rows_here;
       const int orig = valid ? qperm[(size_t)h * N + p0 + ar] : 0;
@@ -303,7 +333,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     // ---- P1: mean and standard deviation of the row's scores, without a pass over them ------------
     // sum_c q.c = q . sum_c c and sum_c (q.c)^2 = q^T (sum_c c c^T) q: the head's centroid moments (a
     // 32-vector and a 32 x 32 matrix, fp32) give both in 1056 multiply-adds per row.  Each column group
-    // takes eight rows of the matrix.  The statistics only place the first histogram range.
+    // takes four rows of the matrix.  The statistics only place the first histogram range.
     {
       const float* mh = sMom;
       float qv[32];
@@ -314,17 +344,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
 #pragma unroll
         for (int e = 0; e < 4; ++e) { qv[q4 * 8 + 2 * e] = bf_lo(ws[e]); qv[q4 * 8 + 2 * e + 1] = bf_hi(ws[e]); }
       }
-      float qa[8];      // elements 8 g .. 8 g + 7 of the row: chunk g
+      constexpr int PER = kR / ST_G;
+      float qa[PER];      // elements PER g .. PER g + PER - 1 of the row
       {
-        const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, g));
-        const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { qa[2 * e] = bf_lo(ws[e]); qa[2 * e + 1] = bf_hi(ws[e]); }
+        const uint2 w = *reinterpret_cast<const uint2*>(sm + OFF_A + sw128(r, g >> 1) + (g & 1) * 8);
+        qa[0] = bf_lo(w.x); qa[1] = bf_hi(w.x); qa[2] = bf_lo(w.y); qa[3] = bf_hi(w.y);
       }
+      static_assert(PER == 4, "eight bytes of the row per group");
       float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4* grow = reinterpret_cast<const float4*>(mh + 32 + (8 * g + i) * 32);
+      for (int i = 0; i < PER; ++i) {
+        const float4* grow = reinterpret_cast<const float4*>(mh + 32 + (PER * g + i) * 32);
         float t0 = 0.f, t1 = 0.f;
 #pragma unroll
         for (int b4 = 0; b4 < 8; ++b4) {
@@ -335,34 +365,36 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
           t1 = fmaf(mm.w, qv[4 * b4 + 3], t1);
         }
         s2 = fmaf(qa[i], t0 + t1, s2);
-        s1 = fmaf(qa[i], mh[8 * g + i], s1);
+        s1 = fmaf(qa[i], mh[PER * g + i], s1);
       }
-      sPart[(1 * 4 + g) * 128 + r] = s1;
-      sPart[(2 * 4 + g) * 128 + r] = s2;
+      sPart[g * 128 + r] = s1;
+      sPart[(ST_G + g) * 128 + r] = s2;
     }
     __syncthreads();
     if (g == 0 && sRowI[R_STATE * 128 + r] == RS_SEARCH) {
       float mean = 0.f, s2 = 0.f;
 #pragma unroll
-      for (int gg = 0; gg < 4; ++gg) {
-        mean += sPart[(1 * 4 + gg) * 128 + r];
-        s2 += sPart[(2 * 4 + gg) * 128 + r];
+      for (int gg = 0; gg < ST_G; ++gg) {
+        mean += sPart[gg * 128 + r];
+        s2 += sPart[(ST_G + gg) * 128 + r];
       }
       const float M = sRowF[R_MAX * 128 + r];
       const float sd = sqrtf(fmaxf(s2 - mean * mean, 1.0e-20f));
       const bool finite = fabsf(M) < INFINITY && fabsf(s2) < INFINITY && fabsf(mean) < INFINITY;
-      // First range: 2.5 standard deviations around the score a fraction ns / N of a bell-shaped
-      // distribution would exceed (inverse normal tail, Abramowitz-Stegun 26.2.23).  Everything above the
-      // range is counted in an overflow bucket.  The range only has to be a good guess: the search continues
-      // above it (up to the bound ||q|| max ||c||) or below it when the running token count says so.
+      // First range: ST_SPAN standard deviations to either side of the score a fraction ns / N of a bell-shaped
+      // distribution would exceed (inverse normal tail, Abramowitz-Stegun 26.2.23; on clustered activations the
+      // thresholds of a tile's rows lie 0.35 to 0.6 deviations apart, centred within 0.15 of it).  Everything
+      // above the range is counted in an overflow bucket.  The range only has to be a good guess: the search continues
+      // above it (up to the bound ||q|| max ||c||) or below it when the running token count says so; the narrower it
+      // is, the finer the buckets and the fewer the candidates.
       const float f = fminf(0.5f, fmaxf((float)ns / (float)N, 1.0e-6f));
       const float tt = sqrtf(-2.0f * __logf(f));
       const float z = tt - (2.515517f + tt * (0.802853f + tt * 0.010328f)) /
                                (1.0f + tt * (1.432788f + tt * (0.189269f + tt * 0.001308f)));
-      float hi = mean + (z + 1.25f) * sd;
+      float hi = mean + (z + ST_SPAN) * sd;
       const int ovf = hi < M ? 1 : 0;
       hi = ovf ? hi : M;
-      const float lo = fminf(mean + (z - 1.25f) * sd, hi);
+      const float lo = fminf(mean + (z - ST_SPAN) * sd, hi);
       sRowF[R_HI * 128 + r] = hi;
       sRowF[R_LO * 128 + r] = lo;
       sRowI[R_OVF * 128 + r] = ovf;
@@ -380,26 +412,28 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
         const bool act = sRowI[R_STATE * 128 + r] == RS_SEARCH;
         const float hi = act ? sRowF[R_HI * 128 + r] : -INFINITY;
         const float inv = act ? sRowF[R_INV * 128 + r] : 1.0f;
-        const float ninv = -inv, hiinv = hi * inv;
         // with an overflow bucket, bucket 0 takes every score above hi and the range starts at bucket 1
         const int ovf = act ? sRowI[R_OVF * 128 + r] : 0;
-        const int bmin = ovf - 1;
-        int* hist_r = sHist + r;
+        const unsigned long long ninv2 = pack2(-inv, -inv), hiinv2 = pack2(hi * inv, hi * inv), magic2 = pack2(12582912.0f, 12582912.0f);
+        const int shift = 0x4B400000 - ovf, bmin = ovf - 1;
+        const uint32_t hist_r = smem_u32(sHist + r);
         stream([&](int cbase, const uint32_t(&v)[32]) {
 #pragma unroll
           for (int j4 = 0; j4 < 32; j4 += 4) {
             const int4 p4 = *reinterpret_cast<const int4*>(sSizeP + cbase + j4);
             const int pp[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
+            for (int e = 0; e < 4; e += 2) {
               // floor by an add rounded toward -inf: 1.5 * 2^23 + t has floor(t) in its low mantissa bits for
               // |t| < 2^22; beyond that the difference keeps the sign of t and is far outside [0, ST_B).
               // t = (hi - s) inv as one multiply-add: a score within a rounding step of a bucket boundary may
               // land in the neighbouring bucket, which only moves the window (the selection is validated
-              // against exact keys afterwards)
-              const float t = __fmaf_rd(__uint_as_float(v[j4 + e]), ninv, hiinv);
-              const int b = max(__float_as_int(__fadd_rd(t, 12582912.0f)) - 0x4B400000 + ovf, bmin);
-              if ((unsigned)b < (unsigned)ST_B) atomicAdd(hist_r + b * 128, pp[e]);
+              // against exact keys afterwards).  Two scores per instruction.
+              const unsigned long long t2 = fma_rm2(pack2(__uint_as_float(v[j4 + e]), __uint_as_float(v[j4 + e + 1])), ninv2, hiinv2);
+              float f0, f1;
+              unpack2(add_rm2(t2, magic2), f0, f1);
+              hist_add(hist_r, max(__float_as_int(f0) - shift, bmin), pp[e]);
+              hist_add(hist_r, max(__float_as_int(f1) - shift, bmin), pp[e + 1]);
             }
           }
         });
@@ -537,7 +571,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     }
     __syncthreads();
 
-    // ---- exact keys of the candidates (four threads share a row) ------------------
+    // ---- exact keys of the candidates (eight threads share a row) -----------------
     {
       const int st = sRowI[R_STATE * 128 + r];
       const int n = sRowI[R_NCAND * 128 + r];
@@ -551,7 +585,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
           q[8 * q4 + 4] = bf_lo(w.z); q[8 * q4 + 5] = bf_hi(w.z);
           q[8 * q4 + 6] = bf_lo(w.w); q[8 * q4 + 7] = bf_hi(w.w);
         }
-        for (int slot = g; slot < n; slot += 4) {
+        for (int slot = g; slot < n; slot += ST_G) {
           const int c = (int)(sCand[cand_at(r, slot)] & 0xFFFFu);
           float acc = 0.f;
 #pragma unroll
@@ -572,8 +606,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     // Walking the candidates in (key descending, index ascending) order until the budget is met selects
     // candidate j iff the tokens above the window plus the sizes of the candidates before j stay below ns.
     // "Before" is a comparison of the entries with their low 16 bits flipped, so every candidate can be
-    // decided on its own: first one thread per row validates the window, then four threads per row take a
-    // quarter of the candidates each.
+    // decided on its own: first one thread per row validates the window, then eight threads per row take an
+    // eighth of the candidates each.
     if (g == 0) {
       int st = sRowI[R_STATE * 128 + r];
       const int n = sRowI[R_NCAND * 128 + r];
@@ -613,7 +647,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       const int n = sRowI[R_NCAND * 128 + r];
       const int running = sRowI[R_SIZEA * 128 + r];
       uint32_t* myUnion = sUnion + (sRowI[R_SEG * 128 + r] & (ST_MAXSEG - 1)) * 64;
-      for (int j = g; j < n; j += 4) {
+      for (int j = g; j < n; j += ST_G) {
         const uint32_t ej = sCand[cand_at(r, j)];
         const uint32_t oj = ej ^ 0xFFFFu;
         int before = running;
@@ -632,7 +666,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       }
     }
     __syncthreads();
-    {
+    if (tid < ST_MAXSEG * 64) {
       // segment bitmaps -> the (zero-initialised) bitmaps of their query clusters
       const int k = tid >> 6, w = tid & 63;
       const uint32_t bits = sUnion[tid];
@@ -703,9 +737,16 @@ extern "C" int t2t_score_select_union(const void* QU, const void* cks, const voi
     return T2T_ERR_CUDA;
   if (cudaFuncSetAttribute(select_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM) != cudaSuccess)
     return T2T_ERR_CUDA;
-  select_tc_kernel<<<dim3(cdiv(cdiv(N, 128), ST_TPC), H), ST_THREADS, ST_SMEM, st>>>(
+  // Tiles per CTA: as many as still leave every SM several CTAs, so that the last wave is short (with four always,
+  // 2 heads x 4096 rows ran on 16 SMs: 263 us).
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int tiles = cdiv(N, 128);
+  const int tpc = max(1, min(ST_MAX_TPC, H * tiles / (4 * sms)));
+  select_tc_kernel<<<dim3(cdiv(tiles, tpc), H), ST_THREADS, ST_SMEM, st>>>(
       (const __nv_bfloat16*)QU, (const __nv_bfloat16*)cks, (const int*)kcounts, (const int*)qperm,
-      (const int*)tile_sizes, ns, (int*)unip, (int*)rowcnt, N, CQ, fixq, mom, d_status);
+      (const int*)tile_sizes, ns, (int*)unip, (int*)rowcnt, N, CQ, tpc, fixq, mom, d_status);
   if (pin_tail > 0) pin_bit_kernel<<<cdiv(H * CQ, 256), 256, 0, st>>>((int*)unip, H * CQ);
   if (cudaGetLastError() != cudaSuccess) return T2T_ERR_CUDA;
   return launch_select_fix((const __nv_bfloat16*)QU, (const __nv_bfloat16*)cks, (const int*)kcounts, ns, (int*)unip,
