@@ -158,18 +158,24 @@ struct Columns {
 };
 
 // One round: the eight disjoint pairs (top, bottom) of a warp.  cx, cy: column numbers of pair lane & 7, whose angle
-// this lane works out.  The angle comes from fp32 arithmetic and one Newton step in fp64 (relative error 1e-13);
-// (c, s) is normalised in fp64 to its last bits, so every rotation is orthogonal to fp64 precision.
+// this lane works out.
+//
+// A round is a chain of dependent steps, and an fp64 step takes about sixteen times as long as an fp32 one, so what
+// steers the rotation stays in fp32 where it can: t = tan of the angle is an fp32 value t0 plus an fp32 correction (one
+// Newton step on gamma (t^2 - 1) + dx t = 0, its residual from exact fp32 products of the leading and trailing parts of
+// gamma and dx; relative error of t below 1e-13).  (c, s) is normalised in fp64 to its last bits, so every rotation is
+// orthogonal to fp64 precision.
 template <int R>
-__device__ __forceinline__ void rotate8(Columns& w, int cx, int cy, double* nrm2, double2* cs, double tiny2, float scale,
-                                        bool& again) {
+__device__ __forceinline__ void rotate8(Columns& w, int cx, int cy, double* nrm2, double2* cs, double tiny2, bool& again) {
   const int lane = threadIdx.x & 31;
+  const double alpha = nrm2[cx], beta = nrm2[cy], dx = beta - alpha;
+  const float dh = (float)dx, dl = (float)(dx - (double)dh);
   double g[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    g[i] = w.t[(i + R) & 7][0] * w.b[(i + 8 - R) & 7][0];
-#pragma unroll
-    for (int m = 1; m < 4; ++m) g[i] = fma(w.t[(i + R) & 7][m], w.b[(i + 8 - R) & 7][m], g[i]);
+    const double(&x)[4] = w.t[(i + R) & 7];
+    const double(&y)[4] = w.b[(i + 8 - R) & 7];
+    g[i] = fma(x[1], y[1], x[0] * y[0]) + fma(x[3], y[3], x[2] * y[2]);
   }
   // eight sums over the warp: lane l ends up with that of pair l & 7
   const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
@@ -181,35 +187,32 @@ __device__ __forceinline__ void rotate8(Columns& w, int cx, int cy, double* nrm2
   double gamma = (b2 ? v[1] : v[0]) + shfl_xor_d(b2 ? v[0] : v[1], 4);
   gamma += shfl_xor_d(gamma, 8);
   gamma += shfl_xor_d(gamma, 16);
-  const double alpha = nrm2[cx], beta = nrm2[cy];
-  const double g2rel = gamma * gamma, ab = alpha * beta;
-  const bool live = alpha > tiny2 && beta > tiny2 && g2rel > 1.0e-27 * ab;
+  const float gh = (float)gamma, gl = (float)(gamma - (double)gh);
+  // the smaller root (in size) of t^2 + dx / gamma t - 1 = 0
+  const float fx = fabsf(dh), fy = 2.0f * fabsf(gh);
+  const float lo = __fdividef(fminf(fx, fy), fmaxf(fx, fy)), root = sqrtf(fmaf(lo, lo, 1.0f));
+  float t0 = __fdividef(fy <= fx ? lo : 1.0f, fy <= fx ? 1.0f + root : lo + root);
+  if (dh != 0.0f && (dh < 0.0f) != (gh < 0.0f)) t0 = -t0;
+  const float q = t0 * t0, p = q - 1.0f;
+  const float pl = (q - (p + 1.0f)) + fmaf(t0, t0, -q);                     // t0^2 - 1 = p + pl
+  const float a1 = gh * p, b1f = dh * t0;
+  const float low = fmaf(gh, p, -a1) + fmaf(dh, t0, -b1f) + fmaf(gh, pl, fmaf(gl, p, dl * t0));
+  const float dt = -__fdividef((a1 + b1f) + low, fmaf(2.0f * gh, t0, dh));
+  const double t = (double)t0 + (double)dt;
+  const double y = (double)rsqrtf(fmaf(t0, t0, 1.0f)), y2 = y * y;
+  const double ty = t * y, h = fma(-fma(t, t, 1.0), y2, 1.0);               // third-order step: error (1e-7)^3
+  const double k = fma(h, 0.375, 0.5);
+  const double g2 = gamma * gamma, ab = alpha * beta;
+  const bool live = alpha > tiny2 && beta > tiny2 && g2 > 1.0e-27 * ab;
   if (!__any_sync(0xffffffffu, live)) return;
-  again = again || (live && g2rel > kJacobiDone2 * ab);
-  double c = 1.0, s = 0.0;
-  if (live) {
-    // tan of the rotation: the smaller root of t^2 + (beta - alpha) / gamma t - 1 = 0
-    const double dx = beta - alpha;
-    const float fd = (float)(dx * scale), fg = (float)(gamma * scale);
-    const float fx = fabsf(fd), fy = 2.0f * fabsf(fg);
-    const float lo = fminf(fx, fy) / fmaxf(fx, fy), root = sqrtf(fmaf(lo, lo, 1.0f));
-    float tf = fy <= fx ? lo / (1.0f + root) : 1.0f / (lo + root);
-    if (fd != 0.0f && (fd < 0.0f) != (fg < 0.0f)) tf = -tf;
-    // Newton on gamma t^2 + dx t - gamma; the slope is at least dx or gamma in size
-    const double t0 = (double)tf;
-    const double res = fma(fma(gamma, t0, dx), t0, -gamma);
-    const double t = t0 - (double)((float)(res * scale) / fmaf(2.0f * fg, tf, fd));
-    const double a = fma(t, t, 1.0);
-    const double y = (double)rsqrtf((float)a);
-    const double h = fma(-a * y, y, 1.0);                  // third-order step: error (1e-7)^3
-    c = fma(y * h, fma(h, 0.375, 0.5), y);
-    s = c * t;
-    if (lane < 8) {
+  again = again || (live && g2 > kJacobiDone2 * ab);
+  if (lane < 8) {
+    cs[lane] = live ? make_double2(fma(y * h, k, y), fma(ty * h, k, ty)) : make_double2(1.0, 0.0);
+    if (live) {
       nrm2[cx] = fmax(fma(-t, gamma, alpha), 0.0);
       nrm2[cy] = fmax(fma(t, gamma, beta), 0.0);
     }
   }
-  if (lane < 8) cs[lane] = make_double2(c, s);
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -232,10 +235,9 @@ __device__ __forceinline__ int bottom_column(int pair, int r) { return (r + (JD 
 // Round R (mod 8) and the hand-over to the next one: one column enters and one leaves each segment of a warp.  The ring
 // runs down the tops (towards pair 0) and up the bottoms: top 1 -> bottom 0, bottom 63 -> top 63.
 template <int R>
-__device__ __forceinline__ void jacobi_round(Columns& w, int& r, double* xch, double* nrm2, double2* cs, double tiny2,
-                                             float scale, bool& again) {
+__device__ __forceinline__ void jacobi_round(Columns& w, int& r, double* xch, double* nrm2, double2* cs, double tiny2, bool& again) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pair = 8 * warp + (lane & 7);
-  rotate8<R>(w, top_column(pair, r), bottom_column(pair, r), nrm2, cs, tiny2, scale, again);
+  rotate8<R>(w, top_column(pair, r), bottom_column(pair, r), nrm2, cs, tiny2, again);
   r = r + 1 < JD - 1 ? r + 1 : 0;
   constexpr int TI = R & 7, TN = (R + 1) & 7, BI = (15 - R) & 7;      // registers of top 0, of top 1, of bottom 7
   double* tops = xch + (R & 1) * 16 * JD;                             // [8 warps][128] column leaving the tops
@@ -275,20 +277,27 @@ __device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
   double2* cs = cs_all + warp * 8;
   __syncthreads();      // W was just written by other threads
   column_norms2(W, nrm2);
+  // a power of two brings the largest squared norm to 2^60 or so: the fp32 part of the angles stays in range
+  double top = 0.0;
+  for (int j = 0; j < JD; ++j) top = fmax(top, nrm2[j]);
+  const int shift = top > 0.0 ? max(-500, min(500, (60 - ilogb(top)) / 2)) : 0;
+  const double up = scalbn(1.0, shift), down = scalbn(1.0, -shift);
+  __syncthreads();      // every thread has read the norms
+  if (tid < JD) nrm2[tid] = nrm2[tid] * up * up;
+  __syncthreads();
   // columns whose squared norm is below (1e-14 of the largest column)^2 are numerically zero: rotating
   // them against each other never settles and changes nothing that is used
   double big = 0.0;
   for (int j = 0; j < JD; ++j) big = fmax(big, nrm2[j]);
   const double tiny2 = 1.0e-28 * big;
-  const float scale = big > 0.0 ? (float)fmin(1.0e18 / big, 1.0e38) : 1.0f;      // keeps the fp32 angles in range
   int r = 0;
   Columns w;
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      w.t[i][m] = W[top_column(8 * warp + i, 0) * JLD + lane + 32 * m];
-      w.b[i][m] = W[bottom_column(8 * warp + i, 0) * JLD + lane + 32 * m];
+      w.t[i][m] = W[top_column(8 * warp + i, 0) * JLD + lane + 32 * m] * up;
+      w.b[i][m] = W[bottom_column(8 * warp + i, 0) * JLD + lane + 32 * m] * up;
     }
   __syncthreads();      // W now carries the columns that change warps
 #pragma unroll 1
@@ -296,14 +305,14 @@ __device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
     bool again = false;
 #pragma unroll 1
     for (int g = 0; g < 16; ++g) {
-      jacobi_round<0>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<1>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<2>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<3>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<4>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<5>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<6>(w, r, W, nrm2, cs, tiny2, scale, again);
-      jacobi_round<7>(w, r, W, nrm2, cs, tiny2, scale, again);
+      jacobi_round<0>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<1>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<2>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<3>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<4>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<5>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<6>(w, r, W, nrm2, cs, tiny2, again);
+      jacobi_round<7>(w, r, W, nrm2, cs, tiny2, again);
     }
     if (!__syncthreads_or(again ? 1 : 0)) break;
     // the running norms pick up rounding
@@ -332,8 +341,8 @@ __device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      W[top_column(8 * warp + i, r) * JLD + lane + 32 * m] = w.t[i][m];
-      W[bottom_column(8 * warp + i, r) * JLD + lane + 32 * m] = w.b[i][m];
+      W[top_column(8 * warp + i, r) * JLD + lane + 32 * m] = w.t[i][m] * down;
+      W[bottom_column(8 * warp + i, r) * JLD + lane + 32 * m] = w.b[i][m] * down;
     }
   __syncthreads();
 }
