@@ -48,7 +48,7 @@ constexpr float ST_SPAN = 0.8f;            // half width of the first histogram 
 constexpr int ST_STRAGGLERS = 8;           // this few unsettled rows of a tile go to the exact kernel instead of another pass
 
 constexpr int OFF_CK = 0;                               // 1024 rows x 128 B: centroid c in row c % 1024, half c / 1024
-constexpr int OFF_A = OFF_CK + 1024 * 128;              // 128 rows x 128 B (first 64 B used)
+constexpr int OFF_A = OFF_CK + 1024 * 128;              // 128 rows x 128 B: this tile's rows in one 64-byte half, the next tile's arrive in the other
 constexpr int OFF_HIST = OFF_A + 128 * 128;             // [ST_B][128] packed (size << 12 | count); after P2 the
 constexpr int OFF_CAND = OFF_HIST;                      //   same bytes hold [128][ST_CAP] cluster | key << 16
 constexpr int OFF_SIZE = OFF_HIST + ST_B * 128 * 4;     // [2048] (cluster size << 12) + 1
@@ -81,7 +81,7 @@ __device__ __forceinline__ int key16_from_score(float s) { return key16_from_hal
 // same slot, hit 32 different banks (the row stride, ST_CAP words, is a multiple of the bank count).
 __device__ __forceinline__ int cand_at(int r, int slot) { return r * ST_CAP + ((slot + r) & (ST_CAP - 1)); }
 
-// Packed fp32 pairs, rounded toward -inf.
+// Packed fp32 pairs: rn to nearest, rm toward -inf.
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -89,6 +89,16 @@ __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
 }
 __device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma_rn2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add_rn2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 __device__ __forceinline__ unsigned long long fma_rm2(unsigned long long a, unsigned long long b, unsigned long long c) {
   unsigned long long r;
@@ -226,6 +236,26 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   constexpr uint32_t idesc = make_idesc_bf16(128, ST_CH, false, false);
   uint32_t ph0 = 0, ph1 = 0;        // phases of this group's two buffer barriers
   bool dead = false;
+  int half = 0;                     // which half of the row tile's lines this tile's rows are in
+
+  // Threads 0..511 fetch the rows of a tile, a 16-byte chunk each: original row of the tile's row tid / 4 (0 past the end)
+  auto row_index = [&](int first) {
+    const int p = first + (tid >> 2);
+    return p < N ? qperm[(size_t)h * N + p] : 0;
+  };
+  auto load_rows = [&](int first, int orig, int hf) {
+    const int ar = tid >> 2, ch = tid & 3;
+    const bool valid = first + ar < N;
+    cp_async16(sA + sw128(ar, hf * 4 + ch), QU + ((size_t)h * N + (valid ? orig : 0)) * kR + ch * 8, valid ? 16u : 0u);
+    cp_async_commit();
+  };
+  int orig_here = 0, orig_next = 0;
+  if (tid < 512) {
+    const int first = blockIdx.x * tpc * 128;
+    orig_here = row_index(first);
+    load_rows(first, orig_here, 0);
+    orig_next = row_index(first + 128);
+  }
 
   // Streams this group's eight chunks through its two TMEM buffers: the MMA of
   // chunk i + 1 runs while chunk i is scanned.  body(cbase, v) sees 32
@@ -235,7 +265,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     tc_fence_after();
 #pragma unroll
     for (int s2 = 0; s2 < 2; ++s2)
-      umma_ss(tmem + g * 2 * ST_CH + b * ST_CH, make_sdesc(sA + s2 * 32, 16, 1024),
+      umma_ss(tmem + g * 2 * ST_CH + b * ST_CH, make_sdesc(sA + half * 64 + s2 * 32, 16, 1024),
               make_sdesc(sCk + (cc & (ST_NCH / 2 - 1)) * (ST_CH * 128) + cc / (ST_NCH / 2) * 64 + s2 * 32, 16, 1024), idesc,
               s2 > 0 ? 1u : 0u);
     umma_commit(bars + g * 2 + b);
@@ -265,16 +295,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
 #pragma unroll 1
   for (int ti = 0; ti < tpc; ++ti) {
     const int p0 = (blockIdx.x * tpc + ti) * 128;    // first sorted row of this tile
-    if (p0 >= N || dead) break;
+    if (p0 >= N || *abort_flag) break;      // (nobody raises the flag between the barrier that ends a tile and here)
     const int rows_here = min(128, N - p0);
-    if (tid < 512) {
-      const int ar = tid >> 2, ch = tid & 3;
-      const bool valid = ar < rows_here;
-      const int orig = valid ? qperm[(size_t)h * N + p0 + ar] : 0;
-      cp_async16(sA + sw128(ar, ch), QU + ((size_t)h * N + orig) * kR + ch * 8, valid ? 16u : 0u);
-      cp_async_commit();
-      if (ch == 0) sRowI[R_ORIG * 128 + ar] = orig;
-    }
+    half = ti & 1;
+    if (tid < 512 && (tid & 3) == 0) sRowI[R_ORIG * 128 + (tid >> 2)] = orig_here;
     if (g == 0) {
       // query cluster of this sorted row: the last t with sPre[t] <= p (empty clusters are skipped)
       int lo = 0, hi = CQ;                               // invariant: sPre[lo] <= p < sPre[hi]
@@ -289,6 +313,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
+    // the next tile's rows travel under this tile's passes (their indices came a tile earlier)
+    if (tid < 512 && ti + 1 < tpc && p0 + 128 < N) {
+      load_rows(p0 + 128, orig_next, half ^ 1);
+      orig_here = orig_next;
+      orig_next = row_index(p0 + 256);
+    }
     if (g == 0) {
       // segment of the row = number of cluster changes before it
       const int clu = sRowI[R_CLU * 128 + r];
@@ -311,7 +341,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       float qn = 0.f;
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4) {
-        const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, q4));
+        const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, half * 4 + q4));
         const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -339,7 +369,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       float qv[32];
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4) {
-        const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, q4));
+        const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, half * 4 + q4));
         const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) { qv[q4 * 8 + 2 * e] = bf_lo(ws[e]); qv[q4 * 8 + 2 * e + 1] = bf_hi(ws[e]); }
@@ -347,7 +377,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       constexpr int PER = kR / ST_G;
       float qa[PER];      // elements PER g .. PER g + PER - 1 of the row
       {
-        const uint2 w = *reinterpret_cast<const uint2*>(sm + OFF_A + sw128(r, g >> 1) + (g & 1) * 8);
+        const uint2 w = *reinterpret_cast<const uint2*>(sm + OFF_A + sw128(r, half * 4 + (g >> 1)) + (g & 1) * 8);
         qa[0] = bf_lo(w.x); qa[1] = bf_hi(w.x); qa[2] = bf_lo(w.y); qa[3] = bf_hi(w.y);
       }
       static_assert(PER == 4, "eight bytes of the row per group");
@@ -519,6 +549,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       const bool act = sRowI[R_STATE * 128 + r] == RS_COLLECT;
       const float thrA = act ? sRowF[R_THRA * 128 + r] : INFINITY;
       const float thrW = act ? sRowF[R_THRW * 128 + r] : INFINITY;
+      const unsigned long long thrA2 = pack2(thrA, thrA), nthrW2 = pack2(-thrW, -thrW), minus1 = pack2(-1.0f, -1.0f);
       int sumA = 0;      // packed: (sizes << 12) + count
       const int nseg = *sNseg;
       const uint32_t* segmask = sSegMask + (warp & 3) * ST_MAXSEG;
@@ -530,15 +561,18 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
         // straight-line over the 32 scores: bit masks of the clusters above the window and of those at or
         // above its lower end; the (few) candidates are appended afterwards from the difference
         // The comparisons as sign bits of differences (a > thrA iff thrA - a < 0; a >= thrW iff not a - thrW < 0),
-        // shifted into the masks from score 31 down to score 0: a subtraction on the FMA pipe and a funnel shift
-        // per bit instead of a compare and a predicated OR on the half-rate ALU pipe.  (Rows that do not collect
+        // shifted into the masks from score 31 down to score 0: half a packed subtraction and a funnel shift per bit
+        // instead of a compare and a predicated OR on the half-rate ALU pipe.  (Rows that do not collect
         // have thrA = thrW = +inf: no bit of either mask.)
         uint32_t wbits = 0u, nbits = 0u;
 #pragma unroll
-        for (int j = 31; j >= 0; --j) {
-          const float a = __uint_as_float(v[j]);
-          wbits = __funnelshift_l(__float_as_uint(thrA - a), wbits, 1);
-          nbits = __funnelshift_l(__float_as_uint(a - thrW), nbits, 1);
+        for (int j = 30; j >= 0; j -= 2) {
+          const unsigned long long a2 = pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+          float w0, w1, n0, n1;
+          unpack2(fma_rn2(a2, minus1, thrA2), w0, w1);
+          unpack2(add_rn2(a2, nthrW2), n0, n1);
+          wbits = __funnelshift_l(__float_as_uint(w0), __funnelshift_l(__float_as_uint(w1), wbits, 1), 1);
+          nbits = __funnelshift_l(__float_as_uint(n0), __funnelshift_l(__float_as_uint(n1), nbits, 1), 1);
         }
         const uint32_t ibits = ~nbits;
         // sizes of the (few) clusters above the window
@@ -579,7 +613,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
         float q[kR];
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
-          const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, q4));
+          const uint4 w = *reinterpret_cast<const uint4*>(sm + OFF_A + sw128(r, half * 4 + q4));
           q[8 * q4 + 0] = bf_lo(w.x); q[8 * q4 + 1] = bf_hi(w.x);
           q[8 * q4 + 2] = bf_lo(w.y); q[8 * q4 + 3] = bf_hi(w.y);
           q[8 * q4 + 4] = bf_lo(w.z); q[8 * q4 + 5] = bf_hi(w.z);

@@ -1273,13 +1273,16 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       const uint2 mw2 = mw_next;
       if (i + 1 < TL_NH) mw_next = *reinterpret_cast<const uint2*>(mrow + (i + 1) * 2);
       float s[TL_H];
-#pragma unroll
-      for (int c = 0; c < TL_H / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tS_lane + b * TL_H + c * 32, v);
+      {
+        uint32_t v0[32], v1[32];
+        tmem_ld32(tS_lane + b * TL_H, v0);
+        tmem_ld32(tS_lane + b * TL_H + 32, v1);
         tmem_wait_ld();
 #pragma unroll
-        for (int k = 0; k < 32; ++k) s[c * 32 + k] = __uint_as_float(v[k]);
+        for (int k = 0; k < 32; ++k) {
+          s[k] = __uint_as_float(v0[k]);
+          s[32 + k] = __uint_as_float(v1[k]);
+        }
       }
       // The scores are rounded to fp16 exactly as the selection saw them, and the members of the row's union
       // become -inf, both on packed pairs: shifting a word of union bits left by 7 - r puts the bits of the
@@ -1328,7 +1331,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       const float nm = (m == -INFINITY) ? 0.f : -m;
       const unsigned long long l2e2 = pack_f2(LOG2E, LOG2E), nm2 = pack_f2(nm, nm);
       const float4* cnt4 = reinterpret_cast<const float4*>(sCnt + i * TL_H);
-      float ps4[4] = {0.f, 0.f, 0.f, 0.f};
+      unsigned long long ps2[2] = {0ull, 0ull};
       uint32_t pk[TL_H / 2];
 #pragma unroll
       for (int k = 0; k < TL_H / 4; ++k) {
@@ -1347,11 +1350,14 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
           p2 = ex2_approx(y2);
           p3 = ex2_approx(y3);
         }
-        ps4[k & 3] = fmaf(p1, cn.y, fmaf(p0, cn.x, ps4[k & 3]));
-        ps4[(k + 2) & 3] = fmaf(p3, cn.w, fmaf(p2, cn.z, ps4[(k + 2) & 3]));
+        ps2[0] = fma_f2(pack_f2(p0, p1), pack_f2(cn.x, cn.y), ps2[0]);
+        ps2[1] = fma_f2(pack_f2(p2, p3), pack_f2(cn.z, cn.w), ps2[1]);
         pk[2 * k] = pack_bf2(p0, p1);
         pk[2 * k + 1] = pack_bf2(p2, p3);
       }
+      float ps4[4];
+      unpack_f2(ps2[0], ps4[0], ps4[1]);
+      unpack_f2(ps2[1], ps4[2], ps4[3]);
       phi += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
       tmem_st32(tS_lane + b * TL_H, pk);
       tmem_wait_st();
