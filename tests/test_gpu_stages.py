@@ -406,8 +406,7 @@ def test_tile_attn_empty_union_is_pure_residual(lib, small_case):
 @pytest.mark.parametrize("H, N", [(1, 1), (2, 127), (3, 129), (1, 2048), (8, 9473), (2, 37889)])
 @pytest.mark.parametrize("Cn", [1, 15, 17, 129, 512, 2048, 2050])
 def test_assign_edges_of_tiles_groups_and_chunks(lib, H, N, Cn):
-    """One and two row tiles per CTA (the last two shapes), ragged rows, centroid counts around a group of 16 and a
-    chunk of 128; a third of the centroids are copies of others - in the same group, in one other group, in many -
+    """Few and many tiles, ragged rows, centroid counts around a group of 16 and a chunk of 128; a third of the centroids are copies of others - in the same group, in one other group, in many -
     and a few rows and centroids are not finite.  Labels equal the all-exact kernel's (checked by the helper)."""
     g = torch.Generator().manual_seed(N + Cn)
     cen = torch.randn(H, Cn, 32, generator=g)

@@ -33,7 +33,8 @@ constexpr int TA_CH = 128;                     // centroids per chunk
 constexpr int TA_G = 16;                       // centroids per group
 constexpr int TA_SA = TA_ROWS * 128;           // 16 KB: rows padded to 128 B
 constexpr int TA_SB = TA_CH * 128;             // 16 KB per stage
-__host__ __device__ constexpr int ta_smem(int tiles) { return tiles * TA_SA + 2 * TA_SB + 128 + 1024; }
+constexpr int TA_SMEM = TA_SA + 2 * TA_SB + 128 + 1024;
+constexpr int TA_THREADS = TA_ROWS;
 
 __device__ __forceinline__ float ta_max3(float a, float b, float c) {
   float r;
@@ -108,23 +109,24 @@ __device__ __forceinline__ void warp_argmin(float& best, int& bi) {
   }
 }
 
-// TILES row tiles of 128 rows per CTA, 128 threads and 128 TMEM columns each; they share the centroid chunks.
+// One tile of 128 rows per CTA, four CTAs to an SM (128 TMEM columns each), each a chain of chunk -> norms -> product ->
+// scan that the others fill.
 //
-// What bounds it: the tensor pipe (three 128 x 128 x 16 steps a chunk and tile, 192 cycles) and the instruction
-// issue of the scan (13 instructions per 16 values plus the updates, which get rare quickly because a CTA starts
-// at the chunk its rows' own position points to: warm-started centroids keep the order of the rows they came from).
-template <int TILES>
-__global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const __nv_bfloat16* __restrict__ X,
-                                                                           const __nv_bfloat16* __restrict__ cen,
-                                                                           int* __restrict__ labels, int N, int Cn,
-                                                                           int pin_begin, int pin_label,
-                                                                           int* __restrict__ settled,
-                                                                           int* __restrict__ status) {
-  constexpr int THREADS = 128 * TILES;
+// What bounds it: instruction issue and the chain.  The scan takes 13 instructions per 16 values plus the updates
+// (three instructions a value in all); a CTA starts at the chunk its rows' own position points to, since warm-started
+// centroids keep the order of the rows they came from, so updates get rare quickly.  The tensor pipe (three
+// 128 x 128 x 16 steps a chunk, 192 cycles) is busy a sixth of the time.  Two tiles per CTA, sharing the centroids and
+// their norms, waited longer at their barriers than they saved: 149 us for 5 x 75,600 rows and 2048 centroids against
+// 141 (512 centroids: 58.5 against 56.8).
+__global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfloat16* __restrict__ X,
+                                                                  const __nv_bfloat16* __restrict__ cen,
+                                                                  int* __restrict__ labels, int N, int Cn, int pin_begin,
+                                                                  int pin_label, int* __restrict__ settled,
+                                                                  int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
-  constexpr int OFF_B = TILES * TA_SA;
+  constexpr int OFF_B = TA_SA;
   const uint32_t sA = base, sB = base + OFF_B;
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + OFF_B + 2 * TA_SB);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
@@ -133,12 +135,12 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
   int* sCount = reinterpret_cast<int*>(bar + 4);      // [2] rows to settle exactly: over two groups, over everything
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.y, row0 = blockIdx.x * (TA_ROWS * TILES);
+  const int h = blockIdx.y, row0 = blockIdx.x * TA_ROWS;
   const __nv_bfloat16* Xh = X + (size_t)h * N * kR;
   const __nv_bfloat16* ch = cen + (size_t)h * Cn * kR;
 
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 128 * TILES);
+    tmem_alloc(tmem_slot, 128);
     tmem_relinquish();
   }
   if (tid == 0) {
@@ -152,8 +154,8 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
   const int lch = tid & 3, lr0 = tid >> 2;     // 4 chunks of 16 B per 64-byte row
   auto load_chunk = [&](int j, int st) {
 #pragma unroll
-    for (int u = 0; u < 4 / TILES; ++u) {
-      const int r = lr0 + 32 * TILES * u;
+    for (int u = 0; u < 4; ++u) {
+      const int r = lr0 + 32 * u;
       const bool valid = j * TA_CH + r < Cn;
       cp_async16(sB + st * TA_SB + sw128(r, lch), ch + (size_t)(valid ? j * TA_CH + r : 0) * kR + lch * 8, valid ? 16u : 0u);
     }
@@ -162,24 +164,23 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
   // the row tiles, with ones in elements 32..34 and zeros up to 47
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const int r = lr0 + 32 * TILES * u;        // row of the CTA
+    const int r = lr0 + 32 * u;
     const bool valid = row0 + r < N;
     cp_async16(sA + sw128(r, lch), Xh + (size_t)(valid ? row0 + r : 0) * kR + lch * 8, valid ? 16u : 0u);
   }
   *reinterpret_cast<uint4*>(sm + sw128(tid, 4)) = make_uint4(0x3F803F80u, 0x00003F80u, 0u, 0u);
   *reinterpret_cast<uint4*>(sm + sw128(tid, 5)) = make_uint4(0u, 0u, 0u, 0u);
-  for (int r = tid; r < 2 * TA_CH; r += THREADS)
+  for (int r = tid; r < 2 * TA_CH; r += TA_THREADS)
     *reinterpret_cast<uint4*>(sm + OFF_B + (r / TA_CH) * TA_SB + sw128(r % TA_CH, 5)) = make_uint4(0u, 0u, 0u, 0u);
 
   // -||c||^2 / 2 of the centroids of chunk j (stage st) as three bf16 pieces; -inf past the last centroid
   float cnmax = 0.f;
   auto augment = [&](int j, int st) {
-    const int r = tid / TILES, part = tid % TILES;
     uint8_t* stage = sm + OFF_B + st * TA_SB;
     float s = 0.f;
 #pragma unroll
-    for (int q4 = 0; q4 < 4 / TILES; ++q4) {
-      const uint4 w = *reinterpret_cast<const uint4*>(stage + sw128(r, part * (4 / TILES) + q4));
+    for (int q4 = 0; q4 < 4; ++q4) {
+      const uint4 w = *reinterpret_cast<const uint4*>(stage + sw128(tid, q4));
       const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -188,27 +189,22 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
         s = fmaf(hi, hi, s);
       }
     }
-    if (TILES == 2) s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if (part == 0) {
-      const bool real = j * TA_CH + r < Cn;
-      // a NaN norm must reach the bound (every row is then settled exactly): compare bits, as atomicMax below does
-      if (real && __float_as_int(s) > __float_as_int(cnmax)) cnmax = s;
-      const float half = -0.5f * s;
-      const uint32_t hi = real ? f_to_bf_bits(half) : 0xFF80u;
-      const float r1 = half - __uint_as_float(hi << 16);
-      const uint32_t mid = real ? f_to_bf_bits(r1) : 0u;
-      const uint32_t lo = real ? f_to_bf_bits(r1 - __uint_as_float(mid << 16)) : 0u;
-      *reinterpret_cast<uint4*>(stage + sw128(r, 4)) = make_uint4(hi | (mid << 16), lo, 0u, 0u);
-    }
+    const bool real = j * TA_CH + tid < Cn;
+    // a NaN norm must reach the bound (every row is then settled exactly): compare bits, as atomicMax below does
+    if (real && __float_as_int(s) > __float_as_int(cnmax)) cnmax = s;
+    const float half = -0.5f * s;
+    const uint32_t hi = real ? f_to_bf_bits(half) : 0xFF80u;
+    const float r1 = half - __uint_as_float(hi << 16);
+    const uint32_t mid = real ? f_to_bf_bits(r1) : 0u;
+    const uint32_t lo = real ? f_to_bf_bits(r1 - __uint_as_float(mid << 16)) : 0u;
+    *reinterpret_cast<uint4*>(stage + sw128(tid, 4)) = make_uint4(hi | (mid << 16), lo, 0u, 0u);
   };
   constexpr uint32_t idesc = make_idesc_bf16(128, TA_CH, false, false);
   auto issue = [&](int st, uint32_t tmem) {     // one thread
 #pragma unroll
-    for (int t = 0; t < TILES; ++t)
-#pragma unroll
-      for (int s2 = 0; s2 < 3; ++s2)
-        umma_ss(tmem + t * 128, make_sdesc(sA + t * TA_SA + s2 * 32, 16, 1024), make_sdesc(sB + st * TA_SB + s2 * 32, 16, 1024),
-                idesc, s2 > 0 ? 1u : 0u);
+    for (int s2 = 0; s2 < 3; ++s2)
+      umma_ss(tmem, make_sdesc(sA + s2 * 32, 16, 1024), make_sdesc(sB + st * TA_SB + s2 * 32, 16, 1024), idesc,
+              s2 > 0 ? 1u : 0u);
     umma_commit(bar);
   };
 
@@ -225,7 +221,7 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t t_lane = tmem_addr(tmem, (warp & 3) * 32, (warp >> 2) * 128);
+  const uint32_t t_lane = tmem_addr(tmem, warp * 32, 0);
   if (tid == 0) issue(0, tmem);
 
   Best b;
@@ -270,8 +266,8 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
       issue((i + 1) & 1, tmem);
     }
   }
-  int* list = reinterpret_cast<int*>(sm + OFF_B);               // [2][THREADS] rows to settle (the stages are free)
-  int2* cand = reinterpret_cast<int2*>(sm + OFF_B + TA_SB);     // [THREADS] first centroids of a row's two groups
+  int* list = reinterpret_cast<int*>(sm + OFF_B);               // [2][TA_THREADS] rows to settle (the stages are free)
+  int2* cand = reinterpret_cast<int2*>(sm + OFF_B + TA_SB);     // [TA_THREADS] first centroids of a row's two groups
   if (dead) {
     if (tid == 0 && status) atomicExch(status, ST_WAIT_TIMEOUT);
     cp_async_wait<0>();
@@ -306,7 +302,7 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
       labels[(size_t)h * N + row] = pinned ? pin_label : b.i1 + bi;
       if (!pinned && !(best - second > eps)) {             // true for NaN as well
         const int mode = b.m1 - b.m3 > eps ? 0 : 1;
-        list[mode * THREADS + atomicAdd(sCount + mode, 1)] = tid;
+        list[mode * TA_THREADS + atomicAdd(sCount + mode, 1)] = tid;
         cand[tid] = make_int2(b.i1, b.i2);
       }
     }
@@ -323,7 +319,7 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
       }
     };
     // a warp per row, a lane per centroid of its two best groups
-    for (int e = warp; e < sCount[0]; e += THREADS / 32) {
+    for (int e = warp; e < sCount[0]; e += TA_THREADS / 32) {
       const int r = list[e];
       const int2 two = cand[r];
       float x[kR];
@@ -339,15 +335,15 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
       if (lane == 0) labels[(size_t)h * N + row0 + r] = di;
     }
     // the whole CTA per row, all centroids
-    float* wd = reinterpret_cast<float*>(sm + OFF_B + TA_SB + THREADS * 8);      // [warps] distances, then indices
-    int* wi = reinterpret_cast<int*>(wd + THREADS / 32);
+    float* wd = reinterpret_cast<float*>(sm + OFF_B + TA_SB + TA_THREADS * 8);      // [warps] distances, then indices
+    int* wi = reinterpret_cast<int*>(wd + TA_THREADS / 32);
     for (int e = 0; e < sCount[1]; ++e) {
-      const int r = list[THREADS + e];
+      const int r = list[TA_THREADS + e];
       float x[kR];
       load_x(r, x);
       float d = INFINITY;
       int di = 0x7fffffff;
-      for (int c = tid; c < Cn; c += THREADS) {
+      for (int c = tid; c < Cn; c += TA_THREADS) {
         const float dc = exact_distance(x, ch + (size_t)c * kR);
         if (dc < d) { d = dc; di = c; }
       }
@@ -355,7 +351,7 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
       if (lane == 0) { wd[warp] = d; wi[warp] = di; }
       __syncthreads();
       if (tid == 0) {
-        for (int w = 1; w < THREADS / 32; ++w)
+        for (int w = 1; w < TA_THREADS / 32; ++w)
           if (wd[w] < d || (wd[w] == d && wi[w] < di)) { d = wd[w]; di = wi[w]; }
         labels[(size_t)h * N + row0 + r] = di == 0x7fffffff ? 0 : di;
       }
@@ -364,7 +360,7 @@ __global__ void __launch_bounds__(128 * TILES, 4 / TILES) assign_tc_kernel(const
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 128 * TILES);
+  if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
 size_t assign_ws_bytes(int H, int N) { return ((size_t)H * N + 1) * sizeof(int); }
@@ -372,22 +368,10 @@ size_t assign_ws_bytes(int H, int N) { return ((size_t)H * N + 1) * sizeof(int);
 int launch_assign(const __nv_bfloat16* X, const __nv_bfloat16* cen, int* labels, int H, int N, int Cn,
                   int pin_begin, int pin_label, int* settled, int* d_status, cudaStream_t st) {
   if (settled && cudaMemsetAsync(settled, 0, sizeof(int), st) != cudaSuccess) return T2T_ERR_CUDA;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Two tiles per CTA halve the work on the centroids and their norms; one tile per CTA gives a small problem
-  // twice the CTAs.
-  if ((long long)H * cdiv(N, 2 * TA_ROWS) >= 2 * sms) {
-    if (cudaFuncSetAttribute(assign_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ta_smem(2)) != cudaSuccess)
-      return T2T_ERR_CUDA;
-    assign_tc_kernel<2><<<dim3(cdiv(N, 2 * TA_ROWS), H), 256, ta_smem(2), st>>>(X, cen, labels, N, Cn, pin_begin,
-                                                                                pin_label, settled, d_status);
-  } else {
-    if (cudaFuncSetAttribute(assign_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ta_smem(1)) != cudaSuccess)
-      return T2T_ERR_CUDA;
-    assign_tc_kernel<1><<<dim3(cdiv(N, TA_ROWS), H), 128, ta_smem(1), st>>>(X, cen, labels, N, Cn, pin_begin,
-                                                                            pin_label, settled, d_status);
-  }
+  if (cudaFuncSetAttribute(assign_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TA_SMEM) != cudaSuccess)
+    return T2T_ERR_CUDA;
+  assign_tc_kernel<<<dim3(cdiv(N, TA_ROWS), H), TA_THREADS, TA_SMEM, st>>>(X, cen, labels, N, Cn, pin_begin, pin_label,
+                                                                           settled, d_status);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
 
