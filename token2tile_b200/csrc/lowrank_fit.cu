@@ -131,6 +131,8 @@ constexpr int J_THREADS = 256;
 constexpr int J_MAX_SWEEPS = 18;
 constexpr double kJacobiDone2 = 9.0e-16;   // (3e-8)^2: see jacobi_orthogonalise
 constexpr int J_SMEM = JD * JLD * 8 + 2 * JD * 8 + 8 * 8 * 16 + 4 * JD * 8 + 64;
+constexpr int F_SMEM = J_SMEM + JD * (JD + 1) / 2 * 8;      // factor_kernel: and a packed triangle
+static_assert(J_SMEM % 16 == 0 && F_SMEM <= 227 * 1024, "shared memory of factor_kernel");
 
 __device__ __forceinline__ double shfl_xor_d(double v, int m) {
   return __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(v), m),
@@ -442,6 +444,156 @@ __device__ __forceinline__ bool cholesky_inverse(double (&e)[16][4], double* Lc,
   return true;
 }
 
+// Sum of v over the CTA (every thread calls it); red: 8 doubles.
+__device__ __forceinline__ double block_sum(double v, double* red) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += shfl_xor_d(v, d);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double sum = 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sum += red[i];
+  return sum;
+}
+
+// The symmetric root of M = L L^T from its Cholesky factor: L^T = P H with P orthogonal and H = M^(1/2), and P is the
+// limit of X <- (X + X^-T) / 2 as well as of X <- X (3 I - X^T X) / 2.  The first form is fast far from the limit and
+// costs nothing for the first step, L^-1 being at hand; the second needs products only and doubles the correct digits
+// once the singular values of X are near one (it converges below sqrt(3), which the first step ensures for condition
+// numbers of M up to a thousand or so).  On entry e holds L^-1 (lower triangle), Lc column k of L at k * JLD; on
+// success H is in out (row-major) and in e.  S: 128 * 129 / 2 doubles.  Returns false when the products do not converge.
+// A singular value that starts above sqrt(3) may end at minus one and leave a symmetric H that is not positive: the
+// caller checks that it is.
+__device__ __forceinline__ bool polar_root(double (&e)[16][4], double inv_norm2, double* X, double* S, double* red,
+                                           double* out) {
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  for (int i = tid; i < JD * JD; i += J_THREADS) out[i] = X[(i & 127) * JLD + (i >> 7)];      // L, needed at the end
+  double part = 0.0;
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const double lt = X[(w + 8 * m) * JLD + l + 32 * n];      // (L^T)_ij
+      part = fma(lt, lt, part);
+    }
+  const double mu = sqrt(sqrt(inv_norm2 / block_sum(part, red)));
+  part = 0.0;
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int i = w + 8 * m, j = l + 32 * n;
+      const double x = 0.5 * (mu * X[i * JLD + j] + (j <= i ? e[m][n] / mu : 0.0));
+      e[m][n] = x;
+      part = fma(x, x, part);
+    }
+  const double scale = sqrt((double)JD / block_sum(part, red));
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) X[(w + 8 * m) * JLD + l + 32 * n] = e[m][n] * scale;
+  __syncthreads();
+  bool done = false;
+#pragma unroll 1
+  for (int step = 0; step < 9 && !done; ++step) {
+#pragma unroll
+    for (int m = 0; m < 16; ++m)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) e[m][n] = 0.0;
+#pragma unroll 2
+    for (int k = 0; k < JD; ++k) {      // X^T X
+      double xb[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) xb[n] = X[k * JLD + l + 32 * n];
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        const double xa = X[k * JLD + w + 8 * m];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) e[m][n] = fma(xa, xb[n], e[m][n]);
+      }
+    }
+    part = 0.0;
+#pragma unroll
+    for (int m = 0; m < 16; ++m)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int i = w + 8 * m, j = l + 32 * n;
+        const double d = e[m][n] - (i == j ? 1.0 : 0.0);
+        part = fma(d, d, part);
+        if (j <= i) S[i * (i + 1) / 2 + j] = e[m][n];
+        e[m][n] = 0.0;
+      }
+    const double off2 = block_sum(part, red);      // (its barriers publish S)
+    if (!(off2 < 1.0e12)) return false;            // diverged, or not a number: the same in every thread
+    done = off2 < 1.0e-14;                         // the step below squares 1e-7
+#pragma unroll 2
+    for (int k = 0; k < JD; ++k) {      // X S
+      double sb[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int j = l + 32 * n;
+        sb[n] = S[j <= k ? k * (k + 1) / 2 + j : j * (j + 1) / 2 + k];
+      }
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        const double xa = X[(w + 8 * m) * JLD + k];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) e[m][n] = fma(xa, sb[n], e[m][n]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 16; ++m)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        double& x = X[(w + 8 * m) * JLD + l + 32 * n];
+        x = fma(-0.5, e[m][n], 1.5 * x);
+      }
+    __syncthreads();
+  }
+  if (!done) return false;
+  // H = L P, symmetric up to rounding
+  for (int i = tid; i < JD * JD; i += J_THREADS) {
+    const int r = i >> 7, c = i & 127;
+    if (c <= r) S[r * (r + 1) / 2 + c] = out[i];
+  }
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) e[m][n] = 0.0;
+  __syncthreads();
+#pragma unroll 1
+  for (int k = 0; k < JD; ++k) {
+    double xb[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) xb[n] = X[k * JLD + l + 32 * n];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      const int i = w + 8 * m;
+      const double la = k <= i ? S[i * (i + 1) / 2 + k] : 0.0;
+#pragma unroll
+      for (int n = 0; n < 4; ++n) e[m][n] = fma(la, xb[n], e[m][n]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) X[(w + 8 * m) * JLD + l + 32 * n] = e[m][n];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int i = w + 8 * m, j = l + 32 * n;
+      e[m][n] = 0.5 * (X[i * JLD + j] + X[j * JLD + i]);
+      out[i * JD + j] = e[m][n];
+    }
+  __syncthreads();
+  return true;
+}
+
 // One CTA per second-moment matrix M (blockIdx.x < H: query side, else key side).
 //   roots    [2 H][128][128] fp64: F with F F^T = M (eigenvalues clamped), row-major
 //   invroots [H][128][128] fp64:   F^-T, query side only
@@ -453,7 +605,8 @@ __device__ __forceinline__ bool cholesky_inverse(double (&e)[16][4], double* Lc,
 // short steps and gives its inverse on the way; it is taken where the clamp cannot matter: where the trace of the
 // inverse (an upper bound of 1 / smallest eigenvalue) is below 1 / kEigFloor.
 // Key side: the symmetric root (another factor would turn the columns that the rotations work on, and with them the
-// signs of the result).
+// signs of the result), from the Cholesky factor where the clamp cannot matter and the products converge, else, and
+// on the query side, from the eigenvectors.
 __global__ void __launch_bounds__(J_THREADS, 1) factor_kernel(const float* __restrict__ partial, int slabs, int H,
                                                               double inv_n, double* __restrict__ roots,
                                                               double* __restrict__ invroots, int* __restrict__ bad) {
@@ -488,26 +641,36 @@ __global__ void __launch_bounds__(J_THREADS, 1) factor_kernel(const float* __res
     const int any_bad = __syncthreads_or(finite ? 0 : 1);
     if (tid == 0) bad[m] = any_bad;
     if (any_bad) return;      // the host raises; nothing below would converge on NaNs
-    if (want_inv) {
+    // key side: a second pass shows that the root is positive definite
+    bool ok = true;
+    int pass = 0;
+#pragma unroll 1
+    for (;; ++pass) {
       double trace = 0.0;
-      const bool ok = cholesky_inverse(e, W, pub, nrm2, &trace);
+      ok = cholesky_inverse(e, W, pub, nrm2, &trace);
       __syncthreads();
-      if (ok && trace < 1.0 / kEigFloor) {
-        for (int i = tid; i < JD * JD; i += J_THREADS) Fo[i] = W[(i & 127) * JLD + (i >> 7)];
-        __syncthreads();
+      if (pass == 0) ok = ok && trace < 1.0 / kEigFloor;
+      if (!ok || pass == 1 || want_inv) break;
+      ok = polar_root(e, trace, W, reinterpret_cast<double*>(jsm + J_SMEM), nrm2, Fo);
+      if (!ok) break;
+    }
+    if (ok) {
+      if (!want_inv) return;
+      for (int i = tid; i < JD * JD; i += J_THREADS) Fo[i] = W[(i & 127) * JLD + (i >> 7)];
+      __syncthreads();
 #pragma unroll
-        for (int a = 0; a < 16; ++a)
+      for (int a = 0; a < 16; ++a)
 #pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            const int i = (tid >> 5) + 8 * a, j = (tid & 31) + 32 * n;
-            W[j * JLD + i] = j <= i ? e[a][n] : 0.0;
-          }
-        __syncthreads();
-        for (int i = tid; i < JD * JD; i += J_THREADS) Io[i] = W[(i >> 7) * JLD + (i & 127)];
-        return;
-      }
+        for (int n = 0; n < 4; ++n) {
+          const int i = (tid >> 5) + 8 * a, j = (tid & 31) + 32 * n;
+          W[j * JLD + i] = j <= i ? e[a][n] : 0.0;
+        }
+      __syncthreads();
+      for (int i = tid; i < JD * JD; i += J_THREADS) Io[i] = W[(i >> 7) * JLD + (i & 127)];
+      return;
     }
   }
+  __syncthreads();
 
   for (int i = tid; i < JD * JD; i += J_THREADS) W[(i >> 7) * JLD + (i & 127)] = moment(i);
   jacobi_orthogonalise(W, nrm2, cs);
@@ -630,7 +793,7 @@ extern "C" int t2t_lowrank_fit_strided(const void* q, const void* k, long long r
   double* invroots = reinterpret_cast<double*>(w + fit_off_inv(H, N));
   const int slabs = gram_slabs(N);
   if (cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(lowrank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, J_SMEM) != cudaSuccess)
     return T2T_ERR_CUDA;
   CUtensorMap mq, mk;
@@ -638,7 +801,7 @@ extern "C" int t2t_lowrank_fit_strided(const void* q, const void* k, long long r
       !make_head_tile_map(&mk, k, (uint64_t)N, (uint64_t)H, GR_ROWS, (uint64_t)row_stride, (uint64_t)head_stride))
     return T2T_ERR_CUDA;
   gram_kernel<<<dim3(slabs, H, 2), 128, GR_SMEM, st>>>(mq, mk, partial, N, d_status);
-  factor_kernel<<<2 * H, J_THREADS, J_SMEM, st>>>(partial, slabs, H, 1.0 / (double)N, roots, invroots, d_bad);
+  factor_kernel<<<2 * H, J_THREADS, F_SMEM, st>>>(partial, slabs, H, 1.0 / (double)N, roots, invroots, d_bad);
   lowrank_kernel<<<H, J_THREADS, J_SMEM, st>>>(roots, invroots, H, d_bad, Uq, Uk);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
