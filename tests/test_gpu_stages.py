@@ -461,3 +461,51 @@ def test_tile_attn_reference_maximum_far_below_later_scores(lib, sizes):
     want = torch.softmax(s, 1) @ v[0].double()
     assert (info["attn_o"][0].double() - want).abs().max() < 2e-2
     assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-2
+
+
+@pytest.mark.parametrize("N", [31, 257, 16384, 16385])
+@pytest.mark.parametrize("Cn", [3, 2048])
+def test_centroid_update_on_both_sides_of_the_chunk_rule(lib, N, Cn):
+    """256 rows per warp up to 16,384 rows, 1024 beyond; ragged ends, labels outside [0, Cn) left out, empty clusters
+    keeping their old centroid.  The sums are exact integers: bit for bit."""
+    H = 2
+    g = torch.Generator().manual_seed(N + Cn)
+    x = torch.randn(H, N, 32, generator=g).to(BF)
+    lab = torch.randint(-1, Cn + 1, (H, N), generator=g).int()
+    old = torch.randn(H, Cn, 32, generator=g).to(BF)
+    fixed = torch.round(x.double() * 32768.0).long()
+    inside = (lab >= 0) & (lab < Cn)
+    sums, counts = torch.zeros(H, Cn + 1, 32, dtype=torch.long), torch.zeros(H, Cn + 1, dtype=torch.long)
+    idx = torch.where(inside, lab, Cn).long()
+    for h in range(H):
+        sums[h].index_add_(0, idx[h], fixed[h])
+        counts[h] = torch.bincount(idx[h], minlength=Cn + 1)
+    counts = counts[:, :Cn]
+    want = (sums[:, :Cn].float() / (32768.0 * counts.float())[..., None]).to(BF)
+    want = torch.where(counts[..., None] > 0, want, old)
+    newc = torch.empty(H, Cn, 32, dtype=BF, device=DEV)
+    got_counts = torch.empty(H, Cn, dtype=torch.int32, device=DEV)
+    ws = torch.empty(lib.t2t_centroid_update_ws_bytes(H, N, Cn), dtype=torch.uint8, device=DEV)
+    xd, ld, od = x.to(DEV), lab.to(DEV), old.to(DEV)
+    _ok(lib.t2t_centroid_update(xd.data_ptr(), ld.data_ptr(), od.data_ptr(), newc.data_ptr(), got_counts.data_ptr(), H, N,
+                                Cn, ws.data_ptr(), ws.numel(), _st()))
+    torch.cuda.synchronize()
+    assert torch.equal(got_counts.cpu().long(), counts)
+    assert torch.equal(newc.cpu(), want)
+
+
+@pytest.mark.parametrize("H, N, CQ", [(1, 2049, 1), (2, 4096, 300), (5, 31000, 97), (40, 15361, 40)])
+@pytest.mark.parametrize("share", [0.0005, 0.015, 0.3])
+def test_select_tiles_per_cta_and_ragged_tiles(lib, H, N, CQ, share):
+    """One, two and eight tiles per CTA (the last one ragged, and the last CTA short), tiles inside one query cluster
+    and tiles spanning many, tiny and large budgets: the same unions and token counts as the all-exact kernel."""
+    g = torch.Generator().manual_seed(N)
+    centres = torch.randn(H, 60, 32, generator=g)
+    pick = lambda n: centres[:, torch.randint(0, 60, (n,), generator=g)]
+    QU = (pick(N) + 0.3 * torch.randn(H, N, 32, generator=g)).to(BF)
+    cks = (0.1 * (pick(2048) + 0.3 * torch.randn(H, 2048, 32, generator=g))).to(BF)
+    counts = torch.bincount(torch.randint(0, 2048, (N,), generator=g), minlength=2048).int()[None].expand(H, -1).contiguous()
+    qlab = torch.randint(0, CQ, (H, N), generator=g)
+    qcounts = torch.stack([torch.bincount(q, minlength=CQ) for q in qlab]).int()
+    qperm = torch.sort(qlab, dim=1, stable=True).indices.int()
+    _select(lib, QU, cks, counts, qperm, qcounts, max(1, int(share * N)))

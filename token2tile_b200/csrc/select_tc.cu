@@ -6,14 +6,14 @@
 // cluster-sorted query order (a tile may span several query clusters: the rows
 // of cluster k form "segment" k of the tile and selections are OR-ed into the
 // segment's bitmap, flushed to the cluster's bitmap at the end).  A tcgen05 MMA
-// (128 x 128 x 32 per chunk of centroids, all 2048 centroids resident in shared
+// (128 x 32 x 32 per chunk of centroids, all 2048 centroids resident in shared
 // memory) gives approximate scores s~ in TMEM, and each row is settled in three
 // steps, two of them streaming passes over the scores:
 //
 //   P1  row mean and deviation from the head's centroid moments (q . mean centroid,
 //       q^T (mean c c^T) q): no pass; the scores lie in [-||q|| max ||c||, ||q|| max ||c||];
-//   P2  size-weighted histogram of s~ over [mean, max] (refined if the threshold
-//       bucket is crowded) -> the bucket [x_lo, x_hi] in which the running token
+//   P2  size-weighted histogram of s~ around the threshold of a bell-shaped distribution
+//       (continued above or below, refined if the threshold bucket is crowded) -> the bucket [x_lo, x_hi] in which the running token
 //       count first reaches ns;
 //   P3  clusters with s~ > x_hi + 2 e' are selected outright (their sizes are
 //       summed exactly), clusters with s~ in [x_lo - 2 e', x_hi + 2 e'] become
@@ -26,6 +26,10 @@
 // cluster below it strictly below, so the result equals the all-exact rule bit
 // for bit.  Rows that do not fit the fast path (more than 64 candidates, no
 // convergence, non-finite scores) are queued for the exact warp-per-row kernel.
+//
+// What bounds it: instruction issue, 21 instructions a score over the two passes, 60 % of the slots used, a third of
+// the warps' time at barriers.  6.15 ms for 40 heads x 75,600 rows (7.7 with 16 warps), 58 us for 2 x 4096 (263 with
+// four tiles to every CTA).
 #include "common.cuh"
 #include "internal.h"
 

@@ -225,7 +225,7 @@ struct RowState {
   float l;      // running denominator
 };
 
-constexpr float kLazy = 8.0f;   // rescale O only when the row maximum grows by more than 2^8
+constexpr float kLazy = 8.0f;   // residual kernel: rescale T only when the row maximum grows by more than 2^8
 
 // Rescale the fp32 accumulator rows in TMEM by `alpha` (per thread = per row).
 __device__ __forceinline__ void rescale_rows(uint32_t tO_lane, float alpha) {

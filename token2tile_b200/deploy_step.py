@@ -22,6 +22,7 @@ CPU path: the module refuses to load without the compiled library.
 from __future__ import annotations
 
 import math
+from concurrent.futures import ThreadPoolExecutor
 
 import torch
 
@@ -370,10 +371,15 @@ class MaskedStepDeploy:
         request; the centroids warm-start every rebuild.  Ends with a host
         synchronisation, like the reference."""
         self._check_qkv(q, k)
-        Uq, Uk = online_u(q, k, self.r)
-        gen = torch.Generator(device="cpu").manual_seed(seed)
-        rows_k = torch.randperm(self.N, generator=gen)[: self.C].sort().values.to(self.dev)
-        rows_q = torch.randperm(self.N, generator=gen)[: self.CQ].sort().values.to(self.dev)
+        def draw():
+            gen = torch.Generator(device="cpu").manual_seed(seed)
+            return [torch.randperm(self.N, generator=gen)[:n].sort().values for n in (self.C, self.CQ)]
+
+        # the draws (1.3 ms at 75,600 rows) run while online_u waits for the fit
+        with ThreadPoolExecutor(max_workers=1) as pool:
+            rows = pool.submit(draw)
+            Uq, Uk = online_u(q, k, self.r)
+            rows_k, rows_q = (r.to(self.dev) for r in rows.result())
         state = self.warm_start(q, k, Uq, Uk, rows_k, rows_q, warm_iters)
         torch.cuda.synchronize(self.dev)
         return state
