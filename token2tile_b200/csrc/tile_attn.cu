@@ -437,8 +437,11 @@ __device__ __forceinline__ void exp2_fma2(float y0, float y1, float& p0, float& 
 // gets short.  That saves every later tile the pass that looks for the maximum (half the tensor-memory loads and a
 // seventh of the instructions).
 //   tile start     l above 2^24 (more than N keys of weight one): m grows by l's exponent e, O and l shrink by 2^-e
-//   first half     a weight sum above 2^24: m becomes the half's maximum, O and l are rescaled, P is computed again
-//                  (the product of the tile before has finished, nothing of this tile has been handed over)
+//   first half     a weight sum above 2^9: m becomes the half's maximum, O and l are rescaled, P is computed again
+//                  (the product of the tile before has finished, nothing of this tile has been handed over).  Range
+//                  would allow 2^24; the weight of a row's maximum is exact in bfloat16 when m is that maximum, and
+//                  that shows where a few keys dominate: 2.3261e-3 against a float64 softmax at 720p (2.3435e-3 with
+//                  2^24, 2.3232e-3 with a maximum per tile), for 1 % of the time.
 //   second half    a weight sum above 2^60: the first half may be in its product already, so O cannot be rescaled,
 //                  and need not be: all earlier weights add up to less than 2^26, 2^-30 of this half's and less than
 //                  an fp32 rounding.  m moves so that the half's maximum weighs 2^56.
@@ -447,7 +450,7 @@ __device__ __forceinline__ void exp2_fma2(float y0, float y1, float& p0, float& 
 // the instructions (every third pair of a full tile that way: attention 10.95 ms at 720p x 40 heads, none: 10.64;
 // 12.0 with the maximum pass.  Fetching the next 32 scores while 32 are weighed: 10.92).
 // MASK: columns >= valid lie past the union and count as -inf.
-constexpr float kSumFirst = 16777216.0f, kSumSecond = 1.152921504606847e18f;      // 2^24, 2^60
+constexpr float kSumFirst = 16777216.0f, kSumGrown = 512.0f, kSumSecond = 1.152921504606847e18f;      // 2^24, 2^9, 2^60
 template <bool MASK>
 __device__ __forceinline__ void load_scores(uint32_t tS_lane, int half, int valid, uint32_t (&v)[2][32]) {
   tmem_ld32(tS_lane + half * 64, v[0]);
@@ -518,7 +521,7 @@ __device__ __forceinline__ void softmax_tile(uint32_t tS_lane, uint32_t tO_lane,
     if (half == 1) load_scores<MASK>(tS_lane, 1, valid, v);
     uint32_t pk[32];
     float sum = weigh(v, rs.m, sc, pk);
-    const bool high = sum > (half == 0 ? kSumFirst : kSumSecond);
+    const bool high = sum > (half == 0 ? kSumGrown : kSumSecond);
     if (__any_sync(0xffffffffu, high)) {
       load_scores<MASK>(tS_lane, half, valid, v);
       const float mx = row_max(v) * sc;
