@@ -48,9 +48,9 @@ int t2t_project(const void* x, const void* U, void* out, int H, int N, int* d_st
 
 /* Projection fit: fp32 Uq, Uk [H,128,32] minimising ||Q K^T - (Q Uq)(K Uk)^T||_F
  * for q, k bf16 [H,N,128].  Second moments on the tensor cores (fp32 slabs of
- * 8192 rows, summed in fp64 in slab order), symmetric roots and singular
- * triplets by an fp64 Jacobi kernel (one CTA per matrix, eigenvalues clamped
- * at 1e-8), all batched over heads on `stream` without a host round trip.
+ * 8192 rows, summed in fp64 in slab order), their factors (eigenvalues clamped
+ * at 1e-8) and singular triplets by fp64 kernels, one CTA per matrix, all
+ * batched over heads on `stream` without a host round trip.
  * d_bad: int [2 H], set to 1 for a head whose q (first H) or k (last H) holds a
  * non-finite value; that head's Uq, Uk are left untouched.  ws:
  * t2t_lowrank_fit_ws_bytes(H, N).  Replaces online_u, deploy_step.py:122-149

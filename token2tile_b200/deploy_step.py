@@ -48,8 +48,8 @@ def lowrank_fit(q, k, r=32, *, check_finite=True):
 
     The second moments Mq = Q^T Q / N, Mk = K^T K / N come from the tensor cores
     (bfloat16 inputs, fp32 slabs summed in fp64 in a fixed order); their
-    symmetric roots and the singular triplets of Mq^(1/2) Mk^(1/2) come from an
-    fp64 Jacobi kernel, one CTA per matrix, batched over heads.  Inputs of
+    factors and the singular triplets of Mq^(1/2) Mk^(1/2) come from fp64
+    kernels, one CTA per matrix, batched over heads.  Inputs of
     another dtype are rounded to bfloat16 first: the operator's own tensors are
     bfloat16, so nothing is lost on its path.
 
