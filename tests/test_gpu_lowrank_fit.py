@@ -105,11 +105,13 @@ def test_fit_rejects_non_finite_inputs():
 
 
 @pytest.mark.parametrize("N", [2048, 2177, 8192 + 1])
-@pytest.mark.parametrize("spread_q, spread_k", [(1.0, 1.0), (3e-3, 1.0), (1e-6, 3e-3), (1.0, 1e-6)])
+@pytest.mark.parametrize("spread_q, spread_k", [(1.0, 1.0), (3e-3, 1.0), (1e-6, 3e-3), (1.0, 1e-6), (1.0, 0.3), (0.3, 0.03)])
 def test_fit_on_both_factor_routes(N, spread_q, spread_k):
-    """Cholesky factor and clamped symmetric root, in every combination of the two sides: smallest second moments of
-    0.3 and 4e-6 (Cholesky: the trace of the inverse is 3e6) and of 5e-13 (below the clamp).  Several and ragged slabs.  The oracle works in float64 on the same bfloat16 values; the kernels' second moments are fp32 sums per
-    slab (2^-24 per addition, 2^-17 for a slab of thousands of rows at worst), and the fit divides by the gap between
+    """Cholesky factor, root by products and clamped root by eigenvectors, with condition numbers of the key side
+    from 2 to 1e12 (the products give up in between) and both sides on either side of the clamp: smallest moments of
+    0.3 and 4e-6 (Cholesky: the trace of the inverse is 3e6) and of 5e-13 (below the clamp).  Several and ragged slabs.
+    The oracle works in float64 on the same bfloat16 values; the kernels' second moments are fp32 sums per slab
+    (2^-24 per addition, 2^-17 for a slab of thousands of rows at worst), and the fit divides by the gap between
     the singular values 32 and 33 (a quarter and more here): 1e-3 of the largest logit, as above."""
     from token2tile_b200.deploy_step import online_u
     g = torch.Generator().manual_seed(N)
