@@ -98,6 +98,35 @@ def test_cfg_reuse_with_refresh_one_rebuilds_every_branch_zero_call():
     assert got == ["rebuild", "reuse", "rebuild", "reuse"]
 
 
+def test_init_state_draws_on_the_calling_thread_while_the_fit_runs(monkeypatch):
+    """The seeded draws come between the launch of the fit and the read of its flags, and on the caller's thread: a
+    fresh thread would set up (and tear down) torch's worker team in every call that draws from more than 32,768 rows."""
+    import threading
+    from token2tile_b200 import deploy_step as ds
+    op = _bare_operator(mask_refresh=1)
+    op.N, op.C, op.CQ, op.r, op.dev = 40000, 2048, 100, 32, torch.device("cpu")
+    seen, randperm = [], torch.randperm
+
+    def record(name, result=None):
+        seen.append((name, threading.get_ident()))
+        return result
+
+    fit = (torch.zeros(1, 128, 32), torch.zeros(1, 128, 32))
+    monkeypatch.setattr(ds, "online_u", lambda q, k, r=32: record("fit", fit))
+    monkeypatch.setattr(ds, "_queue_fit", lambda q, k, r: record("fit", fit + ("flags",)), raising=False)
+    monkeypatch.setattr(ds, "_check_fit", lambda flags, q: record("check"), raising=False)
+    monkeypatch.setattr(torch, "randperm", lambda *a, **kw: record("draw", randperm(*a, **kw)))
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    op._check_qkv = lambda *t: None
+    op.warm_start = lambda q, k, Uq, Uk, rows_k, rows_q, warm_iters: dict(rows_k=rows_k, rows_q=rows_q)
+    got = op.init_state(None, None, seed=5)
+    assert [n for n, _ in seen] == ["fit", "draw", "draw", "check"]
+    assert {t for _, t in seen} == {threading.get_ident()}
+    gen = torch.Generator().manual_seed(5)
+    assert torch.equal(got["rows_k"], randperm(40000, generator=gen)[:2048].sort().values)
+    assert torch.equal(got["rows_q"], randperm(40000, generator=gen)[:100].sort().values)
+
+
 def test_head_ranges_tile_the_heads():
     for H, world in ((40, 1), (40, 2), (40, 4), (40, 8), (12, 5)):
         spans = [parallel.head_range(r, world, H) for r in range(world)]

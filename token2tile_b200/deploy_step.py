@@ -22,7 +22,6 @@ CPU path: the module refuses to load without the compiled library.
 from __future__ import annotations
 
 import math
-from concurrent.futures import ThreadPoolExecutor
 
 import torch
 
@@ -57,6 +56,14 @@ def lowrank_fit(q, k, r=32, *, check_finite=True):
     raises RuntimeError for non-finite inputs, like the reference
     (deploy_step.py:127-132); check_finite=False returns without synchronising
     and leaves the projections of such a head at zero."""
+    Uq, Uk, flags = _queue_fit(q, k, r)
+    if check_finite:
+        _check_fit(flags, q)
+    return Uq, Uk
+
+
+def _queue_fit(q, k, r):
+    """Queues the fit of lowrank_fit; returns Uq, Uk and the flags on the device (2 H non-finite flags, a wait status)."""
     if r != 32:
         raise ValueError("the kernels require r=32")
     if q.dim() != 3 or q.shape[2] != 128 or k.shape != q.shape or not q.is_cuda or k.device != q.device:
@@ -82,15 +89,19 @@ def lowrank_fit(q, k, r=32, *, check_finite=True):
         check(lib.t2t_lowrank_fit_strided(ptr(qb), ptr(kb), lay[0], lay[1], ptr(Uq), ptr(Uk), H, N, ptr(ws), ws.numel(),
                                           ptr(flags), ptr(flags) + 8 * H,
                                           _stream_ptr(torch.cuda.current_stream(dev))), "t2t_lowrank_fit")
-    if check_finite:
-        f = flags.cpu()
-        if int(f[2 * H]) != 0:
-            raise RuntimeError("lowrank_fit: a bounded device wait timed out")
-        for name, part in (("q", f[:H]), ("k", f[H:2 * H])):
-            if bool(part.any()):
-                raise RuntimeError(f"online_u: non-finite {name} input in heads {part.nonzero()[:, 0].tolist()}, "
-                                   f"shape {tuple(q.shape)}")
-    return Uq, Uk
+    return Uq, Uk, flags
+
+
+def _check_fit(flags, q):
+    """Reads the flags of _queue_fit back (a host synchronisation) and raises for what they report."""
+    f = flags.cpu()
+    H = q.shape[0]
+    if int(f[2 * H]) != 0:
+        raise RuntimeError("lowrank_fit: a bounded device wait timed out")
+    for name, part in (("q", f[:H]), ("k", f[H:2 * H])):
+        if bool(part.any()):
+            raise RuntimeError(f"online_u: non-finite {name} input in heads {part.nonzero()[:, 0].tolist()}, "
+                               f"shape {tuple(q.shape)}")
 
 
 def online_u(qf, kf, r=32):
@@ -371,15 +382,13 @@ class MaskedStepDeploy:
         request; the centroids warm-start every rebuild.  Ends with a host
         synchronisation, like the reference."""
         self._check_qkv(q, k)
-        def draw():
-            gen = torch.Generator(device="cpu").manual_seed(seed)
-            return [torch.randperm(self.N, generator=gen)[:n].sort().values for n in (self.C, self.CQ)]
-
-        # the draws (1.3 ms at 75,600 rows) run while online_u waits for the fit
-        with ThreadPoolExecutor(max_workers=1) as pool:
-            rows = pool.submit(draw)
-            Uq, Uk = online_u(q, k, self.r)
-            rows_k, rows_q = (r.to(self.dev) for r in rows.result())
+        Uq, Uk, flags = _queue_fit(q, k, self.r)
+        # The draws run while the fit does.  On this thread: torch.randperm fills ranges above 32,768 with a team of
+        # threads, which a thread of their own would start and tear down on every call.
+        gen = torch.Generator(device="cpu").manual_seed(seed)
+        rows = [torch.randperm(self.N, generator=gen)[:n].sort().values for n in (self.C, self.CQ)]
+        _check_fit(flags, q)
+        rows_k, rows_q = (r.to(self.dev) for r in rows)
         state = self.warm_start(q, k, Uq, Uk, rows_k, rows_q, warm_iters)
         torch.cuda.synchronize(self.dev)
         return state
