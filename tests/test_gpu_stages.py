@@ -427,40 +427,66 @@ def test_assign_edges_of_tiles_groups_and_chunks(lib, H, N, Cn):
     _assign(lib, x.to(BF).to(DEV), finite.to(BF).to(DEV))
 
 
+def _plain_structure(sizes, v):
+    """One head, clusters of consecutive rows, every query cluster executes every key: (km, full union, zero QU)."""
+    N, CQ = v.shape[1], len(sizes)
+    ids = torch.arange(N, dtype=torch.int32)[None]
+    km = dict(qcounts=torch.tensor([sizes], dtype=torch.int32), kcounts=torch.full((1, 2048), 2, dtype=torch.int32),
+              qperm=ids, kperm=ids, qlab=torch.repeat_interleave(torch.arange(CQ), torch.tensor(sizes)).int()[None],
+              V_sorted=v, sumv=torch.zeros(1, 2048, 128, dtype=BF), lam=torch.ones(1))
+    return km, torch.full((1, CQ, 64), -1, dtype=torch.int32), torch.zeros(1, N, 32, dtype=BF)
+
+
 @pytest.mark.parametrize("sizes", [(256, 129, 128, 127, 1, 3455 - 256 * 11), (4096,)])
 def test_tile_attn_reference_maximum_far_below_later_scores(lib, sizes):
-    """The softmax keeps its first tile's maximum as reference and corrects when the weights grow: a slow climb
-    (8 bits a tile: the running sum passes 2^24), jumps inside the first half of a tile (20, 40, 150 bits) and inside
-    the second (70 bits: above 2^60; 140 bits: past the largest float), a fall, and rows that see none of it or all of
-    it upside down.  Against a float64 softmax of the same bfloat16 values; the weights are rounded to bfloat16
-    (2^-9 of values around 1, averaged) and so is the output."""
-    N, H = 4096, 1
+    """The reference of a row follows its maximum: scores that rise inside the first half of a tile (20, 40, 30 bits, the
+    last one right behind a rise in the second half of the tile before), inside the second (70 and 140 bits: past the
+    largest float), that fall by 200 bits and rise by 350, and that climb by 8 bits a tile, the step below which the
+    reference stays; by the sign and size of q[0], rows of one warp see all of it, half, none, or all of it upside down.
+    Against a float64 softmax of the same bfloat16 values; the weights are rounded to bfloat16 (2^-9 of values around 1,
+    averaged) and so is the output."""
+    N = 4096
     sizes = list(sizes) + [256] * 11 if len(sizes) > 1 else list(sizes)
     assert sum(sizes) == N
     g = torch.Generator().manual_seed(N + len(sizes))
     level = torch.zeros(N)
-    for tile, pos, jump in ((2, 10, 20.0), (4, 3, 40.0), (6, 70, 70.0), (9, 100, 140.0), (12, 0, -200.0), (14, 20, 150.0)):
+    for tile, pos, jump in ((2, 10, 20.0), (4, 3, 40.0), (6, 70, 70.0), (7, 20, 30.0), (9, 100, 140.0), (12, 0, -200.0),
+                            (14, 20, 350.0)):
         level[tile * 128 + pos:] += jump
     level[16 * 128:] += 8.0 * (torch.arange(16 * 128) // 128)
     level += 2.0 * torch.randn(N, generator=g)
-    k = 0.1 * torch.randn(H, N, 128, generator=g)
+    k = 0.1 * torch.randn(1, N, 128, generator=g)
     k[0, :, 0] = level * math.sqrt(128.0) / math.log2(math.e) / 16.0
-    q = 0.1 * torch.randn(H, N, 128, generator=g)
+    q = 0.1 * torch.randn(1, N, 128, generator=g)
     q[0, :, 0] = 16.0 * torch.tensor([1.0, 0.5, 0.0, -1.0])[torch.randint(0, 4, (N,), generator=g)]
-    v = torch.randn(H, N, 128, generator=g)
+    v = torch.randn(1, N, 128, generator=g)
     q, k, v = q.to(BF), k.to(BF), v.to(BF)
-    CQ = len(sizes)
-    ids = torch.arange(N, dtype=torch.int32)[None]
-    km = dict(qcounts=torch.tensor([sizes], dtype=torch.int32), kcounts=torch.full((H, 2048), 2, dtype=torch.int32),
-              qperm=ids, kperm=ids, qlab=torch.repeat_interleave(torch.arange(CQ), torch.tensor(sizes)).int()[None],
-              V_sorted=v, sumv=torch.zeros(H, 2048, 128, dtype=BF), lam=torch.ones(H))
-    full = torch.full((H, CQ, 64), -1, dtype=torch.int32)
-    zeros = torch.zeros(H, N, 32, dtype=BF)
+    km, full, zeros = _plain_structure(sizes, v)
     _, info = _tile_attn(lib, q, k, v, zeros, km, zeros[:, :2048].contiguous(), full)
     s = q[0].double() @ k[0].double().T / math.sqrt(128.0)
     want = torch.softmax(s, 1) @ v[0].double()
     assert (info["attn_o"][0].double() - want).abs().max() < 2e-2
     assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-2
+
+
+@pytest.mark.parametrize("sizes", [(4096,), (128,) * 32])
+@pytest.mark.parametrize("tile, pos", [(0, 3), (5, 20), (5, 100), (31, 127)])
+def test_tile_attn_weight_of_a_dominant_key_is_one(lib, sizes, tile, pos):
+    """One key 45 to 56 bits above all others, in the first or second half of an early or late tile, and values of 1e30:
+    its weight is exactly one in bfloat16, so the output is its value bit for bit (the other 4,095 weigh 2^-33 together)
+    and nothing between them leaves the range of fp32."""
+    N = 4096
+    g = torch.Generator().manual_seed(tile)
+    q, k = torch.zeros(1, N, 128), torch.zeros(1, N, 128)
+    q[0, :, 0] = 16.0 + (torch.arange(N) % 32) / 8.0
+    k[0, tile * 128 + pos, 0] = 22.0
+    v = (1.0 + torch.rand(1, N, 128, generator=g)) * torch.where(torch.rand(1, N, 128, generator=g) < 0.5, -1e30, 1e30)
+    q, k, v = q.to(BF), k.to(BF), v.to(BF)
+    km, full, zeros = _plain_structure(list(sizes), v)
+    _, info = _tile_attn(lib, q, k, v, zeros, km, zeros[:, :2048].contiguous(), full)
+    assert torch.equal(info["attn_o"][0], v[0, tile * 128 + pos].expand(N, 128))
+    s = q[0].double() @ k[0].double().T / math.sqrt(128.0)
+    assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-4
 
 
 @pytest.mark.parametrize("N", [31, 257, 16384, 16385])

@@ -225,7 +225,7 @@ struct RowState {
   float l;      // running denominator
 };
 
-constexpr float kLazy = 8.0f;   // residual kernel: rescale T only when the row maximum grows by more than 2^8
+constexpr float kLazy = 8.0f;   // rescale O only when the row maximum grows by more than 2^8
 
 // Rescale the fp32 accumulator rows in TMEM by `alpha` (per thread = per row).
 __device__ __forceinline__ void rescale_rows(uint32_t tO_lane, float alpha) {
@@ -408,7 +408,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-// 2^y for two values y < 127 without the special-function unit: round y to the nearest integer n (the
+// 2^y for two values y <= 8 without the special-function unit: round y to the nearest integer n (the
 // magic-number add leaves n in the low mantissa bits), a cubic for 2^(y - n) on [-0.5, 0.5] (relative error
 // 7.5e-5, well inside a bf16 rounding step), and n added to the exponent field.  Inputs below -125 count as
 // -125 (2^-125 ~ 0).
@@ -427,119 +427,90 @@ __device__ __forceinline__ void exp2_fma2(float y0, float y1, float& p0, float& 
   p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
 }
 
-// Softmax of one 128-column S row held in tensor memory: P = 2^(s * scale - m) packed to bf16 over the columns S
-// occupied, in two halves of 64 columns (half c of S, columns 64 c .., becomes columns 32 c .. of P: always columns
-// that were read before).  `halfway` is called by the whole warp once the first half of P is written, so that the MMA
-// lane can start on it while the rows work on the rest.
-//
-// The reference m is the maximum of the row's first tile and then stays: P, its sum l and O are floating-point
-// numbers, so a reference below the row's later maxima costs no precision, only range, and the sums tell when range
-// gets short.  That saves every later tile the pass that looks for the maximum (half the tensor-memory loads and a
-// seventh of the instructions).
-//   tile start     l above 2^24 (more than N keys of weight one): m grows by l's exponent e, O and l shrink by 2^-e
-//   first half     a weight sum above 2^9: m becomes the half's maximum, O and l are rescaled, P is computed again
-//                  (the product of the tile before has finished, nothing of this tile has been handed over).  Range
-//                  would allow 2^24; the weight of a row's maximum is exact in bfloat16 when m is that maximum, and
-//                  that shows where a few keys dominate: 2.3261e-3 against a float64 softmax at 720p (2.3435e-3 with
-//                  2^24, 2.3232e-3 with a maximum per tile), for 1 % of the time.
-//   second half    a weight sum above 2^60: the first half may be in its product already, so O cannot be rescaled,
-//                  and need not be: all earlier weights add up to less than 2^26, 2^-30 of this half's and less than
-//                  an fp32 rounding.  m moves so that the half's maximum weighs 2^56.
-// All exponentials go to the special-function unit: without the maximum pass the rows are bound by issue slots and the
-// chain of hand-offs (44 % of the slots and a third of each pipe busy), and a polynomial on the FMA pipe costs six times
-// the instructions (every third pair of a full tile that way: attention 10.95 ms at 720p x 40 heads, none: 10.64;
-// 12.0 with the maximum pass.  Fetching the next 32 scores while 32 are weighed: 10.92).
-// MASK: columns >= valid lie past the union and count as -inf.
-constexpr float kSumFirst = 16777216.0f, kSumGrown = 512.0f, kSumSecond = 1.152921504606847e18f;      // 2^24, 2^9, 2^60
-template <bool MASK>
-__device__ __forceinline__ void load_scores(uint32_t tS_lane, int half, int valid, uint32_t (&v)[2][32]) {
-  tmem_ld32(tS_lane + half * 64, v[0]);
-  tmem_ld32(tS_lane + half * 64 + 32, v[1]);
-  tmem_wait_ld();
-  if (MASK) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (half * 64 + c * 32 + j >= valid) v[c][j] = 0xff800000u;      // -inf
-  }
-}
-__device__ __forceinline__ float row_max(const uint32_t (&v)[2][32]) {
-  float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-  for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-      mx4[0] = max3(mx4[0], __uint_as_float(v[c][j]), __uint_as_float(v[c][j + 1]));
-      mx4[1] = max3(mx4[1], __uint_as_float(v[c][j + 2]), __uint_as_float(v[c][j + 3]));
-      mx4[2] = max3(mx4[2], __uint_as_float(v[c][j + 4]), __uint_as_float(v[c][j + 5]));
-      mx4[3] = max3(mx4[3], __uint_as_float(v[c][j + 6]), __uint_as_float(v[c][j + 7]));
-    }
-  return fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-}
-// 64 scores -> 64 weights packed into pk; returns their sum.
-__device__ __forceinline__ float weigh(const uint32_t (&v)[2][32], float m, float sc, uint32_t (&pk)[32]) {
-  const unsigned long long sc2 = pack_f2(sc, sc), nm2 = pack_f2(-m, -m);
-  unsigned long long ls2[2] = {0ull, 0ull};
-#pragma unroll
-  for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      float y0, y1;
-      unpack_f2(fma_f2(pack_f2(__uint_as_float(v[c][2 * j]), __uint_as_float(v[c][2 * j + 1])), sc2, nm2), y0, y1);
-      const float p0 = ex2_approx(y0), p1 = ex2_approx(y1);
-      ls2[j & 1] = add_f2(ls2[j & 1], pack_f2(p0, p1));
-      pk[c * 16 + j] = pack_bf2(p0, p1);
-    }
-  float s0, s1, s2, s3;
-  unpack_f2(ls2[0], s0, s1);
-  unpack_f2(ls2[1], s2, s3);
-  return (s0 + s1) + (s2 + s3);
-}
+// Softmax of one 128-column S row held in tensor memory, in two passes of 32-column chunks so that few
+// registers are live: the row maximum first, then P = 2^(s * scale - m) packed to bf16 over the columns S
+// occupied (chunk c of S, columns 32 c .., becomes columns 16 c .. of P: always columns that were read
+// before).  Two row groups that compute at the same time are bound by the special-function unit (16
+// exponentials per cycle and SM), so every third pair of a full tile takes the FMA-pipe route instead.
+// MASK: columns >= valid lie past the union and count as -inf (all of them through the special-function
+// unit, whose result for -inf is an exact zero).
+// The maximum comes before any weight of the tile: weights stay below 2^kLazy, so O and l keep the range of the values
+// whatever the scores, and a key that dominates its row from beyond that weighs exactly one.  (One pass with the first
+// tile's maximum as reference and corrections by the sums: 10.7 instead of 12.0 ms at 720p x 40 heads, but the largest
+// weight is rounded like any other, 2.326e-3 instead of 2.323e-3 against a float64 softmax, and sums reach 2^60.  One
+// pass that keeps this rule, weighing first and starting over where a weight exceeds 2^kLazy, gains nothing: the first
+// half of P then waits for the second.)
+constexpr int kFmaPairEvery = 3;
+// `halfway` is called by the whole warp once the first 64 columns of P are written, so that the MMA lane can
+// start on them while the rows work on the rest.
 template <bool MASK, typename Halfway>
 __device__ __forceinline__ void softmax_tile(uint32_t tS_lane, uint32_t tO_lane, RowState& rs, int valid, bool first,
                                              float sc, Halfway&& halfway) {
-  uint32_t v[2][32];
+  float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t v[32];
+    tmem_ld32(tS_lane + c * 32, v);
+    tmem_wait_ld();
+    if (MASK) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (c * 32 + j >= valid) v[j] = 0xff800000u;      // -inf
+    }
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      mx4[0] = max3(mx4[0], __uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+      mx4[1] = max3(mx4[1], __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+      mx4[2] = max3(mx4[2], __uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
+      mx4[3] = max3(mx4[3], __uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
+    }
+  }
+  const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc;
   if (first) {
-    load_scores<MASK>(tS_lane, 1, valid, v);
-    const float upper = row_max(v);
-    load_scores<MASK>(tS_lane, 0, valid, v);
-    rs.m = fmaxf(upper, row_max(v)) * sc;
+    rs.m = mx;
   } else {
-    const bool high = rs.l > kSumFirst;
-    if (__any_sync(0xffffffffu, high)) {
-      const int e = high ? min((__float_as_int(rs.l) >> 23) - 127, 126) : 0;
-      const float alpha = __int_as_float((127 - e) << 23);
+    const bool grow = mx > rs.m + kLazy;
+    if (__any_sync(0xffffffffu, grow)) {
+      const float mnew = grow ? mx : rs.m;
+      const float alpha = ex2_approx(rs.m - mnew);
       rescale_rows(tO_lane, alpha);
       rs.l *= alpha;
-      rs.m += (float)e;
+      rs.m = mnew;
     }
-    load_scores<MASK>(tS_lane, 0, valid, v);
   }
+  const unsigned long long sc2 = pack_f2(sc, sc), nm2 = pack_f2(-rs.m, -rs.m);
+  unsigned long long ls2[2] = {0ull, 0ull};
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    if (half == 1) load_scores<MASK>(tS_lane, 1, valid, v);
-    uint32_t pk[32];
-    float sum = weigh(v, rs.m, sc, pk);
-    const bool high = sum > (half == 0 ? kSumGrown : kSumSecond);
-    if (__any_sync(0xffffffffu, high)) {
-      load_scores<MASK>(tS_lane, half, valid, v);
-      const float mx = row_max(v) * sc;
-      if (half == 0) {
-        const float mnew = high ? mx : rs.m;
-        const float alpha = ex2_approx(rs.m - mnew);
-        if (!first) rescale_rows(tO_lane, alpha);
-        rs.l *= alpha;
-        rs.m = mnew;
-      } else if (high) {
-        rs.m = mx - 56.0f;
-      }
-      sum = weigh(v, rs.m, sc, pk);
+  for (int c = 0; c < 4; ++c) {
+    uint32_t v[32];
+    tmem_ld32(tS_lane + c * 32, v);
+    tmem_wait_ld();
+    if (MASK) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (c * 32 + j >= valid) v[j] = 0xff800000u;
     }
-    tmem_st32(tS_lane + half * 32, pk);
-    rs.l += sum;
-    if (half == 0) halfway();
+    uint32_t pk[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      float y0, y1, p0, p1;
+      unpack_f2(fma_f2(pack_f2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), sc2, nm2), y0, y1);
+      if (!MASK && j % kFmaPairEvery == kFmaPairEvery - 1) {
+        exp2_fma2(y0, y1, p0, p1);
+      } else {
+        p0 = ex2_approx(y0);
+        p1 = ex2_approx(y1);
+      }
+      ls2[j & 1] = add_f2(ls2[j & 1], pack_f2(p0, p1));
+      pk[j] = pack_bf2(p0, p1);
+    }
+    tmem_st16(tS_lane + c * 16, pk);
+    if (c == 1) halfway();
   }
+  float s0, s1, s2, s3;
+  unpack_f2(ls2[0], s0, s1);
+  unpack_f2(ls2[1], s2, s3);
+  rs.l += (s0 + s1) + (s2 + s3);
 }
 
 constexpr int A2_COPY_WARPS = 6;
