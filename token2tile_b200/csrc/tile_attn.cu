@@ -1174,10 +1174,13 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       cp_async16(sQ + sw128(r, ch), QU + ((size_t)h * N + max(o4[u], 0)) * kR + ch * 8, o4[u] >= 0 ? 16u : 0u);
     }
     cp_async_commit();
+    // Four counts x y z w are kept as x z y w, every other two quads as z x w y: the weighted sum of a row runs over four
+    // accumulators, two of them per packed multiply-add, and this is the order in which quad k meets them.
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      reinterpret_cast<float4*>(sCnt)[tid + TL_Q * u] =
-          make_float4((float)kz[u].x, (float)kz[u].y, (float)kz[u].z, (float)kz[u].w);
+    for (int u = 0; u < 4; ++u) {
+      const float x = (float)kz[u].x, y = (float)kz[u].y, z = (float)kz[u].z, w = (float)kz[u].w;
+      reinterpret_cast<float4*>(sCnt)[tid + TL_Q * u] = (tid & 2) ? make_float4(z, x, w, y) : make_float4(x, z, y, w);
+    }
     cp_async_wait<0>();
     fence_proxy_async();
   }
@@ -1305,7 +1308,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       const float nm = (m == -INFINITY) ? 0.f : -m;
       const unsigned long long l2e2 = pack_f2(LOG2E, LOG2E), nm2 = pack_f2(nm, nm);
       const float4* cnt4 = reinterpret_cast<const float4*>(sCnt + i * TL_H);
-      unsigned long long ps2[2] = {0ull, 0ull};
+      unsigned long long even2 = 0ull, odd2 = 0ull;      // accumulators 0 and 2, 1 and 3
       uint32_t pk[TL_H / 2];
 #pragma unroll
       for (int k = 0; k < TL_H / 4; ++k) {
@@ -1324,14 +1327,15 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
           p2 = ex2_approx(y2);
           p3 = ex2_approx(y3);
         }
-        ps2[0] = fma_f2(pack_f2(p0, p1), pack_f2(cn.x, cn.y), ps2[0]);
-        ps2[1] = fma_f2(pack_f2(p2, p3), pack_f2(cn.z, cn.w), ps2[1]);
+        unsigned long long& acc = (k & 1) ? odd2 : even2;
+        acc = fma_f2((k & 2) ? pack_f2(p2, p0) : pack_f2(p0, p2), pack_f2(cn.x, cn.y), acc);
+        acc = fma_f2((k & 2) ? pack_f2(p3, p1) : pack_f2(p1, p3), pack_f2(cn.z, cn.w), acc);
         pk[2 * k] = pack_bf2(p0, p1);
         pk[2 * k + 1] = pack_bf2(p2, p3);
       }
       float ps4[4];
-      unpack_f2(ps2[0], ps4[0], ps4[1]);
-      unpack_f2(ps2[1], ps4[2], ps4[3]);
+      unpack_f2(even2, ps4[0], ps4[2]);
+      unpack_f2(odd2, ps4[1], ps4[3]);
       phi += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
       tmem_st32(tS_lane + b * TL_H, pk);
       tmem_wait_st();
