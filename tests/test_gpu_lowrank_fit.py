@@ -127,3 +127,26 @@ def test_fit_on_both_factor_routes(N, spread_q, spread_k):
     want = (q.double() @ _product(oq, ok)) @ k.double().transpose(1, 2)
     got = (q.double() @ _product(Uq, Uk)) @ k.double().transpose(1, 2)
     assert (got - want).abs().max() <= 1e-3 * want.abs().max()
+
+
+@pytest.mark.parametrize("p", [4, 8, 10])
+def test_fit_separates_nearly_equal_singular_values(p):
+    """Second moments that fp32 slabs hold exactly: 8,192 Hadamard rows (one slab, 8192 I) and, on the query side, 300
+    rows of integers times 2^-p (the next slab).  All singular values agree to 7e-4, 3e-6 and 2e-7; the 32 largest span
+    a subspace that is determined to the fp64 rounding over the gap behind them (2^-52 x 128 over 5e-6, 1e-8 and 1e-9),
+    plus the rounding of the fp32 factors."""
+    from token2tile_b200.deploy_step import online_u
+    had = torch.ones(1, 1)
+    while had.shape[0] < 8192:
+        had = torch.cat([torch.cat([had, had], 1), torch.cat([had, -had], 1)])
+    had = had[:, torch.arange(128) * 64 + 1]
+    assert torch.equal(had.double().T @ had.double(), 8192 * torch.eye(128).double())
+    R = torch.randint(-2, 3, (300, 128), generator=torch.Generator().manual_seed(p)).float()
+    q = torch.cat([had, R * 2.0 ** -p])[None].to(BF)
+    k = torch.cat([had, torch.zeros(300, 128)])[None].to(BF)
+    Uq, Uk = online_u(q.to(DEV), k.to(DEV), 32)
+    e, V = torch.linalg.eigh(R.double().T @ R.double())
+    want = V[:, -32:] @ V[:, -32:].T                  # Mq, Mk and their roots share these eigenvectors
+    gap = float(e[-32] - e[-33]) * 4.0 ** -p / 8192 / 2
+    got = _product(Uq, Uk)[0]
+    assert (got - want).abs().max() <= (2.0 ** -52 * 128 / gap + 2.0 ** -22) * want.abs().max()

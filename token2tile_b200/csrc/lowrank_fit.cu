@@ -132,7 +132,8 @@ constexpr int JD = 128;                  // matrix order
 constexpr int JLD = JD + 1;              // column stride in doubles: odd, so that rows can be walked as well as columns
 constexpr int J_THREADS = 256;
 constexpr int J_MAX_SWEEPS = 18;
-constexpr double kJacobiDone2 = 9.0e-16;   // (3e-8)^2: see jacobi_orthogonalise
+constexpr double kJacobiDone2 = 9.0e-16;   // (3e-8)^2, and
+constexpr float kJacobiDoneT = 1.0e-6f;    // the tangent of the angle: see jacobi_orthogonalise
 constexpr int J_SMEM = JD * JLD * 8 + 2 * JD * 8 + 8 * 8 * 16 + 4 * JD * 8 + 64;
 constexpr int F_SMEM = J_SMEM + JD * (JD + 1) / 2 * 8;      // factor_kernel: and a packed triangle
 static_assert(J_SMEM % 16 == 0 && F_SMEM <= 227 * 1024, "shared memory of factor_kernel");
@@ -210,7 +211,7 @@ __device__ __forceinline__ void rotate8(Columns& w, int cx, int cy, double* nrm2
   const double g2 = gamma * gamma, ab = alpha * beta;
   const bool live = alpha > tiny2 && beta > tiny2 && g2 > 1.0e-27 * ab;
   if (!__any_sync(0xffffffffu, live)) return;
-  again = again || (live && g2 > kJacobiDone2 * ab);
+  again = again || (live && (g2 > kJacobiDone2 * ab || fabsf(t0) > kJacobiDoneT));
   if (lane < 8) {
     cs[lane] = live ? make_double2(fma(y * h, k, y), fma(ty * h, k, ty)) : make_double2(1.0, 0.0);
     if (live) {
@@ -274,9 +275,9 @@ __device__ __forceinline__ void jacobi_round(Columns& w, int& r, double* xch, do
 // twice and writing it once (384 KB).  What bounds a round now is its chain of dependent steps: products, a reduction of
 // five shuffles, the angle (worked out once per pair, not by every lane that holds a part of it), the rotation.  The
 // order of the rotations fixes the signs of the result, so it is part of what callers see.
-// A stretch of 128 rounds in which no pair's cosine exceeded sqrt(kJacobiDone2) = 3e-8 leaves cosines of the order of
-// its square (inside a cluster of equal singular values, at most 3e-8), below the rounding of the fp32 factors: it is
-// the last.
+// A stretch of 128 rounds in which no pair turned by more than kJacobiDoneT and no cosine exceeded 3e-8 leaves angles of
+// the order of its square, 128 x 1e-12, below the rounding of the fp32 factors: it is the last.  Small cosines alone do
+// not tell: columns whose lengths agree to 1e-6 have them from the start and may still have to turn by 45 degrees.
 __device__ void jacobi_orthogonalise(double* W, double* nrm2, double2* cs_all) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double2* cs = cs_all + warp * 8;
