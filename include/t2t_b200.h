@@ -258,6 +258,11 @@ int t2t_gather4_selftest(const void* src, int rows, const int* gidx, void* out, 
  * kernel always terminates.  No counterpart in the reference. */
 int t2t_wait_timeout_selftest(int* d_status, int* d_out, cudaStream_t stream);
 
+/* Rotation self-test: for n triples (squared lengths alpha, beta of two columns and
+ * their product gamma, gamma != 0) writes tan, cos and sin of the angle that the
+ * projection fit's Jacobi rounds turn them by.  No counterpart in the reference. */
+int t2t_rotation_selftest(const double* d_pairs, double* d_out, int n, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

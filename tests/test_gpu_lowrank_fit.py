@@ -150,3 +150,24 @@ def test_fit_separates_nearly_equal_singular_values(p):
     gap = float(e[-32] - e[-33]) * 4.0 ** -p / 8192 / 2
     got = _product(Uq, Uk)[0]
     assert (got - want).abs().max() <= (2.0 ** -52 * 128 / gap + 2.0 ** -22) * want.abs().max()
+
+
+def test_rotation_against_float64(lib):
+    """Angles from 1e-12 to 45 degrees, both signs, lengths that agree and that differ by 2^30.  t0 is within a few fp32
+    roundings (3.2e-7 at worst) and the Newton step leaves their square and, in its own correction, another 1e-7 of
+    them: 1e-12 covers it with room.  (c, s) is a rotation to fp64 rounding."""
+    n = 1 << 16
+    g = torch.Generator().manual_seed(3)
+    u = lambda lo, hi: lo + (hi - lo) * torch.rand(n, generator=g, dtype=torch.float64)
+    alpha, beta = 2.0 ** u(30, 60), 2.0 ** u(30, 60)
+    beta = torch.where(torch.arange(n) % 3 == 0, alpha * (1.0 + 2.0 ** u(-40, 0)), beta)
+    gamma = torch.sqrt(alpha * beta) * 10.0 ** u(-13, 0) * torch.where(torch.arange(n) % 2 == 0, 1.0, -1.0)
+    pairs = torch.stack([alpha, beta, gamma], 1).to(DEV)
+    out = torch.empty_like(pairs)
+    assert lib.t2t_rotation_selftest(pairs.data_ptr(), out.data_ptr(), n, torch.cuda.current_stream().cuda_stream) == 0
+    t, c, s = out.cpu().unbind(1)
+    zeta = (beta - alpha) / (2.0 * gamma)
+    want = torch.where(zeta >= 0, 1.0, -1.0) / (zeta.abs() + torch.sqrt(1.0 + zeta * zeta))
+    assert ((t - want) / want).abs().max() < 1e-12
+    assert (c * c + s * s - 1.0).abs().max() < 1e-15
+    assert (s - c * t).abs().max() < 1e-15
