@@ -427,6 +427,59 @@ def test_assign_edges_of_tiles_groups_and_chunks(lib, H, N, Cn):
     _assign(lib, x.to(BF).to(DEV), finite.to(BF).to(DEV))
 
 
+@pytest.mark.parametrize("H, N", [(1, 130), (2, 4096), (1, 37889)])
+@pytest.mark.parametrize("Cn", [48, 2048, 2050])
+@pytest.mark.parametrize("kind", ["constant tail", "noisy tail", "all equal", "two families", "not finite"])
+def test_assign_many_rows_near_many_equal_centroids(lib, H, N, Cn, kind):
+    """Tiles full of rows with more than two groups in reach: a tail of equal rows (and of rows beside them) under centroids
+    drawn from all rows, nothing but equal rows, two sets of equal centroids, and NaN and infinite rows and centroids.
+    Labels equal the all-exact kernel's (checked by the helper)."""
+    g = torch.Generator().manual_seed(N + Cn)
+    x = torch.randn(H, N, 32, generator=g)
+    tail = N if kind == "all equal" else max(100, N // 10)
+    x[:, N - tail:] = x[:, -1:].clone()
+    if kind == "two families":
+        x[:, N - tail::2] = -x[:, -1:].clone()
+    cen = x[:, torch.sort(torch.randint(0, N, (Cn,), generator=g)).values].clone()
+    if kind == "two families":
+        cen[:, ::3], cen[:, 1::3] = x[:, -1:].clone(), -x[:, -1:].clone()
+    if kind == "noisy tail":
+        x[:, N - tail:] += 1e-2 * torch.randn(H, tail, 32, generator=g)
+    if kind == "not finite":
+        x[:, N - 60:, 3] = float("nan")
+        x[:, N - 90:N - 60, 4] = float("inf")
+        cen[0, 5, 0] = float("inf")
+        cen[0, 17, 1] = float("nan")
+    _assign(lib, x.to(BF).to(DEV), cen.to(BF).to(DEV), pin_begin=N - 3, pin_label=1)
+
+
+def test_assign_time_with_a_tail_of_equal_rows(lib):
+    """Padding must not decide how long a call takes: with a tenth of the rows equal (and as many of the centroids), within
+    eight times the call without (about three; settling such rows one by one takes twenty times as long)."""
+    from token2tile_b200.deploy_step import fast_assign
+    g = torch.Generator(device=DEV).manual_seed(4)
+    N = 75600
+    x = torch.randn(1, N, 32, device=DEV, generator=g)
+    rows = torch.randperm(N, device=DEV, generator=g)[:2048].sort().values
+
+    def time(x):
+        x = x.to(BF)
+        cen, out, ms = x[:, rows].contiguous(), torch.empty(1, N, dtype=torch.int32, device=DEV), []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(5):
+                fast_assign(x, cen, out)
+            b.record()
+            b.synchronize()
+            ms.append(a.elapsed_time(b))
+        return min(ms)
+
+    plain = time(x)
+    x[:, N - N // 10:] = x[:, -1:].clone()
+    assert time(x) < 8.0 * plain
+
+
 def _plain_structure(sizes, v):
     """One head, clusters of consecutive rows, every query cluster executes every key: (km, full union, zero QU)."""
     N, CQ = v.shape[1], len(sizes)

@@ -12,8 +12,8 @@
 // the best one.  A label is taken from these approximate values only when every
 // other centroid is further away than twice a bound on |approximate - chain|;
 // otherwise the exact chain decides, over the 32 centroids of the two best groups
-// when the third is out of reach (nearly always), else over all of them.  So the
-// labels are bit-identical to the all-exact kernel.
+// when the third is out of reach (nearly always), else over all centroids in reach.
+// So the labels are bit-identical to the all-exact kernel.
 //
 // Error bound.  With s~ the tensor-core sum and s the real one,
 // |s~ - s| <= kappa * (||x|| ||c|| + ||c||^2 / 2) with kappa = 2^-16 (the measured
@@ -35,6 +35,7 @@ constexpr int TA_SA = TA_ROWS * 128;           // 16 KB: rows padded to 128 B
 constexpr int TA_SB = TA_CH * 128;             // 16 KB per stage
 constexpr int TA_SMEM = TA_SA + 2 * TA_SB + 128 + 1024;
 constexpr int TA_THREADS = TA_ROWS;
+constexpr int TA_FEW = 4;                      // this many rows with more than two groups in reach are settled one by one
 
 __device__ __forceinline__ float ta_max3(float a, float b, float c) {
   float r;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bar + 2);
   int* sCnMax = reinterpret_cast<int*>(bar + 3);
-  int* sCount = reinterpret_cast<int*>(bar + 4);      // [2] rows to settle exactly: over two groups, over everything
+  int* sCount = reinterpret_cast<int*>(bar + 4);      // [2] rows to settle exactly: over two groups, over more
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, row0 = blockIdx.x * TA_ROWS;
@@ -297,12 +298,13 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
       if (b.keep[e] > best) { best = b.keep[e]; bi = e; }
     }
     const int row = row0 + tid;
+    bool wide = false;            // more than two groups in reach
     if (row < N) {
       const bool pinned = pin_begin >= 0 && row >= pin_begin;
       labels[(size_t)h * N + row] = pinned ? pin_label : b.i1 + bi;
       if (!pinned && !(best - second > eps)) {             // true for NaN as well
-        const int mode = b.m1 - b.m3 > eps ? 0 : 1;
-        list[mode * TA_THREADS + atomicAdd(sCount + mode, 1)] = tid;
+        wide = !(b.m1 - b.m3 > eps);
+        list[(wide ? TA_THREADS : 0) + atomicAdd(sCount + (wide ? 1 : 0), 1)] = tid;
         cand[tid] = make_int2(b.i1, b.i2);
       }
     }
@@ -334,10 +336,11 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
       warp_argmin(d, di);
       if (lane == 0) labels[(size_t)h * N + row0 + r] = di;
     }
-    // the whole CTA per row, all centroids
+    // Rows with more than two groups in reach (many equal centroids, or values that are not finite): a few are settled one
+    // after the other by the whole CTA, over all centroids (5.5 us each with 2048).
     float* wd = reinterpret_cast<float*>(sm + OFF_B + TA_SB + TA_THREADS * 8);      // [warps] distances, then indices
     int* wi = reinterpret_cast<int*>(wd + TA_THREADS / 32);
-    for (int e = 0; e < sCount[1]; ++e) {
+    for (int e = 0; sCount[1] <= TA_FEW && e < sCount[1]; ++e) {
       const int r = list[TA_THREADS + e];
       float x[kR];
       load_x(r, x);
@@ -356,6 +359,99 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
         labels[(size_t)h * N + row0 + r] = di == 0x7fffffff ? 0 : di;
       }
       __syncthreads();
+    }
+    // More of them - padding, constant frames: such rows sit together - go through the products once more, with the exact
+    // chain for every centroid whose score is within eps of the row's best.  Of 32 centroids a warp first drops those
+    // whose bits repeat a lower one's (that one ties and wins), then settles either one per step for each of its rows or
+    // all of one row per step, whichever takes fewer steps.  Whole call, 1 head x 75,600 rows, 2048 centroids, a tenth of
+    // the rows equal: 63 us (40 with none equal; 800 when every such row was settled by itself).
+    if (sCount[1] > TA_FEW) {
+      __syncthreads();                                      // the stages are free again
+      const float cut = b.m1 - eps;
+#pragma unroll
+      for (int st = 0; st < 2; ++st)
+        *reinterpret_cast<uint4*>(sm + OFF_B + st * TA_SB + sw128(tid, 5)) = make_uint4(0u, 0u, 0u, 0u);
+      float d = INFINITY;
+      int di = 0x7fffffff, seen = -1;      // seen: a centroid that was settled, copies of which come up most often
+#pragma unroll 1
+      for (int i = 0; i < nch; ++i) {
+        const int st = i & 1;                               // a warp may still read the chunk before
+        const uint8_t* stage = sm + OFF_B + st * TA_SB;
+        load_chunk(i, st);
+        cp_async_wait<0>();
+        __syncthreads();
+        augment(i, st);
+        fence_proxy_async();
+        tc_fence_before();
+        __syncthreads();
+        if (tid == 0) {
+          tc_fence_after();
+          issue(st, tmem);
+        }
+        if (!mbar_wait(bar, ph, abort_flag)) {
+          if (tid == 0 && status) atomicExch(status, ST_WAIT_TIMEOUT);
+          break;
+        }
+        ph ^= 1u;
+        tc_fence_after();
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          uint32_t v[32], near = 0u;
+          tmem_ld32(t_lane + q * 32, v);
+          tmem_wait_ld32(v);
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (!(__uint_as_float(v[e]) < cut)) near |= 1u << e;      // NaN as well
+          if (!wide) near = 0u;
+          const int c0 = i * TA_CH + q * 32;
+          if (c0 + 32 > Cn) near &= c0 < Cn ? (1u << (Cn - c0)) - 1u : 0u;
+          if (!__any_sync(0xffffffffu, near != 0u)) continue;
+          {
+            uint32_t mine[16], hash = 0u;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              const uint4 w = *reinterpret_cast<const uint4*>(stage + sw128(q * 32 + lane, g));
+              mine[4 * g] = w.x; mine[4 * g + 1] = w.y; mine[4 * g + 2] = w.z; mine[4 * g + 3] = w.w;
+            }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) hash = hash * 0x9E3779B1u + mine[k];
+            const int first = __ffs(__match_any_sync(0xffffffffu, hash)) - 1;
+            const uint4* old = reinterpret_cast<const uint4*>(ch + (size_t)max(seen, 0) * kR);
+            bool copy = first < lane, again = seen >= 0;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              const uint4 w = *reinterpret_cast<const uint4*>(stage + sw128(q * 32 + first, g)), o = old[g];
+              copy = copy && mine[4 * g] == w.x && mine[4 * g + 1] == w.y && mine[4 * g + 2] == w.z && mine[4 * g + 3] == w.w;
+              again = again && mine[4 * g] == o.x && mine[4 * g + 1] == o.y && mine[4 * g + 2] == o.z && mine[4 * g + 3] == o.w;
+            }
+            near &= ~__ballot_sync(0xffffffffu, copy || again);
+          }
+          unsigned rows = __ballot_sync(0xffffffffu, near != 0u);
+          if (rows) seen = c0 + __ffs(__reduce_or_sync(0xffffffffu, near)) - 1;
+          float x[kR];
+          if (__popc(rows) > (int)__reduce_max_sync(0xffffffffu, __popc(near))) {
+            load_x(tid, x);
+            for (; near; near &= near - 1u) {
+              const int c = c0 + __ffs(near) - 1;
+              const float dc = exact_distance(x, ch + (size_t)c * kR);
+              if (dc < d) { d = dc; di = c; }
+            }
+            __syncwarp();
+          } else {
+            for (; rows; rows &= rows - 1u) {
+              const int src = __ffs(rows) - 1;
+              load_x(warp * 32 + src, x);
+              const bool mine = (__shfl_sync(0xffffffffu, near, src) >> lane) & 1u;
+              float dc = mine ? exact_distance(x, ch + (size_t)(c0 + lane) * kR) : INFINITY;
+              int dj = c0 + lane;
+              if (!(dc < INFINITY)) { dc = INFINITY; dj = 0x7fffffff; }      // NaN as well
+              warp_argmin(dc, dj);
+              if (lane == src && dc < d) { d = dc; di = dj; }
+            }
+          }
+        }
+      }
+      if (wide) labels[(size_t)h * N + row] = di == 0x7fffffff ? 0 : di;
     }
   }
   tc_fence_before();
