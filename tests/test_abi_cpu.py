@@ -32,6 +32,16 @@ def test_workspace_sizes_are_pure_host_functions(lib):
     assert lib.t2t_centroid_update_ws_bytes(2, 4096, 2048) > 0
 
 
+def test_grouping_takes_few_histograms_where_their_sums_are_what_takes_long(lib):
+    """256 rows per histogram while a thread that adds them up meets at most 64 (once per 1024 clusters), 1024 beyond."""
+    def histograms(H, N, Cn):
+        rest = H * Cn * 4 + H * N * 4               # cluster bases and the permutation, both multiples of 256 bytes here
+        return (lib.t2t_centroid_update_ws_bytes(H, N, Cn) - rest) // (H * Cn * 4)
+
+    assert [histograms(1, N, 2048) for N in (4096, 8192, 16384, 65536)] == [16, 32, 16, 64]
+    assert [histograms(40, N, 512) for N in (4096, 16384, 32768)] == [16, 64, 32]
+
+
 def test_null_and_bad_arguments_are_rejected(lib):
     assert lib.t2t_project(0, 0, 0, 1, 1, 0, 0) == 1
     assert lib.t2t_assign(0, 0, 0, 2, 4096, 32, -1, 0, 0, 0, 0, 0) == 1

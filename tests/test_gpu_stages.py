@@ -542,10 +542,10 @@ def test_tile_attn_weight_of_a_dominant_key_is_one(lib, sizes, tile, pos):
     assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-4
 
 
-@pytest.mark.parametrize("N", [31, 257, 16384, 16385])
-@pytest.mark.parametrize("Cn", [3, 2048])
+@pytest.mark.parametrize("N", [31, 257, 8192, 8193, 16384, 16385])
+@pytest.mark.parametrize("Cn", [3, 1024, 2048])
 def test_centroid_update_on_both_sides_of_the_chunk_rule(lib, N, Cn):
-    """256 rows per warp up to 16,384 rows, 1024 beyond; ragged ends, labels outside [0, Cn) left out, empty clusters
+    """256 rows per warp up to 16,384 rows (8,192 above 1024 clusters), 1024 beyond; ragged ends, labels outside [0, Cn) left out, empty clusters
     keeping their old centroid.  The sums are exact integers: bit for bit."""
     H = 2
     g = torch.Generator().manual_seed(N + Cn)

@@ -116,9 +116,13 @@ __global__ void __launch_bounds__(AS_THREADS) assign_exact_kernel(const __nv_bfl
 // stable grouping: per-chunk histograms -> offsets -> scatter
 // ---------------------------------------------------------------------------
 constexpr int GR_WARPS = 4;
-// Rows per warp: a warp walks its rows 32 at a time, a chain of label -> match -> counter steps of about 100 cycles, and
-// a short problem wants more warps instead (2 heads x 4096 rows ran on two CTAs a side); a long one wants few histograms.
-static int group_chunk(int N) { return N <= 16384 ? 256 : 1024; }
+// Rows per warp.  A warp walks its rows 32 at a time, a chain of label -> match -> counter steps of about 100 cycles, so
+// few rows make short chains; but every chunk of rows is one more histogram for offsets_kernel, whose threads walk all of
+// them once per 1024 clusters.  The line lies where that walk gets longer than the chains get shorter.  Sum of the three
+// kernels in us with 256 / 1024 rows, 1 head (40 heads in brackets): 2048 clusters 18.5 / 28.8 at 4,096 rows, 21.5 / 27.6
+// (26.5 / 29.2) at 8,192, 30.8 / 28.1 (39.5 / 31.2) at 16,384; 512 clusters 15.6 / 21.5 (20.3 / 23.1) at 16,384 and
+// 21.3 / 22.7 (32.6 / 28.2) at 32,760.
+static int group_chunk(int N, int Cn) { return cdiv(N, 256) * cdiv(Cn, 1024) <= 64 ? 256 : 1024; }
 
 // The labels of a warp's IT x 32 rows, all fetched before the first is used; -1 past the end and for a label outside
 // [0, Cn), which is ignored, never indexed.
@@ -164,7 +168,9 @@ __global__ void __launch_bounds__(1024) offsets_kernel(int* __restrict__ chist, 
                                                        int* __restrict__ cbase, int Cn, int nChunk) {
   __shared__ int wsum[32];
   __shared__ int carry_s;
-  constexpr int B = 16;      // histogram entries in flight per thread (the offsets replace them, one batch behind)
+  // histogram entries in flight per thread (the offsets replace them, one batch behind); 16 cost more issue slots than
+  // they hide (2048 clusters, 1 head: 10.2 against 7.6 us at 16 chunks, 35 against 24 at 74; one at a time 7.4 and 31)
+  constexpr int B = 8;
   const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* ch = chist + (size_t)h * nChunk * Cn;
   if (tid == 0) carry_s = 0;
@@ -256,7 +262,7 @@ static void launch_group_of(const int* lab, int* chist, int* counts, int* cbase,
 }
 static void launch_group(const int* lab, int* chist, int* counts, int* cbase, int* perm, int H, int N,
                          int Cn, cudaStream_t st) {
-  if (group_chunk(N) == 256) launch_group_of<8>(lab, chist, counts, cbase, perm, H, N, Cn, st);
+  if (group_chunk(N, Cn) == 256) launch_group_of<8>(lab, chist, counts, cbase, perm, H, N, Cn, st);
   else launch_group_of<32>(lab, chist, counts, cbase, perm, H, N, Cn, st);
 }
 
@@ -493,10 +499,9 @@ struct KmmWs {
 static KmmWs kmm_layout(int H, int N, int CQ, int C, void* base) {
   Carver cv(base);
   KmmWs w;
-  const int nChunk = cdiv(N, group_chunk(N));
   w.qlab1 = cv.take<int>((size_t)H * N);
-  w.chist = cv.take<int>((size_t)H * nChunk * CQ);
-  w.chist_k = cv.take<int>((size_t)H * nChunk * C);
+  w.chist = cv.take<int>((size_t)H * cdiv(N, group_chunk(N, CQ)) * CQ);
+  w.chist_k = cv.take<int>((size_t)H * cdiv(N, group_chunk(N, C)) * C);
   w.cbase_q = cv.take<int>((size_t)H * CQ);
   w.cbase_k = cv.take<int>((size_t)H * C);
   w.cq1 = cv.take<__nv_bfloat16>((size_t)H * CQ * kR);
@@ -528,7 +533,7 @@ struct UpdWs {
 static UpdWs upd_layout(int H, int N, int Cn, void* base) {
   Carver cv(base);
   UpdWs w;
-  w.chist = cv.take<int>((size_t)H * cdiv(N, group_chunk(N)) * Cn);
+  w.chist = cv.take<int>((size_t)H * cdiv(N, group_chunk(N, Cn)) * Cn);
   w.cbase = cv.take<int>((size_t)H * Cn);
   w.perm = cv.take<int>((size_t)H * N);
   w.total = cv.off;
