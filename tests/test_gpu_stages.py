@@ -355,6 +355,29 @@ def _structure(c, ns, pin_tail=0):
     return QU, km, cks, unip
 
 
+@pytest.mark.parametrize("kind", ["two humps", "heavy tails"])
+def test_select_of_unlike_distributions_stays_on_the_tensor_core_path(lib, kind):
+    """Half of the tokens around one centre (two humps of scores, the threshold in the upper one) and rows with Student
+    tails: the first histogram range still brackets the threshold of nearly every row (measured 0.3 % and none queued for
+    the exact kernel; half of the rows with a range of 1.6 deviations instead of 2.5)."""
+    from token2tile_b200.deploy_step import MaskedStepDeploy
+    H, N, CQ = 2, 16384, 128
+    g = torch.Generator().manual_seed(9)
+    rn = lambda *shape: torch.randn(*shape, generator=g)
+    if kind == "two humps":
+        pick = torch.where(torch.rand(N, generator=g) < 0.5, 0, torch.randint(0, 256, (N,), generator=g))
+        base = rn(H, 256, 128)[:, pick]
+        q, k = base + 0.3 * rn(H, N, 128), base + 0.3 * rn(H, N, 128)
+    else:
+        q, k = (rn(H, N, 128) / torch.sqrt((rn(H, N, 3) ** 2).mean(2, keepdim=True) + 0.05) for _ in range(2))
+    q, k, v = (t.to(BF).to(DEV) for t in (q, k, rn(H, N, 128)))
+    op = MaskedStepDeploy(H, N, CQ, s_frac=0.015)
+    op.step(q, k, v, op.init_state(q, k, warm_iters=2))
+    S = op.last_structure
+    _select(lib, op.QU, S["cks"], S["counts"], S["qperm"], S["tile_sizes"], op.ns)
+    assert _select.requeued <= 0.02 * H * N
+
+
 @pytest.mark.parametrize("ns", [204, 20])
 def test_tile_attn_matches_oracle(lib, small_case, ns):
     c = small_case

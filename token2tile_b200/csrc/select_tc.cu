@@ -48,7 +48,13 @@ constexpr int kMomFloats = 32 + 32 * 32;   // per head: mean centroid, second-mo
 constexpr int kMomParts = 8;               // the moments are summed over this many slices of the centroids
 constexpr int ST_MAX_TPC = 8;              // consecutive 128-row tiles of one head per CTA, at most: the head's centroids,
                                            // sizes and prefix sums are staged once for all of them
-constexpr float ST_SPAN = 0.8f;            // half width of the first histogram range, in standard deviations of a row's scores
+// Half width of the first histogram range, in standard deviations of a row's scores.  A narrow range has finer buckets and
+// fewer candidates, but a tile with more than a few rows outside pays a second pass, or leaves them to the exact kernel.
+// 4 heads x 75,600 rows, ms at a budget of 1.5 % / 5 % with 0.8, 1.0 and 1.25: the 3D locality mixture 0.80 / 0.86, 0.81 /
+// 0.89, 0.79 / 0.93; independent normal rows 0.85 / 0.97, 0.88 / 0.99, 0.90 / 1.02; heavy tails (Student, 3 degrees) 1.62 /
+// 1.83, 0.99 / 1.17, 0.97 / 1.31; smooth trajectories 1.05 / 0.80, 1.00 / 0.78, 0.86 / 0.80; half of the rows around one
+// centre 9.62, 1.50, 1.12 at 1.5 % (and 10 with any of them at 5 %: more than ST_CAP candidates).
+constexpr float ST_SPAN = 1.25f;
 constexpr int ST_STRAGGLERS = 8;           // this few unsettled rows of a tile go to the exact kernel instead of another pass
 
 constexpr int OFF_CK = 0;                               // 1024 rows x 128 B: centroid c in row c % 1024, half c / 1024
@@ -416,11 +422,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       const float sd = sqrtf(fmaxf(s2 - mean * mean, 1.0e-20f));
       const bool finite = fabsf(M) < INFINITY && fabsf(s2) < INFINITY && fabsf(mean) < INFINITY;
       // First range: ST_SPAN standard deviations to either side of the score a fraction ns / N of a bell-shaped
-      // distribution would exceed (inverse normal tail, Abramowitz-Stegun 26.2.23; on clustered activations the
-      // thresholds of a tile's rows lie 0.35 to 0.6 deviations apart, centred within 0.15 of it).  Everything
-      // above the range is counted in an overflow bucket.  The range only has to be a good guess: the search continues
-      // above it (up to the bound ||q|| max ||c||) or below it when the running token count says so; the narrower it
-      // is, the finer the buckets and the fewer the candidates.
+      // distribution would exceed (inverse normal tail, Abramowitz-Stegun 26.2.23).  Everything above the range is
+      // counted in an overflow bucket.  The range only has to be a good guess: the search continues above it (up to the
+      // bound ||q|| max ||c||) or below it when the running token count says so.
       const float f = fminf(0.5f, fmaxf((float)ns / (float)N, 1.0e-6f));
       const float tt = sqrtf(-2.0f * __logf(f));
       const float z = tt - (2.515517f + tt * (0.802853f + tt * 0.010328f)) /
