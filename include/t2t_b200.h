@@ -67,7 +67,8 @@ int t2t_lowrank_fit(const void* q, const void* k, float* Uq, float* Uk, int H, i
  * tcgen05 product and re-evaluates by the exact chain only the rows whose two
  * nearest centroids are closer than the product's error bound;
  * t2t_assign_exact evaluates the chain for every pair (slow; the cross-check).
- * Both give identical labels.  ws: t2t_assign_ws_bytes(H, N).  Replaces
+ * Both give identical labels.  ws: t2t_assign_ws_bytes(H, N), an int that
+ * receives the number of rows re-evaluated.  Replaces
  * fast_assign(x, centroids), fast_assign.py:79-106 and assign_kernel,
  * kernels/kmeans_maintain/src/kernels.cu:104-257. */
 size_t t2t_assign_ws_bytes(int H, int N);

@@ -30,6 +30,7 @@ def test_workspace_sizes_are_pure_host_functions(lib):
     ints = lib.t2t_tile_attn_plan_ints(40, 75600, 512)
     assert ints >= 40 * 2049 + 4 * 40 * (512 + 75600 // 256) + 40 * 512
     assert lib.t2t_centroid_update_ws_bytes(2, 4096, 2048) > 0
+    assert lib.t2t_assign_ws_bytes(40, 75600) == 4
 
 
 def test_grouping_takes_few_histograms_where_their_sums_are_what_takes_long(lib):

@@ -781,9 +781,10 @@ extern "C" int t2t_score_select_union(const void* QU, const void* cks, const voi
     return T2T_ERR_CUDA;
   // Tiles per CTA: as many as still leave every SM several CTAs, so that the last wave is short (with four always,
   // 2 heads x 4096 rows ran on 16 SMs: 263 us).
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return T2T_ERR_CUDA;
   const int tiles = cdiv(N, 128);
   const int tpc = max(1, min(ST_MAX_TPC, H * tiles / (4 * sms)));
   select_tc_kernel<<<dim3(cdiv(tiles, tpc), H), ST_THREADS, ST_SMEM, st>>>(

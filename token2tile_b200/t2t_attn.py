@@ -572,8 +572,8 @@ def fast_online_u(qf, kf, r: int = 32):
     (the reference's `_fast_online_u`, t2t_attn.py:211-239, moves the long
     products to fp32 tensor-core GEMMs and keeps only the 128x128
     factorisations in fp64).  Here `online_u` already works that way: both
-    names run the same kernels (tensor-core second moments, fp64 Jacobi
-    factorisations, batched over heads); this one returns as soon as the
+    names run the same kernels (tensor-core second moments, fp64 factors and
+    singular triplets, batched over heads); this one returns as soon as the
     kernels are queued."""
     from .deploy_step import lowrank_fit
     return lowrank_fit(qf, kf, r, check_finite=False)
