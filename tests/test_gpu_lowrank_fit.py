@@ -1,9 +1,10 @@
 """The projection-fit kernels (t2t_lowrank_fit: tensor-core second moments, fp64
-Jacobi factorisations) against the reference's own `online_u` run on the CPU
+factors and singular triplets) against the reference's own `online_u` run on the CPU
 (tests/golden/online_u.pt) and against the oracle.
 
 The factors are defined up to a common sign per component (and a rotation
-inside equal singular values), so the products Uq Uk^T are compared."""
+inside equal singular values), so the products Uq Uk^T are compared; one test
+pins the signs that the order of the rotations gives them."""
 import importlib.util
 from pathlib import Path
 
@@ -171,3 +172,82 @@ def test_rotation_against_float64(lib):
     assert ((t - want) / want).abs().max() < 1e-12
     assert (c * c + s * s - 1.0).abs().max() < 1e-15
     assert (s - c * t).abs().max() < 1e-15
+
+
+def _factors(lib, q, k):
+    """(Uq, Uk, roots [2 H, 128, 128]): the fit by its C entry, with the factors that it left in the workspace."""
+    H, N, _ = q.shape
+    qd, kd = q.to(DEV), k.to(DEV)
+    U = torch.empty(2, H, 128, 32, device=DEV)
+    flags = torch.zeros(2 * H + 1, dtype=torch.int32, device=DEV)
+    ws = torch.empty(lib.t2t_lowrank_fit_ws_bytes(H, N), dtype=torch.uint8, device=DEV)
+    assert lib.t2t_lowrank_fit(qd.data_ptr(), kd.data_ptr(), U[0].data_ptr(), U[1].data_ptr(), H, N, ws.data_ptr(), ws.numel(),
+                               flags.data_ptr(), flags.data_ptr() + 8 * H, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert not bool(flags.any())
+    at = ws.numel() - 3 * H * 128 * 128 * 8            # the last two regions: roots of 2 H matrices, inverses of H
+    return U[0].cpu(), U[1].cpu(), ws[at:at + 2 * H * 128 * 128 * 8].view(torch.float64).view(2 * H, 128, 128).cpu()
+
+
+@pytest.mark.parametrize("spread_q, spread_k, route_q, route_k", [
+    (1.0, 1.0, "cholesky", "products"), (3e-3, 0.3, "cholesky", "products"), (0.3, 0.1, "cholesky", "products"),
+    (1e-6, 1e-6, "eigenvectors", "eigenvectors")])
+def test_fit_takes_the_factor_route_of_its_spread(lib, spread_q, spread_k, route_q, route_k):
+    """The factor shows its route: Cholesky leaves zeros above the diagonal, the products end by averaging the root with
+    its transpose (symmetric bit for bit), and the sum over eigenvectors rounds the two triangles differently.  All of
+    them satisfy F F^T = M to the clamp and to the fp32 sums of the second moments: 256 additions of 16 rows each, every
+    one off by at most 2^-23 of the sum."""
+    g = torch.Generator().manual_seed(31)
+    H, N = 2, 4096
+    ramp = torch.linspace(0.0, 1.0, 128)
+    mix = torch.block_diag(torch.linalg.qr(torch.randn(64, 64, generator=g)).Q, torch.eye(64))
+    make = lambda spread: ((torch.randn(H, N, 128, generator=g) * spread ** ramp) @ mix.T).to(BF)
+    q, k = make(spread_q), make(spread_k)
+    _, _, F = _factors(lib, q, k)
+
+    def route(f):
+        if not bool(torch.triu(f, 1).any()):
+            return "cholesky"
+        return "products" if torch.equal(f, f.T) else "eigenvectors"
+
+    assert [route(F[i]) for i in range(H)] == [route_q] * H
+    assert [route(F[H + i]) for i in range(H)] == [route_k] * H
+    x = torch.cat([q, k]).double()
+    M = x.transpose(1, 2) @ x / N
+    assert (F @ F.transpose(1, 2) - M).abs().max() < 256 * 2.0 ** -23 * M.abs().max() + 1e-8
+
+
+def test_fit_signs_are_those_of_symmetric_roots(lib):
+    """The factors come with the signs (and the order) that one-sided Jacobi gives for symmetric roots on both sides:
+    round-robin rounds over M_q^(1/2) M_k^(1/2), restated here in float64.  Small integers, so that the second moments
+    are the same numbers."""
+    g = torch.Generator().manual_seed(32)
+    N = 4096
+    wide = torch.linspace(6.0, 1.0, 128)
+    k = torch.round(torch.randn(N, 128, generator=g) * wide[torch.randperm(128, generator=g)])
+    q = torch.round(0.5 * k + torch.randn(N, 128, generator=g) * wide)
+    assert q.abs().max() < 256 and k.abs().max() < 256            # exact in bfloat16
+    Uq, Uk, _ = _factors(lib, q[None].to(BF), k[None].to(BF))
+
+    def powers(x):
+        e, V = torch.linalg.eigh(x.double().T @ x.double() / N)
+        return (V * e.sqrt()) @ V.T, (V / e.sqrt()) @ V.T
+
+    (Rq, Iq), (Rk, _) = powers(q), powers(k)
+    W = Rq @ Rk
+    i = torch.arange(1, 64)
+    for sweep in range(14):
+        for r in range(127):
+            x = torch.cat([torch.tensor([127]), (r + i) % 127])
+            y = torch.cat([torch.tensor([r]), (r + 127 - i) % 127])
+            a, b, c = (W[:, x] ** 2).sum(0), (W[:, y] ** 2).sum(0), (W[:, x] * W[:, y]).sum(0)
+            turn = c * c > 1e-27 * a * b
+            zeta = (b - a) / (2.0 * torch.where(turn, c, torch.ones(())))
+            t = torch.where(zeta >= 0, 1.0, -1.0) / (zeta.abs() + torch.sqrt(1.0 + zeta * zeta)) * turn
+            cos = 1.0 / torch.sqrt(1.0 + t * t)
+            W[:, x], W[:, y] = cos * W[:, x] - cos * t * W[:, y], cos * t * W[:, x] + cos * W[:, y]
+    s, order = torch.sort((W * W).sum(0).sqrt(), descending=True, stable=True)
+    w, s = W[:, order[:32]], s[:32]
+    want_q, want_k = Iq @ w / s.sqrt(), Rq @ w / (s * s.sqrt())
+    for got, want in ((Uq[0], want_q), (Uk[0], want_k)):
+        assert (got.double() - want).abs().max() < 1e-5 * want.abs().max()
