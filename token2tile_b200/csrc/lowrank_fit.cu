@@ -23,8 +23,9 @@
 // the same value c, their joint contribution to f(M) is f(c) (I - sum of the other v v^T), whatever basis
 // spans them.
 //
-// Whole fit: 1.86 ms at 2 heads x 4096 rows, 2.18 ms at 40 x 75,600, of which the last kernel's sweeps are 1.5 ms (3.4 and
-// 3.6 ms where every root needs its eigenvectors); 5.9 and 6.3 ms with both roots by Jacobi sweeps through shared memory.
+// Whole fit: 2.2 ms at 2 heads x 4096 rows of clustered activations, 2.4 ms at 40 x 75,600, of which the last kernel's sweeps
+// are 1.4 to 1.5 ms (1.84 ms with independent normal rows, 3.8 to 4.2 where a root needs its eigenvectors); 5.9 to 9.8 ms
+// with both roots by Jacobi sweeps through shared memory.
 #include <cuda.h>
 
 #include "common.cuh"

@@ -27,8 +27,8 @@
 // for bit.  Rows that do not fit the fast path (more than 64 candidates, no
 // convergence, non-finite scores) are queued for the exact warp-per-row kernel.
 //
-// What bounds it: instruction issue, 21 instructions a score over the two passes, 60 % of the slots used, a third of
-// the warps' time at barriers.  6.15 ms for 40 heads x 75,600 rows (7.7 with 16 warps), 58 us for 2 x 4096 (263 with
+// What bounds it: instruction issue, 22 instructions a score over the two passes, 60 % of the slots used, a third of
+// the warps' time at barriers.  6.4 ms for 40 heads x 75,600 rows (7.7 with 16 warps), 64 us for 2 x 4096 (263 with
 // four tiles to every CTA).
 #include "common.cuh"
 #include "internal.h"
