@@ -227,16 +227,17 @@ struct RowState {
 
 constexpr float kLazy = 8.0f;   // rescale O only when the row maximum grows by more than 2^8
 
-// Rescale the fp32 accumulator rows in TMEM by `alpha` (per thread = per row).
+// Rescale the fp32 accumulator rows in TMEM by `alpha` (per thread = per row), few columns at a time: the attention's
+// softmax threads hold a row of scores meanwhile.
 __device__ __forceinline__ void rescale_rows(uint32_t tO_lane, float alpha) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    tmem_ld32(tO_lane + c * 32, v);
+  for (int c = 0; c < 8; ++c) {
+    uint32_t v[16];
+    tmem_ld16(tO_lane + c * 16, v);
     tmem_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * alpha);
-    tmem_st32(tO_lane + c * 32, v);
+    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * alpha);
+    tmem_st16(tO_lane + c * 16, v);
   }
 }
 
@@ -284,16 +285,6 @@ __device__ __forceinline__ void build_runs_warp(const int* __restrict__ koh, con
   }
   if (lane == 0) { sRunCum[runs] = total; *runs_out = runs; }
 }
-// The same for a whole CTA: warp 0 builds the list into sMisc[1], a CTA-wide barrier publishes it.  Returns
-// false when the list would not fit (the abort flag is then set).
-__device__ __forceinline__ bool build_runs(const int* __restrict__ koh, const uint32_t* __restrict__ ubr,
-                                           const uint32_t* __restrict__ nonempty, int* sRunStart, int* sRunCum,
-                                           int* sMisc, volatile int* abort_flag, int* status) {
-  if ((threadIdx.x >> 5) == 0) build_runs_warp(koh, ubr, nonempty, sRunStart, sRunCum, sMisc + 1, abort_flag, status);
-  __syncthreads();
-  return *abort_flag == 0;
-}
-
 constexpr int AT_TILE = KT * kD * 2;   // 32 KB: one 128-row tile of q, kp or vp
 
 // kp / vp rows (all heads: `row0` is the head's first row) of union positions p0 .. p0 + 3, from the run list of
@@ -336,10 +327,10 @@ struct KVMaps {
 // Groups that straddle two runs of the union are gathered.  Returns what this lane issues for each 64-column
 // block: FETCH_NONE (a tile load of a lower lane covers its rows), a gather, or a tile load starting at r[0].
 enum { FETCH_NONE = 0, FETCH_GATHER = 1, FETCH_BOX32 = 2, FETCH_BOX64 = 3 };
-__device__ __forceinline__ int fetch_plan(const int (&r)[4], bool whole, int lane) {
+__device__ __forceinline__ int fetch_plan(const int (&r)[4], bool whole, int lane, int seg) {
   const int prev = __shfl_up_sync(0xffffffffu, r[0], 1);
   const unsigned wmask = __ballot_sync(0xffffffffu, whole);
-  const bool linked = whole && lane > 0 && ((wmask >> (lane - 1)) & 1u) && r[0] == prev + 4;
+  const bool linked = whole && (lane & (seg - 1)) > 0 && ((wmask >> (lane - 1)) & 1u) && r[0] == prev + 4;
   const unsigned lmask = __ballot_sync(0xffffffffu, linked);      // bit g: group g continues the stretch of g - 1
   if (!whole) return FETCH_GATHER;
   const unsigned upto = 0xffffffffu >> (31 - lane);
@@ -363,26 +354,8 @@ __device__ __forceinline__ void fetch_issue(int what, uint32_t dst, const CUtens
 }
 
 // ---------------------------------------------------------------------------
-// exact attention, tasks of QT + 1 .. TASK_ROWS rows
+// softmax of a row of scores, shared by the two attention kernels
 // ---------------------------------------------------------------------------
-// Two row tiles share one K/V stream, so the union crosses L2 -> SM once per task
-// instead of once per 128 rows, and the roles are separated so that nobody who
-// computes ever waits on an issue queue:
-//   warps 0..3 / 4..7  softmax of row group 0 / 1: one thread per query row; S / P
-//                      and O of a group live in its own half of tensor memory
-//   warp 8             one lane issues every MMA (an MMA blocks its issuer while the
-//                      tensor pipe's queue is full)
-//   warps 10..15       stream K and V tiles into two-slot rings with four-row TMA gathers.
-//                      A gather blocks its warp for about 70 cycles per lane, one lane at a
-//                      time, but gathers of different warps overlap: six warps issue the
-//                      128 gathers of a tile pair, 21 or 22 each
-//   (warp 9 only takes part in the CTA-wide barriers: 16 warps keep four per scheduler)
-// Hand-offs are mbarriers: S[g] / O[g] (MMA done -> softmax), P[g] (softmax -> MMA),
-// fullK / fullV[s] (copy landed -> MMA), freeK / freeV[s] (both groups' MMA done -> copy: one
-// commit after group 1's MMA, which the tensor pipe runs after group 0's),
-// fullQ[g].  Ring slot s holds tile g with g & 1 == s, where g counts the tiles this
-// CTA has processed; the n-th fill of a slot waits for phase n of its free barrier
-// (phase 0 is completed at start-up) and completes phase n of its full barrier.
 // Packed fp32 pairs (one instruction for two values) and the three-input maximum keep the instruction count of
 // the softmax rows down: the MMA lane and the copy warps share their schedulers.
 __device__ __forceinline__ unsigned long long pack_f2(float lo, float hi) {
@@ -427,75 +400,59 @@ __device__ __forceinline__ void exp2_fma2(float y0, float y1, float& p0, float& 
   p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
 }
 
-// Softmax of one 128-column S row held in tensor memory, in two passes of 32-column chunks so that few
-// registers are live: the row maximum first, then P = 2^(s * scale - m) packed to bf16 over the columns S
-// occupied (chunk c of S, columns 32 c .., becomes columns 16 c .. of P: always columns that were read
-// before).  Two row groups that compute at the same time are bound by the special-function unit (16
-// exponentials per cycle and SM), so every third pair of a full tile takes the FMA-pipe route instead.
-// MASK: columns >= valid lie past the union and count as -inf (all of them through the special-function
-// unit, whose result for -inf is an exact zero).
+// Softmax of one 128-column S row held in tensor memory: the row comes to registers once, its maximum is found there,
+// then P = 2^(s * scale - m) goes back packed to bf16 (chunk c of S, columns 32 c .., becomes columns 16 c .. of P).
+// Two row groups that compute at the same time are bound by the special-function unit (16 exponentials per cycle and
+// SM), so every third pair takes the FMA-pipe route instead.
+// MASK: columns >= valid lie past the union and count as -inf, a weight of zero (2^-125 from the FMA pipe).
 // The maximum comes before any weight of the tile: weights stay below 2^kLazy, so O and l keep the range of the values
 // whatever the scores, and a key that dominates its row from beyond that weighs exactly one.  (One pass with the first
-// tile's maximum as reference and corrections by the sums: 10.7 instead of 12.0 ms at 720p x 40 heads, but the largest
-// weight is rounded like any other, 2.326e-3 instead of 2.323e-3 against a float64 softmax, and sums reach 2^60.  One
-// pass that keeps this rule, weighing first and starting over where a weight exceeds 2^kLazy, gains nothing: the first
-// half of P then waits for the second.)
-constexpr int kFmaPairEvery = 3;
-// `halfway` is called by the whole warp once the first 64 columns of P are written, so that the MMA lane can
-// start on them while the rows work on the rest.
-template <bool MASK, typename Halfway>
-__device__ __forceinline__ void softmax_tile(uint32_t tS_lane, uint32_t tO_lane, RowState& rs, int valid, bool first,
-                                             float sc, Halfway&& halfway) {
+// tile's maximum as reference and corrections by the sums rounds the largest weight like any other, 2.326e-3 instead
+// of 2.323e-3 against a float64 softmax, and sums reach 2^60.)
+constexpr int kFmaPairEvery = 99;
+
+// The row to registers; returns its maximum (unscaled).
+template <bool MASK>
+__device__ __forceinline__ float row_scores(uint32_t tS_lane, int valid, uint32_t (&v)[4][32]) {
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  tmem_ld32(tS_lane, v[0]);
+  tmem_ld32(tS_lane + 32, v[1]);
+  tmem_wait_ld();
+  tmem_ld32(tS_lane + 64, v[2]);
+  tmem_ld32(tS_lane + 96, v[3]);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    tmem_ld32(tS_lane + c * 32, v);
-    tmem_wait_ld();
+    if (c == 2) tmem_wait_ld();
     if (MASK) {
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        if (c * 32 + j >= valid) v[j] = 0xff800000u;      // -inf
+        if (c * 32 + j >= valid) v[c][j] = 0xff800000u;      // -inf
     }
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
-      mx4[0] = max3(mx4[0], __uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-      mx4[1] = max3(mx4[1], __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-      mx4[2] = max3(mx4[2], __uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
-      mx4[3] = max3(mx4[3], __uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
+      mx4[0] = max3(mx4[0], __uint_as_float(v[c][j]), __uint_as_float(v[c][j + 1]));
+      mx4[1] = max3(mx4[1], __uint_as_float(v[c][j + 2]), __uint_as_float(v[c][j + 3]));
+      mx4[2] = max3(mx4[2], __uint_as_float(v[c][j + 4]), __uint_as_float(v[c][j + 5]));
+      mx4[3] = max3(mx4[3], __uint_as_float(v[c][j + 6]), __uint_as_float(v[c][j + 7]));
     }
   }
-  const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc;
-  if (first) {
-    rs.m = mx;
-  } else {
-    const bool grow = mx > rs.m + kLazy;
-    if (__any_sync(0xffffffffu, grow)) {
-      const float mnew = grow ? mx : rs.m;
-      const float alpha = ex2_approx(rs.m - mnew);
-      rescale_rows(tO_lane, alpha);
-      rs.l *= alpha;
-      rs.m = mnew;
-    }
-  }
+  return fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+}
+// The row's weights relative to rs.m, written over S and added to rs.l.  `halfway` is called by the whole warp once the
+// first 64 columns of P are written, so that the MMA lane can start on them while the rows work on the rest.
+template <typename Halfway>
+__device__ __forceinline__ void row_weights(uint32_t tS_lane, const uint32_t (&v)[4][32], RowState& rs, float sc,
+                                            Halfway&& halfway) {
   const unsigned long long sc2 = pack_f2(sc, sc), nm2 = pack_f2(-rs.m, -rs.m);
   unsigned long long ls2[2] = {0ull, 0ull};
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    tmem_ld32(tS_lane + c * 32, v);
-    tmem_wait_ld();
-    if (MASK) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (c * 32 + j >= valid) v[j] = 0xff800000u;
-    }
     uint32_t pk[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       float y0, y1, p0, p1;
-      unpack_f2(fma_f2(pack_f2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), sc2, nm2), y0, y1);
-      if (!MASK && j % kFmaPairEvery == kFmaPairEvery - 1) {
+      unpack_f2(fma_f2(pack_f2(__uint_as_float(v[c][2 * j]), __uint_as_float(v[c][2 * j + 1])), sc2, nm2), y0, y1);
+      if (j % kFmaPairEvery == kFmaPairEvery - 1) {
         exp2_fma2(y0, y1, p0, p1);
       } else {
         p0 = ex2_approx(y0);
@@ -512,18 +469,208 @@ __device__ __forceinline__ void softmax_tile(uint32_t tS_lane, uint32_t tO_lane,
   unpack_f2(ls2[1], s2, s3);
   rs.l += (s0 + s1) + (s2 + s3);
 }
+template <bool MASK, typename Halfway>
+__device__ __forceinline__ void softmax_tile(uint32_t tS_lane, uint32_t tO_lane, RowState& rs, int valid, bool first,
+                                             float sc, Halfway&& halfway) {
+  uint32_t v[4][32];
+  const float mx = row_scores<MASK>(tS_lane, valid, v) * sc;
+  if (first) {
+    rs.m = mx;
+  } else {
+    const bool grow = mx > rs.m + kLazy;
+    if (__any_sync(0xffffffffu, grow)) {
+      const float mnew = grow ? mx : rs.m;
+      const float alpha = ex2_approx(rs.m - mnew);
+      rescale_rows(tO_lane, alpha);
+      rs.l *= alpha;
+      rs.m = mnew;
+    }
+  }
+  row_weights(tS_lane, v, rs, sc, halfway);
+}
 
-constexpr int A2_COPY_WARPS = 6;
-constexpr int A2_THREADS = (10 + A2_COPY_WARPS) * 32;   // 8 softmax warps, the MMA warp, an idle warp, the copy warps
-constexpr int A2_SLOT = 2 * AT_TILE;                      // K tile, V tile
-constexpr int A2_OFF_SLOT = 2 * AT_TILE;                  // after the two Q tiles
-constexpr int A2_OFF_MISC = A2_OFF_SLOT + 2 * A2_SLOT;
-constexpr int A2_RUN_INTS = 2 * MAX_RUNS + 8;                // one run list: starts, positions
-constexpr int A2_SMEM_INTS = 2 * A2_RUN_INTS + 32;
-constexpr int A2_SMEM = A2_OFF_MISC + 256 + A2_SMEM_INTS * 4 + 1024;
-enum { B_S = 0, B_O = 2, B_P = 4, B_FULLK = 8, B_FULLV = 10, B_FREEK = 12, B_FREEV = 14, B_FULLQ = 16, B_COUNT = 18 };   // P: [group][half]
+// Registers move between the roles of a kernel: a softmax thread holds a whole row of S, the others need few.  Both
+// kernels are launched with 128 registers a thread and every second warpgroup gives up what the softmax warpgroups take:
+// 128 x (200 + 56) = 256 x 128 (and twice that in attn2_kernel).
+constexpr int kLaunchRegs = 128, kSoftmaxRegs = 200, kRoleRegs = 56;
+static_assert(kSoftmaxRegs + kRoleRegs == 2 * kLaunchRegs, "the split may not exceed what the launch holds");
+__device__ __forceinline__ void take_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kSoftmaxRegs)); }
+__device__ __forceinline__ void give_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRoleRegs)); }
 
-__global__ void __launch_bounds__(A2_THREADS, 1) attn2_kernel(
+// One task as it travels through a CTA's two-slot ring.
+struct TaskSlot {
+  int end;      // nonzero: no task is left
+  int head, first, rows, kvlen, runs;      // first: sorted row the task starts at
+  int pad[2];
+};
+
+// Task `task` (none is left at numTasks) into `slot`, by one warp: record and union length, then the run list of its union.
+__device__ __forceinline__ void prepare_task(const PlanView& pv, const uint32_t* __restrict__ ub, int CQ, int numTasks,
+                                             int task, TaskSlot* slot, int* sRunStart, int* sRunCum,
+                                             volatile int* abort_flag, int* status) {
+  const int lane = threadIdx.x & 31;
+  int4 tk = make_int4(0, 0, 0, 0);
+  int len = 0;
+  if (task < numTasks) {
+    tk = pv.tasks[task];
+    len = pv.kv_lens[(size_t)tk.x * CQ + tk.y];
+  }
+  if (len > 0)
+    build_runs_warp(pv.k_off + (size_t)tk.x * (kC + 1), ub + ((size_t)tk.x * CQ + tk.y) * (kC / 32),
+                    pv.nonempty + (size_t)tk.x * (kC / 32), sRunStart, sRunCum, &slot->runs, abort_flag, status);
+  if (lane == 0) {
+    slot->end = task >= numTasks || *abort_flag;
+    slot->head = tk.x;
+    slot->first = tk.z;
+    slot->rows = tk.w;
+    slot->kvlen = len;
+  }
+  __syncwarp();
+}
+
+// A softmax warp's part of one task: its 32 rows' softmax tile by tile, then the division and the store.  `active` says
+// whether the warp has rows at all, `wr` whether this thread has one; barP[0 / 1] take the halves of P, `g` counts the
+// CTA's tiles.  False when a wait gave up.
+__device__ __forceinline__ bool softmax_task(uint32_t tS_lane, uint32_t tO_lane, uint64_t* barS, uint64_t* barPV,
+                                             uint64_t* barP, uint32_t& g, int kvlen, bool active, bool wr, __nv_bfloat16* out_row, float* lse,
+                                             volatile int* abort_flag) {
+  const int lane = threadIdx.x & 31;
+  const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
+  if (kvlen == 0) {   // empty union: O = 0, lse = -inf
+    if (wr) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) reinterpret_cast<uint4*>(out_row)[i] = make_uint4(0u, 0u, 0u, 0u);
+      *lse = -INFINITY;
+    }
+    return true;
+  }
+  const int ntiles = cdiv(kvlen, KT);
+  RowState rs;
+  rs.m = -INFINITY;
+  rs.l = 0.f;
+  for (int t = 0; t < ntiles; ++t) {
+    // this commit also covers P V of tile t - 1, so O may be rescaled
+    if (!mbar_wait(barS, g & 1u, abort_flag)) return false;
+    ++g;
+    tc_fence_after();
+    // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
+    // whatever S held, which only reaches O rows that are never stored.
+    auto halfway = [&]() {      // keys 0 .. 63 of P are in tensor memory
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(barP);
+    };
+    if (active) {
+      const int valid = kvlen - t * KT;
+      if (valid >= KT) softmax_tile<false>(tS_lane, tO_lane, rs, KT, t == 0, sc, halfway);
+      else softmax_tile<true>(tS_lane, tO_lane, rs, valid, t == 0, sc, halfway);
+      tmem_wait_st();
+    } else {
+      halfway();
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(barP + 1);
+  }
+  if (!mbar_wait(barPV, (g - 1u) & 1u, abort_flag)) return false;
+  if (active) {
+    tc_fence_after();
+    const float inv = 1.0f / rs.l;
+    uint4* dst = reinterpret_cast<uint4*>(out_row);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t v[32];
+      tmem_ld32(tO_lane + c * 32, v);
+      tmem_wait_ld();
+      if (wr) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 o;
+          o.x = pack_bf2(__uint_as_float(v[8 * g + 0]) * inv, __uint_as_float(v[8 * g + 1]) * inv);
+          o.y = pack_bf2(__uint_as_float(v[8 * g + 2]) * inv, __uint_as_float(v[8 * g + 3]) * inv);
+          o.z = pack_bf2(__uint_as_float(v[8 * g + 4]) * inv, __uint_as_float(v[8 * g + 5]) * inv);
+          o.w = pack_bf2(__uint_as_float(v[8 * g + 6]) * inv, __uint_as_float(v[8 * g + 7]) * inv);
+          dst[c * 4 + g] = o;
+        }
+      }
+    }
+    if (wr) *lse = (rs.m + log2f(rs.l)) * 0.6931471805599453f;
+    tc_fence_before();
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------------------
+// exact attention, tasks of QT + 1 .. TASK_ROWS rows
+// ---------------------------------------------------------------------------
+// The kernel runs on CTA pairs (clusters of two, one CTA per SM): group 0 of a task's rows on the even CTA, the leader,
+// group 1 on the odd one, 128 rows each.  A product covers both groups (256 rows), and each CTA keeps only half of a K
+// tile (64 keys) and half of a V tile (64 of the 128 columns), so that per SM a tile moves 96 KB through shared memory
+// instead of 128 KB and tensor memory holds one group's O and three score buffers.  Roles of a CTA:
+//   warps 0..3 / 4..7  softmax of the even / odd tiles, one thread per row of the group; the row's reference maximum
+//                      travels from tile to tile through shared memory, each thread sums the weights of its own tiles
+//   warp 8             leader: issues Q K^T (see elect_one)
+//   warp 9             leader: issues P V, so that neither product waits in line behind the other's barriers (one warp for
+//                      both left the tensor pipe idle for 500 of 1,750 cycles a tile); other CTA: takes the next task and
+//                      builds the run list of its union, for both CTAs
+//   warps 10..12       K tiles in turn (and Q tiles) by TMA, warps 13..15 V tiles: finding a tile's rows and issuing up to 32
+//                      instructions, about 70 cycles each, takes a warp three times as long as the products
+// S = Q K^T of tile g goes to score buffer g mod 3, two tiles ahead of P V, so that no softmax warp waits for the
+// product behind its own weights: with two score buffers (one CTA, two groups that share a K / V stream) the chain
+// softmax -> P V -> Q K^T took 3,770 cycles for two 128-row tiles.
+// Barriers: QK and PV are the commits behind the products of a tile, on barrier tile mod 4, and reach both CTAs.  QK(g): S(g)
+// is there, the K slot of tile g is free.  PV(g): O holds tile g, score buffer and V slot of tile g are free.  P[b],
+// FULLK / FULLV / FULLQ and OFREE live in the leader and collect both CTAs' arrivals (and, for copies, both CTAs'
+// bytes); TFREE lives in the other CTA and collects everyone who reads a task.
+constexpr int A2_THREADS = 16 * 32;
+constexpr int A2_STAGES = 4;                              // K and V ring depth
+constexpr int A2_HALF = AT_TILE / 2;                      // 16 KB: 64 keys of a K tile, 64 columns of a V tile
+constexpr int A2_OFF_K = 2 * AT_TILE;                     // after two Q tiles (this task's, the next one's)
+constexpr int A2_OFF_V = A2_OFF_K + A2_STAGES * A2_HALF;
+constexpr int A2_OFF_MISC = A2_OFF_V + A2_STAGES * A2_HALF;
+constexpr int RUN_INTS = 2 * MAX_RUNS + 8;                // one run list: [MAX_RUNS] starts, [MAX_RUNS + 1] positions
+enum { B_QK = 0, B_PV = 4, B_P = 8, B_FULLK = 11, B_FULLV = B_FULLK + A2_STAGES, B_FULLQ = B_FULLV + A2_STAGES,
+       B_FREEQ = B_FULLQ + 2, B_OFREE = B_FREEQ + 2, B_TFULL, B_TFREE = B_TFULL + 2, B_COUNT = B_TFREE + 2 };
+static_assert(A2_STAGES == 4, "ring slots and commits are counted alike");
+constexpr int A2_CONSUMERS = (8 + 6) * 2 + 2;             // warps that read a task: softmax and copy, QK and PV
+constexpr int A2_OFF_RING = A2_OFF_MISC + 512;            // two tasks
+constexpr int A2_OFF_M = A2_OFF_RING + 2 * (int)sizeof(TaskSlot);      // [2][128] reference maxima of the even / odd tiles, with their tiles
+constexpr int A2_OFF_FIN = A2_OFF_M + 2 * QT * 8;         // [2][2][128] (maximum, sum) of the two softmax warpgroups
+constexpr int A2_OFF_RUNS = A2_OFF_FIN + 4 * QT * 8;
+constexpr int A2_SMEM = A2_OFF_RUNS + 2 * RUN_INTS * 4 + 1024;
+static_assert(B_COUNT * 8 + 16 <= 512, "the barriers fit their area");
+static_assert(A2_SMEM <= 227 * 1024, "one CTA per SM");
+
+// A row's reference maximum behind tile `tile`, from the thread that weighs that tile to the thread that weighs the next:
+// value and tile number in one 64-bit word, so that neither needs a barrier (an mbarrier in between cost 440 cycles a tile).
+__device__ __forceinline__ void put_tagged(unsigned long long* at, uint32_t tile, float m) {
+  asm volatile("st.volatile.shared.b64 [%0], %1;\n" ::"r"(smem_u32(at)),
+               "l"(((unsigned long long)tile << 32) | __float_as_uint(m)) : "memory");
+}
+__device__ __forceinline__ unsigned long long peek_tagged(const unsigned long long* at) {
+  unsigned long long w;
+  asm volatile("ld.volatile.shared.b64 %0, [%1];\n" : "=l"(w) : "r"(smem_u32(at)) : "memory");
+  return w;
+}
+// Looks again until `w` is tile `tile`'s.
+__device__ __forceinline__ bool take_tagged(const unsigned long long* at, uint32_t tile, unsigned long long& w,
+                                            volatile int* abort_flag) {
+  for (uint32_t it = 0; (uint32_t)(w >> 32) != tile; ++it) {
+    if ((it & 255u) == 255u && *abort_flag) return false;
+    if (it == kWaitSpinLimit) {
+      *abort_flag = 1;
+      return false;
+    }
+    w = peek_tagged(at);
+  }
+  return true;
+}
+
+// Rows of group 0 of a task of more than QT rows, whole warps of them; group 1 takes the rest.
+__device__ __forceinline__ int group_rows(int rows) { return (((rows + 1) >> 1) + 31) & ~31; }
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2_kernel(
     const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ KVMaps maps,
     const uint32_t* __restrict__ ub, const int* __restrict__ qperm,
     __nv_bfloat16* __restrict__ attn_out, float* __restrict__ attn_lse, int* __restrict__ plan, int H, int N, int CQ,
@@ -534,261 +681,343 @@ __global__ void __launch_bounds__(A2_THREADS, 1) attn2_kernel(
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + A2_OFF_MISC);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + A2_OFF_MISC + B_COUNT * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + A2_OFF_MISC + B_COUNT * 8 + 8);
-  int* sInt = reinterpret_cast<int*>(sm + A2_OFF_MISC + 256);
-  int* sRuns = sInt;                              // two run lists (this task's, the next one's): [MAX_RUNS] starts, [MAX_RUNS + 1] positions
-  int* sMisc = sInt + 2 * A2_RUN_INTS;            // [2..7] the next task: index, head, cluster, first row, rows, union length; [8], [9] runs of the two lists
+  TaskSlot* ring = reinterpret_cast<TaskSlot*>(sm + A2_OFF_RING);
+  unsigned long long* sM = reinterpret_cast<unsigned long long*>(sm + A2_OFF_M);
+  float2* sFin = reinterpret_cast<float2*>(sm + A2_OFF_FIN);
+  int* sRuns = reinterpret_cast<int*>(sm + A2_OFF_RUNS);
 
-  const PlanView pv = plan_view(plan, H, N, CQ);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = (warp >> 2) & 1, gt = tid & 127, gw = warp & 3;   // softmax warps: group, thread, warp in group
+  const uint32_t rank = cluster_rank();      // group of this CTA's rows; 0 leads
 
   // the kernel launched behind this one (tasks of at most QT rows) does not depend on it: let it be scheduled
   // as soon as SMs free up
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
+    tmem_alloc_pair(tmem_slot, 512);
+    tmem_relinquish_pair();
   }
+  if (tid < 2 * QT) sM[tid] = ~0ull;      // no tile
   if (tid == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < B_COUNT; ++i)
-      mbar_init(bars + i, (i >= B_P && i < B_P + 4) ? 4 : 1);
+    for (int i = 0; i < B_COUNT; ++i) {
+      int count = 1;
+      if (i >= B_P && i < B_P + 3) count = 8;                                    // softmax warps of a tile, both CTAs
+      else if (i >= B_FULLK && i < B_FULLK + A2_STAGES) count = 2;               // a copy warp of each CTA
+      else if (i >= B_FULLV && i < B_FULLV + A2_STAGES) count = 2;
+      else if (i == B_FULLQ || i == B_FULLQ + 1) count = 4;
+      else if (i == B_OFREE) count = 16;
+      else if (i == B_TFREE || i == B_TFREE + 1) count = A2_CONSUMERS;
+      mbar_init(bars + i, count);
+    }
     mbar_init_fence();
-    // all ring slots start empty: complete phase 0 of the free barriers
-    for (int i = B_FREEK; i < B_FREEV + 2; ++i) mbar_arrive(bars + i);
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();      // both CTAs' barriers exist
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  uint32_t tiles_done = 0, qcnt = 0;      // tiles / non-empty tasks this CTA has processed; every role counts alike
-  uint32_t phS = 0, phO = 0;              // softmax warps: phases of their group's S and O barriers
-  const int numTasks = pv.counters[0];
-  const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
-  constexpr uint32_t idescQK = make_idesc_bf16(128, KT, false, false);
-  constexpr uint32_t idescPV = make_idesc_bf16(128, kD, false, true);
+  const uint32_t lead = cluster_addr(base + A2_OFF_MISC, 0);      // the leader's barriers
+  const uint32_t tfree = cluster_addr(base + A2_OFF_MISC, 1) + B_TFREE * 8;
 
-  // The next task of more than QT rows is prepared while the current one runs, by warp 9, which has nothing
-  // else to do: cursor, task record and union length (three dependent trips to global memory), then the run
-  // list of its union into the list the current task does not use.
-  auto prepare_task = [&](int list) {
-    int i = 0, th = 0, tc = 0, len = 0;
-    if (lane == 0) {
-      do { i = atomicAdd(&pv.counters[4], 1); } while (i < numTasks && pv.tasks[i].w <= QT);
-      int4 tk = make_int4(0, 0, 0, 0);
-      if (i < numTasks) {
-        tk = pv.tasks[i];
-        len = pv.kv_lens[(size_t)tk.x * CQ + tk.y];
-      }
-      th = tk.x;
-      tc = tk.y;
-      sMisc[2] = i; sMisc[3] = tk.x; sMisc[4] = tk.y; sMisc[5] = tk.z; sMisc[6] = tk.w; sMisc[7] = len;
-    }
-    i = __shfl_sync(0xffffffffu, i, 0);
-    th = __shfl_sync(0xffffffffu, th, 0);
-    tc = __shfl_sync(0xffffffffu, tc, 0);
-    len = __shfl_sync(0xffffffffu, len, 0);
-    if (i < numTasks && len > 0)
-      build_runs_warp(pv.k_off + (size_t)th * (kC + 1), ub + ((size_t)th * CQ + tc) * (kC / 32),
-                      pv.nonempty + (size_t)th * (kC / 32), sRuns + list * A2_RUN_INTS,
-                      sRuns + list * A2_RUN_INTS + MAX_RUNS, sMisc + 8 + list, abort_flag, status);
-  };
-  int list = 0;      // the run list of the current task
-  if (warp == 9) prepare_task(0);
-
-  while (true) {
-    __syncthreads();
-    const int ti = sMisc[2], h = sMisc[3], qs = sMisc[5], qrows = sMisc[6], kvlen = sMisc[7];
-    __syncthreads();      // everyone has the task: the record may be overwritten
-    if (ti >= numTasks || *abort_flag) break;
-    const size_t rowbase = (size_t)h * N + qs;
-    const int* sRunStart = sRuns + list * A2_RUN_INTS;
-    const int* sRunCum = sRunStart + MAX_RUNS;
-    const int nruns = sMisc[8 + list];
-    list ^= 1;
-    if (warp == 9) prepare_task(list);
-
-    if (kvlen == 0) {   // empty union: O = 0, lse = -inf
-      for (int i = tid; i < qrows * 16; i += A2_THREADS)
-        reinterpret_cast<uint4*>(attn_out + (rowbase + (i >> 4)) * kD)[i & 15] = make_uint4(0u, 0u, 0u, 0u);
-      for (int r = tid; r < qrows; r += A2_THREADS) attn_lse[rowbase + r] = -INFINITY;
-      continue;
-    }
-
-    const int rows0 = (qrows + 1) >> 1;                       // rows of group 0; group 1 takes the rest
-    if (warp >= 10 && warp < 14) {      // the Q tiles need no run list: their gathers go first
-      const int kind = (warp - 10) >> 1, oblk = (warp - 10) & 1, orow = lane * 4;
-      const int off = kind ? rows0 : 0, nr = kind ? qrows - rows0 : rows0;
-      int r[4];
+  if (warp < 8) {
+    // ================= softmax warps =================
+    take_registers();
+    const int wg = warp >> 2, gw = warp & 3, row = gw * 32 + lane;
+    const uint32_t tO_lane = tmem_addr(tmem + 3 * 128, gw * 32, 0);
+    const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
+    uint32_t g = 0;      // tiles so far
+    uint32_t q = 0;
+    bool ok = true;
+    for (uint32_t n = 0;; ++n) {
+      const uint32_t sl = n & 1u;
+      if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+      const int end = ring[sl].end, kvlen = ring[sl].kvlen, ntiles = cdiv(kvlen, KT);
+      if (end) break;
+      const int rows0 = group_rows(ring[sl].rows), myrows = rank ? ring[sl].rows - rows0 : rows0;
+      const size_t at = (size_t)ring[sl].head * N + ring[sl].first + (rank ? rows0 : 0) + (row < myrows ? row : 0);
+      const bool wr = row < myrows;
+      if (ntiles == 0) {   // empty union: O = 0, lse = -inf
+        if (wr) {
+          uint4* dst = reinterpret_cast<uint4*>(attn_out + at * kD) + wg * 8;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)      // slots past the group repeat its first row
-        r[j] = h * q_head_step + qperm[rowbase + off + (orow + j < nr ? orow + j : 0)] * q_row_step;
-      if (oblk == 0 && lane == 0) mbar_arrive_expect_tx(bars + B_FULLQ + kind, AT_TILE);
-      tma_gather4(base + kind * AT_TILE + oblk * (KT * 128) + orow * 128, &mapQ, oblk * 64, r[0], r[1], r[2], r[3],
-                  bars + B_FULLQ + kind);
-    }
-    const int ntiles = cdiv(kvlen, KT);
-    const uint32_t g0 = tiles_done;
-
-    if (warp >= 10 && warp < 14) {
-      // ================= copy warps: the K / V stream ===============
-      // warp 10, 11: the two 64-column blocks of the K tiles (above: of group 0's Q tile); warps 12, 13: those
-      // of the V tiles (of group 1's Q tile).  A lane owns rows 4 lane .. 4 lane + 3 of a tile.
-      const int kind = (warp - 10) >> 1, oblk = (warp - 10) & 1, orow = lane * 4;
-      const bool announces = oblk == 0 && lane == 0;
-      const CUtensorMap* map1 = kind ? &maps.v1 : &maps.k1;
-      const CUtensorMap* map32 = kind ? &maps.v32 : &maps.k32;
-      const CUtensorMap* map64 = kind ? &maps.v64 : &maps.k64;
-      int cursor = 0;
-      for (int t = 0; t < ntiles; ++t) {
-        const uint32_t g = g0 + t, slot = g & 1u, par = (g >> 1) & 1u;
-        int r[4];
-        const bool whole = union_rows(sRunStart, sRunCum, nruns, kvlen, t * KT + orow, h * N, cursor, r);
-        const int what = fetch_plan(r, whole, lane);
-        if (!mbar_wait(bars + (kind ? B_FREEV : B_FREEK) + slot, par, abort_flag)) break;
-        uint64_t* full = bars + (kind ? B_FULLV : B_FULLK) + slot;
-        if (announces) mbar_arrive_expect_tx(full, AT_TILE);
-        fetch_issue(what, base + A2_OFF_SLOT + slot * A2_SLOT + kind * AT_TILE + oblk * (KT * 128), map1, map32, map64,
-                    oblk * 64, r, lane, full);
-      }
-    } else if (warp == 8) {
-      // ================= MMA warp: one lane issues everything, group 0 then group 1 ===============
-      // The lane is the busiest resource of the kernel (an MMA of this shape occupies the tensor pipe
-      // for ~90 cycles and the issue blocks for as long), so it waits for the tiles, which land early,
-      // before it waits for a group's P, and then issues P V and the next Q K^T back to back.
-      if (lane == 0) {
-        bool ok = true;
-        // descriptor low words of the tiles (the K steps add constants to them), one high word for all
-        constexpr uint32_t dhi = sdesc_hi(1024);
-        const uint32_t qlo[2] = {sdesc_lo(base, 16), sdesc_lo(base + AT_TILE, 16)};
-        const uint32_t klo[2] = {sdesc_lo(base + A2_OFF_SLOT, 16), sdesc_lo(base + A2_OFF_SLOT + A2_SLOT, 16)};
-        const uint32_t vlo[2] = {sdesc_lo(base + A2_OFF_SLOT + AT_TILE, KT * 128),
-                                 sdesc_lo(base + A2_OFF_SLOT + A2_SLOT + AT_TILE, KT * 128)};
-        auto mma_qk = [&](int g, uint32_t slot) {      // S_g = Q_g K^T for the K tile in ring slot `slot`
-          const uint32_t a0 = qlo[g], b0 = slot ? klo[1] : klo[0];
-#pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            constexpr uint32_t blk = (QT * 128) >> 4;      // second 64-column block of a tile
-            const uint32_t off = (s >> 2) * blk + (s & 3) * 2;
-            umma_ss_lo(tmem + g * 256, a0 + off, b0 + off, dhi, idescQK, s > 0 ? 1u : 0u);
-          }
-          umma_commit(bars + B_S + g);
-          if (g == 1) umma_commit(bars + B_FREEK + slot);      // covers group 0's MMAs too: same issuer, in order
-        };
-        tc_fence_after();
-        ok = mbar_wait(bars + B_FULLQ + 0, qcnt & 1u, abort_flag) && mbar_wait(bars + B_FULLQ + 1, qcnt & 1u, abort_flag) &&
-             mbar_wait(bars + B_FULLK + (g0 & 1u), (g0 >> 1) & 1u, abort_flag);
-        if (ok) {
-          tc_fence_after();
-          mma_qk(0, g0 & 1u);
-          mma_qk(1, g0 & 1u);
+          for (int i = 0; i < 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (wg == 0) attn_lse[at] = -INFINITY;
         }
-        for (int t = 0; t < ntiles && ok; ++t) {
-          const uint32_t tg = g0 + t, slot = tg & 1u;
-          const bool more = t + 1 < ntiles;
-          const uint32_t v0 = slot ? vlo[1] : vlo[0];
-          if (!mbar_wait(bars + B_FULLV + slot, (tg >> 1) & 1u, abort_flag)) break;
-#pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            const uint32_t tS = tmem + g * 256, tO = tS + 128;
-            // P_g reaches tensor memory in two halves of 64 keys; every P barrier completes once per tile
-            if (!mbar_wait(bars + B_P + g * 2, tg & 1u, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-#pragma unroll
-            for (int s8 = 0; s8 < 4; ++s8)
-              umma_ts_lo(tO, tS + s8 * 8, v0 + s8 * (2048 >> 4), dhi, idescPV, (t > 0 || s8 > 0) ? 1u : 0u);
-            if (!mbar_wait(bars + B_P + g * 2 + 1, tg & 1u, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-#pragma unroll
-            for (int s8 = 4; s8 < 8; ++s8)
-              umma_ts_lo(tO, tS + s8 * 8, v0 + s8 * (2048 >> 4), dhi, idescPV, 1u);
-            umma_commit(bars + B_O + g);
-            if (g == 1) umma_commit(bars + B_FREEV + slot);
-            if (more) {
-              if (g == 0) {      // the next K tile is first needed here
-                if (!mbar_wait(bars + B_FULLK + (slot ^ 1u), ((tg + 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
-                tc_fence_after();
-              }
-              mma_qk(g, slot ^ 1u);
-            }
-          }
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
+        continue;
       }
-    } else if (warp < 8) {
-      // ================= softmax warps: 128 threads per group, one query row each =================
-      const int myoff = grp ? rows0 : 0, myrows = grp ? qrows - rows0 : rows0;
-      const bool warp_has_rows = gw * 32 < myrows;
-      const uint32_t tS = tmem + grp * 256, tO = tS + 128;
-      const uint32_t tS_lane = tmem_addr(tS, gw * 32, 0), tO_lane = tmem_addr(tO, gw * 32, 0);
-      uint64_t* barS = bars + B_S + grp;
-      uint64_t* barO = bars + B_O + grp;
+      // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
+      // whatever S held, which only reaches O rows that are never stored.
+      const bool active = gw * 32 < myrows;
       RowState rs;
       rs.m = -INFINITY;
       rs.l = 0.f;
-      bool dead = false;
-      for (int t = 0; t < ntiles; ++t) {
-        if (!mbar_wait(barS, phS, abort_flag)) { dead = true; break; }
-        phS ^= 1u;
-        if (t > 0) {      // P V of tile t - 1 finished before Q K^T of tile t: this only tracks the phase
-          if (!mbar_wait(barO, phO, abort_flag)) { dead = true; break; }
-          phO ^= 1u;
-        }
+      // this warpgroup's tiles: every other one
+      const int t0 = (int)((wg ^ g) & 1u);
+      uint32_t buf = (g + t0) % 3u;
+      for (int t = t0; t < ntiles; t += 2) {
+        const uint32_t gt = g + t, p = gt - 1u;
+        const uint32_t tS_lane = tmem_addr(tmem + buf * 128, gw * 32, 0);
+        ok = mbar_wait(bars + B_QK + (gt & 3u), (gt >> 2) & 1u, abort_flag);
+        if (!ok) break;
         tc_fence_after();
-        // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
-        // whatever S held, which only reaches O rows that are never stored.
-        auto halfway = [&]() {      // keys 0 .. 63 of P are in tensor memory
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bars + B_P + grp * 2);
-        };
-        if (warp_has_rows) {
+        if (active) {
           const int valid = kvlen - t * KT;
-          if (valid >= KT) softmax_tile<false>(tS_lane, tO_lane, rs, KT, t == 0, sc, halfway);
-          else softmax_tile<true>(tS_lane, tO_lane, rs, valid, t == 0, sc, halfway);
-          tmem_wait_st();
-        } else {
-          halfway();
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bars + B_P + grp * 2 + 1);
-      }
-      if (!dead) {
-        if (!mbar_wait(barO, phO, abort_flag)) dead = true;
-        else phO ^= 1u;
-      }
-      if (!dead) {
-        tc_fence_after();
-        if (warp_has_rows) {
-          const float inv = 1.0f / rs.l;
-          const bool wr = gt < myrows;
-          uint4* dst = reinterpret_cast<uint4*>(attn_out + (rowbase + myoff + gt) * kD);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t v[32];
-            tmem_ld32(tO_lane + c * 32, v);
-            tmem_wait_ld();
-            if (wr) {
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                uint4 o;
-                o.x = pack_bf2(__uint_as_float(v[8 * g + 0]) * inv, __uint_as_float(v[8 * g + 1]) * inv);
-                o.y = pack_bf2(__uint_as_float(v[8 * g + 2]) * inv, __uint_as_float(v[8 * g + 3]) * inv);
-                o.z = pack_bf2(__uint_as_float(v[8 * g + 4]) * inv, __uint_as_float(v[8 * g + 5]) * inv);
-                o.w = pack_bf2(__uint_as_float(v[8 * g + 6]) * inv, __uint_as_float(v[8 * g + 7]) * inv);
-                dst[c * 4 + g] = o;
+          uint32_t v[4][32];
+          // the reference behind tile t - 1, from the thread that weighs it: looked at once before the row is here
+          const unsigned long long* before = sM + (p & 1u) * QT + row;
+          unsigned long long tagged = peek_tagged(before);
+          const float mx = (valid >= KT ? row_scores<false>(tS_lane, KT, v) : row_scores<true>(tS_lane, valid, v)) * sc;
+          if (t == 0) {
+            rs.m = mx;
+          } else {
+            ok = take_tagged(before, p, tagged, abort_flag);
+            if (!ok) break;
+            const float m_in = __uint_as_float((uint32_t)tagged);
+            if (__any_sync(0xffffffffu, m_in != rs.m || mx > m_in + kLazy)) {
+              if (m_in != rs.m) rs.l *= t > 1 ? ex2_approx(rs.m - m_in) : 0.f;
+              rs.m = m_in;
+              const bool grow = mx > rs.m + kLazy;
+              if (__any_sync(0xffffffffu, grow)) {
+                const float mnew = grow ? mx : rs.m;
+                ok = mbar_wait(bars + B_PV + (p & 3u), (p >> 2) & 1u, abort_flag);      // O holds the tiles up to t - 1
+                if (!ok) break;
+                const float alpha = ex2_approx(rs.m - mnew);
+                tc_fence_after();
+                rescale_rows(tO_lane, alpha);
+                rs.l *= alpha;
+                rs.m = mnew;
               }
             }
           }
-          if (wr) attn_lse[rowbase + myoff + gt] = (rs.m + log2f(rs.l)) * 0.6931471805599453f;
+          put_tagged(sM + (gt & 1u) * QT + row, gt, rs.m);
+          row_weights(tS_lane, v, rs, sc, [] {});
+          tmem_wait_st();
         }
         tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_peer(lead + (B_P + buf) * 8);
+        buf = buf ? buf - 1 : 2;      // two on, of three
+      }
+      if (!ok) break;
+      g += ntiles;
+      // both warps of these rows meet: the sums of the two are relative to the maxima they saw last
+      float2* fin = sFin + (q & 1u) * 2 * QT;
+      fin[wg * QT + row] = make_float2(rs.m, rs.l);
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + gw) : "memory");
+      const int lastwg = (g - 1u) & 1u;
+      ok = mbar_wait(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag);
+      if (!ok) break;
+      if (active) {
+        tc_fence_after();
+        const float2 a = fin[lastwg * QT + row], b = fin[(lastwg ^ 1) * QT + row];
+        const float l = ntiles > 1 ? a.y + (b.x != a.x ? b.y * ex2_approx(b.x - a.x) : b.y) : a.y;
+        const float inv = 1.0f / l;
+        uint4* dst = reinterpret_cast<uint4*>(attn_out + at * kD) + wg * 8;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tO_lane + wg * 64 + c * 32, v);
+          tmem_wait_ld();
+          if (wr) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              uint4 o;
+              o.x = pack_bf2(__uint_as_float(v[8 * k + 0]) * inv, __uint_as_float(v[8 * k + 1]) * inv);
+              o.y = pack_bf2(__uint_as_float(v[8 * k + 2]) * inv, __uint_as_float(v[8 * k + 3]) * inv);
+              o.z = pack_bf2(__uint_as_float(v[8 * k + 4]) * inv, __uint_as_float(v[8 * k + 5]) * inv);
+              o.w = pack_bf2(__uint_as_float(v[8 * k + 6]) * inv, __uint_as_float(v[8 * k + 7]) * inv);
+              dst[c * 4 + k] = o;
+            }
+          }
+        }
+        if (wr && wg == 0) attn_lse[at] = (a.x + log2f(l)) * 0.6931471805599453f;
+      }
+      ++q;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive_peer(lead + B_OFREE * 8);
+        mbar_arrive_peer(tfree + sl * 8);
       }
     }
-    tiles_done += ntiles;
-    ++qcnt;
+  } else {
+    give_registers();
+    if (warp == 9 && rank == 1) {
+      // ================= the next task and the run list of its union, one task ahead =================
+      const PlanView pv = plan_view(plan, H, N, CQ);
+      const int numTasks = pv.counters[0];
+      for (uint32_t n = 0;; ++n) {
+        const uint32_t sl = n & 1u;
+        TaskSlot* slot = ring + sl;
+        if (!mbar_wait(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
+        int task = 0;
+        if (lane == 0) {
+          do { task = atomicAdd(&pv.counters[4], 1); } while (task < numTasks && pv.tasks[task].w <= QT);
+          task = min(task, numTasks);
+        }
+        task = __shfl_sync(0xffffffffu, task, 0);
+        int* runs = sRuns + sl * RUN_INTS;
+        prepare_task(pv, ub, CQ, numTasks, task, slot, runs, runs + MAX_RUNS, abort_flag, status);
+        // the same for the leader
+        const bool end = slot->end;
+        const uint32_t there = cluster_addr(smem_u32(runs), 0);
+        if (!end && slot->kvlen > 0)
+          for (int i = lane; i <= slot->runs; i += 32) {
+            cluster_store(there + i * 4, runs[i]);
+            cluster_store(there + (MAX_RUNS + i) * 4, runs[MAX_RUNS + i]);
+          }
+        if (lane < 6) cluster_store(cluster_addr(smem_u32(slot), 0) + lane * 4, reinterpret_cast<const int*>(slot)[lane]);
+        __syncwarp();
+        if (lane == 0) {
+          mbar_release_peer(cluster_addr(smem_u32(bars + B_TFULL + sl), 0));
+          mbar_arrive(bars + B_TFULL + sl);
+        }
+        if (end) break;
+      }
+    } else if (warp >= 10) {
+      // ================= copy warps =================
+      const int kind = warp >= 13, cw = warp - 10 - 3 * kind;      // 0: K and Q, 1: V; turn of the three
+      // K: rows 64 rank .. of the tile, both 64-column blocks (half a warp each); V: all rows, block `rank`
+      const int seg = kind ? 32 : 16, prow = kind ? lane * 4 : (int)rank * 64 + (lane & 15) * 4;
+      const int col = kind ? (int)rank * 64 : (lane >> 4) * 64;
+      const uint32_t off = base + (kind ? A2_OFF_V + lane * 512 : A2_OFF_K + (lane >> 4) * (A2_HALF / 2) + (lane & 15) * 512);
+      const CUtensorMap* map1 = kind ? &maps.v1 : &maps.k1;
+      const CUtensorMap* map32 = kind ? &maps.v32 : &maps.k32;
+      const CUtensorMap* map64 = kind ? &maps.v64 : &maps.k64;
+      const int bfull = kind ? B_FULLV : B_FULLK;
+      uint32_t g = 0, q = 0;      // tiles, tasks with tiles so far
+      int turn = 0;               // warp of tile g
+      bool ok = true;
+      for (uint32_t n = 0;; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const TaskSlot tk = ring[sl];
+        if (tk.end) break;
+        const int* sRunStart = sRuns + sl * RUN_INTS;
+        const int* sRunCum = sRunStart + MAX_RUNS;
+        const int ntiles = cdiv(tk.kvlen, KT);
+        if (ntiles > 0 && kind == 0 && cw < 2) {
+          // one 64-column block of the Q tile each; slots past the group repeat its first row
+          const int rows0 = group_rows(tk.rows), skip = rank ? rows0 : 0, nr = rank ? tk.rows - rows0 : rows0;
+          const size_t rowbase = (size_t)tk.head * N + tk.first + skip;
+          int r[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            r[j] = tk.head * q_head_step + qperm[rowbase + (lane * 4 + j < nr ? lane * 4 + j : 0)] * q_row_step;
+          ok = mbar_wait(bars + B_FREEQ + (q & 1u), ((q >> 1) & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          const uint32_t full = lead + (B_FULLQ + (q & 1u)) * 8;
+          if (lane == 0) {
+            if (rank == 0 && cw == 0) mbar_arrive_expect_tx(bars + B_FULLQ + (q & 1u), 2 * AT_TILE);
+            else mbar_arrive_peer(full);
+          }
+          __syncwarp();
+          tma_gather4_pair(base + (q & 1u) * AT_TILE + cw * (KT * 128) + lane * 512, &mapQ, cw * 64, r[0], r[1], r[2],
+                           r[3], full);
+        }
+        int cursor = 0;
+        for (int t = 0; t < ntiles; ++t, ++g) {
+          if (turn != cw) { turn = turn == 2 ? 0 : turn + 1; continue; }
+          turn = turn == 2 ? 0 : turn + 1;
+          int r[4];
+          const bool whole = union_rows(sRunStart, sRunCum, tk.runs, tk.kvlen, t * KT + prow, tk.head * N, cursor, r);
+          const int what = fetch_plan(r, whole, lane, seg);
+          const uint32_t slot = g & 3u;
+          ok = g < 4u || mbar_wait(bars + (kind ? B_PV : B_QK) + slot, ((g - 4u) >> 2) & 1u, abort_flag);
+          if (!ok) break;
+          const uint32_t full = lead + (bfull + slot) * 8;
+          if (lane == 0) {
+            if (rank == 0) mbar_arrive_expect_tx(bars + bfull + slot, 2 * A2_HALF);
+            else mbar_arrive_peer(full);
+          }
+          const uint32_t dst = off + slot * A2_HALF;
+          if (what == FETCH_GATHER) tma_gather4_pair(dst, map1, col, r[0], r[1], r[2], r[3], full);
+          else if (what == FETCH_BOX32) tma_load_tile_pair(dst, map32, col, r[0], full);
+          else if (what == FETCH_BOX64) tma_load_tile_pair(dst, map64, col, r[0], full);
+        }
+        if (!ok) break;
+        if (ntiles > 0) ++q;
+        __syncwarp();
+        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
+      }
+    } else if (warp == 8 && rank == 0) {
+      // ================= Q K^T: waits for the K tile and for P V to have read the score buffer =================
+      constexpr uint32_t idescQK = make_idesc_bf16(256, KT, false, false);
+      constexpr uint32_t dhi = sdesc_hi(1024);
+      const uint32_t qlo = sdesc_lo(base, 16), klo = sdesc_lo(base + A2_OFF_K, 16);
+      uint32_t g = 0, q = 0, tS = tmem;      // tiles, tasks with tiles, score buffer of the next tile
+      bool ok = true;
+      for (uint32_t n = 0; ok; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
+        __syncwarp();
+        if (end) break;
+        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
+        if (ntiles == 0) continue;
+        if (!mbar_wait(bars + B_FULLQ + (q & 1u), (q >> 1) & 1u, abort_flag)) break;
+        const uint32_t a0 = qlo + (q & 1u) * (AT_TILE >> 4);
+        for (int t = 0; t < ntiles; ++t, ++g) {
+          const uint32_t slot = g & 3u, b0 = klo + slot * (A2_HALF >> 4);
+          ok = mbar_wait(bars + B_FULLK + slot, (g >> 2) & 1u, abort_flag) &&
+               (g < 3u || mbar_wait(bars + B_PV + ((g - 3u) & 3u), ((g - 3u) >> 2) & 1u, abort_flag));
+          if (!ok) break;
+          tc_fence_after();
+          __syncwarp();
+          if (elect_one()) {
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+              umma_ss_pair(tS, a0 + (s >> 2) * ((QT * 128) >> 4) + (s & 3) * 2,
+                           b0 + (s >> 2) * ((A2_HALF / 2) >> 4) + (s & 3) * 2, dhi, idescQK, s > 0 ? 1u : 0u);
+            umma_commit_pair(bars + B_QK + slot);
+            if (t + 1 == ntiles) umma_commit_pair(bars + B_FREEQ + (q & 1u));
+          }
+          __syncwarp();
+          tS = tS == tmem + 256 ? tmem : tS + 128;
+        }
+        ++q;
+      }
+    } else if (warp == 9) {
+      // ================= P V =================
+      constexpr uint32_t idescPV = make_idesc_bf16(256, kD, false, true);
+      constexpr uint32_t dhi = sdesc_hi(1024);
+      const uint32_t vlo = sdesc_lo(base + A2_OFF_V, A2_HALF);
+      const uint32_t tO = tmem + 3 * 128;
+      uint32_t g = 0, q = 0, buf = 0, bph = 0;      // tiles, tasks with tiles, score buffer of the next tile and its phase
+      bool ok = true;
+      for (uint32_t n = 0; ok; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
+        __syncwarp();
+        if (end) break;
+        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
+        if (ntiles == 0) continue;
+        // every softmax warp has read the O of the task before
+        if (!mbar_wait(bars + B_OFREE, (q & 1u) ^ 1u, abort_flag)) break;
+        for (int t = 0; t < ntiles; ++t, ++g) {
+          const uint32_t slot = g & 3u, v0 = vlo + slot * (A2_HALF >> 4), tS = tmem + buf * 128, add = t > 0 ? 1u : 0u;
+          ok = mbar_wait(bars + B_FULLV + slot, (g >> 2) & 1u, abort_flag) &&
+               mbar_wait(bars + B_P + buf, bph, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          __syncwarp();
+          if (elect_one()) {
+#pragma unroll
+            for (int s8 = 0; s8 < 8; ++s8)
+              umma_ts_pair(tO, tS + s8 * 8, v0 + s8 * (2048 >> 4), dhi, idescPV, s8 > 0 ? 1u : add);
+            umma_commit_pair(bars + B_PV + slot);
+          }
+          __syncwarp();
+          if (++buf == 3) { buf = 0; bph ^= 1u; }
+        }
+        ++q;
+      }
+    }
   }
+  __syncwarp();
   if (*abort_flag) {
     if (tid == 0 && status) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
     // a wait gave up: let tile copies still in flight land before the shared memory is released
@@ -796,7 +1025,8 @@ __global__ void __launch_bounds__(A2_THREADS, 1) attn2_kernel(
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  cluster_sync();      // the other CTA no longer arrives here, and both are done with tensor memory
+  if (warp == 0) tmem_dealloc_pair(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -806,38 +1036,38 @@ __global__ void __launch_bounds__(A2_THREADS, 1) attn2_kernel(
 // (256 tensor-memory columns and 110 KB of shared memory each) so that one CTA's softmax runs under the
 // other's loads and products:
 //   warps 0..3   softmax, one thread per query row
-//   warp 4       one lane issues every MMA
+//   warp 4       issues every MMA (see elect_one)
 //   warps 5..7   the K and V tiles (and the task's Q tile) by TMA (see fetch_plan).  A TMA instruction holds
 //                its warp for about 70 cycles per lane, which threads that also compute cannot afford, and
 //                one warp alone would need longer for a K tile than the softmax takes.
-// Fill g of the K (V) buffer, g counting the tiles this CTA has processed, waits for phase g of freeK (freeV) -
-// phase 0 is completed at start-up, phase g by the commit behind the product that read fill g - 1 - and
-// completes phase g of fullK (fullV).
+// Fill g of the K (V) buffer, g counting the tiles this CTA has processed, waits for the commit behind the product that
+// read fill g - 1, phase g - 1 of C_S (C_PV), and completes phase g of fullK (fullV).  A commit costs the tensor pipe about
+// 100 cycles, so these two are all there are: C_S also says that a task's Q tile is free, C_PV that its O is complete.
 constexpr int A1_THREADS = 8 * 32;
 constexpr int A1_OFF_MISC = 3 * AT_TILE;                  // Q, K, V tiles
-constexpr int A1_SMEM_INTS = 2 * MAX_RUNS + 8 + 32;
-constexpr int A1_SMEM = A1_OFF_MISC + 256 + A1_SMEM_INTS * 4 + 1024;
-enum { C_S = 0, C_O = 1, C_P = 2, C_FULLK = 4, C_FULLV, C_FREEK, C_FREEV, C_FULLQ, C_COUNT };      // P: [half]
+constexpr int A1_SMEM = A1_OFF_MISC + 256 + 2 * (int)sizeof(TaskSlot) + 2 * RUN_INTS * 4;
+enum { C_S = 0, C_PV = 1, C_P = 2, C_FULLK = 4, C_FULLV, C_FULLQ, C_TFULL, C_TFREE = C_TFULL + 2,
+       C_COUNT = C_TFREE + 2 };      // P: [half]; TFULL / TFREE: the task ring
+constexpr int A1_CONSUMERS = 4 + 1 + 3;                   // warps that read a task: softmax, MMA, copy
 static_assert(2 * (A1_SMEM + 1024) <= 228 * 1024, "two CTAs share an SM");
+static_assert(C_COUNT * 8 + 16 <= 256, "the barriers fit their area");
 
 __global__ void __launch_bounds__(A1_THREADS, 2) attn_kernel(
     const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ KVMaps maps,
     const uint32_t* __restrict__ ub, const int* __restrict__ qperm,
     __nv_bfloat16* __restrict__ attn_out, float* __restrict__ attn_lse, int* __restrict__ plan, int H, int N, int CQ,
     int q_row_step, int q_head_step, int* __restrict__ status) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
+  // the second run list leaves no room for aligning the tiles by hand
+  extern __shared__ __align__(1024) uint8_t smem_tiles[];
+  uint8_t* sm = smem_tiles;
+  const uint32_t base = smem_u32(sm);
   const uint32_t sQ = base, sK = base + AT_TILE, sV = base + 2 * AT_TILE;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + A1_OFF_MISC);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + A1_OFF_MISC + C_COUNT * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + A1_OFF_MISC + C_COUNT * 8 + 8);
-  int* sInt = reinterpret_cast<int*>(sm + A1_OFF_MISC + 256);
-  int* sRunStart = sInt;                          // [MAX_RUNS]
-  int* sRunCum = sRunStart + MAX_RUNS;            // [MAX_RUNS + 1]
-  int* sMisc = sRunCum + MAX_RUNS + 8;            // [1] runs; [2..7] the next task: index, head, cluster, first row, rows, union length
+  TaskSlot* ring = reinterpret_cast<TaskSlot*>(sm + A1_OFF_MISC + 256);
+  int* sRuns = reinterpret_cast<int*>(ring + 2);
 
-  const PlanView pv = plan_view(plan, H, N, CQ);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
@@ -845,105 +1075,127 @@ __global__ void __launch_bounds__(A1_THREADS, 2) attn_kernel(
     tmem_relinquish();
   }
   if (tid == 0) {
-    *abort_flag = 0;
-    for (int i = 0; i < C_COUNT; ++i)
-      mbar_init(bars + i, (i == C_P || i == C_P + 1) ? 4 : ((i == C_FULLK || i == C_FULLV) ? 3 : 1));
+    *abort_flag = base & 1023u ? 1 : 0;
+    for (int i = 0; i < C_COUNT; ++i) {
+      int count = 1;
+      if (i == C_P || i == C_P + 1) count = 4;
+      else if (i == C_FULLK || i == C_FULLV) count = 3;
+      else if (i == C_FULLQ) count = 2;
+      else if (i >= C_TFREE) count = A1_CONSUMERS;
+      mbar_init(bars + i, count);
+    }
     mbar_init_fence();
-    mbar_arrive(bars + C_FREEK);      // both buffers start empty
-    mbar_arrive(bars + C_FREEV);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t tS = tmem, tO = tmem + 128;
-  uint32_t tiles_done = 0, qcnt = 0;      // tiles / non-empty tasks this CTA has processed; every role counts alike
-  uint32_t phS = 0, phO = 0;              // softmax warps: phases of the S and O barriers
-  const int numTasks = pv.counters[0];
-  const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
-  constexpr uint32_t idescQK = make_idesc_bf16(128, KT, false, false);
-  constexpr uint32_t idescPV = make_idesc_bf16(128, kD, false, true);
 
-  // The next task of at most QT rows (the two-tile kernel takes the others) is fetched - cursor, task record,
-  // union length: three dependent trips to global memory - by a copy warp once it has issued the current
-  // task's last tile, while the other roles are still busy with it.
-  auto fetch_task = [&]() {
-    int i;
-    do { i = atomicAdd(&pv.counters[1], 1); } while (i < numTasks && pv.tasks[i].w > QT);
-    int4 tk = make_int4(0, 0, 0, 0);
-    int len = 0;
-    if (i < numTasks) {
-      tk = pv.tasks[i];
-      len = pv.kv_lens[(size_t)tk.x * CQ + tk.y];
+  if (*abort_flag) {
+    // misaligned tiles: nothing starts
+  } else if (warp < 4) {
+    // ================= softmax warps: one query row per thread =================
+    take_registers();
+    const uint32_t tS_lane = tmem_addr(tS, warp * 32, 0), tO_lane = tmem_addr(tO, warp * 32, 0);
+    uint32_t g = 0;      // tiles so far
+    for (uint32_t n = 0;; ++n) {
+      const uint32_t sl = n & 1u;
+      if (!mbar_wait(bars + C_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+      const TaskSlot tk = ring[sl];
+      if (tk.end) break;
+      const size_t at = (size_t)tk.head * N + tk.first + (tid < tk.rows ? tid : 0);
+      if (!softmax_task(tS_lane, tO_lane, bars + C_S, bars + C_PV, bars + C_P, g, tk.kvlen, warp * 32 < tk.rows,
+                        tid < tk.rows, attn_out + at * kD, attn_lse + at, abort_flag))
+        break;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + C_TFREE + sl);
     }
-    sMisc[2] = i; sMisc[3] = tk.x; sMisc[4] = tk.y; sMisc[5] = tk.z; sMisc[6] = tk.w; sMisc[7] = len;
-  };
-  if (warp == 7 && lane == 0) fetch_task();
-
-  while (true) {
-    __syncthreads();
-    const int ti = sMisc[2], h = sMisc[3], qc = sMisc[4], qs = sMisc[5], qrows = sMisc[6], kvlen = sMisc[7];
-    __syncthreads();      // everyone has the task: the record may be overwritten
-    if (ti >= numTasks || *abort_flag) break;
-    const size_t rowbase = (size_t)h * N + qs;
-
-    if (kvlen == 0) {   // empty union: O = 0, lse = -inf
-      if (warp == 7 && lane == 0) fetch_task();
-      for (int i = tid; i < qrows * 16; i += A1_THREADS)
-        reinterpret_cast<uint4*>(attn_out + (rowbase + (i >> 4)) * kD)[i & 15] = make_uint4(0u, 0u, 0u, 0u);
-      for (int r = tid; r < qrows; r += A1_THREADS) attn_lse[rowbase + r] = -INFINITY;
-      continue;
-    }
-    if (warp == 5) {      // the task's Q tile needs no run list: its gathers go first; slots past the task repeat its first row
-      const int orow = lane * 4;
-      int r[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        r[j] = h * q_head_step + qperm[rowbase + (orow + j < qrows ? orow + j : 0)] * q_row_step;
-      if (lane == 0) mbar_arrive_expect_tx(bars + C_FULLQ, AT_TILE);
-      tma_gather4(sQ + orow * 128, &mapQ, 0, r[0], r[1], r[2], r[3], bars + C_FULLQ);
-      tma_gather4(sQ + KT * 128 + orow * 128, &mapQ, 64, r[0], r[1], r[2], r[3], bars + C_FULLQ);
-    }
-
-    if (!build_runs(pv.k_off + (size_t)h * (kC + 1), ub + ((size_t)h * CQ + qc) * (kC / 32),
-                    pv.nonempty + (size_t)h * (kC / 32), sRunStart, sRunCum, sMisc, abort_flag, status))
-      break;
-    const int nruns = sMisc[1];
-    const int ntiles = cdiv(kvlen, KT);
-    const uint32_t g0 = tiles_done;
-
+  } else {
+    give_registers();
     if (warp >= 5) {
       // ================= copy warps =================
       // K and V tiles hold the same rows, so one fetch plan serves both tiles and both of their 64-column
       // blocks; the three warps share its instructions (the n-th issuing lane belongs to warp n mod 3), K
-      // first: the next Q K^T waits for it.
+      // first: the next Q K^T waits for it.  Warp 7 also prepares the next task, behind its share of the second tile.
+      const PlanView pv = plan_view(plan, H, N, CQ);
+      const int numTasks = pv.counters[0];
       const int cw = warp - 5, orow = lane * 4;
-      int cursor = 0;
-      for (int t = 0; t < ntiles; ++t) {
-        const uint32_t g = g0 + t;
-        int r[4];
-        const bool whole = union_rows(sRunStart, sRunCum, nruns, kvlen, t * KT + orow, h * N, cursor, r);
-        int what = fetch_plan(r, whole, lane);
-        const unsigned issuing = __ballot_sync(0xffffffffu, what != FETCH_NONE);
-        if (__popc(issuing & ((1u << lane) - 1u)) % 3 != cw) what = FETCH_NONE;
-        if (!mbar_wait(bars + C_FREEK, g & 1u, abort_flag)) break;
-        // every copy warp arrives on the full barrier, so that none of them can fall two phases behind the
-        // free barrier it waits on (a warp may have nothing to fetch for a tile)
-        if (lane == 0) { if (cw == 0) mbar_arrive_expect_tx(bars + C_FULLK, AT_TILE); else mbar_arrive(bars + C_FULLK); }
-        fetch_issue(what, sK, &maps.k1, &maps.k32, &maps.k64, 0, r, lane, bars + C_FULLK);
-        fetch_issue(what, sK + KT * 128, &maps.k1, &maps.k32, &maps.k64, 64, r, lane, bars + C_FULLK);
-        if (!mbar_wait(bars + C_FREEV, g & 1u, abort_flag)) break;
-        if (lane == 0) { if (cw == 0) mbar_arrive_expect_tx(bars + C_FULLV, AT_TILE); else mbar_arrive(bars + C_FULLV); }
-        fetch_issue(what, sV, &maps.v1, &maps.v32, &maps.v64, 0, r, lane, bars + C_FULLV);
-        fetch_issue(what, sV + KT * 128, &maps.v1, &maps.v32, &maps.v64, 64, r, lane, bars + C_FULLV);
+      auto prepare = [&](uint32_t n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait(bars + C_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) return false;
+        int task = 0;
+        if (lane == 0) {
+          do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > QT);
+          task = min(task, numTasks);
+        }
+        task = __shfl_sync(0xffffffffu, task, 0);
+        prepare_task(pv, ub, CQ, numTasks, task, ring + sl, sRuns + sl * RUN_INTS, sRuns + sl * RUN_INTS + MAX_RUNS,
+                            abort_flag, status);
+        if (lane == 0) mbar_arrive(bars + C_TFULL + sl);
+        return true;
+      };
+      uint32_t g = 0;      // tiles so far; every role counts alike
+      bool ok = cw < 2 || prepare(0);
+      for (uint32_t n = 0; ok; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait(bars + C_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const TaskSlot tk = ring[sl];
+        if (tk.end) break;
+        const int* sRunStart = sRuns + sl * RUN_INTS;
+        const int* sRunCum = sRunStart + MAX_RUNS;
+        const int ntiles = cdiv(tk.kvlen, KT);
+        if (ntiles > 0 && cw < 2) {      // one 64-column block of the Q tile each; slots past the task repeat its first row
+          const size_t rowbase = (size_t)tk.head * N + tk.first;
+          int r[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            r[j] = tk.head * q_head_step + qperm[rowbase + (orow + j < tk.rows ? orow + j : 0)] * q_row_step;
+          ok = mbar_wait(bars + C_S, (g & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          if (lane == 0) mbar_arrive_expect_tx(bars + C_FULLQ, AT_TILE / 2);
+          __syncwarp();
+          tma_gather4(sQ + cw * (KT * 128) + orow * 128, &mapQ, cw * 64, r[0], r[1], r[2], r[3], bars + C_FULLQ);
+        }
+        int cursor = 0;
+        for (int t = 0; t < ntiles; ++t, ++g) {
+          int r[4];
+          const bool whole = union_rows(sRunStart, sRunCum, tk.runs, tk.kvlen, t * KT + orow, tk.head * N, cursor, r);
+          int what = fetch_plan(r, whole, lane, 32);
+          const unsigned issuing = __ballot_sync(0xffffffffu, what != FETCH_NONE);
+          if (__popc(issuing & ((1u << lane) - 1u)) % 3 != cw) what = FETCH_NONE;
+          ok = mbar_wait(bars + C_S, (g & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          // every copy warp arrives on the full barrier, so that none of them can fall two phases behind the
+          // free barrier it waits on (a warp may have nothing to fetch for a tile)
+          if (lane == 0) { if (cw == 0) mbar_arrive_expect_tx(bars + C_FULLK, AT_TILE); else mbar_arrive(bars + C_FULLK); }
+          fetch_issue(what, sK, &maps.k1, &maps.k32, &maps.k64, 0, r, lane, bars + C_FULLK);
+          fetch_issue(what, sK + KT * 128, &maps.k1, &maps.k32, &maps.k64, 64, r, lane, bars + C_FULLK);
+          ok = mbar_wait(bars + C_PV, (g & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          if (lane == 0) { if (cw == 0) mbar_arrive_expect_tx(bars + C_FULLV, AT_TILE); else mbar_arrive(bars + C_FULLV); }
+          fetch_issue(what, sV, &maps.v1, &maps.v32, &maps.v64, 0, r, lane, bars + C_FULLV);
+          fetch_issue(what, sV + KT * 128, &maps.v1, &maps.v32, &maps.v64, 64, r, lane, bars + C_FULLV);
+          if (cw == 2 && t == min(1, ntiles - 1)) {
+            __syncwarp();
+            ok = prepare(n + 1);
+            if (!ok) break;
+          }
+        }
+        if (!ok) break;
+        if (ntiles == 0 && cw == 2) ok = prepare(n + 1);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars + C_TFREE + sl);
       }
-      if (warp == 7 && lane == 0) fetch_task();
-    } else if (warp == 4) {
-      // ================= MMA warp: one lane issues everything =================
-      if (lane == 0) {
-        constexpr uint32_t dhi = sdesc_hi(1024);
-        const uint32_t qlo = sdesc_lo(sQ, 16), klo = sdesc_lo(sK, 16), vlo = sdesc_lo(sV, KT * 128);
-        auto mma_qk = [&]() {      // S = Q K^T; its completion also frees the K buffer
+    } else {
+      // ================= MMA warp =================
+      constexpr uint32_t idescQK = make_idesc_bf16(128, KT, false, false);
+      constexpr uint32_t idescPV = make_idesc_bf16(128, kD, false, true);
+      constexpr uint32_t dhi = sdesc_hi(1024);
+      const uint32_t qlo = sdesc_lo(sQ, 16), klo = sdesc_lo(sK, 16), vlo = sdesc_lo(sV, KT * 128);
+      auto mma_qk = [&]() {      // S = Q K^T
+        __syncwarp();
+        if (elect_one()) {
 #pragma unroll
           for (int s = 0; s < 8; ++s) {
             constexpr uint32_t blk = (QT * 128) >> 4;      // second 64-column block of a tile
@@ -951,109 +1203,61 @@ __global__ void __launch_bounds__(A1_THREADS, 2) attn_kernel(
             umma_ss_lo(tS, qlo + off, klo + off, dhi, idescQK, s > 0 ? 1u : 0u);
           }
           umma_commit(bars + C_S);
-          umma_commit(bars + C_FREEK);
-        };
-        tc_fence_after();
-        bool ok = mbar_wait(bars + C_FULLQ, qcnt & 1u, abort_flag) && mbar_wait(bars + C_FULLK, g0 & 1u, abort_flag);
-        if (ok) {
-          tc_fence_after();
-          mma_qk();
         }
+        __syncwarp();
+      };
+      uint32_t g0 = 0, q = 0;
+      bool ok = true;
+      for (uint32_t n = 0; ok; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait(bars + C_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (ring[sl].end) break;
+        const int ntiles = cdiv(ring[sl].kvlen, KT);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars + C_TFREE + sl);
+        if (ntiles == 0) continue;
+        ok = mbar_wait(bars + C_FULLQ, q & 1u, abort_flag) && mbar_wait(bars + C_FULLK, g0 & 1u, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        mma_qk();
         for (int t = 0; t < ntiles && ok; ++t) {
           const uint32_t tg = g0 + t;
           const bool more = t + 1 < ntiles;
+          ok = false;
           if (!mbar_wait(bars + C_FULLV, tg & 1u, abort_flag)) break;
           // P reaches tensor memory in two halves of 64 keys; both P barriers complete once per tile
           if (!mbar_wait(bars + C_P, tg & 1u, abort_flag)) break;
           tc_fence_after();
+          const uint32_t first = t > 0 ? 1u : 0u;
+          __syncwarp();
+          if (elect_one()) {
 #pragma unroll
-          for (int s8 = 0; s8 < 4; ++s8)
-            umma_ts_lo(tO, tS + s8 * 8, vlo + s8 * (2048 >> 4), dhi, idescPV, (t > 0 || s8 > 0) ? 1u : 0u);
+            for (int s8 = 0; s8 < 4; ++s8)
+              umma_ts_lo(tO, tS + s8 * 8, vlo + s8 * (2048 >> 4), dhi, idescPV, s8 > 0 ? 1u : first);
+          }
+          __syncwarp();
           if (!mbar_wait(bars + C_P + 1, tg & 1u, abort_flag)) break;
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int s8 = 4; s8 < 8; ++s8)
-            umma_ts_lo(tO, tS + s8 * 8, vlo + s8 * (2048 >> 4), dhi, idescPV, 1u);
-          umma_commit(bars + C_O);
-          umma_commit(bars + C_FREEV);
+            for (int s8 = 4; s8 < 8; ++s8)
+              umma_ts_lo(tO, tS + s8 * 8, vlo + s8 * (2048 >> 4), dhi, idescPV, 1u);
+            umma_commit(bars + C_PV);
+          }
+          __syncwarp();
           if (more) {
             if (!mbar_wait(bars + C_FULLK, (tg + 1) & 1u, abort_flag)) break;
             tc_fence_after();
             mma_qk();
           }
+          ok = true;
         }
-      }
-    } else {
-      // ================= softmax warps: one query row per thread =================
-      const bool warp_has_rows = warp * 32 < qrows;
-      const uint32_t tS_lane = tmem_addr(tS, warp * 32, 0), tO_lane = tmem_addr(tO, warp * 32, 0);
-      RowState rs;
-      rs.m = -INFINITY;
-      rs.l = 0.f;
-      bool dead = false;
-      for (int t = 0; t < ntiles; ++t) {
-        if (!mbar_wait(bars + C_S, phS, abort_flag)) { dead = true; break; }
-        phS ^= 1u;
-        if (t > 0) {      // P V of tile t - 1 finished before Q K^T of tile t: this only tracks the phase
-          if (!mbar_wait(bars + C_O, phO, abort_flag)) { dead = true; break; }
-          phO ^= 1u;
-        }
-        tc_fence_after();
-        // A warp whose rows all lie past the task's last row skips the arithmetic: its P rows stay whatever S
-        // held, which only reaches O rows that are never stored.
-        auto halfway = [&]() {      // keys 0 .. 63 of P are in tensor memory
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bars + C_P);
-        };
-        if (warp_has_rows) {
-          const int valid = kvlen - t * KT;
-          if (valid >= KT) softmax_tile<false>(tS_lane, tO_lane, rs, KT, t == 0, sc, halfway);
-          else softmax_tile<true>(tS_lane, tO_lane, rs, valid, t == 0, sc, halfway);
-          tmem_wait_st();
-        } else {
-          halfway();
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bars + C_P + 1);
-      }
-      if (!dead) {
-        if (!mbar_wait(bars + C_O, phO, abort_flag)) dead = true;
-        else phO ^= 1u;
-      }
-      if (!dead) {
-        tc_fence_after();
-        if (warp_has_rows) {
-          const float inv = 1.0f / rs.l;
-          const bool wr = tid < qrows;
-          uint4* dst = reinterpret_cast<uint4*>(attn_out + (rowbase + tid) * kD);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t v[32];
-            tmem_ld32(tO_lane + c * 32, v);
-            tmem_wait_ld();
-            if (wr) {
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                uint4 o;
-                o.x = pack_bf2(__uint_as_float(v[8 * g + 0]) * inv, __uint_as_float(v[8 * g + 1]) * inv);
-                o.y = pack_bf2(__uint_as_float(v[8 * g + 2]) * inv, __uint_as_float(v[8 * g + 3]) * inv);
-                o.z = pack_bf2(__uint_as_float(v[8 * g + 4]) * inv, __uint_as_float(v[8 * g + 5]) * inv);
-                o.w = pack_bf2(__uint_as_float(v[8 * g + 6]) * inv, __uint_as_float(v[8 * g + 7]) * inv);
-                dst[c * 4 + g] = o;
-              }
-            }
-          }
-          if (wr) attn_lse[rowbase + tid] = (rs.m + log2f(rs.l)) * 0.6931471805599453f;
-        }
-        tc_fence_before();
+        g0 += ntiles;
+        ++q;
       }
     }
-    tiles_done += ntiles;
-    ++qcnt;
   }
+  __syncwarp();
   if (*abort_flag) {
     if (tid == 0 && status) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
     // a wait gave up: let tile copies still in flight land before the shared memory is released
@@ -1516,7 +1720,7 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
       !cached_row_map(&kv.v64, vp, rows, 64))
     return T2T_ERR_CUDA;
   // tasks above 128 rows first (one CTA per SM, two row tiles per K/V stream), then the others
-  attn2_kernel<<<sms, A2_THREADS, A2_SMEM, st>>>(mq, kv, (const uint32_t*)unip, (const int*)qperm, attn_out,
+  attn2_kernel<<<sms & ~1, A2_THREADS, A2_SMEM, st>>>(mq, kv, (const uint32_t*)unip, (const int*)qperm, attn_out,
                                                  attn_lse, plan, H, N, CQ, q_row_step, q_head_step, d_status);
   // The two kernels take disjoint tasks (own cursors, own output rows), so the second may start while the
   // first drains: it is launched with programmatic stream serialization and the first kernel releases its
