@@ -201,12 +201,14 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
     *reinterpret_cast<uint4*>(stage + sw128(tid, 4)) = make_uint4(hi | (mid << 16), lo, 0u, 0u);
   };
   constexpr uint32_t idesc = make_idesc_bf16(128, TA_CH, false, false);
-  auto issue = [&](int st, uint32_t tmem) {     // one thread
+  auto issue = [&](int st, uint32_t tmem) {     // one warp (see elect_one)
+    const uint32_t a0 = sdesc_lo(sA, 16), b0 = sdesc_lo(sB + st * TA_SB, 16);
+    if (elect_one()) {
 #pragma unroll
-    for (int s2 = 0; s2 < 3; ++s2)
-      umma_ss(tmem, make_sdesc(sA + s2 * 32, 16, 1024), make_sdesc(sB + st * TA_SB + s2 * 32, 16, 1024), idesc,
-              s2 > 0 ? 1u : 0u);
-    umma_commit(bar);
+      for (int s2 = 0; s2 < 3; ++s2) umma_ss_lo(tmem, a0 + s2 * 2, b0 + s2 * 2, sdesc_hi(1024), idesc, s2 > 0 ? 1u : 0u);
+      umma_commit(bar);
+    }
+    __syncwarp();
   };
 
   const int nch = cdiv(Cn, TA_CH);
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t t_lane = tmem_addr(tmem, warp * 32, 0);
-  if (tid == 0) issue(0, tmem);
+  if (warp == 0) issue(0, tmem);
 
   Best b;
   b.m1 = b.m2 = b.m3 = -INFINITY;
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
     }
     tc_fence_before();
     __syncthreads();              // every row has read the scores, the next chunk's rows are complete
-    if (tid == 0 && i + 1 < nch) {
+    if (warp == 0 && i + 1 < nch) {
       tc_fence_after();
       issue((i + 1) & 1, tmem);
     }
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0) {
           tc_fence_after();
           issue(st, tmem);
         }

@@ -270,26 +270,30 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   // Streams this group's eight chunks through its two TMEM buffers: the MMA of
   // chunk i + 1 runs while chunk i is scanned.  body(cbase, v) sees 32
   // consecutive approximate scores of this thread's row.
-  auto issue = [&](int i) {        // called by the group's first thread
+  const uint32_t alo0 = sdesc_lo(sA, 16), clo0 = sdesc_lo(sCk, 16);
+  auto issue = [&](int i) {        // called by the group's first warp (see elect_one)
     const int cc = g + ST_G * i, b = i & 1;
+    const uint32_t a0 = alo0 + half * 4;
+    const uint32_t c0 = clo0 + (cc & (ST_NCH / 2 - 1)) * ((ST_CH * 128) >> 4) + cc / (ST_NCH / 2) * 4;
+    const uint32_t d = tmem + g * 2 * ST_CH + b * ST_CH;
     tc_fence_after();
+    if (elect_one()) {
 #pragma unroll
-    for (int s2 = 0; s2 < 2; ++s2)
-      umma_ss(tmem + g * 2 * ST_CH + b * ST_CH, make_sdesc(sA + half * 64 + s2 * 32, 16, 1024),
-              make_sdesc(sCk + (cc & (ST_NCH / 2 - 1)) * (ST_CH * 128) + cc / (ST_NCH / 2) * 64 + s2 * 32, 16, 1024), idesc,
-              s2 > 0 ? 1u : 0u);
-    umma_commit(bars + g * 2 + b);
+      for (int s2 = 0; s2 < 2; ++s2) umma_ss_lo(d, a0 + s2 * 2, c0 + s2 * 2, sdesc_hi(1024), idesc, s2 > 0 ? 1u : 0u);
+      umma_commit(bars + g * 2 + b);
+    }
+    __syncwarp();
   };
   auto stream = [&](auto&& body) {
     if (dead) return;
-    if (r == 0) issue(0);
+    if ((warp & 3) == 0) issue(0);
 #pragma unroll 1
     for (int i = 0; i < ST_NCH / ST_G; ++i) {
       const int cc = g + ST_G * i, b = i & 1;
       // every warp of the group has finished reading the other buffer (chunk i - 1): refill it
       tc_fence_before();
       wg_sync(g);
-      if (r == 0 && i + 1 < ST_NCH / ST_G) issue(i + 1);
+      if ((warp & 3) == 0 && i + 1 < ST_NCH / ST_G) issue(i + 1);
       if (!mbar_wait(bars + g * 2 + b, b ? ph1 : ph0, abort_flag)) { dead = true; break; }
       if (b) ph1 ^= 1u; else ph0 ^= 1u;
       tc_fence_after();

@@ -33,6 +33,7 @@ namespace t2t {
 
 constexpr int QT = 128;          // query rows per tensor-core tile (one thread per row)
 constexpr int TASK_ROWS = 256;   // query rows per task: tasks above QT rows run as two tiles sharing one K/V stream
+constexpr int PAIR_ROWS = 128;
 constexpr int KT = 128;          // keys per tile
 constexpr int MAX_RUNS = 1024;   // runs of selected clusters in one union
 constexpr int PLAN_SORT_MAX = 2048;
@@ -668,7 +669,7 @@ __device__ __forceinline__ bool take_tagged(const unsigned long long* at, uint32
 }
 
 // Rows of group 0 of a task of more than QT rows, whole warps of them; group 1 takes the rest.
-__device__ __forceinline__ int group_rows(int rows) { return (((rows + 1) >> 1) + 31) & ~31; }
+__device__ __forceinline__ int group_rows(int rows) { return min((((rows + 1) >> 1) + 31) & ~31, rows); }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2_kernel(
     const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ KVMaps maps,
@@ -734,7 +735,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
       const int end = ring[sl].end, kvlen = ring[sl].kvlen, ntiles = cdiv(kvlen, KT);
       if (end) break;
       const int rows0 = group_rows(ring[sl].rows), myrows = rank ? ring[sl].rows - rows0 : rows0;
-      const size_t at = (size_t)ring[sl].head * N + ring[sl].first + (rank ? rows0 : 0) + (row < myrows ? row : 0);
+      const size_t at = (size_t)ring[sl].head * N + ring[sl].first + (row < myrows ? (rank ? rows0 : 0) + row : 0);
       const bool wr = row < myrows;
       if (ntiles == 0) {   // empty union: O = 0, lse = -inf
         if (wr) {
@@ -854,7 +855,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         if (!mbar_wait(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
-          do { task = atomicAdd(&pv.counters[4], 1); } while (task < numTasks && pv.tasks[task].w <= QT);
+          do { task = atomicAdd(&pv.counters[4], 1); } while (task < numTasks && pv.tasks[task].w <= PAIR_ROWS);
           task = min(task, numTasks);
         }
         task = __shfl_sync(0xffffffffu, task, 0);
@@ -900,8 +901,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         const int ntiles = cdiv(tk.kvlen, KT);
         if (ntiles > 0 && kind == 0 && cw < 2) {
           // one 64-column block of the Q tile each; slots past the group repeat its first row
-          const int rows0 = group_rows(tk.rows), skip = rank ? rows0 : 0, nr = rank ? tk.rows - rows0 : rows0;
-          const size_t rowbase = (size_t)tk.head * N + tk.first + skip;
+          const int rows0 = group_rows(tk.rows), nr = rank ? tk.rows - rows0 : rows0;
+          const size_t rowbase = (size_t)tk.head * N + tk.first + (rank && nr > 0 ? rows0 : 0);
           int r[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
@@ -1126,7 +1127,7 @@ __global__ void __launch_bounds__(A1_THREADS, 2) attn_kernel(
         if (!mbar_wait(bars + C_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) return false;
         int task = 0;
         if (lane == 0) {
-          do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > QT);
+          do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > PAIR_ROWS);
           task = min(task, numTasks);
         }
         task = __shfl_sync(0xffffffffu, task, 0);
@@ -1289,7 +1290,7 @@ constexpr int TL_OFF_CNT = TL_OFF_V + TL_STAGES * TL_SV;
 constexpr int TL_OFF_BAR = TL_OFF_CNT + kC * 4;
 // 97 KB: two CTAs share an SM, and no more than two (tensor memory holds two 256-column allocations)
 constexpr int TL_SMEM = TL_OFF_BAR + 128 + 1024;
-constexpr int TL_THREADS = 160;           // warps 0..3: one softmax thread per row; warp 4: the MMA lane
+constexpr int TL_THREADS = 160;           // warps 0..3: one softmax thread per row; warp 4: the products
 static_assert(TL_NH % 2 == 0 && TL_NH >= 4, "the two score regions alternate");
 static_assert(3 * TL_SMEM > 227 * 1024, "at most two CTAs may share an SM");
 
@@ -1397,45 +1398,53 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
   constexpr uint32_t idescT = make_idesc_bf16(128, kD, false, true);
   constexpr float LOG2E = 1.4426950408889634f;
 
-  auto issue_scores = [&](int step) {   // S_(step & 1) = QU cks_step^T, K = 32
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const uint64_t ad = make_sdesc(sQ + s * 32, 16, 1024);
-      const uint64_t bd = make_sdesc(sC + (step % TL_STAGES) * TL_SC + s * 32, 16, 1024);
-      umma_ss(tS + (step & 1) * TL_H, ad, bd, idescS, s > 0 ? 1u : 0u);
-    }
-  };
-
-  // value sums of one step: 64 rows x 256 B as two 64-column blocks, one TMA tile load each
-  auto load_v = [&](int step) {
-    uint64_t* bar = vFull + step % TL_STAGES;
-    const uint32_t dst = sV + (step % TL_STAGES) * TL_SV;
-    mbar_arrive_expect_tx(bar, TL_SV);
-    tma_load_tile(dst, &mapSumv, 0, h * kC + step * TL_H, bar);
-    tma_load_tile(dst + TL_H * 128, &mapSumv, 64, h * kC + step * TL_H, bar);
-  };
-  if (tid == TL_Q) {
-    // ---- MMA lane ----
-    load_v(0);
-    issue_scores(0);
-    umma_commit(sReady + 0);
-    issue_scores(1);
-    umma_commit(sReady + 1);
-    for (int i = 0; i < TL_NH; ++i) {
-      const int b = i & 1;
-      if (!mbar_wait(pReady + b, (i >> 1) & 1, abort_flag)) break;
-      tc_fence_after();
-      // every softmax thread has seen the commit behind the product of step i - 2: its stage is free
-      if (i + 1 < TL_NH) load_v(i + 1);
-      if (!mbar_wait(vFull + i % TL_STAGES, (i / TL_STAGES) & 1, abort_flag)) break;
-      const uint32_t vb = sV + (i % TL_STAGES) * TL_SV;
-#pragma unroll
-      for (int s8 = 0; s8 < TL_H / 16; ++s8) {
-        const uint64_t bd = make_sdesc(vb + s8 * 2048, TL_H * 128, 1024);
-        umma_ts(tO, tS + b * TL_H + s8 * 8, bd, idescT, (i > 0 || s8 > 0) ? 1u : 0u);
+  if (warp == 4) {
+    // ---- MMA warp: one elected lane issues (see elect_one) ----
+    constexpr uint32_t dhi = sdesc_hi(1024);
+    const uint32_t qlo = sdesc_lo(sQ, 16), clo = sdesc_lo(sC, 16), vlo = sdesc_lo(sV, TL_H * 128);
+    // value sums of one step: 64 rows x 256 B as two 64-column blocks, one TMA tile load each
+    auto load_v = [&](int step, int st) {
+      uint64_t* bar = vFull + st;
+      const uint32_t dst = sV + st * TL_SV;
+      if (elect_one()) {
+        mbar_arrive_expect_tx(bar, TL_SV);
+        tma_load_tile(dst, &mapSumv, 0, h * kC + step * TL_H, bar);
+        tma_load_tile(dst + TL_H * 128, &mapSumv, 64, h * kC + step * TL_H, bar);
       }
-      if (i + 2 < TL_NH) issue_scores(i + 2);
+      __syncwarp();
+    };
+    // S_(step & 1) = QU cks_step^T, K = 32
+    auto scores = [&](int b, int st) {
+      const uint32_t c0 = clo + st * (TL_SC >> 4);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) umma_ss_lo(tS + b * TL_H, qlo + k * 2, c0 + k * 2, dhi, idescS, k > 0 ? 1u : 0u);
       umma_commit(sReady + b);
+    };
+    load_v(0, 0);
+    if (elect_one()) {
+      scores(0, 0);
+      scores(1, 1);
+    }
+    __syncwarp();
+    int st = 0;      // stage of step i
+    for (int i = 0; i < TL_NH; ++i) {
+      const int b = i & 1, st1 = st == TL_STAGES - 1 ? 0 : st + 1, st2 = st1 == TL_STAGES - 1 ? 0 : st1 + 1;
+      if (!mbar_wait(pReady + b, (i >> 1) & 1, abort_flag)) break;
+      // every softmax thread has seen the commit behind the product of step i - 2: its stage is free
+      if (i + 1 < TL_NH) load_v(i + 1, st1);
+      if (!mbar_wait(vFull + st, (i / TL_STAGES) & 1, abort_flag)) break;
+      tc_fence_after();
+      const uint32_t v0 = vlo + st * (TL_SV >> 4), first = i > 0 ? 1u : 0u;
+      __syncwarp();
+      if (elect_one()) {
+#pragma unroll
+        for (int s8 = 0; s8 < TL_H / 16; ++s8)
+          umma_ts_lo(tO, tS + b * TL_H + s8 * 8, v0 + s8 * (2048 >> 4), dhi, idescT, s8 > 0 ? 1u : first);
+        if (i + 2 < TL_NH) scores(b, st2);
+        else umma_commit(sReady + b);
+      }
+      __syncwarp();
+      st = st1;
     }
   }
   bool dead = false;
