@@ -565,6 +565,60 @@ def test_tile_attn_weight_of_a_dominant_key_is_one(lib, sizes, tile, pos):
     assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-4
 
 
+@pytest.mark.parametrize("largest", [128, 300])
+def test_tile_attn_unions_of_many_forms(lib, largest):
+    """Tasks of 1 to `largest` rows, several to a CTA, with unions of no key, of one, of 127 / 128 / 129 / 256, of clusters
+    of one key each with gaps (more than 32 runs in a tile), of long stretches at odd offsets, of everything; empty
+    clusters inside.  Against a float64 softmax over the union: the weights and the output are rounded to bfloat16."""
+    H, N = 12, 6000
+    g = torch.Generator().manual_seed(largest)
+    kc = torch.zeros(H, 2048, dtype=torch.int32)
+    for h in range(H):
+        kc[h, :600] = 1
+        kc[h, 600:1200] = torch.randint(0, 4, (600,), generator=g).int()
+        kc[h, 1200] = 128
+        kc[h, 1202:1220] = torch.randint(30, 140, (18,), generator=g).int()
+        kc[h, 2047] = N - int(kc[h].sum())
+    assert int(kc.min()) == 0 and int(kc[:, 2047].min()) > 256
+    edge = [1, 31, 32, 33, 64, 127, 128] + ([129, 160, 255, 256, 257, 300] if largest > 128 else [])
+    sizes = list(edge)
+    while N - sum(sizes) > largest:
+        sizes.append(int(torch.randint(1, largest + 1, (1,), generator=g)))
+    sizes.append(N - sum(sizes))
+    CQ = len(sizes)
+    sel = torch.zeros(H, CQ, 2048, dtype=torch.bool)
+    for h in range(H):
+        for c in range(CQ):
+            kind = (c + h) % 10
+            if kind == 1: sel[h, c, 5] = True
+            elif kind in (2, 3, 4): sel[h, c, 7:7 + 127 + (kind - 2)] = True
+            elif kind == 5: sel[h, c, 0:600:2] = True
+            elif kind == 6: sel[h, c, 600:1200:2] = True
+            elif kind == 7: sel[h, c, [3, 1200, 1203, 1204, 1205, 1210, 2047]] = True
+            elif kind == 8: sel[h, c] = True
+            elif kind == 9: sel[h, c] = torch.rand(2048, generator=g) < 0.2
+            if kind == 4 and c % 2: sel[h, c, 1200] = True
+    bits = (sel.view(H, CQ, 64, 32).long() << torch.arange(32)).sum(-1)
+    union = torch.where(bits >= 2 ** 31, bits - 2 ** 32, bits).int()
+    q, k, v = (torch.randn(H, N, 128, generator=g).to(BF) for _ in range(3))
+    km, _, zeros = _plain_structure(sizes, v[:1])
+    km = {key: t.expand(H, *t.shape[1:]).contiguous() for key, t in km.items() if key != "lam"}
+    km.update(lam=torch.ones(H), kcounts=kc, V_sorted=v)
+    _, info = _tile_attn(lib, q, k, v, torch.zeros(H, N, 32, dtype=BF), km, torch.zeros(H, 2048, 32, dtype=BF), union)
+    lab = torch.repeat_interleave(torch.arange(CQ), torch.tensor(sizes))
+    for h in range(H):
+        inside = torch.repeat_interleave(sel[h], kc[h].long(), dim=1)[lab].to(DEV)
+        s = q[h].to(DEV).double() @ k[h].to(DEV).double().T / math.sqrt(128.0)
+        s = torch.where(inside, s, -math.inf)
+        some = inside.any(1)
+        want = torch.where(some[:, None], torch.softmax(s, 1), 0.0) @ v[h].to(DEV).double()
+        lse = torch.logsumexp(s, 1).cpu()
+        assert (info["attn_o"][h].double() - want.cpu()).abs().max() < 2e-2
+        fin = some.cpu()
+        assert torch.equal(torch.isfinite(info["lse"][h]), fin)
+        assert (info["lse"][h].double() - lse)[fin].abs().max() < 1e-2
+
+
 @pytest.mark.parametrize("N", [31, 257, 8192, 8193, 16384, 16385])
 @pytest.mark.parametrize("Cn", [3, 1024, 2048])
 def test_centroid_update_on_both_sides_of_the_chunk_rule(lib, N, Cn):

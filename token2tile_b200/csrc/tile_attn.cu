@@ -13,14 +13,12 @@
 //
 // One thread owns one query row (TMEM lane), so row maxima and sums need no
 // shuffles.  K/V rows of a union are contiguous runs in the cluster-major
-// copies kp/vp; the attention kernels fetch them with TMA row gathers (four
-// rows per instruction) straight into 128-byte-swizzled tiles, the residual
-// kernel with 16-byte cp.async.  Tasks of up to 128 query rows run in
-// attn_kernel, two CTAs to an SM (256 TMEM columns each) so that the softmax
-// of one overlaps the MMAs and loads of the other; tasks of 129..256 rows run
-// in attn2_kernel, one warp-specialised CTA per SM whose two row groups share
-// one K/V stream.  Every mbarrier wait is bounded; on a timeout the CTA raises
-// a status word and leaves.
+// copies kp/vp, fetched into 128-byte-swizzled tiles by TMA tile loads, TMA
+// row gathers (four rows per instruction) and 16-byte cp.async.  Tasks of
+// 129..256 query rows run in attn2_kernel on CTA pairs that share every
+// product, tasks of up to 128 rows in attn_kernel, one CTA per SM; both are
+// warp-specialised and persistent.  Every mbarrier wait is bounded; on a
+// timeout the CTA raises a status word and leaves.
 #include <cuda.h>
 
 #include <mutex>
@@ -344,16 +342,6 @@ __device__ __forceinline__ int fetch_plan(const int (&r)[4], bool whole, int lan
   if (k < k32) return ((k - k64) & 7) == 0 ? FETCH_BOX32 : FETCH_NONE;
   return FETCH_GATHER;
 }
-// One lane's part of one 64-column block (`dst`: the block's first byte; bytes are counted on `full`).
-__device__ __forceinline__ void fetch_issue(int what, uint32_t dst, const CUtensorMap* map1, const CUtensorMap* map32,
-                                            const CUtensorMap* map64, int col, const int (&r)[4], int lane,
-                                            uint64_t* full) {
-  const uint32_t mine = dst + lane * 512;
-  if (what == FETCH_GATHER) tma_gather4(mine, map1, col, r[0], r[1], r[2], r[3], full);
-  else if (what == FETCH_BOX32) tma_load_tile(mine, map32, col, r[0], full);
-  else if (what == FETCH_BOX64) tma_load_tile(mine, map64, col, r[0], full);
-}
-
 // ---------------------------------------------------------------------------
 // softmax of a row of scores, shared by the two attention kernels
 // ---------------------------------------------------------------------------
@@ -403,15 +391,12 @@ __device__ __forceinline__ void exp2_fma2(float y0, float y1, float& p0, float& 
 
 // Softmax of one 128-column S row held in tensor memory: the row comes to registers once, its maximum is found there,
 // then P = 2^(s * scale - m) goes back packed to bf16 (chunk c of S, columns 32 c .., becomes columns 16 c .. of P).
-// Two row groups that compute at the same time are bound by the special-function unit (16 exponentials per cycle and
-// SM), so every third pair takes the FMA-pipe route instead.
-// MASK: columns >= valid lie past the union and count as -inf, a weight of zero (2^-125 from the FMA pipe).
+// All exponentials use the special-function unit (16 per cycle and SM, 1,024 cycles a tile).
+// MASK: columns >= valid lie past the union and count as -inf, a weight of zero.
 // The maximum comes before any weight of the tile: weights stay below 2^kLazy, so O and l keep the range of the values
 // whatever the scores, and a key that dominates its row from beyond that weighs exactly one.  (One pass with the first
 // tile's maximum as reference and corrections by the sums rounds the largest weight like any other, 2.326e-3 instead
 // of 2.323e-3 against a float64 softmax, and sums reach 2^60.)
-constexpr int kFmaPairEvery = 99;
-
 // The row to registers; returns its maximum (unscaled).
 template <bool MASK>
 __device__ __forceinline__ float row_scores(uint32_t tS_lane, int valid, uint32_t (&v)[4][32]) {
@@ -439,11 +424,8 @@ __device__ __forceinline__ float row_scores(uint32_t tS_lane, int valid, uint32_
   }
   return fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
 }
-// The row's weights relative to rs.m, written over S and added to rs.l.  `halfway` is called by the whole warp once the
-// first 64 columns of P are written, so that the MMA lane can start on them while the rows work on the rest.
-template <typename Halfway>
-__device__ __forceinline__ void row_weights(uint32_t tS_lane, const uint32_t (&v)[4][32], RowState& rs, float sc,
-                                            Halfway&& halfway) {
+// The row's weights relative to rs.m, written over S and added to rs.l.
+__device__ __forceinline__ void row_weights(uint32_t tS_lane, const uint32_t (&v)[4][32], RowState& rs, float sc) {
   const unsigned long long sc2 = pack_f2(sc, sc), nm2 = pack_f2(-rs.m, -rs.m);
   unsigned long long ls2[2] = {0ull, 0ull};
 #pragma unroll
@@ -451,48 +433,22 @@ __device__ __forceinline__ void row_weights(uint32_t tS_lane, const uint32_t (&v
     uint32_t pk[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      float y0, y1, p0, p1;
+      float y0, y1;
       unpack_f2(fma_f2(pack_f2(__uint_as_float(v[c][2 * j]), __uint_as_float(v[c][2 * j + 1])), sc2, nm2), y0, y1);
-      if (j % kFmaPairEvery == kFmaPairEvery - 1) {
-        exp2_fma2(y0, y1, p0, p1);
-      } else {
-        p0 = ex2_approx(y0);
-        p1 = ex2_approx(y1);
-      }
+      const float p0 = ex2_approx(y0), p1 = ex2_approx(y1);
       ls2[j & 1] = add_f2(ls2[j & 1], pack_f2(p0, p1));
       pk[j] = pack_bf2(p0, p1);
     }
     tmem_st16(tS_lane + c * 16, pk);
-    if (c == 1) halfway();
   }
   float s0, s1, s2, s3;
   unpack_f2(ls2[0], s0, s1);
   unpack_f2(ls2[1], s2, s3);
   rs.l += (s0 + s1) + (s2 + s3);
 }
-template <bool MASK, typename Halfway>
-__device__ __forceinline__ void softmax_tile(uint32_t tS_lane, uint32_t tO_lane, RowState& rs, int valid, bool first,
-                                             float sc, Halfway&& halfway) {
-  uint32_t v[4][32];
-  const float mx = row_scores<MASK>(tS_lane, valid, v) * sc;
-  if (first) {
-    rs.m = mx;
-  } else {
-    const bool grow = mx > rs.m + kLazy;
-    if (__any_sync(0xffffffffu, grow)) {
-      const float mnew = grow ? mx : rs.m;
-      const float alpha = ex2_approx(rs.m - mnew);
-      rescale_rows(tO_lane, alpha);
-      rs.l *= alpha;
-      rs.m = mnew;
-    }
-  }
-  row_weights(tS_lane, v, rs, sc, halfway);
-}
-
 // Registers move between the roles of a kernel: a softmax thread holds a whole row of S, the others need few.  Both
 // kernels are launched with 128 registers a thread and every second warpgroup gives up what the softmax warpgroups take:
-// 128 x (200 + 56) = 256 x 128 (and twice that in attn2_kernel).
+// 256 x (200 + 56) = 512 x 128.
 constexpr int kLaunchRegs = 128, kSoftmaxRegs = 200, kRoleRegs = 56;
 static_assert(kSoftmaxRegs + kRoleRegs == 2 * kLaunchRegs, "the split may not exceed what the launch holds");
 __device__ __forceinline__ void take_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kSoftmaxRegs)); }
@@ -527,79 +483,6 @@ __device__ __forceinline__ void prepare_task(const PlanView& pv, const uint32_t*
     slot->kvlen = len;
   }
   __syncwarp();
-}
-
-// A softmax warp's part of one task: its 32 rows' softmax tile by tile, then the division and the store.  `active` says
-// whether the warp has rows at all, `wr` whether this thread has one; barP[0 / 1] take the halves of P, `g` counts the
-// CTA's tiles.  False when a wait gave up.
-__device__ __forceinline__ bool softmax_task(uint32_t tS_lane, uint32_t tO_lane, uint64_t* barS, uint64_t* barPV,
-                                             uint64_t* barP, uint32_t& g, int kvlen, bool active, bool wr, __nv_bfloat16* out_row, float* lse,
-                                             volatile int* abort_flag) {
-  const int lane = threadIdx.x & 31;
-  const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
-  if (kvlen == 0) {   // empty union: O = 0, lse = -inf
-    if (wr) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) reinterpret_cast<uint4*>(out_row)[i] = make_uint4(0u, 0u, 0u, 0u);
-      *lse = -INFINITY;
-    }
-    return true;
-  }
-  const int ntiles = cdiv(kvlen, KT);
-  RowState rs;
-  rs.m = -INFINITY;
-  rs.l = 0.f;
-  for (int t = 0; t < ntiles; ++t) {
-    // this commit also covers P V of tile t - 1, so O may be rescaled
-    if (!mbar_wait(barS, g & 1u, abort_flag)) return false;
-    ++g;
-    tc_fence_after();
-    // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
-    // whatever S held, which only reaches O rows that are never stored.
-    auto halfway = [&]() {      // keys 0 .. 63 of P are in tensor memory
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(barP);
-    };
-    if (active) {
-      const int valid = kvlen - t * KT;
-      if (valid >= KT) softmax_tile<false>(tS_lane, tO_lane, rs, KT, t == 0, sc, halfway);
-      else softmax_tile<true>(tS_lane, tO_lane, rs, valid, t == 0, sc, halfway);
-      tmem_wait_st();
-    } else {
-      halfway();
-    }
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(barP + 1);
-  }
-  if (!mbar_wait(barPV, (g - 1u) & 1u, abort_flag)) return false;
-  if (active) {
-    tc_fence_after();
-    const float inv = 1.0f / rs.l;
-    uint4* dst = reinterpret_cast<uint4*>(out_row);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t v[32];
-      tmem_ld32(tO_lane + c * 32, v);
-      tmem_wait_ld();
-      if (wr) {
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 o;
-          o.x = pack_bf2(__uint_as_float(v[8 * g + 0]) * inv, __uint_as_float(v[8 * g + 1]) * inv);
-          o.y = pack_bf2(__uint_as_float(v[8 * g + 2]) * inv, __uint_as_float(v[8 * g + 3]) * inv);
-          o.z = pack_bf2(__uint_as_float(v[8 * g + 4]) * inv, __uint_as_float(v[8 * g + 5]) * inv);
-          o.w = pack_bf2(__uint_as_float(v[8 * g + 6]) * inv, __uint_as_float(v[8 * g + 7]) * inv);
-          dst[c * 4 + g] = o;
-        }
-      }
-    }
-    if (wr) *lse = (rs.m + log2f(rs.l)) * 0.6931471805599453f;
-    tc_fence_before();
-  }
-  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -671,6 +554,142 @@ __device__ __forceinline__ bool take_tagged(const unsigned long long* at, uint32
 // Rows of group 0 of a task of more than QT rows, whole warps of them; group 1 takes the rest.
 __device__ __forceinline__ int group_rows(int rows) { return min((((rows + 1) >> 1) + 31) & ~31, rows); }
 
+// The softmax warps of both kernels: warps 0..3 weigh a row's even tiles, warps 4..7 its odd ones (see attn2_kernel).
+// `rank`, `lead` and `tfree` are the group of this CTA's rows and the cluster addresses of the pair's barriers.
+template <bool PAIR>
+__device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* ring, unsigned long long* sM, float2* sFin,
+                                             uint32_t tmem, uint32_t rank, uint32_t lead, uint32_t tfree,
+                                             __nv_bfloat16* __restrict__ attn_out, float* __restrict__ attn_lse, int N,
+                                             volatile int* abort_flag) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wg = warp >> 2, gw = warp & 3, row = gw * 32 + lane;
+  const uint32_t tO_lane = tmem_addr(tmem + 3 * 128, gw * 32, 0);
+  const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
+  // arrival on this CTA's barrier `own`, or on that of the pair at the cluster address `at`
+  auto arrive = [&](int own, uint32_t at) {
+    if (PAIR) mbar_arrive_peer(at); else mbar_arrive(bars + own);
+  };
+  uint32_t g = 0;      // tiles so far
+  uint32_t q = 0;
+  bool ok = true;
+  for (uint32_t n = 0;; ++n) {
+    const uint32_t sl = n & 1u;
+    if (!(PAIR ? mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)
+               : mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)))
+      break;
+    const int end = ring[sl].end, kvlen = ring[sl].kvlen, ntiles = cdiv(kvlen, KT);
+    if (end) break;
+    const int rows0 = PAIR ? group_rows(ring[sl].rows) : ring[sl].rows, myrows = rank ? ring[sl].rows - rows0 : rows0;
+    const size_t at = (size_t)ring[sl].head * N + ring[sl].first + (row < myrows ? (rank ? rows0 : 0) + row : 0);
+    const bool wr = row < myrows;
+    if (ntiles == 0) {   // empty union: O = 0, lse = -inf
+      if (wr) {
+        uint4* dst = reinterpret_cast<uint4*>(attn_out + at * kD) + wg * 8;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (wg == 0) attn_lse[at] = -INFINITY;
+      }
+      __syncwarp();
+      if (lane == 0) arrive(B_TFREE + sl, tfree + sl * 8);
+      continue;
+    }
+    // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
+    // whatever S held, which only reaches O rows that are never stored.
+    const bool active = gw * 32 < myrows;
+    RowState rs;
+    rs.m = -INFINITY;
+    rs.l = 0.f;
+    // this warpgroup's tiles: every other one
+    const int t0 = (int)((wg ^ g) & 1u);
+    uint32_t buf = (g + t0) % 3u;
+    for (int t = t0; t < ntiles; t += 2) {
+      const uint32_t gt = g + t, p = gt - 1u;
+      const uint32_t tS_lane = tmem_addr(tmem + buf * 128, gw * 32, 0);
+      ok = mbar_wait(bars + B_QK + (gt & 3u), (gt >> 2) & 1u, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      if (active) {
+        const int valid = kvlen - t * KT;
+        uint32_t v[4][32];
+        // the reference behind tile t - 1, from the thread that weighs it: looked at once before the row is here
+        const unsigned long long* before = sM + (p & 1u) * QT + row;
+        unsigned long long tagged = peek_tagged(before);
+        const float mx = (valid >= KT ? row_scores<false>(tS_lane, KT, v) : row_scores<true>(tS_lane, valid, v)) * sc;
+        if (t == 0) {
+          rs.m = mx;
+        } else {
+          ok = take_tagged(before, p, tagged, abort_flag);
+          if (!ok) break;
+          const float m_in = __uint_as_float((uint32_t)tagged);
+          if (__any_sync(0xffffffffu, m_in != rs.m || mx > m_in + kLazy)) {
+            if (m_in != rs.m) rs.l *= t > 1 ? ex2_approx(rs.m - m_in) : 0.f;
+            rs.m = m_in;
+            const bool grow = mx > rs.m + kLazy;
+            if (__any_sync(0xffffffffu, grow)) {
+              const float mnew = grow ? mx : rs.m;
+              ok = mbar_wait(bars + B_PV + (p & 3u), (p >> 2) & 1u, abort_flag);      // O holds the tiles up to t - 1
+              if (!ok) break;
+              const float alpha = ex2_approx(rs.m - mnew);
+              tc_fence_after();
+              rescale_rows(tO_lane, alpha);
+              rs.l *= alpha;
+              rs.m = mnew;
+            }
+          }
+        }
+        put_tagged(sM + (gt & 1u) * QT + row, gt, rs.m);
+        row_weights(tS_lane, v, rs, sc);
+        tmem_wait_st();
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive(B_P + buf, lead + (B_P + buf) * 8);
+      buf = buf ? buf - 1 : 2;      // two on, of three
+    }
+    if (!ok) break;
+    g += ntiles;
+    // both warps of these rows meet: the sums of the two are relative to the maxima they saw last
+    float2* fin = sFin + (q & 1u) * 2 * QT;
+    fin[wg * QT + row] = make_float2(rs.m, rs.l);
+    asm volatile("bar.sync %0, 64;\n" ::"r"(1 + gw) : "memory");
+    const int lastwg = (g - 1u) & 1u;
+    ok = mbar_wait(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag);
+    if (!ok) break;
+    if (active) {
+      tc_fence_after();
+      const float2 a = fin[lastwg * QT + row], b = fin[(lastwg ^ 1) * QT + row];
+      const float l = ntiles > 1 ? a.y + (b.x != a.x ? b.y * ex2_approx(b.x - a.x) : b.y) : a.y;
+      const float inv = 1.0f / l;
+      uint4* dst = reinterpret_cast<uint4*>(attn_out + at * kD) + wg * 8;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t v[32];
+        tmem_ld32(tO_lane + wg * 64 + c * 32, v);
+        tmem_wait_ld();
+        if (wr) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            uint4 o;
+            o.x = pack_bf2(__uint_as_float(v[8 * k + 0]) * inv, __uint_as_float(v[8 * k + 1]) * inv);
+            o.y = pack_bf2(__uint_as_float(v[8 * k + 2]) * inv, __uint_as_float(v[8 * k + 3]) * inv);
+            o.z = pack_bf2(__uint_as_float(v[8 * k + 4]) * inv, __uint_as_float(v[8 * k + 5]) * inv);
+            o.w = pack_bf2(__uint_as_float(v[8 * k + 6]) * inv, __uint_as_float(v[8 * k + 7]) * inv);
+            dst[c * 4 + k] = o;
+          }
+        }
+      }
+      if (wr && wg == 0) attn_lse[at] = (a.x + log2f(l)) * 0.6931471805599453f;
+    }
+    ++q;
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) {
+      arrive(B_OFREE, lead + B_OFREE * 8);
+      arrive(B_TFREE + sl, tfree + sl * 8);
+    }
+  }
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2_kernel(
     const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ KVMaps maps,
     const uint32_t* __restrict__ ub, const int* __restrict__ qperm,
@@ -723,126 +742,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
   if (warp < 8) {
     // ================= softmax warps =================
     take_registers();
-    const int wg = warp >> 2, gw = warp & 3, row = gw * 32 + lane;
-    const uint32_t tO_lane = tmem_addr(tmem + 3 * 128, gw * 32, 0);
-    const float sc = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
-    uint32_t g = 0;      // tiles so far
-    uint32_t q = 0;
-    bool ok = true;
-    for (uint32_t n = 0;; ++n) {
-      const uint32_t sl = n & 1u;
-      if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
-      const int end = ring[sl].end, kvlen = ring[sl].kvlen, ntiles = cdiv(kvlen, KT);
-      if (end) break;
-      const int rows0 = group_rows(ring[sl].rows), myrows = rank ? ring[sl].rows - rows0 : rows0;
-      const size_t at = (size_t)ring[sl].head * N + ring[sl].first + (row < myrows ? (rank ? rows0 : 0) + row : 0);
-      const bool wr = row < myrows;
-      if (ntiles == 0) {   // empty union: O = 0, lse = -inf
-        if (wr) {
-          uint4* dst = reinterpret_cast<uint4*>(attn_out + at * kD) + wg * 8;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
-          if (wg == 0) attn_lse[at] = -INFINITY;
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
-        continue;
-      }
-      // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
-      // whatever S held, which only reaches O rows that are never stored.
-      const bool active = gw * 32 < myrows;
-      RowState rs;
-      rs.m = -INFINITY;
-      rs.l = 0.f;
-      // this warpgroup's tiles: every other one
-      const int t0 = (int)((wg ^ g) & 1u);
-      uint32_t buf = (g + t0) % 3u;
-      for (int t = t0; t < ntiles; t += 2) {
-        const uint32_t gt = g + t, p = gt - 1u;
-        const uint32_t tS_lane = tmem_addr(tmem + buf * 128, gw * 32, 0);
-        ok = mbar_wait(bars + B_QK + (gt & 3u), (gt >> 2) & 1u, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        if (active) {
-          const int valid = kvlen - t * KT;
-          uint32_t v[4][32];
-          // the reference behind tile t - 1, from the thread that weighs it: looked at once before the row is here
-          const unsigned long long* before = sM + (p & 1u) * QT + row;
-          unsigned long long tagged = peek_tagged(before);
-          const float mx = (valid >= KT ? row_scores<false>(tS_lane, KT, v) : row_scores<true>(tS_lane, valid, v)) * sc;
-          if (t == 0) {
-            rs.m = mx;
-          } else {
-            ok = take_tagged(before, p, tagged, abort_flag);
-            if (!ok) break;
-            const float m_in = __uint_as_float((uint32_t)tagged);
-            if (__any_sync(0xffffffffu, m_in != rs.m || mx > m_in + kLazy)) {
-              if (m_in != rs.m) rs.l *= t > 1 ? ex2_approx(rs.m - m_in) : 0.f;
-              rs.m = m_in;
-              const bool grow = mx > rs.m + kLazy;
-              if (__any_sync(0xffffffffu, grow)) {
-                const float mnew = grow ? mx : rs.m;
-                ok = mbar_wait(bars + B_PV + (p & 3u), (p >> 2) & 1u, abort_flag);      // O holds the tiles up to t - 1
-                if (!ok) break;
-                const float alpha = ex2_approx(rs.m - mnew);
-                tc_fence_after();
-                rescale_rows(tO_lane, alpha);
-                rs.l *= alpha;
-                rs.m = mnew;
-              }
-            }
-          }
-          put_tagged(sM + (gt & 1u) * QT + row, gt, rs.m);
-          row_weights(tS_lane, v, rs, sc, [] {});
-          tmem_wait_st();
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_peer(lead + (B_P + buf) * 8);
-        buf = buf ? buf - 1 : 2;      // two on, of three
-      }
-      if (!ok) break;
-      g += ntiles;
-      // both warps of these rows meet: the sums of the two are relative to the maxima they saw last
-      float2* fin = sFin + (q & 1u) * 2 * QT;
-      fin[wg * QT + row] = make_float2(rs.m, rs.l);
-      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + gw) : "memory");
-      const int lastwg = (g - 1u) & 1u;
-      ok = mbar_wait(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag);
-      if (!ok) break;
-      if (active) {
-        tc_fence_after();
-        const float2 a = fin[lastwg * QT + row], b = fin[(lastwg ^ 1) * QT + row];
-        const float l = ntiles > 1 ? a.y + (b.x != a.x ? b.y * ex2_approx(b.x - a.x) : b.y) : a.y;
-        const float inv = 1.0f / l;
-        uint4* dst = reinterpret_cast<uint4*>(attn_out + at * kD) + wg * 8;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t v[32];
-          tmem_ld32(tO_lane + wg * 64 + c * 32, v);
-          tmem_wait_ld();
-          if (wr) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              uint4 o;
-              o.x = pack_bf2(__uint_as_float(v[8 * k + 0]) * inv, __uint_as_float(v[8 * k + 1]) * inv);
-              o.y = pack_bf2(__uint_as_float(v[8 * k + 2]) * inv, __uint_as_float(v[8 * k + 3]) * inv);
-              o.z = pack_bf2(__uint_as_float(v[8 * k + 4]) * inv, __uint_as_float(v[8 * k + 5]) * inv);
-              o.w = pack_bf2(__uint_as_float(v[8 * k + 6]) * inv, __uint_as_float(v[8 * k + 7]) * inv);
-              dst[c * 4 + k] = o;
-            }
-          }
-        }
-        if (wr && wg == 0) attn_lse[at] = (a.x + log2f(l)) * 0.6931471805599453f;
-      }
-      ++q;
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive_peer(lead + B_OFREE * 8);
-        mbar_arrive_peer(tfree + sl * 8);
-      }
-    }
+    softmax_role<true>(bars, ring, sM, sFin, tmem, rank, lead, tfree, attn_out, attn_lse, N, abort_flag);
   } else {
     give_registers();
     if (warp == 9 && rank == 1) {
@@ -1033,56 +933,110 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
 // ---------------------------------------------------------------------------
 // exact attention, tasks of at most QT rows
 // ---------------------------------------------------------------------------
-// The same roles as attn2_kernel with one row group and single K, V and Q buffers, two CTAs to an SM
-// (256 tensor-memory columns and 110 KB of shared memory each) so that one CTA's softmax runs under the
-// other's loads and products:
-//   warps 0..3   softmax, one thread per query row
-//   warp 4       issues every MMA (see elect_one)
-//   warps 5..7   the K and V tiles (and the task's Q tile) by TMA (see fetch_plan).  A TMA instruction holds
-//                its warp for about 70 cycles per lane, which threads that also compute cannot afford, and
-//                one warp alone would need longer for a K tile than the softmax takes.
-// Fill g of the K (V) buffer, g counting the tiles this CTA has processed, waits for the commit behind the product that
-// read fill g - 1, phase g - 1 of C_S (C_PV), and completes phase g of fullK (fullV).  A commit costs the tensor pipe about
-// 100 cycles, so these two are all there are: C_S also says that a task's Q tile is free, C_PV that its O is complete.
-constexpr int A1_THREADS = 8 * 32;
-constexpr int A1_OFF_MISC = 3 * AT_TILE;                  // Q, K, V tiles
-constexpr int A1_SMEM = A1_OFF_MISC + 256 + 2 * (int)sizeof(TaskSlot) + 2 * RUN_INTS * 4;
-enum { C_S = 0, C_PV = 1, C_P = 2, C_FULLK = 4, C_FULLV, C_FULLQ, C_TFULL, C_TFREE = C_TFULL + 2,
-       C_COUNT = C_TFREE + 2 };      // P: [half]; TFULL / TFREE: the task ring
-constexpr int A1_CONSUMERS = 4 + 1 + 3;                   // warps that read a task: softmax, MMA, copy
-static_assert(2 * (A1_SMEM + 1024) <= 228 * 1024, "two CTAs share an SM");
-static_assert(C_COUNT * 8 + 16 <= 256, "the barriers fit their area");
+// attn2_kernel's pipeline on one CTA per SM: three score buffers and O fill tensor memory, the softmax of a tile belongs
+// to one of two warpgroups, S = Q K^T runs two tiles ahead of P V.  A CTA keeps whole K and V tiles, 64 KB a tile for 128
+// rows, so the loads bound it: tile loads (TMA) where 32 or more rows of the union are contiguous; of the groups of four
+// rows between them a third comes by TMA gathers and the rest by 16-byte cp.async (26 and 28 B/clk alone).
+// 404 k tiles at 720p x 40 heads take 3.35 ms, 2,300 cycles a tile and SM (3.70 with two CTAs per SM, single K / V buffers
+// and the rows found by every copy warp), 321 k at 480p x 40 and 5 % 2.87 ms (3.28), 49 tasks at 2 x 4096 30 us less.
+// With 64-row tile loads from any rows instead it would be 2.8 and 2.25 ms, with next to no loads 2.5 and 2.1.
+//   warps 0..7   softmax (see softmax_role)
+//   warp 8 / 9   issue Q K^T / P V
+//   warp 10      the next task, the run list of its union, its Q tile
+//   warp 11      the source rows of the next tiles and how they are fetched (see fetch_plan), a ring of A1_PLANS of them
+//   warps 12, 13 the K tiles, warps 14, 15 the V tiles, half of a tile's copies each
+// Barriers as in attn2_kernel; FULLK / FULLV take an arrival that announces the bytes of the TMA copies and one of every
+// thread that copies, by the hardware once the thread's cp.async rows have landed.  PLAN / PFREE[g mod 8]: tile g's rows
+// are there, its copy warps have read them.
+constexpr int A1_THREADS = 16 * 32;
+constexpr int A1_KST = 3, A1_VST = 2;                     // K and V ring depth; one Q tile
+constexpr int A1_TEAM = 2;                                // warps that share a K tile, a V tile
+constexpr int A1_PLANS = 8;
+struct TilePlan {
+  int rows[QT];                      // source row of every row of the tile
+  unsigned gathers, box32, box64;    // four-row groups that are gathered, that start a 32- or 64-row tile load
+  unsigned pad;
+};
+// Groups gathered by TMA rather than cp.async: 3.34 / 2.87 ms (720p / 480p) with a third of them, 3.44 / 2.91 with half,
+// 3.36 / 3.01 with all, 3.4 / 3.2 with none.
+constexpr unsigned kGatherByTma = 0x92492492u;
+constexpr unsigned kSecondHalf = 0xccccccccu;             // groups whose copies the second warp of a team starts
+enum { B_PLAN = B_COUNT, B_PFREE = B_PLAN + A1_PLANS, A1_BARS = B_PFREE + A1_PLANS };
+constexpr int A1_OFF_K = AT_TILE;
+constexpr int A1_OFF_V = A1_OFF_K + A1_KST * AT_TILE;
+constexpr int A1_OFF_MISC = A1_OFF_V + A1_VST * AT_TILE;
+constexpr int A1_OFF_RING = A1_OFF_MISC + 512;
+constexpr int A1_OFF_M = A1_OFF_RING + 2 * (int)sizeof(TaskSlot);
+constexpr int A1_OFF_FIN = A1_OFF_M + 2 * QT * 8;
+constexpr int A1_OFF_ROWS = A1_OFF_FIN + 4 * QT * 8;      // [128] source rows of the Q tile
+constexpr int A1_OFF_PLAN = A1_OFF_ROWS + QT * 4;
+constexpr int A1_OFF_RUNS = A1_OFF_PLAN + A1_PLANS * (int)sizeof(TilePlan);
+constexpr int A1_SMEM = A1_OFF_RUNS + 2 * RUN_INTS * 4 + 1024;
+constexpr int A1_CONSUMERS = 8 + 2 + 1 + 2 * A1_TEAM;     // warps that read a task: softmax, QK and PV, rows, copy
+static_assert(A1_SMEM <= 227 * 1024, "one CTA per SM");
+static_assert(A1_KST <= 4 && A1_VST <= 4, "the commits of four tiles are told apart");
+static_assert(A1_BARS * 8 + 16 <= 512 && A1_OFF_PLAN % 16 == 0, "the barriers fit their area");
 
-__global__ void __launch_bounds__(A1_THREADS, 2) attn_kernel(
-    const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ KVMaps maps,
-    const uint32_t* __restrict__ ub, const int* __restrict__ qperm,
+// The four-row groups in `groups` of a 128-row tile, by one warp: cp.async of rows `rows[0..127]` (from `src`, whole rows of
+// 128 columns) into the 128-byte-swizzled tile at `dst`.  A half-warp takes two of a group's rows, a lane 16 bytes of each.
+__device__ __forceinline__ void copy_groups(uint32_t dst, const __nv_bfloat16* __restrict__ src, const int* rows,
+                                            unsigned groups, int lane) {
+  const int two = (lane >> 4) * 2, ch = lane & 15;
+  const uint32_t at = dst + (ch >> 3) * (QT * 128) + two * 128, swz = ((ch & 7) ^ two) << 4;
+  const __nv_bfloat16* from = src + ch * 8;
+  while (groups) {
+    int i[4];
+    int2 two_rows[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      i[k] = __ffs(groups) - 1;
+      groups &= groups - 1;
+      two_rows[k] = *reinterpret_cast<const int2*>(rows + max(i[k], 0) * 4 + two);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i[k] < 0) break;
+      const uint32_t d = at + i[k] * 512, sw = swz ^ ((i[k] & 1) << 6);
+      cp_async16(d + sw, from + (size_t)two_rows[k].x * kD);
+      cp_async16(d + 128 + (sw ^ 16u), from + (size_t)two_rows[k].y * kD);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
+    const __grid_constant__ KVMaps maps, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kp,
+    const __nv_bfloat16* __restrict__ vp, const uint32_t* __restrict__ ub, const int* __restrict__ qperm,
     __nv_bfloat16* __restrict__ attn_out, float* __restrict__ attn_lse, int* __restrict__ plan, int H, int N, int CQ,
     int q_row_step, int q_head_step, int* __restrict__ status) {
-  // the second run list leaves no room for aligning the tiles by hand
-  extern __shared__ __align__(1024) uint8_t smem_tiles[];
-  uint8_t* sm = smem_tiles;
-  const uint32_t base = smem_u32(sm);
-  const uint32_t sQ = base, sK = base + AT_TILE, sV = base + 2 * AT_TILE;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + A1_OFF_MISC);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + A1_OFF_MISC + C_COUNT * 8);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + A1_OFF_MISC + C_COUNT * 8 + 8);
-  TaskSlot* ring = reinterpret_cast<TaskSlot*>(sm + A1_OFF_MISC + 256);
-  int* sRuns = reinterpret_cast<int*>(ring + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + A1_OFF_MISC + A1_BARS * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + A1_OFF_MISC + A1_BARS * 8 + 8);
+  TaskSlot* ring = reinterpret_cast<TaskSlot*>(sm + A1_OFF_RING);
+  unsigned long long* sM = reinterpret_cast<unsigned long long*>(sm + A1_OFF_M);
+  float2* sFin = reinterpret_cast<float2*>(sm + A1_OFF_FIN);
+  int* sRuns = reinterpret_cast<int*>(sm + A1_OFF_RUNS);
+  TilePlan* plans = reinterpret_cast<TilePlan*>(sm + A1_OFF_PLAN);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  if (tid < 2 * QT) sM[tid] = ~0ull;      // no tile
   if (tid == 0) {
-    *abort_flag = base & 1023u ? 1 : 0;
-    for (int i = 0; i < C_COUNT; ++i) {
+    *abort_flag = 0;
+    for (int i = 0; i < A1_BARS; ++i) {
       int count = 1;
-      if (i == C_P || i == C_P + 1) count = 4;
-      else if (i == C_FULLK || i == C_FULLV) count = 3;
-      else if (i == C_FULLQ) count = 2;
-      else if (i >= C_TFREE) count = A1_CONSUMERS;
+      if (i >= B_P && i < B_P + 3) count = 4;                                    // softmax warps of a tile
+      else if (i >= B_FULLK && i < B_FULLK + A1_KST) count = 1 + 32 * A1_TEAM;
+      else if (i >= B_FULLV && i < B_FULLV + A1_VST) count = 1 + 32 * A1_TEAM;
+      else if (i == B_OFREE) count = 8;
+      else if (i >= B_PFREE) count = 2 * A1_TEAM;
+      else if (i == B_TFREE || i == B_TFREE + 1) count = A1_CONSUMERS;
       mbar_init(bars + i, count);
     }
     mbar_init_fence();
@@ -1091,182 +1045,244 @@ __global__ void __launch_bounds__(A1_THREADS, 2) attn_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tO = tmem + 128;
 
-  if (*abort_flag) {
-    // misaligned tiles: nothing starts
-  } else if (warp < 4) {
-    // ================= softmax warps: one query row per thread =================
+  if (warp < 8) {
+    // ================= softmax warps =================
     take_registers();
-    const uint32_t tS_lane = tmem_addr(tS, warp * 32, 0), tO_lane = tmem_addr(tO, warp * 32, 0);
-    uint32_t g = 0;      // tiles so far
-    for (uint32_t n = 0;; ++n) {
-      const uint32_t sl = n & 1u;
-      if (!mbar_wait(bars + C_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
-      const TaskSlot tk = ring[sl];
-      if (tk.end) break;
-      const size_t at = (size_t)tk.head * N + tk.first + (tid < tk.rows ? tid : 0);
-      if (!softmax_task(tS_lane, tO_lane, bars + C_S, bars + C_PV, bars + C_P, g, tk.kvlen, warp * 32 < tk.rows,
-                        tid < tk.rows, attn_out + at * kD, attn_lse + at, abort_flag))
-        break;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + C_TFREE + sl);
-    }
+    softmax_role<false>(bars, ring, sM, sFin, tmem, 0u, 0u, 0u, attn_out, attn_lse, N, abort_flag);
   } else {
     give_registers();
-    if (warp >= 5) {
-      // ================= copy warps =================
-      // K and V tiles hold the same rows, so one fetch plan serves both tiles and both of their 64-column
-      // blocks; the three warps share its instructions (the n-th issuing lane belongs to warp n mod 3), K
-      // first: the next Q K^T waits for it.  Warp 7 also prepares the next task, behind its share of the second tile.
+    if (warp == 10) {
+      // ================= the next task, the run list of its union and its Q tile =================
       const PlanView pv = plan_view(plan, H, N, CQ);
       const int numTasks = pv.counters[0];
-      const int cw = warp - 5, orow = lane * 4;
-      auto prepare = [&](uint32_t n) {
+      int* sRows = reinterpret_cast<int*>(sm + A1_OFF_ROWS);
+      const uint32_t q_last = (uint32_t)((H - 1) * q_head_step + (N - 1) * q_row_step);      // see kv_last
+      uint32_t nq = 0;      // tasks with tiles so far
+      for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + C_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) return false;
+        if (!mbar_wait(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
           do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > PAIR_ROWS);
           task = min(task, numTasks);
         }
         task = __shfl_sync(0xffffffffu, task, 0);
-        prepare_task(pv, ub, CQ, numTasks, task, ring + sl, sRuns + sl * RUN_INTS, sRuns + sl * RUN_INTS + MAX_RUNS,
-                            abort_flag, status);
-        if (lane == 0) mbar_arrive(bars + C_TFULL + sl);
-        return true;
-      };
-      uint32_t g = 0;      // tiles so far; every role counts alike
-      bool ok = cw < 2 || prepare(0);
-      for (uint32_t n = 0; ok; ++n) {
+        int* runs = sRuns + sl * RUN_INTS;
+        prepare_task(pv, ub, CQ, numTasks, task, ring + sl, runs, runs + MAX_RUNS, abort_flag, status);
+        const TaskSlot tk = ring[sl];
+        if (lane == 0) mbar_arrive(bars + B_TFULL + sl);
+        if (tk.end) break;
+        if (tk.kvlen == 0) continue;
+        // slots past the task repeat its first row; warps of slots past it compute nothing and need no rows
+        const size_t rowbase = (size_t)tk.head * N + tk.first;
+        int r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int row = tk.head * q_head_step + qperm[rowbase + (lane * 4 + j < tk.rows ? lane * 4 + j : 0)] * q_row_step;
+          r[j] = (int)min((uint32_t)row, q_last);
+        }
+        reinterpret_cast<int4*>(sRows)[lane] = make_int4(r[0], r[1], r[2], r[3]);
+        __syncwarp();
+        if (!mbar_wait(bars + B_FREEQ, (nq & 1u) ^ 1u, abort_flag)) break;
+        copy_groups(base, q, sRows, 0xffffffffu >> (32 - 8 * cdiv(tk.rows, 32)), lane);
+        cp_async_commit();
+        cp_async_wait<0>();
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars + B_FULLQ);
+        ++nq;
+      }
+    } else if (warp == 11) {
+      // ================= rows of the next tiles =================
+      const uint32_t kv_last = (uint32_t)H * (uint32_t)N - 1u;
+      uint32_t g = 0;             // tiles so far
+      bool ok = true;
+      for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + C_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const TaskSlot tk = ring[sl];
         if (tk.end) break;
         const int* sRunStart = sRuns + sl * RUN_INTS;
         const int* sRunCum = sRunStart + MAX_RUNS;
         const int ntiles = cdiv(tk.kvlen, KT);
-        if (ntiles > 0 && cw < 2) {      // one 64-column block of the Q tile each; slots past the task repeat its first row
-          const size_t rowbase = (size_t)tk.head * N + tk.first;
-          int r[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            r[j] = tk.head * q_head_step + qperm[rowbase + (orow + j < tk.rows ? orow + j : 0)] * q_row_step;
-          ok = mbar_wait(bars + C_S, (g & 1u) ^ 1u, abort_flag);
-          if (!ok) break;
-          if (lane == 0) mbar_arrive_expect_tx(bars + C_FULLQ, AT_TILE / 2);
-          __syncwarp();
-          tma_gather4(sQ + cw * (KT * 128) + orow * 128, &mapQ, cw * 64, r[0], r[1], r[2], r[3], bars + C_FULLQ);
-        }
-        int cursor = 0;
+        int first = 0;            // run of the tile's first row
         for (int t = 0; t < ntiles; ++t, ++g) {
+          // lane j holds the position of run first + j: the run of this lane's first row is found among those, or
+          // stepped to from the last one
+          const int p0 = t * KT + lane * 4;
+          const int cum = first + lane < tk.runs ? sRunCum[first + lane] : 0x7fffffff;
+          int cursor = 0;
+#pragma unroll
+          for (int d = 16; d > 0; d >>= 1)
+            if (__shfl_sync(0xffffffffu, cum, cursor + d) <= p0) cursor += d;
+          cursor += first;
           int r[4];
-          const bool whole = union_rows(sRunStart, sRunCum, tk.runs, tk.kvlen, t * KT + orow, tk.head * N, cursor, r);
-          int what = fetch_plan(r, whole, lane, 32);
-          const unsigned issuing = __ballot_sync(0xffffffffu, what != FETCH_NONE);
-          if (__popc(issuing & ((1u << lane) - 1u)) % 3 != cw) what = FETCH_NONE;
-          ok = mbar_wait(bars + C_S, (g & 1u) ^ 1u, abort_flag);
+          const bool whole = union_rows(sRunStart, sRunCum, tk.runs, tk.kvlen, p0, tk.head * N, cursor, r);
+          const int what = fetch_plan(r, whole, lane, 32);
+          first = __shfl_sync(0xffffffffu, cursor, 31);
+          const unsigned gathers = __ballot_sync(0xffffffffu, what == FETCH_GATHER);
+          const unsigned b32 = __ballot_sync(0xffffffffu, what == FETCH_BOX32), b64 = __ballot_sync(0xffffffffu, what == FETCH_BOX64);
+          TilePlan* plan = plans + (g & (A1_PLANS - 1));
+          ok = mbar_wait(bars + B_PFREE + (g & (A1_PLANS - 1)), ((g / A1_PLANS) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
-          // every copy warp arrives on the full barrier, so that none of them can fall two phases behind the
-          // free barrier it waits on (a warp may have nothing to fetch for a tile)
-          if (lane == 0) { if (cw == 0) mbar_arrive_expect_tx(bars + C_FULLK, AT_TILE); else mbar_arrive(bars + C_FULLK); }
-          fetch_issue(what, sK, &maps.k1, &maps.k32, &maps.k64, 0, r, lane, bars + C_FULLK);
-          fetch_issue(what, sK + KT * 128, &maps.k1, &maps.k32, &maps.k64, 64, r, lane, bars + C_FULLK);
-          ok = mbar_wait(bars + C_PV, (g & 1u) ^ 1u, abort_flag);
-          if (!ok) break;
-          if (lane == 0) { if (cw == 0) mbar_arrive_expect_tx(bars + C_FULLV, AT_TILE); else mbar_arrive(bars + C_FULLV); }
-          fetch_issue(what, sV, &maps.v1, &maps.v32, &maps.v64, 0, r, lane, bars + C_FULLV);
-          fetch_issue(what, sV + KT * 128, &maps.v1, &maps.v32, &maps.v64, 64, r, lane, bars + C_FULLV);
-          if (cw == 2 && t == min(1, ntiles - 1)) {
-            __syncwarp();
-            ok = prepare(n + 1);
-            if (!ok) break;
+          // cp.async has no bounds of its own: a plan that does not match kp / vp stays inside them
+#pragma unroll
+          for (int j = 0; j < 4; ++j) r[j] = (int)min((uint32_t)r[j], kv_last);
+          reinterpret_cast<int4*>(plan->rows)[lane] = make_int4(r[0], r[1], r[2], r[3]);
+          if (lane == 0) {
+            plan->gathers = gathers;
+            plan->box32 = b32;
+            plan->box64 = b64;
           }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bars + B_PLAN + (g & (A1_PLANS - 1)));
         }
         if (!ok) break;
-        if (ntiles == 0 && cw == 2) ok = prepare(n + 1);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bars + C_TFREE + sl);
+        if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
       }
-    } else {
-      // ================= MMA warp =================
-      constexpr uint32_t idescQK = make_idesc_bf16(128, KT, false, false);
-      constexpr uint32_t idescPV = make_idesc_bf16(128, kD, false, true);
-      constexpr uint32_t dhi = sdesc_hi(1024);
-      const uint32_t qlo = sdesc_lo(sQ, 16), klo = sdesc_lo(sK, 16), vlo = sdesc_lo(sV, KT * 128);
-      auto mma_qk = [&]() {      // S = Q K^T
+    } else if (warp >= 12) {
+      // ================= copy warps =================
+      const int kind = (warp - 12) / A1_TEAM, member = (warp - 12) % A1_TEAM;      // 0: K, 1: V
+      const uint32_t depth = kind ? A1_VST : A1_KST;
+      const __nv_bfloat16* src = kind ? vp : kp;
+      const CUtensorMap* map1 = kind ? &maps.v1 : &maps.k1;
+      const CUtensorMap* map32 = kind ? &maps.v32 : &maps.k32;
+      const CUtensorMap* map64 = kind ? &maps.v64 : &maps.k64;
+      uint32_t g = 0, slot = 0;                        // tiles so far, ring slot of the next one
+      // the lanes whose copies this warp starts: of each fetch and kind of copy about half
+      const unsigned mine_mask = member ? kSecondHalf : ~kSecondHalf;
+      bool ok = true;
+      for (uint32_t n = 0;; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
-        if (elect_one()) {
-#pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            constexpr uint32_t blk = (QT * 128) >> 4;      // second 64-column block of a tile
-            const uint32_t off = (s >> 2) * blk + (s & 3) * 2;
-            umma_ss_lo(tS, qlo + off, klo + off, dhi, idescQK, s > 0 ? 1u : 0u);
+        if (end) break;
+        if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
+        for (int t = 0; t < ntiles; ++t, ++g, slot = slot + 1 == depth ? 0 : slot + 1) {
+          const TilePlan* plan = plans + (g & (A1_PLANS - 1));
+          ok = mbar_wait(bars + B_PLAN + (g & (A1_PLANS - 1)), (g / A1_PLANS) & 1u, abort_flag);
+          if (!ok) break;
+          const int4 r = reinterpret_cast<const int4*>(plan->rows)[lane];
+          const unsigned gathers = plan->gathers, b32 = plan->box32, b64 = plan->box64;
+          ok = g < depth || mbar_wait(bars + (kind ? B_PV : B_QK) + ((g - depth) & 3u), ((g - depth) >> 2) & 1u, abort_flag);
+          if (!ok) break;
+          uint64_t* full = bars + (kind ? B_FULLV : B_FULLK) + slot;
+          const uint32_t dst = base + (kind ? A1_OFF_V : A1_OFF_K) + slot * AT_TILE, mine = dst + lane * 512;
+          if (member == 0 && lane == 0) {
+            const uint32_t bytes = (4u * __popc(gathers & kGatherByTma) + 32u * __popc(b32) + 64u * __popc(b64)) * kD * 2;
+            if (bytes) mbar_arrive_expect_tx(full, bytes); else mbar_arrive(full);
           }
-          umma_commit(bars + C_S);
+          __syncwarp();
+          if (((b32 | b64) & mine_mask) >> lane & 1u) {
+            const CUtensorMap* map = (b64 >> lane) & 1u ? map64 : map32;
+            tma_load_tile(mine, map, 0, r.x, full);
+            tma_load_tile(mine + KT * 128, map, 64, r.x, full);
+          } else if ((gathers & kGatherByTma & mine_mask) >> lane & 1u) {
+            tma_gather4(mine, map1, 0, r.x, r.y, r.z, r.w, full);
+            tma_gather4(mine + KT * 128, map1, 64, r.x, r.y, r.z, r.w, full);
+          }
+          __syncwarp();
+          copy_groups(dst, src, plan->rows, gathers & ~kGatherByTma & mine_mask, lane);
+          cp_async_arrive(full);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bars + B_PFREE + (g & (A1_PLANS - 1)));
         }
-        __syncwarp();
-      };
-      uint32_t g0 = 0, q = 0;
+        if (!ok) break;
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+    } else if (warp == 8) {
+      // ================= Q K^T: waits for the K tile and for P V to have read the score buffer =================
+      constexpr uint32_t idescQK = make_idesc_bf16(128, KT, false, false);
+      constexpr uint32_t dhi = sdesc_hi(1024);
+      const uint32_t qlo = sdesc_lo(base, 16), klo = sdesc_lo(base + A1_OFF_K, 16);
+      uint32_t g = 0, nq = 0, tS = tmem;      // tiles, tasks with tiles, score buffer of the next tile
+      uint32_t ks = 0, kph = 0;               // K slot and its phase
       bool ok = true;
       for (uint32_t n = 0; ok; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + C_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
-        if (ring[sl].end) break;
-        const int ntiles = cdiv(ring[sl].kvlen, KT);
+        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bars + C_TFREE + sl);
+        if (end) break;
+        if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
         if (ntiles == 0) continue;
-        ok = mbar_wait(bars + C_FULLQ, q & 1u, abort_flag) && mbar_wait(bars + C_FULLK, g0 & 1u, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        mma_qk();
-        for (int t = 0; t < ntiles && ok; ++t) {
-          const uint32_t tg = g0 + t;
-          const bool more = t + 1 < ntiles;
-          ok = false;
-          if (!mbar_wait(bars + C_FULLV, tg & 1u, abort_flag)) break;
-          // P reaches tensor memory in two halves of 64 keys; both P barriers complete once per tile
-          if (!mbar_wait(bars + C_P, tg & 1u, abort_flag)) break;
+        if (!mbar_wait(bars + B_FULLQ, nq & 1u, abort_flag)) break;
+        for (int t = 0; t < ntiles; ++t, ++g) {
+          const uint32_t b0 = klo + ks * (AT_TILE >> 4);
+          ok = mbar_wait(bars + B_FULLK + ks, kph, abort_flag) &&
+               (g < 3u || mbar_wait(bars + B_PV + ((g - 3u) & 3u), ((g - 3u) >> 2) & 1u, abort_flag));
+          if (!ok) break;
+          fence_proxy_async();      // rows that came by cp.async
           tc_fence_after();
-          const uint32_t first = t > 0 ? 1u : 0u;
           __syncwarp();
           if (elect_one()) {
 #pragma unroll
-            for (int s8 = 0; s8 < 4; ++s8)
-              umma_ts_lo(tO, tS + s8 * 8, vlo + s8 * (2048 >> 4), dhi, idescPV, s8 > 0 ? 1u : first);
+            for (int s = 0; s < 8; ++s) {
+              const uint32_t off = (s >> 2) * ((QT * 128) >> 4) + (s & 3) * 2;      // 64-column block, 16 columns
+              umma_ss_lo(tS, qlo + off, b0 + off, dhi, idescQK, s > 0 ? 1u : 0u);
+            }
+            umma_commit(bars + B_QK + (g & 3u));
+            if (t + 1 == ntiles) umma_commit(bars + B_FREEQ);
           }
           __syncwarp();
-          if (!mbar_wait(bars + C_P + 1, tg & 1u, abort_flag)) break;
-          tc_fence_after();
-          if (elect_one()) {
-#pragma unroll
-            for (int s8 = 4; s8 < 8; ++s8)
-              umma_ts_lo(tO, tS + s8 * 8, vlo + s8 * (2048 >> 4), dhi, idescPV, 1u);
-            umma_commit(bars + C_PV);
-          }
-          __syncwarp();
-          if (more) {
-            if (!mbar_wait(bars + C_FULLK, (tg + 1) & 1u, abort_flag)) break;
-            tc_fence_after();
-            mma_qk();
-          }
-          ok = true;
+          tS = tS == tmem + 256 ? tmem : tS + 128;
+          if (++ks == A1_KST) { ks = 0; kph ^= 1u; }
         }
-        g0 += ntiles;
-        ++q;
+        ++nq;
+      }
+    } else {
+      // ================= P V =================
+      constexpr uint32_t idescPV = make_idesc_bf16(128, kD, false, true);
+      constexpr uint32_t dhi = sdesc_hi(1024);
+      const uint32_t vlo = sdesc_lo(base + A1_OFF_V, KT * 128);
+      const uint32_t tO = tmem + 3 * 128;
+      uint32_t g = 0, nq = 0, buf = 0, bph = 0;      // tiles, tasks with tiles, score buffer of the next tile and its phase
+      uint32_t vs = 0, vph = 0;                      // V slot and its phase
+      bool ok = true;
+      for (uint32_t n = 0; ok; ++n) {
+        const uint32_t sl = n & 1u;
+        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
+        __syncwarp();
+        if (end) break;
+        if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
+        if (ntiles == 0) continue;
+        // every softmax warp has read the O of the task before
+        if (!mbar_wait(bars + B_OFREE, (nq & 1u) ^ 1u, abort_flag)) break;
+        for (int t = 0; t < ntiles; ++t, ++g) {
+          const uint32_t v0 = vlo + vs * (AT_TILE >> 4), tS = tmem + buf * 128, add = t > 0 ? 1u : 0u;
+          ok = mbar_wait(bars + B_FULLV + vs, vph, abort_flag) && mbar_wait(bars + B_P + buf, bph, abort_flag);
+          if (!ok) break;
+          fence_proxy_async();      // rows that came by cp.async
+          tc_fence_after();
+          __syncwarp();
+          if (elect_one()) {
+#pragma unroll
+            for (int s8 = 0; s8 < 8; ++s8)
+              umma_ts_lo(tO, tS + s8 * 8, v0 + s8 * (2048 >> 4), dhi, idescPV, s8 > 0 ? 1u : add);
+            umma_commit(bars + B_PV + (g & 3u));
+          }
+          __syncwarp();
+          if (++buf == 3) { buf = 0; bph ^= 1u; }
+          if (++vs == A1_VST) { vs = 0; vph ^= 1u; }
+        }
+        ++nq;
       }
     }
   }
   __syncwarp();
   if (*abort_flag) {
     if (tid == 0 && status) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
-    // a wait gave up: let tile copies still in flight land before the shared memory is released
+    // a wait gave up: let copies still in flight land before the shared memory is released
     for (int i = 0; i < 100; ++i) __nanosleep(1000);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256);
+  if (warp == 0) tmem_dealloc(tmem, 512);
   // This kernel may have started while the kernel launched before it (the tasks above QT rows) was still
   // running.  No CTA leaves before that grid has completed and its results are visible, so that this grid's
   // completion, which later work in the stream waits for, implies the other's.  (Without a programmatic
@@ -1736,7 +1752,7 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
   // dependents at once.  Their CTAs cannot share an SM (shared memory), so the second kernel's CTAs move in
   // as the first kernel's CTAs run out of tasks and exit.  Later work in the stream waits for both as usual.
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * sms);
+  cfg.gridDim = dim3(sms);
   cfg.blockDim = dim3(A1_THREADS);
   cfg.dynamicSmemBytes = A1_SMEM;
   cfg.stream = st;
@@ -1745,8 +1761,9 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, attn_kernel, mq, kv, (const uint32_t*)unip, (const int*)qperm, attn_out, attn_lse,
-                         plan, H, N, CQ, q_row_step, q_head_step, d_status) != cudaSuccess)
+  if (cudaLaunchKernelEx(&cfg, attn_kernel, kv, (const __nv_bfloat16*)q, (const __nv_bfloat16*)kp, (const __nv_bfloat16*)vp,
+                         (const uint32_t*)unip, (const int*)qperm, attn_out, attn_lse, plan, H, N, CQ, q_row_step,
+                         q_head_step, d_status) != cudaSuccess)
     return T2T_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
