@@ -245,14 +245,21 @@ __device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr, uint32_t lbo_bytes)
 __host__ __device__ constexpr uint32_t sdesc_hi(uint32_t sbo_bytes) {
   return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
 }
+// K-major operand of 64-byte rows (32 16-bit elements) under 64-byte swizzle: 8-row groups 512 B apart.
+__host__ __device__ constexpr uint32_t sdesc_hi_64b() { return (512u >> 4) | (1u << 14) | (4u << 29); }
+// The operands' tiles may be laid out differently (ahi, bhi).
+__device__ __forceinline__ void umma_ss_lo2(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %6, 0;\n"
+      " mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %4};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n" ::"r"(d_tmem),
+      "r"(alo), "r"(blo), "r"(ahi), "r"(bhi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 __device__ __forceinline__ void umma_ss_lo(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc,
                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n"
-      " mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}\n" ::"r"(d_tmem),
-      "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
-      : "memory");
+  umma_ss_lo2(d_tmem, alo, hi, blo, hi, idesc, accumulate);
 }
 __device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t blo, uint32_t hi, uint32_t idesc,
                                            uint32_t accumulate) {

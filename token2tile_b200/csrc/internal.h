@@ -26,6 +26,9 @@ bool make_row_gather_map(void* map_out, const void* base, uint64_t rows);
 // Same matrix, box of 64 columns x `box_rows` rows: plain tile loads of contiguous rows.
 bool make_row_tile_map(void* map_out, const void* base, uint64_t rows, uint32_t box_rows);
 
+// The bf16 matrix base [rows, 32] with a box of 32 columns x `box_rows` rows and 64-byte swizzle: operand tiles of 64-byte rows.
+bool make_rank_tile_map(void* map_out, const void* base, uint64_t rows, uint32_t box_rows);
+
 // A bf16 tensor of `heads` x `rows_per_head` rows of 128 elements (row (h, n) at base + h * head_stride +
 // n * row_stride, strides in elements) as a 3D tensor with a 64-column x `box_rows`-row x 1-head box: tile
 // loads that never cross a head, rows past the head's last row read as zeros.

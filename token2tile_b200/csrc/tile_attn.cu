@@ -1298,17 +1298,17 @@ constexpr int TL_H = 64;                  // centroids per step
 constexpr int TL_NH = kC / TL_H;          // steps per CTA
 constexpr int TL_STAGES = 3;              // ring depth of the centroid and value-sum tiles
 constexpr int TL_SQ = TL_Q * 128;         // 16 KB: QU rows padded to 128 B
-constexpr int TL_SC = TL_H * 128;         // 8 KB per stage: cks rows padded to 128 B
+constexpr int TL_SC = TL_H * kR * 2;      // 4 KB per stage: cks rows of 64 B
 constexpr int TL_SV = TL_H * kD * 2;      // 16 KB per stage
 constexpr int TL_OFF_C = TL_SQ;
 constexpr int TL_OFF_V = TL_OFF_C + TL_STAGES * TL_SC;
 constexpr int TL_OFF_CNT = TL_OFF_V + TL_STAGES * TL_SV;
 constexpr int TL_OFF_BAR = TL_OFF_CNT + kC * 4;
-// 97 KB: two CTAs share an SM, and no more than two (tensor memory holds two 256-column allocations)
+// 85 KB: two CTAs share an SM, and no more than two (tensor memory holds two 256-column allocations)
 constexpr int TL_SMEM = TL_OFF_BAR + 128 + 1024;
 constexpr int TL_THREADS = 160;           // warps 0..3: one softmax thread per row; warp 4: the products
 static_assert(TL_NH % 2 == 0 && TL_NH >= 4, "the two score regions alternate");
-static_assert(3 * TL_SMEM > 227 * 1024, "at most two CTAs may share an SM");
+static_assert(3 * TL_SMEM > 228 * 1024, "at most two CTAs may share an SM");
 
 // Work is pipelined over steps of 64 centroids.  Tensor memory holds two 64-column score regions and the
 // 128-column accumulator T.  For step i (region b = i & 1):
@@ -1316,17 +1316,16 @@ static_assert(3 * TL_SMEM > 227 * 1024, "at most two CTAs may share an SM");
 //   softmax rows  wait sReady[b]; p = exp2(S_b - m) masked by the row's union, packed to bf16 into S_b;
 //                 arrive on pReady[b]
 //   MMA lane      wait pReady[b]; T += P_b sumv_i; S_b = QU cks_{i+2}^T; commit on sReady[b]
-// so the tensor work of one region runs under the softmax of the other.  Two rings feed the products.  The
-// softmax threads issue the cp.async copies of cks_{i+3} at the start of step i, into the stage that
-// sReady[b] has just declared free, and before arriving on pReady[b] they wait for the copy issued one step
-// earlier (cks_{i+2}), which the MMA lane is about to read.  The MMA lane itself fetches sumv_{i+1} with two
-// TMA tile loads once pReady[b] of step i shows that every row has seen the commit behind the product of
-// step i - 2, and waits for sumv_i on the stage's byte-counting barrier before T += P_b sumv_i.
+// so the tensor work of one region runs under the softmax of the other.  The MMA lane also feeds the products by TMA
+// tile loads, on byte-counting barriers: once pReady[b] of step i shows that every row has seen the commit behind the
+// products up to cks_i and sumv_{i-2}, it fetches cks_{i+3} and sumv_{i+1} into the stages those held.  (With the softmax
+// threads copying cks by cp.async, each waited for its copy and fenced the proxies in every step: 3.10 ms at 720p x 40
+// heads instead of 2.93.)
 __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
-    const __grid_constant__ CUtensorMap mapSumv, const __nv_bfloat16* __restrict__ attn_out,
+    const __grid_constant__ CUtensorMap mapSumv, const __grid_constant__ CUtensorMap mapCks,
+    const __nv_bfloat16* __restrict__ attn_out,
     const float* __restrict__ attn_lse,
-    const __nv_bfloat16* __restrict__ QU, const __nv_bfloat16* __restrict__ cks,
-    const int* __restrict__ ksz, const uint32_t* __restrict__ ub,
+    const __nv_bfloat16* __restrict__ QU, const int* __restrict__ ksz, const uint32_t* __restrict__ ub,
     const int* __restrict__ qlab, const int* __restrict__ qperm, const float* __restrict__ lam_s,
     const float* __restrict__ tailw_ptr, __nv_bfloat16* __restrict__ out, long long out_row_stride,
     long long out_head_stride, int N, int CQ,
@@ -1337,10 +1336,11 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
   const uint32_t sQ = base, sC = base + TL_OFF_C, sV = base + TL_OFF_V;
   float* sCnt = reinterpret_cast<float*>(sm + TL_OFF_CNT);
   uint64_t* sReady = reinterpret_cast<uint64_t*>(sm + TL_OFF_BAR);        // [2], one arrival (tcgen05.commit)
-  uint64_t* pReady = sReady + 2;                                          // [2], 128 arrivals
+  uint64_t* pReady = sReady + 2;                                          // [2], one arrival of every softmax warp
   uint64_t* vFull = sReady + 4;                                           // [TL_STAGES], bytes of one value-sum tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + TL_OFF_BAR + 64);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + TL_OFF_BAR + 80);
+  uint64_t* cFull = vFull + TL_STAGES;                                    // [TL_STAGES], bytes of one centroid tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + TL_OFF_BAR + 96);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + TL_OFF_BAR + 104);
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool soft = warp < 4;
@@ -1353,9 +1353,9 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
     *abort_flag = 0;
     mbar_init(sReady + 0, 1);
     mbar_init(sReady + 1, 1);
-    mbar_init(pReady + 0, TL_Q);
-    mbar_init(pReady + 1, TL_Q);
-    for (int st = 0; st < TL_STAGES; ++st) mbar_init(vFull + st, 1);
+    mbar_init(pReady + 0, TL_Q / 32);
+    mbar_init(pReady + 1, TL_Q / 32);
+    for (int st = 0; st < 2 * TL_STAGES; ++st) mbar_init(vFull + st, 1);
     mbar_init_fence();
   }
   const int j = qs + tid;
@@ -1364,23 +1364,8 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
   const int label = active ? qlab[(size_t)h * N + orig] : 0;
   const uint32_t* mrow = ub + ((size_t)h * CQ + label) * (kC / 32);
 
-  auto load_c = [&](int step) {   // centroid rows of one step: 64 rows x 64 B into 128-byte rows
-    const int ch = tid & 3, r0 = tid >> 2;
-    const __nv_bfloat16* src = cks + ((size_t)h * kC + step * TL_H) * kR + ch * 8;
-    const uint32_t dst = sC + (step % TL_STAGES) * TL_SC;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int r = r0 + 32 * u;
-      cp_async16(dst + sw128(r, ch), src + (size_t)r * kR, 16u);
-    }
-  };
   if (soft) {
-    // group 0: the copies that depend on nothing (centroids of steps 0..2) go first
-    load_c(0);
-    load_c(1);
-    load_c(2);
-    cp_async_commit();
-    // group 1: QU rows of the 128 sorted queries (64 B each, 4 chunks), behind the loads of their indices
+    // QU rows of the 128 sorted queries (64 B each, 4 chunks), behind the loads of their indices
     const int ch = tid & 3, r0 = tid >> 2;
     int o4[4];
 #pragma unroll
@@ -1429,26 +1414,40 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       }
       __syncwarp();
     };
+    auto load_c = [&](int step, int st) {
+      if (elect_one()) {
+        mbar_arrive_expect_tx(cFull + st, TL_SC);
+        tma_load_tile(sC + st * TL_SC, &mapCks, 0, h * kC + step * TL_H, cFull + st);
+      }
+      __syncwarp();
+    };
     // S_(step & 1) = QU cks_step^T, K = 32
     auto scores = [&](int b, int st) {
       const uint32_t c0 = clo + st * (TL_SC >> 4);
 #pragma unroll
-      for (int k = 0; k < 2; ++k) umma_ss_lo(tS + b * TL_H, qlo + k * 2, c0 + k * 2, dhi, idescS, k > 0 ? 1u : 0u);
+      for (int k = 0; k < 2; ++k)
+        umma_ss_lo2(tS + b * TL_H, qlo + k * 2, dhi, c0 + k * 2, sdesc_hi_64b(), idescS, k > 0 ? 1u : 0u);
       umma_commit(sReady + b);
     };
+    for (int step = 0; step < TL_STAGES; ++step) load_c(step, step);
     load_v(0, 0);
-    if (elect_one()) {
+    const bool there = mbar_wait(cFull + 0, 0, abort_flag) && mbar_wait(cFull + 1, 0, abort_flag);
+    tc_fence_after();
+    __syncwarp();
+    if (there && elect_one()) {
       scores(0, 0);
       scores(1, 1);
     }
     __syncwarp();
     int st = 0;      // stage of step i
-    for (int i = 0; i < TL_NH; ++i) {
+    for (int i = 0; there && i < TL_NH; ++i) {
       const int b = i & 1, st1 = st == TL_STAGES - 1 ? 0 : st + 1, st2 = st1 == TL_STAGES - 1 ? 0 : st1 + 1;
       if (!mbar_wait(pReady + b, (i >> 1) & 1, abort_flag)) break;
-      // every softmax thread has seen the commit behind the product of step i - 2: its stage is free
+      // every softmax thread has seen the commit behind S_i and the product of step i - 2: their stages are free
       if (i + 1 < TL_NH) load_v(i + 1, st1);
+      if (i + TL_STAGES < TL_NH) load_c(i + TL_STAGES, st);
       if (!mbar_wait(vFull + st, (i / TL_STAGES) & 1, abort_flag)) break;
+      if (i + 2 < TL_NH && !mbar_wait(cFull + st2, ((i + 2) / TL_STAGES) & 1, abort_flag)) break;
       tc_fence_after();
       const uint32_t v0 = vlo + st * (TL_SV >> 4), first = i > 0 ? 1u : 0u;
       __syncwarp();
@@ -1473,9 +1472,6 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       const int b = i & 1;
       if (!mbar_wait(sReady + b, (i >> 1) & 1, abort_flag)) { dead = true; break; }
       tc_fence_after();
-      // the stage of cks_i is free now
-      if (i + 3 < TL_NH) load_c(i + 3);
-      cp_async_commit();
       const uint2 mw2 = mw_next;
       if (i + 1 < TL_NH) mw_next = *reinterpret_cast<const uint2*>(mrow + (i + 1) * 2);
       float s[TL_H];
@@ -1568,11 +1564,9 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
       phi += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
       tmem_st32(tS_lane + b * TL_H, pk);
       tmem_wait_st();
-      // cks_{i+2} (issued one step ago) must have landed before the MMA lane reads it
-      cp_async_wait<1>();
-      fence_proxy_async();
       tc_fence_before();
-      mbar_arrive(pReady + b);
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(pReady + b);
     }
     // the row of the exact part is fetched while the last products finish
     const uint4* src = reinterpret_cast<const uint4*>(attn_out + ((size_t)h * N + (active ? j : 0)) * kD);
@@ -1620,9 +1614,13 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
         }
       }
     }
-    cp_async_wait<0>();
   }
-  if (*abort_flag && (tid & 31) == 0 && status) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
+  __syncwarp();
+  if (*abort_flag) {
+    if ((tid & 31) == 0 && status) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
+    // a wait gave up: let tile copies still in flight land before the shared memory is released
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 256);
@@ -1659,26 +1657,29 @@ const DeviceFacts* device_facts() {
   return f;
 }
 
-// Tensor maps are pure functions of (base address, rows, box rows): the operator passes the same few buffers on
+// Tensor maps are pure functions of (base address, rows, columns, box rows): the operator passes the same few buffers on
 // every call, so the last encodings are kept.
 struct MapSlot {
   const void* base;
   uint64_t rows;
   uint32_t box_rows;
+  int cols;
   CUtensorMap map;
 };
 std::mutex g_map_mutex;
-bool cached_row_map(CUtensorMap* out, const void* base, uint64_t rows, uint32_t box_rows) {
+bool cached_row_map(CUtensorMap* out, const void* base, uint64_t rows, uint32_t box_rows, int cols = kD) {
   static MapSlot slots[32] = {};
   static unsigned next = 0;
   std::lock_guard<std::mutex> lock(g_map_mutex);
   for (const MapSlot& s : slots)
-    if (s.base == base && s.rows == rows && s.box_rows == box_rows && s.base != nullptr) { *out = s.map; return true; }
+    if (s.base == base && s.rows == rows && s.box_rows == box_rows && s.cols == cols && s.base != nullptr) { *out = s.map; return true; }
   MapSlot fresh;
   fresh.base = base;
   fresh.rows = rows;
   fresh.box_rows = box_rows;
-  if (!make_row_tile_map(&fresh.map, base, rows, box_rows)) return false;
+  fresh.cols = cols;
+  if (!(cols == kD ? make_row_tile_map(&fresh.map, base, rows, box_rows) : make_rank_tile_map(&fresh.map, base, rows, box_rows)))
+    return false;
   slots[next++ % 32] = fresh;
   *out = fresh.map;
   return true;
@@ -1791,10 +1792,11 @@ extern "C" int t2t_tile_attn_merge_strided(const void* QU, const void* cks, cons
   split_ws(ws, H, N, &attn_out, &attn_lse);
   if (!device_facts()) return T2T_ERR_CUDA;
   // the value sums as an [H * 2048, 128] matrix, fetched 64 rows x 64 columns at a time
-  CUtensorMap msv;
-  if (!cached_row_map(&msv, sumv, (uint64_t)H * kC, TL_H)) return T2T_ERR_CUDA;
+  CUtensorMap msv, mck;
+  if (!cached_row_map(&msv, sumv, (uint64_t)H * kC, TL_H) || !cached_row_map(&mck, cks, (uint64_t)H * kC, TL_H, kR))
+    return T2T_ERR_CUDA;
   tail_kernel<<<dim3(cdiv(N, TL_Q), H), TL_THREADS, TL_SMEM, st>>>(
-      msv, attn_out, attn_lse, (const __nv_bfloat16*)QU, (const __nv_bfloat16*)cks, (const int*)kcounts, (const uint32_t*)unip, (const int*)qlab, (const int*)qperm, (const float*)lam, tailw,
+      msv, mck, attn_out, attn_lse, (const __nv_bfloat16*)QU, (const int*)kcounts, (const uint32_t*)unip, (const int*)qlab, (const int*)qperm, (const float*)lam, tailw,
       (__nv_bfloat16*)out, out_row_stride, out_head_stride, N, CQ, d_status);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
