@@ -27,9 +27,10 @@
 // for bit.  Rows that do not fit the fast path (more than 64 candidates, no
 // convergence, non-finite scores) are queued for the exact warp-per-row kernel.
 //
-// What bounds it: instruction issue, 22 instructions a score over the two passes, 60 % of the slots used, a third of
-// the warps' time at barriers.  6.4 ms for 40 heads x 75,600 rows (7.7 with 16 warps), 64 us for 2 x 4096 (263 with
-// four tiles to every CTA).
+// What bounds it: instruction issue, integer and compare instructions above all (half rate), and the warps' time at
+// barriers.  5.2 ms for 40 heads x 75,600 rows (6.06 with clamped and predicated histogram updates and the buckets
+// scanned one by one, 7.7 with 16 warps), 2.83 for 40 x 32,760 at 5 % (3.39), 52 us for 2 x 4096 (263 with four tiles to
+// every CTA).
 #include "common.cuh"
 #include "internal.h"
 
@@ -41,6 +42,7 @@ constexpr int ST_THREADS = ST_G * 128;     // 32 warps: the passes are chains of
 constexpr int ST_CH = 32;                  // centroids per MMA chunk
 constexpr int ST_NCH = kC / ST_CH;         // 64: eight per column group, double-buffered in TMEM
 constexpr int ST_B = 64;                   // histogram buckets
+constexpr int ST_HB = ST_B + 3;            // histogram rows: scores above the range, its buckets, scores below it (two)
 constexpr int ST_CAP = 64;                 // candidates per row
 constexpr int ST_REFINE = 40;              // refine the bucket when it alone holds more clusters than this
 constexpr int ST_MAX_ITERS = 5;
@@ -53,15 +55,17 @@ constexpr int ST_MAX_TPC = 8;              // consecutive 128-row tiles of one h
 // 4 heads x 75,600 rows, ms at a budget of 1.5 % / 5 % with 0.8, 1.0 and 1.25: the 3D locality mixture 0.80 / 0.86, 0.81 /
 // 0.89, 0.79 / 0.93; independent normal rows 0.85 / 0.97, 0.88 / 0.99, 0.90 / 1.02; heavy tails (Student, 3 degrees) 1.62 /
 // 1.83, 0.99 / 1.17, 0.97 / 1.31; smooth trajectories 1.05 / 0.80, 1.00 / 0.78, 0.86 / 0.80; half of the rows around one
-// centre 9.62, 1.50, 1.12 at 1.5 % (and 10 with any of them at 5 %: more than ST_CAP candidates).
+// centre 9.62, 1.50, 1.12 at 1.5 % (and 10 with any of them at 5 %: more than ST_CAP candidates).  Those are times of
+// predicated histogram updates; inputs like these take 0.66 / 0.76, 0.64 / 0.74, 0.62 / 0.71, 0.73 / 0.64 and 0.81 / 1.39
+// now (0.81 / 0.95, 0.82 / 0.93, 0.77 / 0.90, 0.82 / 0.71, 0.93 / 1.59 then).
 constexpr float ST_SPAN = 1.25f;
 constexpr int ST_STRAGGLERS = 8;           // this few unsettled rows of a tile go to the exact kernel instead of another pass
 
 constexpr int OFF_CK = 0;                               // 1024 rows x 128 B: centroid c in row c % 1024, half c / 1024
 constexpr int OFF_A = OFF_CK + 1024 * 128;              // 128 rows x 128 B: this tile's rows in one 64-byte half, the next tile's arrive in the other
-constexpr int OFF_HIST = OFF_A + 128 * 128;             // [ST_B][128] packed (size << 12 | count); after P2 the
+constexpr int OFF_HIST = OFF_A + 128 * 128;             // [ST_HB][128] packed (size << 12 | count); after P2 the
 constexpr int OFF_CAND = OFF_HIST;                      //   same bytes hold [128][ST_CAP] cluster | key << 16
-constexpr int OFF_SIZE = OFF_HIST + ST_B * 128 * 4;     // [2048] (cluster size << 12) + 1
+constexpr int OFF_SIZE = OFF_HIST + ST_HB * 128 * 4;    // [2048] (cluster size << 12) + 1
 constexpr int OFF_PART = OFF_SIZE + kC * 4;             // [2][ST_G][128] per-group partial sums
 constexpr int OFF_ROW = OFF_PART + 2 * ST_G * 128 * 4;        // [17][128] per-row scalars
 constexpr int ST_MAXSEG = 8;                            // query clusters one tile may span on the fast path
@@ -115,20 +119,17 @@ __device__ __forceinline__ unsigned long long fma_rm2(unsigned long long a, unsi
   asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ unsigned long long add_rm2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+// a b + c, clamped to [0, 1] (NaN to 0).
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-
-// Adds to bucket `b` of the histogram column at `col` if there is such a bucket.  (As a conditional atomicAdd this was a
-// branch around every update, 3.4 control instructions a score; predicated it is one.)
-__device__ __forceinline__ void hist_add(uint32_t col, int b, int value) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.lt.u32 p, %1, %3;\n"
-      " @p red.shared::cta.add.u32 [%0], %2;\n}\n" ::"r"(col + (uint32_t)b * 512u),
-      "r"(b), "r"(value), "n"(ST_B)
-      : "memory");
+// Adds to row f of the histogram column at `col`.  Every score is added somewhere: scores outside the range have rows of
+// their own, which costs less than a predicate (compare, clamp and predicate were three of six half-rate instructions a
+// score; 697 instead of 780 us at 5 heads x 75,600, 2.93 instead of 3.39 ms at 40 x 32,760 and 5 %).
+__device__ __forceinline__ void hist_add(uint32_t col, int f, int value) {
+  asm volatile("red.shared::cta.add.u32 [%0], %1;\n" ::"r"(col + (uint32_t)f * 512u), "r"(value) : "memory");
 }
 
 __device__ __forceinline__ void wg_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
@@ -440,25 +441,26 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       sRowF[R_HI * 128 + r] = hi;
       sRowF[R_LO * 128 + r] = lo;
       sRowI[R_OVF * 128 + r] = ovf;
-      sRowF[R_INV * 128 + r] = hi > lo ? (float)(ST_B - ovf) / (hi - lo) : 0.f;
+      sRowF[R_INV * 128 + r] = hi > lo ? (float)ST_B / (hi - lo) : 0.f;
       if (!finite) sRowI[R_STATE * 128 + r] = RS_QUEUE + 1;
     }
 
     // ---- P2: histogram search for the threshold bucket --------------------------
     for (int it = 0; it < ST_MAX_ITERS; ++it) {
-      for (int i = tid; i < ST_B * 128; i += ST_THREADS) sHist[i] = 0;
+      for (int i = tid; i < (ST_B + 1) * 128; i += ST_THREADS) sHist[i] = 0;
       __syncthreads();
       {
-        // bucket = floor((hi - s) * inv): s > hi gives a negative bucket; rows that are not searching get
-        // hi = -inf and fall out the same way
+        // Histogram row floor((hi - s) inv) + 1, clamped to 0 (above hi) and 65 or 66 (below lo) by a saturating
+        // multiply-add: u = ((hi - s) inv + 1) / 66 in [0, 1], and 66 u rounded down by an add to 1.5 * 2^23.  A score
+        // within a few rounding steps of a bucket boundary may land in the neighbouring bucket, which only moves the
+        // window (the selection is validated against exact keys afterwards).  Rows that are not searching get u = 1.
         const bool act = sRowI[R_STATE * 128 + r] == RS_SEARCH;
-        const float hi = act ? sRowF[R_HI * 128 + r] : -INFINITY;
-        const float inv = act ? sRowF[R_INV * 128 + r] : 1.0f;
-        // with an overflow bucket, bucket 0 takes every score above hi and the range starts at bucket 1
-        const int ovf = act ? sRowI[R_OVF * 128 + r] : 0;
-        const unsigned long long ninv2 = pack2(-inv, -inv), hiinv2 = pack2(hi * inv, hi * inv), magic2 = pack2(12582912.0f, 12582912.0f);
-        const int shift = 0x4B400000 - ovf, bmin = ovf - 1;
-        const uint32_t hist_r = smem_u32(sHist + r);
+        const float hi = act ? sRowF[R_HI * 128 + r] : 0.f;
+        const float inv = act ? sRowF[R_INV * 128 + r] : 0.f;
+        constexpr float kRows = (float)(ST_B + 2);
+        const float slope = -inv * (1.0f / kRows), at0 = act ? fmaf(hi, inv, 1.0f) * (1.0f / kRows) : 1.0f;
+        const unsigned long long rows2 = pack2(kRows, kRows), magic2 = pack2(12582912.0f, 12582912.0f);
+        const uint32_t hist_r = smem_u32(sHist + r) - 0x4B400000u * 512u;
         stream([&](int cbase, const uint32_t(&v)[32]) {
 #pragma unroll
           for (int j4 = 0; j4 < 32; j4 += 4) {
@@ -466,16 +468,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
             const int pp[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
             for (int e = 0; e < 4; e += 2) {
-              // floor by an add rounded toward -inf: 1.5 * 2^23 + t has floor(t) in its low mantissa bits for
-              // |t| < 2^22; beyond that the difference keeps the sign of t and is far outside [0, ST_B).
-              // t = (hi - s) inv as one multiply-add: a score within a rounding step of a bucket boundary may
-              // land in the neighbouring bucket, which only moves the window (the selection is validated
-              // against exact keys afterwards).  Two scores per instruction.
-              const unsigned long long t2 = fma_rm2(pack2(__uint_as_float(v[j4 + e]), __uint_as_float(v[j4 + e + 1])), ninv2, hiinv2);
+              const float u0 = fma_sat(__uint_as_float(v[j4 + e]), slope, at0), u1 = fma_sat(__uint_as_float(v[j4 + e + 1]), slope, at0);
               float f0, f1;
-              unpack2(add_rm2(t2, magic2), f0, f1);
-              hist_add(hist_r, max(__float_as_int(f0) - shift, bmin), pp[e]);
-              hist_add(hist_r, max(__float_as_int(f1) - shift, bmin), pp[e + 1]);
+              unpack2(fma_rm2(pack2(u0, u1), rows2, magic2), f0, f1);
+              hist_add(hist_r, __float_as_int(f0), pp[e]);
+              hist_add(hist_r, __float_as_int(f1), pp[e + 1]);
             }
           }
         });
@@ -493,12 +490,21 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
           const int p = sHist[r];
           if (cum + (p >> 12) >= ns) above = true; else cum += p >> 12;
         }
-        for (int b = ovf; b < ST_B && !above; ++b) {
-          const int p = sHist[b * 128 + r];
-          if (cum + (p >> 12) >= ns) { bstar = b - ovf; cnt = p & 4095; break; }
-          cum += p >> 12;
+        // eight buckets at a time, so that their loads overlap
+        for (int b0 = 0; b0 < ST_B && !above && bstar < 0; b0 += 8) {
+          int p[8], sum = 0;
+#pragma unroll
+          for (int b = 0; b < 8; ++b) p[b] = sHist[(b0 + b + 1) * 128 + r];
+#pragma unroll
+          for (int b = 0; b < 8; ++b) sum += p[b] >> 12;
+          if (cum + sum < ns) { cum += sum; continue; }
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            if (bstar >= 0) break;
+            if (cum + (p[b] >> 12) >= ns) { bstar = b0 + b; cnt = p[b] & 4095; } else cum += p[b] >> 12;
+          }
         }
-        const float w = (hi - lo) / (float)(ST_B - ovf);
+        const float w = (hi - lo) / (float)ST_B;
         if (above) {
           // continue between hi and the row maximum (nothing has been added to cum)
           if (it + 1 < ST_MAX_ITERS) {
