@@ -742,24 +742,47 @@ __global__ void pin_bit_kernel(int* __restrict__ unip, int rows) {
 
 // First two moments of a head's scaled key centroids, as kMomParts partial sums (one CTA per slice of
 // C / kMomParts centroids): mom[h][p] = { sum_c c / C (32), sum_c c c^T / C (32 x 32) } over the slice.
+// Bound by shared-memory loads: a warp takes four rows of the matrix and a quarter of the slice, so that a centroid costs
+// it two loads for four products (one row a warp over the whole slice, two loads a product: 12 us at 2 heads, 36 at 40).
+// The kernel also clears the unions and the queue's counts for the selection behind it.
 __global__ void __launch_bounds__(1024) centroid_moments_kernel(const __nv_bfloat16* __restrict__ cks,
-                                                                float* __restrict__ mom) {
-  constexpr int SLICE = kC / kMomParts;
-  __shared__ float sc[SLICE][kR + 1];
-  const int h = blockIdx.y, part = blockIdx.x, a = threadIdx.x >> 5, b = threadIdx.x & 31;
+                                                                float* __restrict__ mom, int* __restrict__ unip, int CQ,
+                                                                int* __restrict__ fixq, int N) {
+  constexpr int SLICE = kC / kMomParts, QUARTER = SLICE / 4, LD = kR + 4;
+  __shared__ __align__(16) float sc[SLICE][LD];
+  static_assert(SLICE * LD >= 4 * (kR * kR + kR), "the quarters' sums take the centroids' place");
+  const int h = blockIdx.y, part = blockIdx.x, warp = threadIdx.x >> 5, b = threadIdx.x & 31;
   const __nv_bfloat16* ch = cks + ((size_t)h * kC + (size_t)part * SLICE) * kR;
   for (int i = threadIdx.x; i < SLICE * kR; i += 1024) sc[i >> 5][i & 31] = bf_to_f(ch[i]);      // coalesced
+  for (int i = part * 1024 + threadIdx.x; i < CQ * 64; i += kMomParts * 1024) unip[(size_t)h * CQ * 64 + i] = 0;
+  if (part == 0 && threadIdx.x == 0) fixq[(size_t)h * (2 * (size_t)N + 1)] = 0;
   __syncthreads();
-  float g0 = 0.f, g1 = 0.f, m0 = 0.f;
-#pragma unroll 4
-  for (int c = 0; c < SLICE; c += 2) {
-    g0 = fmaf(sc[c][a], sc[c][b], g0);
-    g1 = fmaf(sc[c + 1][a], sc[c + 1][b], g1);
-    m0 += sc[c][b] + sc[c + 1][b];
+  const int a0 = 4 * (warp & 7), c0 = (warp >> 3) * QUARTER;
+  float g[4] = {0.f, 0.f, 0.f, 0.f}, m0 = 0.f;
+#pragma unroll 8
+  for (int c = c0; c < c0 + QUARTER; ++c) {
+    const float4 x = *reinterpret_cast<const float4*>(&sc[c][a0]);
+    const float y = sc[c][b];
+    g[0] = fmaf(x.x, y, g[0]);
+    g[1] = fmaf(x.y, y, g[1]);
+    g[2] = fmaf(x.z, y, g[2]);
+    g[3] = fmaf(x.w, y, g[3]);
+    m0 += y;
   }
+  __syncthreads();
+  float (*part_sum)[kR * kR + kR] = reinterpret_cast<float (*)[kR * kR + kR]>(&sc[0][0]);
+  float* mine = part_sum[warp >> 3];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) mine[(a0 + i) * 32 + b] = g[i];
+  if ((warp & 7) == 0) mine[kR * kR + b] = m0;
+  __syncthreads();
   float* mh = mom + ((size_t)h * kMomParts + part) * kMomFloats;
-  mh[32 + a * 32 + b] = (g0 + g1) * (1.0f / kC);
-  if (a == 0) mh[b] = m0 * (1.0f / kC);
+  const int i = threadIdx.x;
+  mh[32 + i] = ((part_sum[0][i] + part_sum[1][i]) + (part_sum[2][i] + part_sum[3][i])) * (1.0f / kC);
+  if (i < kR) {
+    const int j = kR * kR + i;
+    mh[i] = ((part_sum[0][j] + part_sum[1][j]) + (part_sum[2][j] + part_sum[3][j])) * (1.0f / kC);
+  }
 }
 
 static size_t select_queue_bytes(int H, int N) { return ((size_t)H * (2 * (size_t)N + 1) * sizeof(int) + 255) & ~(size_t)255; }
@@ -783,10 +806,7 @@ extern "C" int t2t_score_select_union(const void* QU, const void* cks, const voi
                                         st);
   int* fixq = (int*)ws;
   float* mom = reinterpret_cast<float*>((char*)ws + select_queue_bytes(H, N));
-  centroid_moments_kernel<<<dim3(kMomParts, H), 1024, 0, st>>>((const __nv_bfloat16*)cks, mom);
-  if (cudaMemsetAsync(fixq, 0, select_queue_bytes(H, N), st) != cudaSuccess ||
-      cudaMemsetAsync(unip, 0, (size_t)H * CQ * 64 * sizeof(int), st) != cudaSuccess)
-    return T2T_ERR_CUDA;
+  centroid_moments_kernel<<<dim3(kMomParts, H), 1024, 0, st>>>((const __nv_bfloat16*)cks, mom, (int*)unip, CQ, fixq, N);
   if (cudaFuncSetAttribute(select_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM) != cudaSuccess)
     return T2T_ERR_CUDA;
   // Tiles per CTA: as many as still leave every SM several CTAs, so that the last wave is short (with four always,

@@ -35,12 +35,12 @@ constexpr int PAIR_ROWS = 128;
 constexpr int KT = 128;          // keys per tile
 constexpr int MAX_RUNS = 1024;   // runs of selected clusters in one union
 constexpr int PLAN_SORT_MAX = 2048;
-constexpr int PLAN_HDR = 8;      // counters: [0] tasks, [1] cursor of the one-tile kernel, [2..3] executed pairs (lo, hi),
-                                 //           [4] cursor of the two-tile kernel
+constexpr int PLAN_THREADS = 1024;
+constexpr int PLAN_HDR = 8;      // counters: [0] tasks, [1] cursor of attn_kernel, [2] cursor of attn2_kernel
 
 // Layout of the plan (an int32 array owned by a structure snapshot): first row of every key cluster in kp / vp,
-// one bit per key cluster saying whether it holds any token, the counters (on a 16-byte boundary: the pair
-// count is a 64-bit atomic), the tasks, and the union length of every query cluster.
+// one bit per key cluster saying whether it holds any token, the counters (on a 16-byte boundary, as the tasks behind
+// them), the tasks, and the union length of every query cluster.
 __host__ __device__ inline size_t plan_nonempty_offset(int H) { return (size_t)H * (kC + 1); }
 __host__ __device__ inline size_t plan_counter_offset(int H) { return (plan_nonempty_offset(H) + (size_t)H * (kC / 32) + 3) & ~(size_t)3; }
 __host__ __device__ inline size_t plan_task_offset(int H) { return plan_counter_offset(H) + PLAN_HDR; }
@@ -72,62 +72,51 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // ---------------------------------------------------------------------------
 // plan: key-cluster offsets, union lengths, tasks (most work first inside a head)
 // ---------------------------------------------------------------------------
-// Exclusive prefix of v over the 256 threads of the CTA (every thread calls it); scratch holds 8 ints.
-__device__ __forceinline__ int block_prefix_256(int v, int* scratch, int& total) {
+// Exclusive prefix of v over the PLAN_THREADS threads of the CTA (every thread calls it); scratch holds 32 ints.
+__device__ __forceinline__ int block_prefix(int v, int* scratch, int& total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int inc = warp_incl_scan(v, lane);
   __syncthreads();
   if (lane == 31) scratch[w] = inc;
   __syncthreads();
-  int before = 0, all = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int part = scratch[i];
-    before += i < w ? part : 0;
-    all += part;
-  }
-  total = all;
-  return before + inc - v;
+  const int part = scratch[lane], parts = warp_incl_scan(part, lane);
+  total = __shfl_sync(0xffffffffu, parts, 31);
+  return __shfl_sync(0xffffffffu, parts - part, w) + inc - v;
 }
+static_assert(PLAN_THREADS == 32 * 32 && kC == 2 * PLAN_THREADS, "a warp scans the warps' sums; two key clusters a thread");
 
 // One CTA per head.  A query cluster of n rows gives ceil(n / TASK_ROWS) tasks: full ones first, the remainder
 // last (a remainder of at most QT rows costs one row tile instead of two).
-__global__ void __launch_bounds__(256) plan_kernel(const int* __restrict__ qcount, const int* __restrict__ kcount,
-                                                   const uint32_t* __restrict__ ubits, int H, int N, int CQ,
-                                                   int* __restrict__ plan) {
+// Bound by the latency of its steps (H CTAs in all): with 256 threads, which also went through the heads before theirs
+// one after the other, 114 us at 40 heads of 720p and 20 at 2 x 4096.
+__global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(const int* __restrict__ qcount, const int* __restrict__ kcount,
+                                                            const uint32_t* __restrict__ ubits, int H, int N, int CQ,
+                                                            int* __restrict__ plan) {
   __shared__ int s_off[kC + 1];
   __shared__ unsigned long long s_key[PLAN_SORT_MAX];
-  __shared__ int s_scan[8];
+  __shared__ int s_scan[32];
   const PlanView pv = plan_view(plan, H, N, CQ);
   const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-  // first kp / vp row of every key cluster (eight consecutive clusters per thread) and the non-empty bits
+  // first kp / vp row of every key cluster (two consecutive clusters per thread) and the non-empty bits
   {
-    int c8[8], sum = 0;
-    uint32_t some = 0u;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      c8[i] = kcount[(size_t)h * kC + tid * 8 + i];
-      sum += c8[i];
-      some |= (c8[i] > 0 ? 1u : 0u) << i;
-    }
+    const int2 c2 = make_int2(kcount[(size_t)h * kC + tid * 2], kcount[(size_t)h * kC + tid * 2 + 1]);
     int total;
-    int run = block_prefix_256(sum, s_scan, total);
+    const int run = block_prefix(c2.x + c2.y, s_scan, total);
+    s_off[tid * 2] = run;
+    s_off[tid * 2 + 1] = run + c2.x;
+    if (tid == PLAN_THREADS - 1) s_off[kC] = total;
+    // sixteen neighbouring threads hold the bits of one 32-cluster word
+    uint32_t word = ((c2.x > 0 ? 1u : 0u) | (c2.y > 0 ? 2u : 0u)) << (2 * (tid & 15));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { s_off[tid * 8 + i] = run; run += c8[i]; }
-    if (tid == 255) s_off[kC] = run;
-    // four neighbouring threads hold the four bytes of one 32-cluster word
-    uint32_t word = some << (8 * (tid & 3));
-    word |= __shfl_xor_sync(0xffffffffu, word, 1);
-    word |= __shfl_xor_sync(0xffffffffu, word, 2);
-    if ((tid & 3) == 0) pv.nonempty[(size_t)h * (kC / 32) + (tid >> 2)] = word;
+    for (int d = 8; d > 0; d >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, d);
+    if ((tid & 15) == 0) pv.nonempty[(size_t)h * (kC / 32) + (tid >> 4)] = word;
   }
   __syncthreads();
-  for (int i = tid; i <= kC; i += 256) pv.k_off[(size_t)h * (kC + 1) + i] = s_off[i];
+  for (int i = tid; i <= kC; i += PLAN_THREADS) pv.k_off[(size_t)h * (kC + 1) + i] = s_off[i];
 
-  // tokens in the union of every query cluster (a warp per cluster), and the pairs the head executes
-  unsigned long long pairs = 0;
-  for (int c = warp; c < CQ; c += 8) {
+  // tokens in the union of every query cluster (a warp per cluster)
+  for (int c = warp; c < CQ; c += PLAN_THREADS / 32) {
     const int n = qcount[(size_t)h * CQ + c];
     int len = 0;
     if (n > 0) {
@@ -142,34 +131,29 @@ __global__ void __launch_bounds__(256) plan_kernel(const int* __restrict__ qcoun
       }
     }
     len = __reduce_add_sync(0xffffffffu, len);
-    if (lane == 0) {
-      pv.kv_lens[(size_t)h * CQ + c] = len;
-      pairs += (unsigned long long)n * (unsigned long long)len;
-    }
+    if (lane == 0) pv.kv_lens[(size_t)h * CQ + c] = len;
   }
-  if (lane == 0 && pairs) atomicAdd(reinterpret_cast<unsigned long long*>(pv.counters + 2), pairs);
-  __syncthreads();
 
   // the task array is head-major (the K / V rows of a head stay in L2 while its unions are read):
   // count the tasks of the heads before this one
-  int first = 0, mine = 0;
-  for (int hh = 0; hh <= h; ++hh) {
-    int cnt = 0;
-    for (int c = tid; c < CQ; c += 256) cnt += cdiv(qcount[(size_t)hh * CQ + c], TASK_ROWS);
-    int total;
-    block_prefix_256(cnt, s_scan, total);
-    if (hh < h) first += total; else mine = total;
+  int first, mine;
+  {
+    int before = 0, own = 0;
+    for (int i = tid; i < h * CQ; i += PLAN_THREADS) before += cdiv(qcount[i], TASK_ROWS);
+    for (int i = tid; i < CQ; i += PLAN_THREADS) own += cdiv(qcount[(size_t)h * CQ + i], TASK_ROWS);
+    block_prefix(before, s_scan, first);
+    block_prefix(own, s_scan, mine);
   }
   if (h == H - 1 && tid == 0) pv.counters[0] = first + mine;
 
   int rows_before = 0, tasks_before = 0;
-  for (int c0 = 0; c0 < CQ; c0 += 256) {
+  for (int c0 = 0; c0 < CQ; c0 += PLAN_THREADS) {
     const int c = c0 + tid;
     const int n = c < CQ ? qcount[(size_t)h * CQ + c] : 0;
     const int nt = cdiv(n, TASK_ROWS);
     int tot_rows, tot_tasks;
-    const int row0 = rows_before + block_prefix_256(n, s_scan, tot_rows);
-    const int task0 = tasks_before + block_prefix_256(nt, s_scan, tot_tasks);
+    const int row0 = rows_before + block_prefix(n, s_scan, tot_rows);
+    const int task0 = tasks_before + block_prefix(nt, s_scan, tot_tasks);
     for (int i = 0; i < nt; ++i)
       pv.tasks[first + task0 + i] = make_int4(h, c, row0 + i * TASK_ROWS, min(TASK_ROWS, n - i * TASK_ROWS));
     rows_before += tot_rows;
@@ -181,7 +165,7 @@ __global__ void __launch_bounds__(256) plan_kernel(const int* __restrict__ qcoun
   // most work first (rows x union length); equal work keeps its order
   int pow2 = 2;
   while (pow2 < mine) pow2 <<= 1;
-  for (int i = tid; i < pow2; i += 256) {
+  for (int i = tid; i < pow2; i += PLAN_THREADS) {
     unsigned long long key = 0ull;
     if (i < mine) {
       const int4 t = pv.tasks[first + i];
@@ -193,7 +177,7 @@ __global__ void __launch_bounds__(256) plan_kernel(const int* __restrict__ qcoun
   __syncthreads();
   for (int span = 2; span <= pow2; span <<= 1) {
     for (int step = span >> 1; step > 0; step >>= 1) {
-      for (int i = tid; i < pow2; i += 256) {
+      for (int i = tid; i < pow2; i += PLAN_THREADS) {
         const int j = i ^ step;
         if (j > i) {
           const unsigned long long x = s_key[i], y = s_key[j];
@@ -204,16 +188,33 @@ __global__ void __launch_bounds__(256) plan_kernel(const int* __restrict__ qcoun
       __syncthreads();
     }
   }
-  int4 keep[PLAN_SORT_MAX / 256];
+  int4 keep[PLAN_SORT_MAX / PLAN_THREADS];
   int k = 0;
-  for (int i = tid; i < mine; i += 256) keep[k++] = pv.tasks[first + (int)(0xFFFFFFFFu - (unsigned)(s_key[i] & 0xFFFFFFFFull))];
+  for (int i = tid; i < mine; i += PLAN_THREADS) keep[k++] = pv.tasks[first + (int)(0xFFFFFFFFu - (unsigned)(s_key[i] & 0xFFFFFFFFull))];
   __syncthreads();
   k = 0;
-  for (int i = tid; i < mine; i += 256) pv.tasks[first + i] = keep[k++];
+  for (int i = tid; i < mine; i += PLAN_THREADS) pv.tasks[first + i] = keep[k++];
 }
 
-__global__ void plan_info_kernel(const int* __restrict__ counters, int* __restrict__ info) {
-  if (threadIdx.x < 4) info[threadIdx.x] = threadIdx.x == 0 ? counters[0] : (threadIdx.x < 3 ? counters[threadIdx.x + 1] : 0);
+// info: tasks, executed (query, key) pairs (low and high word), 0
+__global__ void __launch_bounds__(1024) plan_info_kernel(PlanView pv, int CQ, int* __restrict__ info) {
+  __shared__ unsigned long long s_pairs;
+  if (threadIdx.x == 0) s_pairs = 0ull;
+  __syncthreads();
+  const int tasks = pv.counters[0];
+  unsigned long long pairs = 0ull;
+  for (int i = threadIdx.x; i < tasks; i += 1024) {
+    const int4 t = pv.tasks[i];
+    pairs += (unsigned long long)t.w * (unsigned long long)pv.kv_lens[(size_t)t.x * CQ + t.y];
+  }
+  atomicAdd(&s_pairs, pairs);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    info[0] = tasks;
+    info[1] = (int)(uint32_t)s_pairs;
+    info[2] = (int)(uint32_t)(s_pairs >> 32);
+    info[3] = 0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -755,7 +756,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         if (!mbar_wait(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
-          do { task = atomicAdd(&pv.counters[4], 1); } while (task < numTasks && pv.tasks[task].w <= PAIR_ROWS);
+          do { task = atomicAdd(&pv.counters[2], 1); } while (task < numTasks && pv.tasks[task].w <= PAIR_ROWS);
           task = min(task, numTasks);
         }
         task = __shfl_sync(0xffffffffu, task, 0);
@@ -1702,9 +1703,7 @@ static void split_ws(void* ws, int H, int N, __nv_bfloat16** attn_out, float** a
 extern "C" int t2t_tile_attn_plan(const void* tile_sizes, const void* kcounts, const void* unip, int* plan, int H,
                                   int N, int CQ, cudaStream_t st) {
   if (!tile_sizes || !kcounts || !unip || !plan || H <= 0 || N <= 0 || CQ <= 0) return T2T_ERR_ARG;
-  const PlanView pv = plan_view(plan, H, N, CQ);
-  if (cudaMemsetAsync(pv.counters, 0, PLAN_HDR * sizeof(int), st) != cudaSuccess) return T2T_ERR_CUDA;
-  plan_kernel<<<H, 256, 0, st>>>((const int*)tile_sizes, (const int*)kcounts, (const uint32_t*)unip, H, N, CQ, plan);
+  plan_kernel<<<H, PLAN_THREADS, 0, st>>>((const int*)tile_sizes, (const int*)kcounts, (const uint32_t*)unip, H, N, CQ, plan);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
 
@@ -1729,10 +1728,8 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
   float* attn_lse;
   split_ws(ws, H, N, &attn_out, &attn_lse);
   const PlanView pv = plan_view(plan, H, N, CQ);
-  // the task cursor is the only per-dispatch state of a prepared plan
-  if (cudaMemsetAsync(pv.counters + 1, 0, sizeof(int), st) != cudaSuccess ||
-      cudaMemsetAsync(pv.counters + 4, 0, sizeof(int), st) != cudaSuccess)
-    return T2T_ERR_CUDA;
+  // the task cursors are the only per-dispatch state of a prepared plan
+  if (cudaMemsetAsync(pv.counters + 1, 0, 2 * sizeof(int), st) != cudaSuccess) return T2T_ERR_CUDA;
   const DeviceFacts* facts = device_facts();
   if (!facts) return T2T_ERR_CUDA;
   const int sms = facts->sms;
@@ -1818,6 +1815,6 @@ extern "C" int t2t_tile_attn(const void* q, const void* kp, const void* vp, cons
 extern "C" int t2t_tile_attn_plan_info(const int* plan, int H, int N, int CQ, int* d_info, cudaStream_t st) {
   if (!plan || !d_info) return T2T_ERR_ARG;
   const PlanView pv = plan_view(const_cast<int*>(plan), H, N, CQ);
-  plan_info_kernel<<<1, 32, 0, st>>>(pv.counters, d_info);
+  plan_info_kernel<<<1, 1024, 0, st>>>(pv, CQ, d_info);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
