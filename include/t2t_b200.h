@@ -259,6 +259,16 @@ int t2t_gather4_selftest(const void* src, int rows, const int* gidx, void* out, 
  * kernel always terminates.  No counterpart in the reference. */
 int t2t_wait_timeout_selftest(int* d_status, int* d_out, cudaStream_t stream);
 
+/* Give-up path of the attention kernels' softmax warps: one CTA runs them on a task of 128 rows and
+ * two key tiles.  `commits` says which products are reported complete (bits 0, 1: the scores of tile 0,
+ * 1; bits 2, 3: the weighted sum behind tile 0, 1), `handed` which lanes of a warp find a row's maximum
+ * behind tile 0 in place beforehand.  What is missing never comes: the waits for it run out within
+ * milliseconds, d_left[0..7] = 1 (every warp left), *d_status becomes 1 (wait timed out).  out [128, 128]
+ * bf16 and lse [128] are written if nothing is missing: ones, log 256.  The kernel always terminates.  No
+ * counterpart in the reference. */
+int t2t_softmax_give_up_selftest(int commits, unsigned handed, void* out, float* lse, int* d_left, int* d_status,
+                                 cudaStream_t stream);
+
 /* Rotation self-test: for n triples (squared lengths alpha, beta of two columns and
  * their product gamma, gamma != 0) writes tan, cos and sin of the angle that the
  * projection fit's Jacobi rounds turn them by.  No counterpart in the reference. */

@@ -60,6 +60,28 @@ def test_bounded_wait_gives_up_cleanly(lib):
     assert float((torch.ones(4, device=DEV) * 2).sum()) == 8.0      # the device still works
 
 
+def _softmax_give_up(lib, commits, handed):
+    out = torch.full((128, 128), -1.0, dtype=BF, device=DEV)
+    lse = torch.full((128,), -1.0, device=DEV)
+    left = torch.zeros(8, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    _ok(lib.t2t_softmax_give_up_selftest(commits, handed, out.data_ptr(), lse.data_ptr(), left.data_ptr(),
+                                         status.data_ptr(), _st()))
+    torch.cuda.synchronize()
+    assert left.tolist() == [1] * 8
+    return int(status.item()), out.float().cpu(), lse.cpu()
+
+
+@pytest.mark.parametrize("commits, handed", [(0, 0), (0, 0xffffffff), (2, 0), (2, 1), (2, 0x55555555), (2, 0xffff0000),
+                                             (2, 0xfffffffe)])
+def test_softmax_warps_give_up_as_warps(lib, commits, handed):
+    """No scores at all, or those of tile 1 alone, with the maximum behind tile 0 there for no lane of a warp, one, half of
+    them, all but one: the lanes that have it must not go on to warp-collective instructions without the others."""
+    status, out, lse = _softmax_give_up(lib, commits, handed)
+    assert status == 1 and bool((out == -1).all()) and bool((lse == -1).all())
+    assert float((torch.ones(4, device=DEV) * 2).sum()) == 8.0      # the device still works
+
+
 def test_umma_selftest(lib):
     g = torch.Generator().manual_seed(7)
     A = (torch.randn(128, 128, generator=g) * 0.5).to(BF)

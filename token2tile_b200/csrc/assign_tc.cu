@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
       augment(jn, (i + 1) & 1);
       fence_proxy_async();
     }
-    if (!mbar_wait(bar, ph, abort_flag)) { dead = true; break; }
+    if (!mbar_wait_warp(bar, ph, abort_flag)) { dead = true; break; }
     ph ^= 1u;
     tc_fence_after();
     const int cbase = j * TA_CH;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(TA_THREADS, 4) assign_tc_kernel(const __nv_bfl
           tc_fence_after();
           issue(st, tmem);
         }
-        if (!mbar_wait(bar, ph, abort_flag)) {
+        if (!mbar_wait_warp(bar, ph, abort_flag)) {
           if (tid == 0 && status) atomicExch(status, ST_WAIT_TIMEOUT);
           break;
         }

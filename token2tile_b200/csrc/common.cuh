@@ -114,7 +114,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait.  Returns false when it gave up (or another thread already
+// Bounded wait of one thread.  Returns false when it gave up (or another thread already
 // raised `*abort_flag`); the caller must then leave its loops, skip further
 // waits and fall through to the kernel's common exit so TMEM is released.
 // The bound is `limit` tries or `limit` x 1024 cycles, whichever comes first (about two seconds for
@@ -134,6 +134,52 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_wait_limited(bar, parity, abort_flag, kWaitSpinLimit);
+}
+// The same wait by a whole warp: votes give all of its lanes one answer, so that a caller may go on to warp-collective
+// instructions (votes, elect.sync, tcgen05.ld / st, named barriers) or leave for its exit as a warp.  Lane by lane, the limit
+// or the abort flag can be seen by some lanes while others still see the phase complete, and a collective with lanes missing
+// may never end.  The vote on a look takes its predicate as it comes, without a detour over a register: 0.5 % of the exact
+// attention's time (1.5 % with one vote on the answer of mbar_wait_limited).
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " vote.sync.all.pred p, p, 0xffffffff;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_wait_warp(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      " vote.sync.all.pred p, p, 0xffffffff;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitHintNs)
+      : "memory");
+  return ok != 0;
+}
+// `tries` looks once, with a vote, and may park.
+template <typename Try>
+__device__ __forceinline__ bool keep_trying_warp(Try&& tries, volatile int* abort_flag, uint32_t limit) {
+  const long long t0 = clock64();
+  for (uint32_t it = 0; it < limit; ++it) {
+    if (tries()) return true;
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+    if (__any_sync(0xffffffffu, clock64() - t0 > ((long long)limit << 10))) break;
+  }
+  *abort_flag = 1;
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                               uint32_t limit = kWaitSpinLimit) {
+  if (mbar_test_warp(bar, parity)) return true;
+  return keep_trying_warp([&] { return mbar_try_wait_warp(bar, parity); }, abort_flag, limit);
 }
 
 // ---- TMA row gather ----------------------------------------------------------
@@ -305,28 +351,21 @@ __device__ __forceinline__ void mbar_arrive_peer(uint32_t bar) {
 __device__ __forceinline__ void mbar_release_peer(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-// mbar_wait for a barrier of this CTA that threads of the other CTA arrive on as well.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+// mbar_wait_warp for a barrier of this CTA that threads of the other CTA arrive on as well.
+__device__ __forceinline__ bool mbar_try_wait_warp_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n .reg .pred p;\n"
       " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
+      " vote.sync.all.pred p, p, 0xffffffff;\n"
       " selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
       : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitHintNs)
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (uint32_t it = 0; it < kWaitSpinLimit; ++it) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > ((long long)kWaitSpinLimit << 10)) break;
-  }
-  *abort_flag = 1;
-  return false;
+__device__ __forceinline__ bool mbar_wait_warp_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return keep_trying_warp([&] { return mbar_try_wait_warp_cluster(bar, parity); }, abort_flag, kWaitSpinLimit);
 }
 // tma_gather4 / tma_load_tile into this CTA's shared memory with the bytes counted on a barrier of either CTA.
 __device__ __forceinline__ void tma_gather4_pair(uint32_t dst, const void* map, int col, int r0, int r1, int r2, int r3,

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) gram_kernel(const __grid_constant__ CUten
     umma_commit(done);
   }
   __syncwarp();
-  const bool ok = mbar_wait(done, 0, abort_flag);
+  const bool ok = mbar_wait_warp(done, 0, abort_flag);
   tc_fence_after();
   if (ok) {
     float* dst = partial + ((size_t)m * slabs + slab) * (kD * kD) + (size_t)tid * kD;

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(128) project_kernel(const __nv_bfloat16* __res
     }
     umma_commit(bar);
   }
-  const bool ok = mbar_wait(bar, 0, abort_flag);
+  const bool ok = mbar_wait_warp(bar, 0, abort_flag);
   tc_fence_after();
   if (ok) {
     uint32_t v[32];
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(128) umma_selftest_kernel(const __nv_bfloat16*
     }
     umma_commit(bars + 0);
   }
-  bool ok = mbar_wait(bars + 0, 0, abort_flag);
+  bool ok = mbar_wait_warp(bars + 0, 0, abort_flag);
   tc_fence_after();
   if (ok) {
     uint32_t p[64];
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(128) umma_selftest_kernel(const __nv_bfloat16*
     }
     umma_commit(bars + 1);
   }
-  ok = ok && mbar_wait(bars + 1, 0, abort_flag);
+  ok = ok && mbar_wait_warp(bars + 1, 0, abort_flag);
   tc_fence_after();
   if (ok) {
 #pragma unroll

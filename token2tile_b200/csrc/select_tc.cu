@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
       tc_fence_before();
       wg_sync(g);
       if ((warp & 3) == 0 && i + 1 < ST_NCH / ST_G) issue(i + 1);
-      if (!mbar_wait(bars + g * 2 + b, b ? ph1 : ph0, abort_flag)) { dead = true; break; }
+      if (!mbar_wait_warp(bars + g * 2 + b, b ? ph1 : ph0, abort_flag)) { dead = true; break; }
       if (b) ph1 ^= 1u; else ph0 ^= 1u;
       tc_fence_after();
       uint32_t v[32];

@@ -538,26 +538,25 @@ __device__ __forceinline__ unsigned long long peek_tagged(const unsigned long lo
   asm volatile("ld.volatile.shared.b64 %0, [%1];\n" : "=l"(w) : "r"(smem_u32(at)) : "memory");
   return w;
 }
-// Looks again until `w` is tile `tile`'s.
+// Looks until `w` is tile `tile`'s in every lane: one answer for the warp, as in mbar_wait_warp.
 __device__ __forceinline__ bool take_tagged(const unsigned long long* at, uint32_t tile, unsigned long long& w,
-                                            volatile int* abort_flag) {
-  for (uint32_t it = 0; (uint32_t)(w >> 32) != tile; ++it) {
-    if ((it & 255u) == 255u && *abort_flag) return false;
-    if (it == kWaitSpinLimit) {
-      *abort_flag = 1;
-      return false;
-    }
+                                            volatile int* abort_flag, uint32_t limit) {
+  for (uint32_t it = 0; it < limit; ++it) {
+    if (__all_sync(0xffffffffu, (uint32_t)(w >> 32) == tile)) return true;
+    if ((it & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
     w = peek_tagged(at);
   }
-  return true;
+  *abort_flag = 1;
+  return false;
 }
 
 // Rows of group 0 of a task of more than QT rows, whole warps of them; group 1 takes the rest.
 __device__ __forceinline__ int group_rows(int rows) { return min((((rows + 1) >> 1) + 31) & ~31, rows); }
 
 // The softmax warps of both kernels: warps 0..3 weigh a row's even tiles, warps 4..7 its odd ones (see attn2_kernel).
-// `rank`, `lead` and `tfree` are the group of this CTA's rows and the cluster addresses of the pair's barriers.
-template <bool PAIR>
+// `rank`, `lead` and `tfree` are the group of this CTA's rows and the cluster addresses of the pair's barriers; `LIMIT` bounds
+// the waits.
+template <bool PAIR, uint32_t LIMIT = kWaitSpinLimit>
 __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* ring, unsigned long long* sM, float2* sFin,
                                              uint32_t tmem, uint32_t rank, uint32_t lead, uint32_t tfree,
                                              __nv_bfloat16* __restrict__ attn_out, float* __restrict__ attn_lse, int N,
@@ -575,8 +574,8 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
   bool ok = true;
   for (uint32_t n = 0;; ++n) {
     const uint32_t sl = n & 1u;
-    if (!(PAIR ? mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)
-               : mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)))
+    if (!(PAIR ? mbar_wait_warp_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)
+               : mbar_wait_warp(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag, LIMIT)))
       break;
     const int end = ring[sl].end, kvlen = ring[sl].kvlen, ntiles = cdiv(kvlen, KT);
     if (end) break;
@@ -606,7 +605,7 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
     for (int t = t0; t < ntiles; t += 2) {
       const uint32_t gt = g + t, p = gt - 1u;
       const uint32_t tS_lane = tmem_addr(tmem + buf * 128, gw * 32, 0);
-      ok = mbar_wait(bars + B_QK + (gt & 3u), (gt >> 2) & 1u, abort_flag);
+      ok = mbar_wait_warp(bars + B_QK + (gt & 3u), (gt >> 2) & 1u, abort_flag, LIMIT);
       if (!ok) break;
       tc_fence_after();
       if (active) {
@@ -619,16 +618,18 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
         if (t == 0) {
           rs.m = mx;
         } else {
-          ok = take_tagged(before, p, tagged, abort_flag);
-          if (!ok) break;
-          const float m_in = __uint_as_float((uint32_t)tagged);
-          if (__any_sync(0xffffffffu, m_in != rs.m || mx > m_in + kLazy)) {
+          // one vote in the common case: the reference is there in every lane and stays
+          const float seen = __uint_as_float((uint32_t)tagged);
+          if (__any_sync(0xffffffffu, (uint32_t)(tagged >> 32) != p || seen != rs.m || mx > seen + kLazy)) {
+            ok = take_tagged(before, p, tagged, abort_flag, LIMIT);
+            if (!ok) break;
+            const float m_in = __uint_as_float((uint32_t)tagged);
             if (m_in != rs.m) rs.l *= t > 1 ? ex2_approx(rs.m - m_in) : 0.f;
             rs.m = m_in;
             const bool grow = mx > rs.m + kLazy;
             if (__any_sync(0xffffffffu, grow)) {
               const float mnew = grow ? mx : rs.m;
-              ok = mbar_wait(bars + B_PV + (p & 3u), (p >> 2) & 1u, abort_flag);      // O holds the tiles up to t - 1
+              ok = mbar_wait_warp(bars + B_PV + (p & 3u), (p >> 2) & 1u, abort_flag, LIMIT);      // O holds the tiles up to t - 1
               if (!ok) break;
               const float alpha = ex2_approx(rs.m - mnew);
               tc_fence_after();
@@ -654,7 +655,7 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
     fin[wg * QT + row] = make_float2(rs.m, rs.l);
     asm volatile("bar.sync %0, 64;\n" ::"r"(1 + gw) : "memory");
     const int lastwg = (g - 1u) & 1u;
-    ok = mbar_wait(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag);
+    ok = mbar_wait_warp(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag, LIMIT);
     if (!ok) break;
     if (active) {
       tc_fence_after();
@@ -753,7 +754,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
       for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
         TaskSlot* slot = ring + sl;
-        if (!mbar_wait(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
           do { task = atomicAdd(&pv.counters[2], 1); } while (task < numTasks && pv.tasks[task].w <= PAIR_ROWS);
@@ -794,7 +795,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
       bool ok = true;
       for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const TaskSlot tk = ring[sl];
         if (tk.end) break;
         const int* sRunStart = sRuns + sl * RUN_INTS;
@@ -808,7 +809,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             r[j] = tk.head * q_head_step + qperm[rowbase + (lane * 4 + j < nr ? lane * 4 + j : 0)] * q_row_step;
-          ok = mbar_wait(bars + B_FREEQ + (q & 1u), ((q >> 1) & 1u) ^ 1u, abort_flag);
+          ok = mbar_wait_warp(bars + B_FREEQ + (q & 1u), ((q >> 1) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
           const uint32_t full = lead + (B_FULLQ + (q & 1u)) * 8;
           if (lane == 0) {
@@ -827,7 +828,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
           const bool whole = union_rows(sRunStart, sRunCum, tk.runs, tk.kvlen, t * KT + prow, tk.head * N, cursor, r);
           const int what = fetch_plan(r, whole, lane, seg);
           const uint32_t slot = g & 3u;
-          ok = g < 4u || mbar_wait(bars + (kind ? B_PV : B_QK) + slot, ((g - 4u) >> 2) & 1u, abort_flag);
+          ok = g < 4u || mbar_wait_warp(bars + (kind ? B_PV : B_QK) + slot, ((g - 4u) >> 2) & 1u, abort_flag);
           if (!ok) break;
           const uint32_t full = lead + (bfull + slot) * 8;
           if (lane == 0) {
@@ -853,21 +854,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
       bool ok = true;
       for (uint32_t n = 0; ok; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
         if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
         if (ntiles == 0) continue;
-        if (!mbar_wait(bars + B_FULLQ + (q & 1u), (q >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_FULLQ + (q & 1u), (q >> 1) & 1u, abort_flag)) break;
         const uint32_t a0 = qlo + (q & 1u) * (AT_TILE >> 4);
         for (int t = 0; t < ntiles; ++t, ++g) {
           const uint32_t slot = g & 3u, b0 = klo + slot * (A2_HALF >> 4);
-          ok = mbar_wait(bars + B_FULLK + slot, (g >> 2) & 1u, abort_flag) &&
-               (g < 3u || mbar_wait(bars + B_PV + ((g - 3u) & 3u), ((g - 3u) >> 2) & 1u, abort_flag));
+          ok = mbar_wait_warp(bars + B_FULLK + slot, (g >> 2) & 1u, abort_flag) &&
+               (g < 3u || mbar_wait_warp(bars + B_PV + ((g - 3u) & 3u), ((g - 3u) >> 2) & 1u, abort_flag));
           if (!ok) break;
           tc_fence_after();
-          __syncwarp();
           if (elect_one()) {
 #pragma unroll
             for (int s = 0; s < 8; ++s)
@@ -891,21 +891,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
       bool ok = true;
       for (uint32_t n = 0; ok; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp_cluster(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
         if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
         if (ntiles == 0) continue;
         // every softmax warp has read the O of the task before
-        if (!mbar_wait(bars + B_OFREE, (q & 1u) ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_OFREE, (q & 1u) ^ 1u, abort_flag)) break;
         for (int t = 0; t < ntiles; ++t, ++g) {
           const uint32_t slot = g & 3u, v0 = vlo + slot * (A2_HALF >> 4), tS = tmem + buf * 128, add = t > 0 ? 1u : 0u;
-          ok = mbar_wait(bars + B_FULLV + slot, (g >> 2) & 1u, abort_flag) &&
-               mbar_wait(bars + B_P + buf, bph, abort_flag);
+          ok = mbar_wait_warp(bars + B_FULLV + slot, (g >> 2) & 1u, abort_flag) &&
+               mbar_wait_warp(bars + B_P + buf, bph, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          __syncwarp();
           if (elect_one()) {
 #pragma unroll
             for (int s8 = 0; s8 < 8; ++s8)
@@ -1062,7 +1061,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
       uint32_t nq = 0;      // tasks with tiles so far
       for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
           do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > PAIR_ROWS);
@@ -1085,7 +1084,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
         }
         reinterpret_cast<int4*>(sRows)[lane] = make_int4(r[0], r[1], r[2], r[3]);
         __syncwarp();
-        if (!mbar_wait(bars + B_FREEQ, (nq & 1u) ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_FREEQ, (nq & 1u) ^ 1u, abort_flag)) break;
         copy_groups(base, q, sRows, 0xffffffffu >> (32 - 8 * cdiv(tk.rows, 32)), lane);
         cp_async_commit();
         cp_async_wait<0>();
@@ -1101,7 +1100,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
       bool ok = true;
       for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const TaskSlot tk = ring[sl];
         if (tk.end) break;
         const int* sRunStart = sRuns + sl * RUN_INTS;
@@ -1125,7 +1124,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
           const unsigned gathers = __ballot_sync(0xffffffffu, what == FETCH_GATHER);
           const unsigned b32 = __ballot_sync(0xffffffffu, what == FETCH_BOX32), b64 = __ballot_sync(0xffffffffu, what == FETCH_BOX64);
           TilePlan* plan = plans + (g & (A1_PLANS - 1));
-          ok = mbar_wait(bars + B_PFREE + (g & (A1_PLANS - 1)), ((g / A1_PLANS) & 1u) ^ 1u, abort_flag);
+          ok = mbar_wait_warp(bars + B_PFREE + (g & (A1_PLANS - 1)), ((g / A1_PLANS) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
           // cp.async has no bounds of its own: a plan that does not match kp / vp stays inside them
 #pragma unroll
@@ -1157,18 +1156,18 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
       bool ok = true;
       for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
         if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
         for (int t = 0; t < ntiles; ++t, ++g, slot = slot + 1 == depth ? 0 : slot + 1) {
           const TilePlan* plan = plans + (g & (A1_PLANS - 1));
-          ok = mbar_wait(bars + B_PLAN + (g & (A1_PLANS - 1)), (g / A1_PLANS) & 1u, abort_flag);
+          ok = mbar_wait_warp(bars + B_PLAN + (g & (A1_PLANS - 1)), (g / A1_PLANS) & 1u, abort_flag);
           if (!ok) break;
           const int4 r = reinterpret_cast<const int4*>(plan->rows)[lane];
           const unsigned gathers = plan->gathers, b32 = plan->box32, b64 = plan->box64;
-          ok = g < depth || mbar_wait(bars + (kind ? B_PV : B_QK) + ((g - depth) & 3u), ((g - depth) >> 2) & 1u, abort_flag);
+          ok = g < depth || mbar_wait_warp(bars + (kind ? B_PV : B_QK) + ((g - depth) & 3u), ((g - depth) >> 2) & 1u, abort_flag);
           if (!ok) break;
           uint64_t* full = bars + (kind ? B_FULLV : B_FULLK) + slot;
           const uint32_t dst = base + (kind ? A1_OFF_V : A1_OFF_K) + slot * AT_TILE, mine = dst + lane * 512;
@@ -1205,21 +1204,20 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
       bool ok = true;
       for (uint32_t n = 0; ok; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
         if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
         if (ntiles == 0) continue;
-        if (!mbar_wait(bars + B_FULLQ, nq & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_FULLQ, nq & 1u, abort_flag)) break;
         for (int t = 0; t < ntiles; ++t, ++g) {
           const uint32_t b0 = klo + ks * (AT_TILE >> 4);
-          ok = mbar_wait(bars + B_FULLK + ks, kph, abort_flag) &&
-               (g < 3u || mbar_wait(bars + B_PV + ((g - 3u) & 3u), ((g - 3u) >> 2) & 1u, abort_flag));
+          ok = mbar_wait_warp(bars + B_FULLK + ks, kph, abort_flag) &&
+               (g < 3u || mbar_wait_warp(bars + B_PV + ((g - 3u) & 3u), ((g - 3u) >> 2) & 1u, abort_flag));
           if (!ok) break;
           fence_proxy_async();      // rows that came by cp.async
           tc_fence_after();
-          __syncwarp();
           if (elect_one()) {
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
@@ -1246,21 +1244,20 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
       bool ok = true;
       for (uint32_t n = 0; ok; ++n) {
         const uint32_t sl = n & 1u;
-        if (!mbar_wait(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_TFULL + sl, (n >> 1) & 1u, abort_flag)) break;
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
         if (lane == 0) mbar_arrive(bars + B_TFREE + sl);
         if (ntiles == 0) continue;
         // every softmax warp has read the O of the task before
-        if (!mbar_wait(bars + B_OFREE, (nq & 1u) ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(bars + B_OFREE, (nq & 1u) ^ 1u, abort_flag)) break;
         for (int t = 0; t < ntiles; ++t, ++g) {
           const uint32_t v0 = vlo + vs * (AT_TILE >> 4), tS = tmem + buf * 128, add = t > 0 ? 1u : 0u;
-          ok = mbar_wait(bars + B_FULLV + vs, vph, abort_flag) && mbar_wait(bars + B_P + buf, bph, abort_flag);
+          ok = mbar_wait_warp(bars + B_FULLV + vs, vph, abort_flag) && mbar_wait_warp(bars + B_P + buf, bph, abort_flag);
           if (!ok) break;
           fence_proxy_async();      // rows that came by cp.async
           tc_fence_after();
-          __syncwarp();
           if (elect_one()) {
 #pragma unroll
             for (int s8 = 0; s8 < 8; ++s8)
@@ -1289,6 +1286,72 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
   // completion, which later work in the stream waits for, implies the other's.  (Without a programmatic
   // launch the instruction returns at once.)
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+// softmax_role on one task of two tiles where some of the commits it waits for never come (a bit of `commits` each: QK of
+// tile 0 and 1, PV of tile 0 and 1) and only the lanes in `handed` find the maximum behind tile 0 in place: every warp has to
+// leave within its limits.  All scores are 0, O holds 256.
+__global__ void __launch_bounds__(256, 1) softmax_give_up_selftest_kernel(int commits, unsigned handed,
+                                                                          __nv_bfloat16* __restrict__ attn_out,
+                                                                          float* __restrict__ attn_lse,
+                                                                          int* __restrict__ left, int* __restrict__ status) {
+  __shared__ uint64_t bars[B_COUNT];
+  __shared__ TaskSlot ring[2];
+  __shared__ unsigned long long sM[2 * QT];
+  __shared__ float2 sFin[4 * QT];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    tmem_alloc(&tmem_slot, 512);
+    tmem_relinquish();
+  }
+  sM[tid] = tid < QT && (handed >> lane & 1u) ? 0ull : ~0ull;      // tile 0, maximum 0
+  if (tid == 0) {
+    abort_word = 0;
+    for (int i = 0; i < B_COUNT; ++i) {
+      int count = 1;
+      if (i >= B_P && i < B_P + 3) count = 4;
+      else if (i == B_OFREE) count = 8;
+      else if (i == B_TFREE || i == B_TFREE + 1) count = A1_CONSUMERS;
+      mbar_init(bars + i, count);
+    }
+    mbar_init_fence();
+    ring[0] = TaskSlot{0, 0, 0, QT, 2 * KT, 1, {0, 0}};
+    ring[1] = TaskSlot{1, 0, 0, 0, 0, 0, {0, 0}};
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  if (warp < 4) {
+    for (int col = 0; col < 512; col += 16) {
+      uint32_t v[16];
+      for (int j = 0; j < 16; ++j) v[j] = col < 384 ? 0u : __float_as_uint(256.0f);
+      tmem_st16(tmem_addr(tmem, warp * 32, col), v);
+    }
+    tmem_wait_st();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (tid == 0) {
+    mbar_arrive(bars + B_TFULL);
+    mbar_arrive(bars + B_TFULL + 1);
+    for (int t = 0; t < 2; ++t) {
+      if (commits >> t & 1) mbar_arrive(bars + B_QK + t);
+      if (commits >> (2 + t) & 1) mbar_arrive(bars + B_PV + t);
+    }
+  }
+  __syncwarp();
+  softmax_role<false, 1u << 10>(bars, ring, sM, sFin, tmem, 0u, 0u, 0u, attn_out, attn_lse, QT, abort_flag);
+  __syncwarp();
+  if (lane == 0) left[warp] = 1;
+  if (*abort_flag && tid == 0) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -1432,7 +1495,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
     };
     for (int step = 0; step < TL_STAGES; ++step) load_c(step, step);
     load_v(0, 0);
-    const bool there = mbar_wait(cFull + 0, 0, abort_flag) && mbar_wait(cFull + 1, 0, abort_flag);
+    const bool there = mbar_wait_warp(cFull + 0, 0, abort_flag) && mbar_wait_warp(cFull + 1, 0, abort_flag);
     tc_fence_after();
     __syncwarp();
     if (there && elect_one()) {
@@ -1443,15 +1506,14 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
     int st = 0;      // stage of step i
     for (int i = 0; there && i < TL_NH; ++i) {
       const int b = i & 1, st1 = st == TL_STAGES - 1 ? 0 : st + 1, st2 = st1 == TL_STAGES - 1 ? 0 : st1 + 1;
-      if (!mbar_wait(pReady + b, (i >> 1) & 1, abort_flag)) break;
+      if (!mbar_wait_warp(pReady + b, (i >> 1) & 1, abort_flag)) break;
       // every softmax thread has seen the commit behind S_i and the product of step i - 2: their stages are free
       if (i + 1 < TL_NH) load_v(i + 1, st1);
       if (i + TL_STAGES < TL_NH) load_c(i + TL_STAGES, st);
-      if (!mbar_wait(vFull + st, (i / TL_STAGES) & 1, abort_flag)) break;
-      if (i + 2 < TL_NH && !mbar_wait(cFull + st2, ((i + 2) / TL_STAGES) & 1, abort_flag)) break;
+      if (!mbar_wait_warp(vFull + st, (i / TL_STAGES) & 1, abort_flag)) break;
+      if (i + 2 < TL_NH && !mbar_wait_warp(cFull + st2, ((i + 2) / TL_STAGES) & 1, abort_flag)) break;
       tc_fence_after();
       const uint32_t v0 = vlo + st * (TL_SV >> 4), first = i > 0 ? 1u : 0u;
-      __syncwarp();
       if (elect_one()) {
 #pragma unroll
         for (int s8 = 0; s8 < TL_H / 16; ++s8)
@@ -1471,7 +1533,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
     uint2 mw_next = *reinterpret_cast<const uint2*>(mrow);   // union bits of the step's 64 centroids
     for (int i = 0; i < TL_NH; ++i) {
       const int b = i & 1;
-      if (!mbar_wait(sReady + b, (i >> 1) & 1, abort_flag)) { dead = true; break; }
+      if (!mbar_wait_warp(sReady + b, (i >> 1) & 1, abort_flag)) { dead = true; break; }
       tc_fence_after();
       const uint2 mw2 = mw_next;
       if (i + 1 < TL_NH) mw_next = *reinterpret_cast<const uint2*>(mrow + (i + 1) * 2);
@@ -1524,7 +1586,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
         if (i > 0) {
           // T is rescaled in place: the product of step i - 1 may still be running, its commit is the
           // next completion of the other region's barrier (the same one step i + 1 waits for)
-          if (!mbar_wait(sReady + (b ^ 1), (((i - 1) >> 1) + 1) & 1, abort_flag)) { dead = true; break; }
+          if (!mbar_wait_warp(sReady + (b ^ 1), (((i - 1) >> 1) + 1) & 1, abort_flag)) { dead = true; break; }
           tc_fence_after();
           rescale_rows(tO_lane, alpha);
         }
@@ -1577,8 +1639,8 @@ __global__ void __launch_bounds__(TL_THREADS, 2) tail_kernel(
     const float lam = lam_s[h], tw = *tailw_ptr;
     const float le = active ? attn_lse[(size_t)h * N + j] : 0.f;
     // the last commit on each region's barrier covers every product
-    if (!dead) dead = !mbar_wait(sReady + 0, (TL_NH >> 1) & 1, abort_flag);
-    if (!dead) dead = !mbar_wait(sReady + 1, (TL_NH >> 1) & 1, abort_flag);
+    if (!dead) dead = !mbar_wait_warp(sReady + 0, (TL_NH >> 1) & 1, abort_flag);
+    if (!dead) dead = !mbar_wait_warp(sReady + 1, (TL_NH >> 1) & 1, abort_flag);
     tc_fence_after();
     if (!dead) {
       // merge with the exact part (natural-log units from here on); rows past N
@@ -1816,5 +1878,12 @@ extern "C" int t2t_tile_attn_plan_info(const int* plan, int H, int N, int CQ, in
   if (!plan || !d_info) return T2T_ERR_ARG;
   const PlanView pv = plan_view(const_cast<int*>(plan), H, N, CQ);
   plan_info_kernel<<<1, 1024, 0, st>>>(pv, CQ, d_info);
+  return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
+}
+
+extern "C" int t2t_softmax_give_up_selftest(int commits, unsigned handed, void* out, float* lse, int* d_left, int* d_status,
+                                            cudaStream_t st) {
+  if (!out || !lse || !d_left || !d_status) return T2T_ERR_ARG;
+  softmax_give_up_selftest_kernel<<<1, 256, 0, st>>>(commits, handed, (__nv_bfloat16*)out, lse, d_left, d_status);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
