@@ -261,10 +261,11 @@ int t2t_wait_timeout_selftest(int* d_status, int* d_out, cudaStream_t stream);
 
 /* Give-up path of the attention kernels' softmax warps: one CTA runs them on a task of 128 rows and
  * two key tiles.  `commits` says which products are reported complete (bits 0, 1: the scores of tile 0,
- * 1; bits 2, 3: the weighted sum behind tile 0, 1), `handed` which lanes of a warp find a row's maximum
- * behind tile 0 in place beforehand.  What is missing never comes: the waits for it run out within
+ * 1; bits 2, 3: the weighted sum behind tile 0, 1); bit 4 makes the scores of tile 1 1000 instead of 0 in
+ * the odd rows.  `handed` says which lanes of a warp find a row's maximum behind tile 0 in place beforehand.  What is missing never comes: the waits for it run out within
  * milliseconds, d_left[0..7] = 1 (every warp left), *d_status becomes 1 (wait timed out).  out [128, 128]
- * bf16 and lse [128] are written if nothing is missing: ones, log 256.  The kernel always terminates.  No
+ * bf16 and lse [128] are written if nothing is missing: ones, log 256 (odd rows with bit 4: zeros, 1000 /
+ * sqrt(128) + log 128).  The kernel always terminates.  No
  * counterpart in the reference. */
 int t2t_softmax_give_up_selftest(int commits, unsigned handed, void* out, float* lse, int* d_left, int* d_status,
                                  cudaStream_t stream);

@@ -82,6 +82,27 @@ def test_softmax_warps_give_up_as_warps(lib, commits, handed):
     assert float((torch.ones(4, device=DEV) * 2).sum()) == 8.0      # the device still works
 
 
+@pytest.mark.parametrize("commits, handed", [(1, 0), (2, 0xffffffff), (3, 0), (7, 0), (19, 0), (1 | 16, 0)])
+def test_softmax_warps_do_not_wait_for_a_warp_that_gave_up(lib, commits, handed):
+    """One of the two warps of a row leaves at a wait that runs out (the scores of tile 1, of tile 0, the weighted sum that
+    a rising maximum rescales) when the other has finished its tile and comes to where their sums are joined; or both are
+    through and the last weighted sum never comes."""
+    status, out, lse = _softmax_give_up(lib, commits, handed)
+    assert status == 1 and bool((out == -1).all()) and bool((lse == -1).all())
+    assert float((torch.ones(4, device=DEV) * 2).sum()) == 8.0      # the device still works
+
+
+@pytest.mark.parametrize("commits", [15, 31])
+def test_softmax_warps_join_their_sums_when_nothing_is_missing(lib, commits):
+    """256 equal scores: weights of one that sum to 256, half from either warp.  Scores of 1000 in the odd rows of tile 1:
+    tile 0 and the O it left weigh 2^-127.5, the second warp's 128 keys are all there is."""
+    status, out, lse = _softmax_give_up(lib, commits, 0)
+    odd = (torch.arange(128) % 2 == 1) & (commits == 31)
+    assert status == 0 and torch.equal(out, torch.where(odd, 0.0, 1.0)[:, None].expand(128, 128))
+    want = torch.where(odd, 1000.0 / math.sqrt(128.0) + math.log(128.0), math.log(256.0))
+    assert (lse - want).abs().max() < 1e-4
+
+
 def test_umma_selftest(lib):
     g = torch.Generator().manual_seed(7)
     A = (torch.randn(128, 128, generator=g) * 0.5).to(BF)

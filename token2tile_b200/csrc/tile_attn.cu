@@ -507,7 +507,8 @@ __device__ __forceinline__ void prepare_task(const PlanView& pv, const uint32_t*
 // Barriers: QK and PV are the commits behind the products of a tile, on barrier tile mod 4, and reach both CTAs.  QK(g): S(g)
 // is there, the K slot of tile g is free.  PV(g): O holds tile g, score buffer and V slot of tile g are free.  P[b],
 // FULLK / FULLV / FULLQ and OFREE live in the leader and collect both CTAs' arrivals (and, for copies, both CTAs'
-// bytes); TFREE lives in the other CTA and collects everyone who reads a task.
+// bytes); TFREE lives in the other CTA and collects everyone who reads a task.  MEET[w]: the two softmax warps of
+// rows 32 w .. have laid down their sums of a task.
 constexpr int A2_THREADS = 16 * 32;
 constexpr int A2_STAGES = 4;                              // K and V ring depth
 constexpr int A2_HALF = AT_TILE / 2;                      // 16 KB: 64 keys of a K tile, 64 columns of a V tile
@@ -516,7 +517,8 @@ constexpr int A2_OFF_V = A2_OFF_K + A2_STAGES * A2_HALF;
 constexpr int A2_OFF_MISC = A2_OFF_V + A2_STAGES * A2_HALF;
 constexpr int RUN_INTS = 2 * MAX_RUNS + 8;                // one run list: [MAX_RUNS] starts, [MAX_RUNS + 1] positions
 enum { B_QK = 0, B_PV = 4, B_P = 8, B_FULLK = 11, B_FULLV = B_FULLK + A2_STAGES, B_FULLQ = B_FULLV + A2_STAGES,
-       B_FREEQ = B_FULLQ + 2, B_OFREE = B_FREEQ + 2, B_TFULL, B_TFREE = B_TFULL + 2, B_COUNT = B_TFREE + 2 };
+       B_FREEQ = B_FULLQ + 2, B_OFREE = B_FREEQ + 2, B_TFULL, B_TFREE = B_TFULL + 2, B_MEET = B_TFREE + 2,
+       B_COUNT = B_MEET + 4 };
 static_assert(A2_STAGES == 4, "ring slots and commits are counted alike");
 constexpr int A2_CONSUMERS = (8 + 6) * 2 + 2;             // warps that read a task: softmax and copy, QK and PV
 constexpr int A2_OFF_RING = A2_OFF_MISC + 512;            // two tasks
@@ -650,10 +652,14 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
     }
     if (!ok) break;
     g += ntiles;
-    // both warps of these rows meet: the sums of the two are relative to the maxima they saw last
+    // both warps of these rows meet, by a wait with a limit as everywhere (the other one may have left at a wait that gave
+    // up): the sums of the two are relative to the maxima they saw last
     float2* fin = sFin + (q & 1u) * 2 * QT;
     fin[wg * QT + row] = make_float2(rs.m, rs.l);
-    asm volatile("bar.sync %0, 64;\n" ::"r"(1 + gw) : "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bars + B_MEET + gw);
+    ok = mbar_wait_warp(bars + B_MEET + gw, q & 1u, abort_flag, LIMIT);
+    if (!ok) break;
     const int lastwg = (g - 1u) & 1u;
     ok = mbar_wait_warp(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag, LIMIT);
     if (!ok) break;
@@ -724,6 +730,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
     for (int i = 0; i < B_COUNT; ++i) {
       int count = 1;
       if (i >= B_P && i < B_P + 3) count = 8;                                    // softmax warps of a tile, both CTAs
+      else if (i >= B_MEET) count = 2;                                           // the softmax warps of the same rows
       else if (i >= B_FULLK && i < B_FULLK + A2_STAGES) count = 2;               // a copy warp of each CTA
       else if (i >= B_FULLV && i < B_FULLV + A2_STAGES) count = 2;
       else if (i == B_FULLQ || i == B_FULLQ + 1) count = 4;
@@ -1032,6 +1039,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
     for (int i = 0; i < A1_BARS; ++i) {
       int count = 1;
       if (i >= B_P && i < B_P + 3) count = 4;                                    // softmax warps of a tile
+      else if (i >= B_MEET && i < B_MEET + 4) count = 2;                         // the softmax warps of the same rows
       else if (i >= B_FULLK && i < B_FULLK + A1_KST) count = 1 + 32 * A1_TEAM;
       else if (i >= B_FULLV && i < B_FULLV + A1_VST) count = 1 + 32 * A1_TEAM;
       else if (i == B_OFREE) count = 8;
@@ -1290,7 +1298,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
 
 // softmax_role on one task of two tiles where some of the commits it waits for never come (a bit of `commits` each: QK of
 // tile 0 and 1, PV of tile 0 and 1) and only the lanes in `handed` find the maximum behind tile 0 in place: every warp has to
-// leave within its limits.  All scores are 0, O holds 256.
+// leave within its limits.  All scores are 0 (bit 4 of `commits`: 1000 for the odd rows of tile 1), O holds 256.
 __global__ void __launch_bounds__(256, 1) softmax_give_up_selftest_kernel(int commits, unsigned handed,
                                                                           __nv_bfloat16* __restrict__ attn_out,
                                                                           float* __restrict__ attn_lse,
@@ -1313,6 +1321,7 @@ __global__ void __launch_bounds__(256, 1) softmax_give_up_selftest_kernel(int co
     for (int i = 0; i < B_COUNT; ++i) {
       int count = 1;
       if (i >= B_P && i < B_P + 3) count = 4;
+      else if (i >= B_MEET) count = 2;
       else if (i == B_OFREE) count = 8;
       else if (i == B_TFREE || i == B_TFREE + 1) count = A1_CONSUMERS;
       mbar_init(bars + i, count);
@@ -1328,7 +1337,8 @@ __global__ void __launch_bounds__(256, 1) softmax_give_up_selftest_kernel(int co
   if (warp < 4) {
     for (int col = 0; col < 512; col += 16) {
       uint32_t v[16];
-      for (int j = 0; j < 16; ++j) v[j] = col < 384 ? 0u : __float_as_uint(256.0f);
+      const bool high = (commits & 16) && (lane & 1) && col >= 128 && col < 256;
+      for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(col >= 384 ? 256.0f : high ? 1000.0f : 0.0f);
       tmem_st16(tmem_addr(tmem, warp * 32, col), v);
     }
     tmem_wait_st();
