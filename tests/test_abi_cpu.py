@@ -59,6 +59,17 @@ def test_null_and_bad_arguments_are_rejected(lib):
     assert lib.t2t_rotation_selftest(0, 0, 1, 0) == 1
 
 
+def test_readers_of_a_shared_task_release_it_at_cluster_scope():
+    """The other CTA of a pair overwrites a task's slot behind the TFREE barrier.  No run can show a missing order, so the
+    source is read: every arrival there is a release at cluster scope, the wait in front of the stores an acquire."""
+    text = (ROOT / "token2tile_b200" / "csrc" / "tile_attn.cu").read_text()
+    pair = text[text.index("attn2_kernel("):text.index("exact attention, tasks of at most QT rows")]
+    role = text[text.index("void softmax_role("):text.index("attn2_kernel(")]
+    arrivals = re.findall(r"(mbar_\w+|arrive)\([^;]*\btfree\b", role + pair)
+    assert len(arrivals) >= 4 and set(arrivals) == {"mbar_release_peer"}
+    assert re.findall(r"(mbar_wait\w*)\(bars \+ B_TFREE", pair) == ["mbar_wait_warp_cluster"]
+
+
 def test_operator_dir_points_at_the_sources():
     import token2tile_b200
     d = Path(token2tile_b200.operator_dir())

@@ -343,8 +343,9 @@ __device__ __forceinline__ void cluster_store(uint32_t caddr, int v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(caddr), "r"(v) : "memory");
 }
 // The barrier operands below are cluster addresses.  mbar_arrive_peer orders nothing between the CTAs (what it reports is
-// tensor memory, ordered by tcgen05 fences, or copies in flight); mbar_release_peer publishes this thread's shared-memory
-// stores to the other CTA, which costs a fence of about 1,500 cycles.
+// tensor memory, ordered by tcgen05 fences, or copies in flight); mbar_release_peer orders this thread's loads and stores so
+// far, and those its warp has synchronised with it, before whatever the other CTA does behind mbar_wait_warp_cluster.  It
+// costs a fence of about 1,500 cycles, more with stores in flight.
 __device__ __forceinline__ void mbar_arrive_peer(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }

@@ -507,8 +507,10 @@ __device__ __forceinline__ void prepare_task(const PlanView& pv, const uint32_t*
 // Barriers: QK and PV are the commits behind the products of a tile, on barrier tile mod 4, and reach both CTAs.  QK(g): S(g)
 // is there, the K slot of tile g is free.  PV(g): O holds tile g, score buffer and V slot of tile g are free.  P[b],
 // FULLK / FULLV / FULLQ and OFREE live in the leader and collect both CTAs' arrivals (and, for copies, both CTAs'
-// bytes); TFREE lives in the other CTA and collects everyone who reads a task.  MEET[w]: the two softmax warps of
-// rows 32 w .. have laid down their sums of a task.
+// bytes); TFREE lives in the other CTA, which overwrites both CTAs' copies of a task behind it, and collects everyone who reads
+// one: releases at cluster scope, once per warp and task and where their fence is not waited for (a softmax warp's before its
+// stores, those of QK and PV behind their products).  MEET[w]: the two softmax warps of rows 32 w .. have laid down their
+// sums of a task.
 constexpr int A2_THREADS = 16 * 32;
 constexpr int A2_STAGES = 4;                              // K and V ring depth
 constexpr int A2_HALF = AT_TILE / 2;                      // 16 KB: 64 keys of a K tile, 64 columns of a V tile
@@ -571,6 +573,10 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
   auto arrive = [&](int own, uint32_t at) {
     if (PAIR) mbar_arrive_peer(at); else mbar_arrive(bars + own);
   };
+  // the task's slot and run list may be overwritten
+  auto release_task = [&](uint32_t sl) {
+    if (PAIR) mbar_release_peer(tfree + sl * 8); else mbar_arrive(bars + B_TFREE + sl);
+  };
   uint32_t g = 0;      // tiles so far
   uint32_t q = 0;
   bool ok = true;
@@ -592,7 +598,7 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
         if (wg == 0) attn_lse[at] = -INFINITY;
       }
       __syncwarp();
-      if (lane == 0) arrive(B_TFREE + sl, tfree + sl * 8);
+      if (lane == 0) release_task(sl);
       continue;
     }
     // A warp whose rows all lie past the group's last row skips the arithmetic: its P rows stay
@@ -660,6 +666,7 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
     if (lane == 0) mbar_arrive(bars + B_MEET + gw);
     ok = mbar_wait_warp(bars + B_MEET + gw, q & 1u, abort_flag, LIMIT);
     if (!ok) break;
+    if (lane == 0) release_task(sl);      // the task is in registers; before the stores below, which a release would wait for
     const int lastwg = (g - 1u) & 1u;
     ok = mbar_wait_warp(bars + B_PV + ((g - 1u) & 3u), ((g - 1u) >> 2) & 1u, abort_flag, LIMIT);
     if (!ok) break;
@@ -691,10 +698,7 @@ __device__ __forceinline__ void softmax_role(uint64_t* bars, const TaskSlot* rin
     ++q;
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) {
-      arrive(B_OFREE, lead + B_OFREE * 8);
-      arrive(B_TFREE + sl, tfree + sl * 8);
-    }
+    if (lane == 0) arrive(B_OFREE, lead + B_OFREE * 8);
   }
 }
 
@@ -761,7 +765,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
       for (uint32_t n = 0;; ++n) {
         const uint32_t sl = n & 1u;
         TaskSlot* slot = ring + sl;
-        if (!mbar_wait_warp(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp_cluster(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
           do { task = atomicAdd(&pv.counters[2], 1); } while (task < numTasks && pv.tasks[task].w <= PAIR_ROWS);
@@ -850,7 +854,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         if (!ok) break;
         if (ntiles > 0) ++q;
         __syncwarp();
-        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
+        if (lane == 0) mbar_release_peer(tfree + sl * 8);
       }
     } else if (warp == 8 && rank == 0) {
       // ================= Q K^T: waits for the K tile and for P V to have read the score buffer =================
@@ -865,8 +869,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
-        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
-        if (ntiles == 0) continue;
+        if (ntiles == 0) {
+          if (lane == 0) mbar_release_peer(tfree + sl * 8);
+          continue;
+        }
         if (!mbar_wait_warp(bars + B_FULLQ + (q & 1u), (q >> 1) & 1u, abort_flag)) break;
         const uint32_t a0 = qlo + (q & 1u) * (AT_TILE >> 4);
         for (int t = 0; t < ntiles; ++t, ++g) {
@@ -887,6 +893,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
           tS = tS == tmem + 256 ? tmem : tS + 128;
         }
         ++q;
+        if (ok && lane == 0) mbar_release_peer(tfree + sl * 8);
       }
     } else if (warp == 9) {
       // ================= P V =================
@@ -902,8 +909,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         const int end = ring[sl].end, ntiles = cdiv(ring[sl].kvlen, KT);
         __syncwarp();
         if (end) break;
-        if (lane == 0) mbar_arrive_peer(tfree + sl * 8);
-        if (ntiles == 0) continue;
+        if (ntiles == 0) {
+          if (lane == 0) mbar_release_peer(tfree + sl * 8);
+          continue;
+        }
         // every softmax warp has read the O of the task before
         if (!mbar_wait_warp(bars + B_OFREE, (q & 1u) ^ 1u, abort_flag)) break;
         for (int t = 0; t < ntiles; ++t, ++g) {
@@ -922,6 +931,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
           if (++buf == 3) { buf = 0; bph ^= 1u; }
         }
         ++q;
+        if (ok && lane == 0) mbar_release_peer(tfree + sl * 8);
       }
     }
   }
