@@ -270,6 +270,12 @@ int t2t_wait_timeout_selftest(int* d_status, int* d_out, cudaStream_t stream);
 int t2t_softmax_give_up_selftest(int commits, unsigned handed, void* out, float* lse, int* d_left, int* d_status,
                                  cudaStream_t stream);
 
+/* Give-up path of the selection's column groups: one CTA runs four passes of eight chunks in each of its
+ * eight groups; chunk `stuck` of the first group (none if negative) is never reported, and its wait runs out
+ * within milliseconds.  d_left[0..31] = 1 + the chunks a warp scanned, *d_status becomes 1 (wait timed out)
+ * unless nothing is missing.  The kernel always terminates.  No counterpart in the reference. */
+int t2t_select_give_up_selftest(int stuck, int* d_left, int* d_status, cudaStream_t stream);
+
 /* Rotation self-test: for n triples (squared lengths alpha, beta of two columns and
  * their product gamma, gamma != 0) writes tan, cos and sin of the angle that the
  * projection fit's Jacobi rounds turn them by.  No counterpart in the reference. */

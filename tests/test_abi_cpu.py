@@ -56,6 +56,7 @@ def test_null_and_bad_arguments_are_rejected(lib):
     assert lib.t2t_gather4_selftest(0, 0, 0, 0, 0, 0) == 1
     assert lib.t2t_wait_timeout_selftest(0, 0, 0) == 1
     assert lib.t2t_softmax_give_up_selftest(0, 0, 0, 0, 0, 0, 0) == 1
+    assert lib.t2t_select_give_up_selftest(0, 0, 0, 0) == 1
     assert lib.t2t_rotation_selftest(0, 0, 1, 0) == 1
 
 

@@ -103,6 +103,23 @@ def test_softmax_warps_join_their_sums_when_nothing_is_missing(lib, commits):
     assert (lse - want).abs().max() < 1e-4
 
 
+@pytest.mark.parametrize("stuck", [-1, 0, 1, 5, 7])
+def test_selection_groups_outlive_a_group_that_gave_up(lib, stuck):
+    """One column group's wait runs out while the others are at work: their warps see the abort flag at different chunks and
+    must still meet at their groups' barriers until the last of them is through."""
+    left = torch.zeros(32, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for _ in range(8):
+        left.zero_()
+        _ok(lib.t2t_select_give_up_selftest(stuck, left.data_ptr(), status.data_ptr(), _st()))
+        torch.cuda.synchronize()
+        assert left[:4].tolist() == [1 + stuck if stuck >= 0 else 33] * 4
+        assert 1 <= int(left.min()) and int(left.max()) <= 33
+        assert stuck >= 0 or left.tolist() == [33] * 32
+    assert int(status.item()) == (1 if stuck >= 0 else 0)
+    assert float((torch.ones(4, device=DEV) * 2).sum()) == 8.0      # the device still works
+
+
 def test_umma_selftest(lib):
     g = torch.Generator().manual_seed(7)
     A = (torch.randn(128, 128, generator=g) * 0.5).to(BF)

@@ -134,6 +134,32 @@ __device__ __forceinline__ void hist_add(uint32_t col, int f, int value) {
 
 __device__ __forceinline__ void wg_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
 
+// One pass of column group `g` over its chunks through two buffers: chunk i + 1 is produced (`issue`, by the group's first
+// warp, which reports it on the buffer's barrier) while chunk i is scanned (`body`).  A warp whose wait gave up, in this pass
+// or an earlier one, scans nothing more but keeps meeting its group at the group's barrier: the warps of a group may see the
+// abort flag at different chunks, and one that left the loop would be waited for there without a limit.
+template <uint32_t LIMIT = kWaitSpinLimit, typename Issue, typename Body>
+__device__ __forceinline__ void stream_chunks(uint64_t* bars, int g, bool& dead, volatile int* abort_flag, Issue&& issue,
+                                              Body&& body) {
+  static_assert(ST_NCH / ST_G % 4 == 0, "a pass leaves the phases of both barriers as it found them");
+  const bool first = ((threadIdx.x >> 5) & 3) == 0;
+  if (first && !dead) issue(0);
+#pragma unroll 1
+  for (int i = 0; i < ST_NCH / ST_G; ++i) {
+    const int b = i & 1;
+    // every warp of the group has finished reading the other buffer (chunk i - 1): refill it
+    tc_fence_before();
+    wg_sync(g);
+    if (dead) continue;
+    if (first && i + 1 < ST_NCH / ST_G) issue(i + 1);
+    if (!mbar_wait_warp(bars + g * 2 + b, (i >> 1) & 1, abort_flag, LIMIT)) { dead = true; continue; }
+    tc_fence_after();
+    body(i, b);
+  }
+  tc_fence_before();
+  wg_sync(g);
+}
+
 __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     const __nv_bfloat16* __restrict__ QU, const __nv_bfloat16* __restrict__ cks,
     const int* __restrict__ kcounts, const int* __restrict__ qperm, const int* __restrict__ tile_sizes,
@@ -245,7 +271,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   const int ns = *ns_ptr;
   const float cmaxnorm = sqrtf(__int_as_float(*sCmax));
   constexpr uint32_t idesc = make_idesc_bf16(128, ST_CH, false, false);
-  uint32_t ph0 = 0, ph1 = 0;        // phases of this group's two buffer barriers
   bool dead = false;
   int half = 0;                     // which half of the row tile's lines this tile's rows are in
 
@@ -268,9 +293,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     orig_next = row_index(first + 128);
   }
 
-  // Streams this group's eight chunks through its two TMEM buffers: the MMA of
-  // chunk i + 1 runs while chunk i is scanned.  body(cbase, v) sees 32
-  // consecutive approximate scores of this thread's row.
+  // Streams this group's eight chunks through its two TMEM buffers (see stream_chunks): body(cbase, v) sees 32 consecutive
+  // approximate scores of this thread's row.
   const uint32_t alo0 = sdesc_lo(sA, 16), clo0 = sdesc_lo(sCk, 16);
   auto issue = [&](int i) {        // called by the group's first warp (see elect_one)
     const int cc = g + ST_G * i, b = i & 1;
@@ -286,25 +310,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
     __syncwarp();
   };
   auto stream = [&](auto&& body) {
-    if (dead) return;
-    if ((warp & 3) == 0) issue(0);
-#pragma unroll 1
-    for (int i = 0; i < ST_NCH / ST_G; ++i) {
-      const int cc = g + ST_G * i, b = i & 1;
-      // every warp of the group has finished reading the other buffer (chunk i - 1): refill it
-      tc_fence_before();
-      wg_sync(g);
-      if ((warp & 3) == 0 && i + 1 < ST_NCH / ST_G) issue(i + 1);
-      if (!mbar_wait_warp(bars + g * 2 + b, b ? ph1 : ph0, abort_flag)) { dead = true; break; }
-      if (b) ph1 ^= 1u; else ph0 ^= 1u;
-      tc_fence_after();
+    stream_chunks(bars, g, dead, abort_flag, issue, [&](int i, int b) {
       uint32_t v[32];
       tmem_ld32(t_lane + b * ST_CH, v);
       tmem_wait_ld();
-      body(cc * ST_CH, v);
-    }
-    tc_fence_before();
-    wg_sync(g);
+      body((g + ST_G * i) * ST_CH, v);
+    });
   };
 
 #pragma unroll 1
@@ -734,6 +745,39 @@ __global__ void __launch_bounds__(ST_THREADS, 1) select_tc_kernel(
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+// Four passes of stream_chunks where group 0's chunk `stuck` is never reported, while the other groups are at work (a chunk
+// takes them some 50 us, 20 of them in the wait, so that its warps meet the abort flag in different chunks): every warp has to
+// leave.  left[warp] = 1 + the chunks it scanned.
+__global__ void __launch_bounds__(ST_THREADS, 1) select_give_up_selftest_kernel(int stuck, int* __restrict__ left,
+                                                                                int* __restrict__ status) {
+  __shared__ uint64_t bars[2 * ST_G];
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
+  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7;
+  if (tid == 0) {
+    abort_word = 0;
+    for (int i = 0; i < 2 * ST_G; ++i) mbar_init(bars + i, 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  bool dead = false;
+  int scanned = 0;
+  for (int pass = 0; pass < 4; ++pass)
+    stream_chunks<1u << 10>(bars, g, dead, abort_flag, [&](int i) {
+      if (elect_one()) {
+        __nanosleep(20000);
+        if (g > 0 || i != stuck) mbar_arrive(bars + g * 2 + (i & 1));
+      }
+      __syncwarp();
+    }, [&](int, int) {
+      __nanosleep(10000 + 7000 * (warp & 3));
+      ++scanned;
+    });
+  if ((tid & 31) == 0) left[warp] = 1 + scanned;
+  __syncthreads();
+  if (tid == 0 && *abort_flag) atomicCAS(status, ST_OK, ST_WAIT_TIMEOUT);
+}
+
 // pin_tail: every query cluster executes the reserved last key cluster
 __global__ void pin_bit_kernel(int* __restrict__ unip, int rows) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -824,4 +868,10 @@ extern "C" int t2t_score_select_union(const void* QU, const void* cks, const voi
   if (cudaGetLastError() != cudaSuccess) return T2T_ERR_CUDA;
   return launch_select_fix((const __nv_bfloat16*)QU, (const __nv_bfloat16*)cks, (const int*)kcounts, ns, (int*)unip,
                            (int*)rowcnt, H, N, CQ, fixq, st);
+}
+
+extern "C" int t2t_select_give_up_selftest(int stuck, int* d_left, int* d_status, cudaStream_t st) {
+  if (!d_left || !d_status) return T2T_ERR_ARG;
+  select_give_up_selftest_kernel<<<1, ST_THREADS, 0, st>>>(stuck, d_left, d_status);
+  return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
