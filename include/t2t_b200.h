@@ -276,6 +276,12 @@ int t2t_softmax_give_up_selftest(int commits, unsigned handed, void* out, float*
  * unless nothing is missing.  The kernel always terminates.  No counterpart in the reference. */
 int t2t_select_give_up_selftest(int stuck, int* d_left, int* d_status, cudaStream_t stream);
 
+/* What the attention entry points check of their two kernels before the first launch on a device, for a
+ * kernel built with `regs` registers a thread: 0 if the split of registers between its warps holds,
+ * T2T_ERR_CUDA otherwise (its warps would wait for registers that do not exist).  Host only.  No counterpart
+ * in the reference. */
+int t2t_register_split_selftest(int regs);
+
 /* Rotation self-test: for n triples (squared lengths alpha, beta of two columns and
  * their product gamma, gamma != 0) writes tan, cos and sin of the angle that the
  * projection fit's Jacobi rounds turn them by.  No counterpart in the reference. */

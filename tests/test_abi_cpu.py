@@ -60,6 +60,12 @@ def test_null_and_bad_arguments_are_rejected(lib):
     assert lib.t2t_rotation_selftest(0, 0, 1, 0) == 1
 
 
+def test_kernels_built_with_other_register_counts_are_refused(lib):
+    """The attention kernels' warps trade registers out of 128 a thread; registers are allocated in eights."""
+    assert [lib.t2t_register_split_selftest(r) for r in (128, 121)] == [0, 0]
+    assert [lib.t2t_register_split_selftest(r) for r in (0, 64, 104, 120, 129, 255)] == [2] * 6
+
+
 def test_readers_of_a_shared_task_release_it_at_cluster_scope():
     """The other CTA of a pair overwrites a task's slot behind the TFREE barrier.  No run can show a missing order, so the
     source is read: every arrival there is a release at cluster scope, the wait in front of the stores an acquire."""

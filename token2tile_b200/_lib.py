@@ -56,6 +56,7 @@ SIGNATURES = {
     "t2t_wait_timeout_selftest": (_I, [_P, _P, _P]),
     "t2t_softmax_give_up_selftest": (_I, [_I, C.c_uint, _P, _P, _P, _P, _P]),
     "t2t_select_give_up_selftest": (_I, [_I, _P, _P, _P]),
+    "t2t_register_split_selftest": (_I, [_I]),
     "t2t_rotation_selftest": (_I, [_P, _P, _I, _P]),
 }
 

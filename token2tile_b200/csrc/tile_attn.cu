@@ -452,6 +452,9 @@ __device__ __forceinline__ void row_weights(uint32_t tS_lane, const uint32_t (&v
 // 256 x (200 + 56) = 512 x 128.
 constexpr int kLaunchRegs = 128, kSoftmaxRegs = 200, kRoleRegs = 56;
 static_assert(kSoftmaxRegs + kRoleRegs == 2 * kLaunchRegs, "the split may not exceed what the launch holds");
+// Whether a kernel that was built with `regs` registers a thread is launched with kLaunchRegs (registers come in eights).
+// With fewer, which other compiler flags can bring about, take_registers would wait for what its CTA does not have.
+inline bool split_fits(int regs) { return ((regs + 7) & ~7) == kLaunchRegs; }
 __device__ __forceinline__ void take_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kSoftmaxRegs)); }
 __device__ __forceinline__ void give_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRoleRegs)); }
 
@@ -1734,6 +1737,10 @@ const DeviceFacts* device_facts() {
         cudaFuncSetAttribute(attn2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, A2_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM) != cudaSuccess)
       return nullptr;
+    cudaFuncAttributes small, large;
+    if (cudaFuncGetAttributes(&small, attn_kernel) != cudaSuccess || cudaFuncGetAttributes(&large, attn2_kernel) != cudaSuccess ||
+        !split_fits(small.numRegs) || !split_fits(large.numRegs))
+      return nullptr;
     f->sms = sms;
     f->ready = true;
   }
@@ -1900,6 +1907,8 @@ extern "C" int t2t_tile_attn_plan_info(const int* plan, int H, int N, int CQ, in
   plan_info_kernel<<<1, 1024, 0, st>>>(pv, CQ, d_info);
   return cudaGetLastError() == cudaSuccess ? T2T_OK : T2T_ERR_CUDA;
 }
+
+extern "C" int t2t_register_split_selftest(int regs) { return split_fits(regs) ? T2T_OK : T2T_ERR_CUDA; }
 
 extern "C" int t2t_softmax_give_up_selftest(int commits, unsigned handed, void* out, float* lse, int* d_left, int* d_status,
                                             cudaStream_t st) {
