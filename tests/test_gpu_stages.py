@@ -625,11 +625,8 @@ def test_tile_attn_weight_of_a_dominant_key_is_one(lib, sizes, tile, pos):
     assert (info["lse"][0].double() - torch.logsumexp(s, 1)).abs().max() < 1e-4
 
 
-@pytest.mark.parametrize("largest", [128, 300])
-def test_tile_attn_unions_of_many_forms(lib, largest):
-    """Tasks of 1 to `largest` rows, several to a CTA, with unions of no key, of one, of 127 / 128 / 129 / 256, of clusters
-    of one key each with gaps (more than 32 runs in a tile), of long stretches at odd offsets, of everything; empty
-    clusters inside.  Against a float64 softmax over the union: the weights and the output are rounded to bfloat16."""
+def _unions_of_many_forms(largest):
+    """(key cluster sizes, query cluster sizes, selected clusters, the same as bitmaps, generator) of twelve heads."""
     H, N = 12, 6000
     g = torch.Generator().manual_seed(largest)
     kc = torch.zeros(H, 2048, dtype=torch.int32)
@@ -660,12 +657,22 @@ def test_tile_attn_unions_of_many_forms(lib, largest):
             if kind == 4 and c % 2: sel[h, c, 1200] = True
     bits = (sel.view(H, CQ, 64, 32).long() << torch.arange(32)).sum(-1)
     union = torch.where(bits >= 2 ** 31, bits - 2 ** 32, bits).int()
+    return kc, sizes, sel, union, g
+
+
+@pytest.mark.parametrize("largest", [128, 300])
+def test_tile_attn_unions_of_many_forms(lib, largest):
+    """Tasks of 1 to `largest` rows, several to a CTA, with unions of no key, of one, of 127 / 128 / 129 / 256, of clusters
+    of one key each with gaps (more than 32 runs in a tile), of long stretches at odd offsets, of everything; empty
+    clusters inside.  Against a float64 softmax over the union: the weights and the output are rounded to bfloat16."""
+    kc, sizes, sel, union, g = _unions_of_many_forms(largest)
+    H, N = len(kc), sum(sizes)
     q, k, v = (torch.randn(H, N, 128, generator=g).to(BF) for _ in range(3))
     km, _, zeros = _plain_structure(sizes, v[:1])
     km = {key: t.expand(H, *t.shape[1:]).contiguous() for key, t in km.items() if key != "lam"}
     km.update(lam=torch.ones(H), kcounts=kc, V_sorted=v)
     _, info = _tile_attn(lib, q, k, v, torch.zeros(H, N, 32, dtype=BF), km, torch.zeros(H, 2048, 32, dtype=BF), union)
-    lab = torch.repeat_interleave(torch.arange(CQ), torch.tensor(sizes))
+    lab = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes))
     for h in range(H):
         inside = torch.repeat_interleave(sel[h], kc[h].long(), dim=1)[lab].to(DEV)
         s = q[h].to(DEV).double() @ k[h].to(DEV).double().T / math.sqrt(128.0)
@@ -677,6 +684,56 @@ def test_tile_attn_unions_of_many_forms(lib, largest):
         fin = some.cpu()
         assert torch.equal(torch.isfinite(info["lse"][h]), fin)
         assert (info["lse"][h].double() - lse)[fin].abs().max() < 1e-2
+
+
+@pytest.mark.parametrize("largest", [128, 300])
+def test_tile_attn_meets_every_row_of_a_union_once(lib, largest):
+    """The same unions, with keys and values that show a row that is missing, read twice or taken from its neighbour, however
+    long the union is: in an average of thousands of normal values one row for another moves an output by 6e-3 at most, less
+    than the bound above.
+
+    Values: q = 0, so every weight is one and the output is what a union holds of each of 128 codes (a random one per key,
+    one-hot), divided by its length: whole numbers below 2^24, so the same bits as the count rounded once each by the
+    division, the product and bfloat16.  Keys: a code's score is 8 / log2(e) or 0, by random bits of the query, so that
+    one key for another of other score changes its logsumexp by a 6000th or more (fp32 sums 6,000 weights to within 1e-5 and
+    rounds the result to 1e-6)."""
+    kc, sizes, sel, union, g = _unions_of_many_forms(largest)
+    H, N = len(kc), sum(sizes)
+    code = torch.randint(0, 128, (H, N), generator=g)
+    onehot = torch.nn.functional.one_hot(code, 128)
+    km, _, _ = _plain_structure(sizes, torch.zeros(1, N, 128, dtype=BF))
+    km = {key: t.expand(H, *t.shape[1:]).contiguous() for key, t in km.items() if key != "lam"}
+    km.update(lam=torch.ones(H), kcounts=kc, V_sorted=onehot.to(BF))
+    rest = torch.zeros(H, N, 32, dtype=BF), km, torch.zeros(H, 2048, 32, dtype=BF), union
+    # per query cluster: which keys its union holds, and how many of each code
+    keys = torch.stack([torch.repeat_interleave(sel[h], kc[h].long(), dim=1) for h in range(H)])
+    counts = keys.float() @ onehot.float()
+    length = keys.sum(-1)
+    lab = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes))
+    average = lambda counts, length: (counts * (1.0 / length.clamp(min=1).float())[..., None]).to(BF)
+    _, info = _tile_attn(lib, torch.zeros(H, N, 128, dtype=BF), torch.randn(H, N, 128, generator=g).to(BF),
+                         km["V_sorted"], *rest)
+    assert torch.equal(info["attn_o"], average(counts, length)[:, lab])
+
+    q = 16.0 * torch.randint(0, 2, (H, N, 128), generator=g).to(BF)
+    k = onehot.to(BF) * (8.0 * math.log(2.0) * math.sqrt(128.0) / 16.0)
+    _, info = _tile_attn(lib, q, k, km["V_sorted"], *rest)
+    weight = torch.exp(q.double() * float(k.max()) / math.sqrt(128.0))      # of a key by its code
+    lse = lambda counts: (counts.double()[:, lab] * weight).sum(-1).log()
+    some = length[:, lab] > 0
+    assert torch.equal(torch.isfinite(info["lse"]), some)
+    assert (info["lse"].double() - lse(counts))[some].abs().max() < 2e-5
+
+    # both would see one key of the longest union replaced by its neighbour
+    long = (length == N) & (torch.tensor(sizes) > 8)
+    a = 2 * N // 3
+    b = a + 1 + int((code[:, a + 1:] != code[:, a:a + 1]).long().argmax(1).max())
+    wrong = counts - onehot[:, None, a] + onehot[:, None, b]
+    moved = (code[:, a] != code[:, b])[:, None] & long
+    assert bool(moved.any()) and bool((average(wrong, length) != average(counts, length)).any(-1)[moved].all())
+    moved = moved[:, lab]
+    change = (lse(wrong) - lse(counts)).abs()
+    assert float((change > 4e-5)[moved].double().mean()) > 0.3
 
 
 @pytest.mark.parametrize("N", [31, 257, 8192, 8193, 16384, 16385])
