@@ -30,8 +30,7 @@
 namespace t2t {
 
 constexpr int QT = 128;          // query rows per tensor-core tile (one thread per row)
-constexpr int TASK_ROWS = 256;   // query rows per task: tasks above QT rows run as two tiles sharing one K/V stream
-constexpr int PAIR_ROWS = 128;
+constexpr int TASK_ROWS = 256;   // query rows per task: tasks above QT rows run in attn2_kernel, the others in attn_kernel
 constexpr int KT = 128;          // keys per tile
 constexpr int MAX_RUNS = 1024;   // runs of selected clusters in one union
 constexpr int PLAN_SORT_MAX = 2048;
@@ -771,7 +770,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
         if (!mbar_wait_warp_cluster(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
-          do { task = atomicAdd(&pv.counters[2], 1); } while (task < numTasks && pv.tasks[task].w <= PAIR_ROWS);
+          do { task = atomicAdd(&pv.counters[2], 1); } while (task < numTasks && pv.tasks[task].w <= QT);
           task = min(task, numTasks);
         }
         task = __shfl_sync(0xffffffffu, task, 0);
@@ -1085,7 +1084,7 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
         if (!mbar_wait_warp(bars + B_TFREE + sl, ((n >> 1) & 1u) ^ 1u, abort_flag)) break;
         int task = 0;
         if (lane == 0) {
-          do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > PAIR_ROWS);
+          do { task = atomicAdd(&pv.counters[1], 1); } while (task < numTasks && pv.tasks[task].w > QT);
           task = min(task, numTasks);
         }
         task = __shfl_sync(0xffffffffu, task, 0);
@@ -1172,7 +1171,8 @@ __global__ void __launch_bounds__(A1_THREADS, 1) attn_kernel(
       const CUtensorMap* map32 = kind ? &maps.v32 : &maps.k32;
       const CUtensorMap* map64 = kind ? &maps.v64 : &maps.k64;
       uint32_t g = 0, slot = 0;                        // tiles so far, ring slot of the next one
-      // the lanes whose copies this warp starts: of each fetch and kind of copy about half
+      // the lanes whose copies this warp starts: half of the four-row groups (tile loads mostly start at multiples of four groups
+      // and then are the first warp's)
       const unsigned mine_mask = member ? kSecondHalf : ~kSecondHalf;
       bool ok = true;
       for (uint32_t n = 0;; ++n) {
@@ -1808,7 +1808,7 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
                                            int* plan, int H, int N, int CQ, void* ws, size_t ws_bytes,
                                            int* d_status, cudaStream_t st) {
   if (!q || !kp || !vp || !unip || !qperm || !plan || !ws || H <= 0 || N <= 0 || CQ <= 0) return T2T_ERR_ARG;
-  // q rows are fetched by TMA row gathers from a [rows, 128] view of the tensor: whole rows between rows
+  // q rows are fetched by TMA row gathers and 16-byte copies from a [rows, 128] view of the tensor: whole rows between rows
   if (q_row_stride < kD || q_head_stride <= 0 || (q_row_stride % kD) || (q_head_stride % kD)) return T2T_ERR_ARG;
   const int q_row_step = (int)(q_row_stride / kD), q_head_step = (int)(q_head_stride / kD);
   const uint64_t q_rows = (uint64_t)(H - 1) * q_head_step + (uint64_t)(N - 1) * q_row_step + 1;
@@ -1822,7 +1822,7 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
   const DeviceFacts* facts = device_facts();
   if (!facts) return T2T_ERR_CUDA;
   const int sms = facts->sms;
-  // tensor maps over q, kp, vp as [H * N, 128] matrices: the kernel fetches tile rows four at a time
+  // tensor maps over q, kp, vp as matrices of whole rows: boxes of one row (four-row gathers), 32 and 64 rows
   CUtensorMap mq;
   KVMaps kv;
   const uint64_t rows = (uint64_t)H * (uint64_t)N;
@@ -1831,7 +1831,7 @@ extern "C" int t2t_tile_attn_exact_strided(const void* q, long long q_row_stride
       !cached_row_map(&kv.v1, vp, rows, 1) || !cached_row_map(&kv.v32, vp, rows, 32) ||
       !cached_row_map(&kv.v64, vp, rows, 64))
     return T2T_ERR_CUDA;
-  // tasks above 128 rows first (one CTA per SM, two row tiles per K/V stream), then the others
+  // tasks above 128 rows first (CTA pairs, one CTA per SM with one of a task's two row tiles), then the others
   attn2_kernel<<<sms & ~1, A2_THREADS, A2_SMEM, st>>>(mq, kv, (const uint32_t*)unip, (const int*)qperm, attn_out,
                                                  attn_lse, plan, H, N, CQ, q_row_step, q_head_step, d_status);
   // The two kernels take disjoint tasks (own cursors, own output rows), so the second may start while the
