@@ -35,8 +35,8 @@ sys.path.insert(0, str(ROOT))
 WORKLOAD = dict(name="wan2.1-14b-720p-self-attention-layer", H=40, grid="720p", N=75600, CQ=512, D=128,
                 s_frac=0.015)
 KERNELS_REBUILD = 2 + 18 + 3 + 1 + 1 + 3  # project, kmeans (3 assign, 3x3 grouping, 3 means, 3 value stats), centroid moments+select+fix, gather, plan, attention (two kernels) + merge
-KERNELS_REUSE = 1 + 1 + 3 + 3   # project q, gather k, value stats, attention (two kernels) + merge
-ATTN_DRAM_BYTES_480P_8H = 444.2e6      # attn2_kernel (206.6 MB) + attn_kernel (210.9 MB), H 8, N 32,760 (ncu)
+KERNELS_REUSE = 1 + 1 + 4 + 3   # project q, gather k, value stats (cluster bases, sums, maximum, scale), attention (two kernels) + merge
+ATTN_DRAM_BYTES_480P_8H = 402.6e6      # attn2_kernel (203.4 MB) + attn_kernel (199.2 MB), H 8, N 32,760 (ncu)
 METRIC = "t2t_attn_ms_per_layer"
 UNIT = "ms/layer"
 

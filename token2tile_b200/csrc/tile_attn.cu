@@ -956,8 +956,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(A2_THREADS, 1) attn2
 // to one of two warpgroups, S = Q K^T runs two tiles ahead of P V.  A CTA keeps whole K and V tiles, 64 KB a tile for 128
 // rows, so the loads bound it: tile loads (TMA) where 32 or more rows of the union are contiguous; of the groups of four
 // rows between them a third comes by TMA gathers and the rest by 16-byte cp.async (26 and 28 B/clk alone).
-// 404 k tiles at 720p x 40 heads take 3.35 ms, 2,300 cycles a tile and SM (3.70 with two CTAs per SM, single K / V buffers
-// and the rows found by every copy warp), 321 k at 480p x 40 and 5 % 2.87 ms (3.28), 49 tasks at 2 x 4096 30 us less.
+// 404 k tiles at 720p x 40 heads take 3.4 ms, 2,300 cycles a tile and SM (3.70 with two CTAs per SM, single K / V buffers
+// and the rows found by every copy warp), 321 k at 480p x 40 and 5 % 2.9 ms (3.28), 49 tasks at 2 x 4096 30 us less.
 // With 64-row tile loads from any rows instead it would be 2.8 and 2.25 ms, with next to no loads 2.5 and 2.1.
 //   warps 0..7   softmax (see softmax_role)
 //   warp 8 / 9   issue Q K^T / P V
